@@ -126,6 +126,45 @@ static int parse_chunk(szp_b200_ctx *ctx, Arena &A, const unsigned char *pay, un
   return 0;
 }
 
+// First blocks of every chunk of the candidates T = T0 + blockIdx.x (thread t:
+// chunk t).  A chunk whose walk stops
+// (bit count byte at or past the bound, or above 32) within kProbeBlocks full
+// blocks marks the candidate: bad[T] = 1.
+constexpr int kProbeBlocks = 16;
+
+__global__ void chunk_probe_kernel(const unsigned char *__restrict__ cmp, unsigned long long bound,
+                                   unsigned long long nb, int B, bool tags, int T0, unsigned *__restrict__ bad) {
+  const int T = T0 + (int)blockIdx.x, t = (int)threadIdx.x;
+  const unsigned long long hdr = (unsigned long long)T * 8;
+  if (t >= T || hdr >= bound) return;
+  const unsigned long long bpt = (nb + T - 1) / T, b0 = (unsigned long long)t * bpt;
+  if (b0 >= nb) return;
+  // the chunk's last block may be shorter: only the blocks before it
+  const unsigned long long nbc = (nb - b0 < bpt ? nb - b0 : bpt) - 1;
+  unsigned long long p = 0;
+  for (int k = 0; k < 8; k++) p |= (unsigned long long)cmp[8 * t + k] << (8 * k);
+  const unsigned char *pay = cmp + hdr;
+  const unsigned long long lim = bound - hdr;
+  for (int k = 0; k < kProbeBlocks && (unsigned long long)k < nbc; k++) {
+    const unsigned bc = p + 4 < lim ? pay[p + 4] : 255u;
+    if (bc > 32u) { bad[T] = 1u; return; }
+    p += block_bytes((unsigned)B, bc, tags);
+  }
+}
+
+// Whether the chunks of a whole parse start where the table says: *bad = 1
+// where one does not.
+__global__ void chunk_verify_kernel(const unsigned char *__restrict__ cmp, const unsigned long long *__restrict__ offs,
+                                    unsigned long long nb, int T, unsigned *__restrict__ bad) {
+  const int t = (int)threadIdx.x;
+  if (t >= T) return;
+  const unsigned long long b0 = (unsigned long long)t * ((nb + T - 1) / T);
+  if (b0 >= nb) return;
+  unsigned long long v = 0;
+  for (int k = 0; k < 8; k++) v |= (unsigned long long)cmp[8 * t + k] << (8 * k);
+  if (offs[b0] != v) *bad = 1u;
+}
+
 // Thread count and block offsets of an OpenMP-layout stream by the
 // reference's detection rule.  cmp: the stream (its offset table first),
 // len: its bytes, n: elements; first_try: 1 for the topology stream, 2 for
@@ -145,8 +184,32 @@ static int detect_chunks(szp_b200_ctx *ctx, Arena &A, const unsigned char *cmp, 
   if (cuda_fail(cudaMemcpyAsync(tab.data(), cmp, (size_t)tmax * 8, cudaMemcpyDeviceToHost, s), "D2H") ||
       cuda_fail(cudaStreamSynchronize(s), "table"))
     return -1;
-  auto try_T = [&](int T, unsigned long long bound, bool *ok) -> int {
+  // the payload of candidate T as one walk, its chunk starts checked
+  unsigned *flag = A.take<unsigned>(kMaxTableThreads + 2);   // [1 .. 128] probed candidates, [0] a failed check
+  if (!flag) { set_error("scratch arena too small for the chunk parser"); return -1; }
+  if (cuda_fail(cudaMemsetAsync(flag, 0, (kMaxTableThreads + 2) * 4, s), "memset")) return -1;
+  auto whole_T = [&](int T, unsigned long long bound, bool *ok) -> int {
     *ok = false;
+    const unsigned long long hdr = (unsigned long long)T * 8;
+    if (hdr >= bound || tab[0] != 0) return 0;
+    const size_t mark = A.used;
+    if (parse_stream(ctx, A, cmp + hdr, bound - hdr, n, nullptr, B, tags, false, d_offs, d_status, B == 1)) return -1;
+    A.used = mark;
+    if (cuda_fail(cudaMemsetAsync(flag, 0, 4, s), "memset")) return -1;
+    chunk_verify_kernel<<<1, kMaxTableThreads, 0, s>>>(cmp, d_offs, nb, T, flag);
+    ctx->launches += 1;
+    unsigned *h_flag = reinterpret_cast<unsigned *>(ctx->h_words + 22);
+    if (cuda_fail(cudaGetLastError(), "chunk check") ||
+        cuda_fail(cudaMemcpyAsync(ctx->h_words + 20, d_status, 16, cudaMemcpyDeviceToHost, s), "D2H") ||
+        cuda_fail(cudaMemcpyAsync(h_flag, flag, 4, cudaMemcpyDeviceToHost, s), "D2H") ||
+        cuda_fail(cudaStreamSynchronize(s), "parse"))
+      return -1;
+    *ok = ctx->h_words[20] != 0 && ctx->h_words[21] == 0 && *h_flag == 0;
+    return 0;
+  };
+  auto try_T = [&](int T, unsigned long long bound, bool *ok) -> int {
+    if (whole_T(T, bound, ok)) return -1;
+    if (*ok || T == 1) return 0;   // one chunk: the walk was the chunk's own
     const unsigned long long hdr = (unsigned long long)T * 8;
     if (hdr >= bound) return 0;
     const unsigned long long bpt = (nb + T - 1) / T;
@@ -162,11 +225,19 @@ static int detect_chunks(szp_b200_ctx *ctx, Arena &A, const unsigned char *cmp, 
     return 0;
   };
   if (tab[0] == 0) {
-    for (int T = first_try; T <= tmax; T++) {
-      bool valid = true;
-      for (int k = 1; k < T; k++)
-        if (tab[k] > maxc || tab[k] < tab[k - 1]) { valid = false; break; }
-      if (!valid) break;
+    int tlast = 1;   // candidates whose table is non-decreasing and bounded
+    while (tlast < tmax && tab[tlast] <= maxc && tab[tlast] >= tab[tlast - 1]) tlast++;
+    std::vector<unsigned> bad(tlast + 1, 0u);
+    if (B > 1 && tlast > first_try) {
+      chunk_probe_kernel<<<tlast - first_try + 1, kMaxTableThreads, 0, s>>>(cmp, bound, nb, B, tags, first_try, flag);
+      ctx->launches += 1;
+      if (cuda_fail(cudaGetLastError(), "chunk probe") ||
+          cuda_fail(cudaMemcpyAsync(bad.data(), flag, bad.size() * 4, cudaMemcpyDeviceToHost, s), "D2H") ||
+          cuda_fail(cudaStreamSynchronize(s), "chunk probe"))
+        return -1;
+    }
+    for (int T = first_try; T <= tlast; T++) {
+      if (bad[T]) continue;
       bool ok = false;
       if (try_T(T, bound, &ok)) return -1;
       if (ok) return T;
@@ -289,7 +360,7 @@ int szp_b200_container_decompress_dev(szp_b200_ctx *ctx, const unsigned char *d_
   }
   const unsigned long long nbs = (E + B - 1) / B;
   const size_t need = a256((nb + nbs + 1) * 8) + parse_scratch_bytes(topo_size, B, true) +
-                      (E ? parse_scratch_bytes(sort_len, B, false) : 0) + a256(nb * 8) + 16384;
+                      (E ? parse_scratch_bytes(sort_len, B, false) : 0) + a256(nb * 8) + 16384 + 1024;
   // the decompression reserves its own scratch: keep the index in the io arena
   if (!ctx->io.reserve(a256((nb + nbs + 1) * 8) + 256)) return -1;
   unsigned long long *idx = ctx->io.take<unsigned long long>(nb + nbs + 1);
