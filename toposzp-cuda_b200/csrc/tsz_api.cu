@@ -66,12 +66,13 @@ int ctx_reserve_for(szp_b200_ctx *ctx, unsigned long long n, int B) {
   const unsigned long long nb = (n + B - 1) / B;
   // the largest scratch of a fused compression and of a fused decompression
   // with post-processing and device stream parsing
-  const size_t comp = a256(n * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 2 +
+  const size_t comp = a256(n * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 3 +
                       rank_scratch_bytes(n, ctx->sm_count) + 8192;
   const size_t dec = post_scratch_bytes(n) + a256(n * 4) + a256(n) + 8192 + a256(2 * nb * 8) +
                      parse_scratch_bytes(stream_bound(n, B, true) - 8, B, true) +
                      parse_scratch_bytes(stream_bound(n, B, false) - 8, B, false);
   if (!ctx->scratch.reserve(comp > dec ? comp : dec)) return -1;
+  if (rank_bits_reserve(ctx)) return -1;
   return post_words(ctx, n) ? 0 : -1;
 }
 
@@ -104,16 +105,17 @@ int encode_pass(szp_b200_ctx *ctx, int mode, const float *d_data, const int *d_i
                 const unsigned char *d_types, unsigned long long n, int B, float eb,
                 const Geom &g, unsigned char *d_stream, unsigned long long stream_cap,
                 unsigned long long *d_blk_off, int cp_mode, void *d_cp, unsigned long long cp_cap,
-                unsigned long long totals_out[3]) {
+                unsigned long long totals_out[3], const RankBits *rb) {
   cudaStream_t s = ctx->stream;
   const unsigned long long nb = (n + B - 1) / B;
   const int TB = enc_tile_blocks(B);
   const unsigned long long ntiles = (nb + TB - 1) / TB;
   TileDesc *desc = ctx->scratch.take<TileDesc>(ntiles + 1);
   if (!desc) { set_error("scratch arena too small for tile descriptors"); return -1; }
-  unsigned long long *w = ctx->d_words;  // [0..2] totals, [3] tile counter, [4] err
+  // [0..2] totals, [3] tile counter, [4] err, [8..11] statistics of the rank bits
+  unsigned long long *w = ctx->d_words;
   if (cuda_fail(cudaMemsetAsync(desc, 0, (ntiles + 1) * sizeof(TileDesc), s), "memset") ||
-      cuda_fail(cudaMemsetAsync(w, 0, 8 * sizeof(unsigned long long), s), "memset"))
+      cuda_fail(cudaMemsetAsync(w, 0, (rb ? 12 : 8) * sizeof(unsigned long long), s), "memset"))
     return -1;
   if (d_stream && cuda_fail(cudaMemsetAsync(d_stream, 0, 8, s), "memset")) return -1;
   EncArgs a{};
@@ -135,13 +137,14 @@ int encode_pass(szp_b200_ctx *ctx, int mode, const float *d_data, const int *d_i
   a.cp_mode = cp_mode;
   a.cp_out = d_cp;
   a.cp_cap = cp_cap;
+  if (rb) a.rb = *rb;
   int grid = (int)std::min<unsigned long long>(ntiles, (unsigned long long)ctx->sm_count * 8ull);
   if (grid < 1) grid = 1;
   if (cuda_fail(enc64_applies(a, mode) ? launch_enc64_from(a, s, ctx->sm_count) : launch_encode(mode, a, s, grid),
                 "encode launch"))
     return -1;
   ctx->launches += 1;
-  if (cuda_fail(cudaMemcpyAsync(ctx->h_words, w, 8 * sizeof(unsigned long long),
+  if (cuda_fail(cudaMemcpyAsync(ctx->h_words, w, 12 * sizeof(unsigned long long),
                                 cudaMemcpyDeviceToHost, s), "D2H totals") ||
       cuda_fail(cudaStreamSynchronize(s), "encode"))
     return -1;
@@ -163,8 +166,9 @@ int encode_pass(szp_b200_ctx *ctx, int mode, const float *d_data, const int *d_i
 // the launches finish (the caller waits for the copy stream).
 static int encode_topo_chunked(szp_b200_ctx *ctx, const float *h_src, float *d_data, unsigned long long n, int B,
                                float eb, const Geom &g, unsigned char *d_stream, unsigned long long stream_cap,
-                               unsigned long long *d_blk_off, void *d_cp, unsigned long long cp_cap,
-                               unsigned long long totals_out[3], unsigned char *h_out, size_t out_cap) {
+                               unsigned long long *d_blk_off, int cp_mode, void *d_cp, unsigned long long cp_cap,
+                               unsigned long long totals_out[3], unsigned char *h_out, size_t out_cap,
+                               const RankBits *rb) {
   cudaStream_t s = ctx->stream;
   cudaStream_t cs = copy_stream(ctx);
   if (!cs) return -1;
@@ -191,7 +195,7 @@ static int encode_topo_chunked(szp_b200_ctx *ctx, const float *h_src, float *d_d
   if (!desc) { set_error("scratch arena too small for tile descriptors"); return -1; }
   unsigned long long *w = ctx->d_words;  // [0..2] totals, [3] tile counter, [4] err
   if (cuda_fail(cudaMemsetAsync(desc, 0, (ntiles + 1) * sizeof(TileDesc), s), "memset") ||
-      cuda_fail(cudaMemsetAsync(w, 0, 8 * sizeof(unsigned long long), s), "memset") ||
+      cuda_fail(cudaMemsetAsync(w, 0, 12 * sizeof(unsigned long long), s), "memset") ||
       cuda_fail(cudaMemsetAsync(d_stream, 0, 8, s), "memset"))
     return -1;
   EncArgs a{};
@@ -208,9 +212,10 @@ static int encode_topo_chunked(szp_b200_ctx *ctx, const float *h_src, float *d_d
   a.err = reinterpret_cast<int *>(w + 4);
   a.total = w;
   a.desc = desc;
-  a.cp_mode = kCpPairs;
+  a.cp_mode = cp_mode;
   a.cp_out = d_cp;
   a.cp_cap = cp_cap;
+  if (rb) a.rb = *rb;
   unsigned long long done = 0;
   int parts = 0;
   for (int k = 0; k < K; k++) {
@@ -241,7 +246,7 @@ static int encode_topo_chunked(szp_b200_ctx *ctx, const float *h_src, float *d_d
       parts++;
     }
   }
-  if (cuda_fail(cudaMemcpyAsync(ctx->h_words, w, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
+  if (cuda_fail(cudaMemcpyAsync(ctx->h_words, w, 12 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
                 "D2H totals"))
     return -1;
   // as each launch finishes, its part of the stream leaves for the host on a
@@ -715,13 +720,20 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
   const int B = blockSize;
   const unsigned long long nb = (n + B - 1) / B;
   const unsigned long long kcap = n;
-  const size_t need = a256(kcap * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 2 +
+  const size_t need = a256(kcap * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 3 +
                       rank_scratch_bytes(kcap, ctx->sm_count) + 8192;
   if (!ctx->scratch.reserve(need)) return -1;
   Arena &A = ctx->scratch;
   uint2 *pairs = A.take<uint2>(kcap);
   int *sp = A.take<int>(n);
   unsigned long long tot[3];
+  // From 2^18 values on the encoder sets the rank's bits itself and hands
+  // over the extrema's codes (in the pairs' place): no pair is written or
+  // read.  Below, the pairs are few and the rank picks its way by their count.
+  RankBits rb;
+  const EncArgs probe = [&] { EncArgs e{}; e.B = B; e.data = d_data; e.out = d_topo + 8; e.cp_mode = kCpBits; return e; }();
+  const bool bits = n >= (1ull << 18) && enc64_applies(probe, kEncClassify) && rank_bits_begin(ctx, absErrBound, &rb);
+  const int cp_mode = bits ? kCpBits : kCpPairs;
   tl_begin(ctx);
   // a field still on the host (h_src) is copied in parts that overlap the encoder
   const bool chunked = h_src && B <= 256 && n >= (1ull << 24);
@@ -731,10 +743,10 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
     return -1;
   if (chunked ? encode_topo_chunked(ctx, h_src, const_cast<float *>(d_data), n, B, absErrBound, g, d_topo,
                                     stream_bound(n, B, true), reinterpret_cast<unsigned long long *>(d_blk_index),
-                                    pairs, kcap, tot, h_topo, topo_cap)
+                                    cp_mode, pairs, kcap, tot, h_topo, topo_cap, bits ? &rb : nullptr)
               : encode_pass(ctx, kEncClassify, d_data, nullptr, nullptr, n, B, absErrBound, g, d_topo,
                             stream_bound(n, B, true), reinterpret_cast<unsigned long long *>(d_blk_index),
-                            kCpPairs, pairs, kcap, tot))
+                            cp_mode, pairs, kcap, tot, bits ? &rb : nullptr))
     return -1;
   tl_mark(ctx, "encode_topo");
   sizes->topo_bytes = 8 + tot[0];
@@ -752,8 +764,28 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
       return -1;
   }
   const unsigned long long K = tot[1], E = tot[2];
+  int left = bits && K == 0 ? 0 : 1;   // 1: to be ranked from pairs
+  if (bits && K) {
+    unsigned h_stat[8];
+    memcpy(h_stat, ctx->h_words + kRbStatWord, sizeof(h_stat));
+    left = rank_bits_finish(ctx, rb, h_stat, absErrBound, reinterpret_cast<const unsigned *>(pairs), nullptr, K, E, sp);
+    if (left < 0) return -1;
+  } else if (bits) {
+    ctx->rank_bits_dirty = false;      // nothing was set
+  }
   if (E == 0) return 0;
-  if (rank_positions(ctx, pairs, nullptr, K, E, absErrBound, sp)) return -1;
+  if (left) {
+    if (bits) {
+      // values the bits do not cover: the same encoding once more, for its pairs
+      if (ctx->d2h_stream && cuda_fail(cudaStreamSynchronize(ctx->d2h_stream), "sync")) return -1;
+      if (ctx->copy_stream && cuda_fail(cudaStreamSynchronize(ctx->copy_stream), "sync")) return -1;
+      if (encode_pass(ctx, kEncClassify, d_data, nullptr, nullptr, n, B, absErrBound, g, d_topo,
+                      stream_bound(n, B, true), reinterpret_cast<unsigned long long *>(d_blk_index), kCpPairs, pairs,
+                      kcap, tot))
+        return -1;
+    }
+    if (rank_positions(ctx, pairs, nullptr, K, E, absErrBound, sp, !bits)) return -1;
+  }
   tl_mark(ctx, "rank");
   unsigned long long st[3];
   if (encode_pass(ctx, kEncInts, nullptr, sp, nullptr, E, B, absErrBound, g, d_sort,

@@ -301,8 +301,9 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
 // Back half of a tile: look-back for the tile's stream and CP offsets, block
 // index, write-out of the image and copy-out of the staged pairs.  Ends with
 // a CTA barrier.
+template <bool BITS>
 __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, const unsigned char *img,
-                                         const uint2 *stage, E64Sh &sh) {
+                                         const uint2 *stage, E64Sh &sh, unsigned &nmax, unsigned &cmax) {
   const int tid = threadIdx.x;
   const long long n = (long long)a.n;
   const long long nblocks = (n + 63) / 64;
@@ -357,8 +358,22 @@ __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, con
     const unsigned t0b = head + 16u * nq;
     if (t0b + tid < tile_bytes) dst[t0b + tid] = img[t0b + tid];
   }
-  // critical-point pairs in raster order
-  {
+  if (BITS) {
+    // every value's bit; the extrema's codes in raster order
+    const unsigned long long cb = sh.gcnt >> 32, eb0 = sh.gcnt & 0xffffffffull;
+    const unsigned ntc = sh.tile_cps;
+    for (unsigned k = tid; k < ntc; k += kE64Threads) {
+      const uint2 pr = stage[k];
+      const unsigned ext = pr.y == kNoExtremum ? kNoExtremum : (unsigned)eb0 + pr.y;
+      rb_set(a.rb, pr.x, ext);
+      if (cb + k < kRankSmall) a.rb.first[cb + k] = make_uint2(pr.x, ext);
+      nmax = max(nmax, ~pr.x);
+      cmax = max(cmax, pr.x);
+      if (ext != kNoExtremum && eb0 + pr.y < a.cp_cap) a.code_out[eb0 + pr.y] = pr.x;
+    }
+    if (tid == 0 && eb0 + sh.tile_ext > a.cp_cap) atomicExch(a.err, kErrCapacity);
+  } else {
+    // critical-point pairs in raster order
     const unsigned long long cb = sh.gcnt >> 32;
     const uint32_t eb0 = (uint32_t)(sh.gcnt & 0xffffffffull);
     const unsigned ntc = sh.tile_cps;
@@ -378,7 +393,7 @@ __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, con
 // Persistent CTAs claim tiles in order; each keeps two images and runs one
 // tile behind (tile k's aggregate is published before tile k-1 looks back),
 // so a look-back only ever waits for tiles held by running CTAs.
-template <bool D3>
+template <bool D3, bool BITS>
 __global__ void __launch_bounds__(kE64Threads, 4) enc64_kernel(Enc64Args a) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   __shared__ E64Sh sh[2];
@@ -387,6 +402,7 @@ __global__ void __launch_bounds__(kE64Threads, 4) enc64_kernel(Enc64Args a) {
   const long long tend = a.tile_hi ? (long long)a.tile_hi : ntiles;
   long long prev = -1;
   int cur = 0;
+  unsigned nmax = 0, cmax = 0;
   while (true) {
     if (threadIdx.x == 0) s_claim = (long long)a.tile_lo + (long long)atomicAdd(a.tile_ctr, 1u);
     __syncthreads();
@@ -397,12 +413,13 @@ __global__ void __launch_bounds__(kE64Threads, 4) enc64_kernel(Enc64Args a) {
     __syncthreads();
     if (prev >= 0) {
       const unsigned char *pp = smem_dyn + (size_t)(cur ^ 1) * kE64Part;
-      e64_back(a, prev, pp, reinterpret_cast<const uint2 *>(pp + kE64Img), sh[cur ^ 1]);
+      e64_back<BITS>(a, prev, pp, reinterpret_cast<const uint2 *>(pp + kE64Img), sh[cur ^ 1], nmax, cmax);
     }
     if (!more) break;
     prev = tile;
     cur ^= 1;
   }
+  if (BITS) rb_extent(a.rb, nmax, cmax);
 }
 
 unsigned long long enc64_tiles(unsigned long long n) { return (n + kE64Tile - 1) / kE64Tile; }
@@ -411,7 +428,8 @@ size_t enc64_smem_bytes() { return 2 * (size_t)kE64Part; }
 
 static cudaError_t launch_enc64(const Enc64Args &a, cudaStream_t s, int sm_count) {
   const size_t smem = enc64_smem_bytes();
-  auto k = a.g.nd == 3 ? enc64_kernel<true> : enc64_kernel<false>;
+  auto k = a.code_out ? (a.g.nd == 3 ? enc64_kernel<true, true> : enc64_kernel<false, true>)
+                      : (a.g.nd == 3 ? enc64_kernel<true, false> : enc64_kernel<false, false>);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
@@ -476,7 +494,7 @@ int selftest_lookback(int spin_limit, int *status, float *ms) {
 }
 
 bool enc64_applies(const EncArgs &a, int mode) {
-  return mode == kEncClassify && a.B == 64 && a.cp_mode == kCpPairs && a.out != nullptr &&
+  return mode == kEncClassify && a.B == 64 && (a.cp_mode == kCpPairs || a.cp_mode == kCpBits) && a.out != nullptr &&
          (reinterpret_cast<uintptr_t>(a.data) & 15) == 0 && enc_tile_blocks(64) == kE64Blocks;
 }
 
@@ -497,7 +515,12 @@ cudaError_t launch_enc64_from(const EncArgs &e, cudaStream_t s, int sm_count) {
   a.tile_hi = e.tile_hi;
   a.err = e.err;
   a.total = e.total;
-  a.cp_out = reinterpret_cast<uint2 *>(e.cp_out);
+  if (e.cp_mode == kCpBits) {
+    a.code_out = reinterpret_cast<unsigned *>(e.cp_out);
+    a.rb = e.rb;
+  } else {
+    a.cp_out = reinterpret_cast<uint2 *>(e.cp_out);
+  }
   a.cp_cap = e.cp_cap;
   a.spin_limit = 0;
   return launch_enc64(a, s, sm_count);

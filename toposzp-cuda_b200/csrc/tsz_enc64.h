@@ -18,7 +18,9 @@ struct Enc64Args {
   unsigned long long tile_hi;
   int *err;                     // status word
   unsigned long long *total;    // [payload bytes, cps, extrema]
-  uint2 *cp_out;                // critical-point pairs {value code, extremum index or ~0}
+  uint2 *cp_out;                // critical-point pairs {value code, extremum index or ~0}, or null:
+  unsigned *code_out;           // extremum codes in raster order, every value's bit in rb
+  RankBits rb;
   unsigned long long cp_cap;
   int spin_limit;               // look-back polls before giving up (0: default)
   unsigned long long base;      // global index of local element 0 (a slab of a larger field; 0 otherwise):
@@ -26,7 +28,7 @@ struct Enc64Args {
                                 // base + local through data (indexed by global element)
 };
 
-// The fused topology encoder with pairs output applies to blockSize 64 and a
+// The fused topology encoder (pairs, or bits and codes) applies to blockSize 64 and a
 // 16-byte aligned field; its tiles are the general encoder's (2048 elements).
 bool enc64_applies(const EncArgs &a, int mode);
 // Launches it over the tiles of a (persistent grid sized by occupancy).

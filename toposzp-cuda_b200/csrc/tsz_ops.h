@@ -35,14 +35,34 @@ int encode_pass(szp_b200_ctx *ctx, int mode, const float *d_data, const int *d_i
                 const unsigned char *d_types, unsigned long long n, int B, float eb,
                 const Geom &g, unsigned char *d_stream, unsigned long long stream_cap,
                 unsigned long long *d_blk_off, int cp_mode, void *d_cp, unsigned long long cp_cap,
-                unsigned long long totals_out[3]);
+                unsigned long long totals_out[3], const RankBits *rb = nullptr);
+
+// Sort positions from a bitmap over the values (tsz_rankbits.cuh).  begin:
+// the bits of a call with bound eb, false when they do not apply; its values
+// then are set by an encode_pass with rb (kCpBits) or by rank_bits_pairs.
+// finish: positions of the E extrema, from their codes in raster order or
+// from K pairs, h_stat the call's statistics; enqueued, and the bits cleared.
+// Returns 0, -1 on an error, or 1 when the values are left to the bucket
+// ranking (which needs pairs).
+constexpr int kRbStatWord = 8;   // of d_words: RankBits::stat (32 bytes)
+int rank_bits_reserve(szp_b200_ctx *ctx);
+bool rank_bits_begin(szp_b200_ctx *ctx, float eb, RankBits *rb);
+int rank_bits_finish(szp_b200_ctx *ctx, const RankBits &rb, const unsigned *h_stat, float eb, const unsigned *d_codes,
+                     const uint2 *d_pairs, unsigned long long K, unsigned long long E, int *d_sp);
+int rank_bits_from_pairs(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long long K, unsigned long long E, float eb,
+                         int *d_sp);
+// rb: the bits that the pairs set, to be cleared (null: none)
+int rank_small(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long long K, float eb, int *d_sp,
+               const RankBits *rb = nullptr);
+size_t rank_bits_scratch_bytes();
 
 // Dense rank of every extremum inside its quantization bin.
 //   pairs[k] = (orderable value code, extremum index or kNoExtremum), k < K
 //   writes sp[e] for every extremum e < E.  bins come from the value
 //   (bin = quant_bin(value, eb)); mode_given_bins = true uses bins[k] instead.
+// (try_bits: through the bitmap over the values where it applies)
 int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
-                   unsigned long long K, unsigned long long E, float eb, int *d_sp);
+                   unsigned long long K, unsigned long long E, float eb, int *d_sp, bool try_bits = true);
 
 // Post-processing of a decoded field in place (serial raster semantics of the
 // reference drivers).  types: u8 per element (or int when types_i != null).

@@ -121,6 +121,8 @@ static void ctx_free(szp_b200_ctx *c) {
   c->scratch.release();
   if (c->post_S) cudaFree(c->post_S);
   c->post_S = nullptr;
+  if (c->rank_bits) cudaFree(c->rank_bits);
+  c->rank_bits = nullptr;
   c->io.release();
   if (c->h_words) cudaFreeHost(c->h_words);
   if (c->d_words) cudaFree(c->d_words);

@@ -44,6 +44,8 @@ struct szp_b200_ctx {
   unsigned long long *post_S = nullptr;    // post-processing result words (generation-tagged)
   unsigned long long post_S_cap = 0;
   unsigned post_gen = 0;
+  unsigned *rank_bits = nullptr;           // bitmap of the rank stage, zero between calls unless dirty
+  bool rank_bits_dirty = false;
   // stage timeline of the last call (CUDA events on the workspace stream)
   static constexpr int kMaxStages = 24;
   cudaEvent_t ev[kMaxStages + 1] = {};

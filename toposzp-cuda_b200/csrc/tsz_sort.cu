@@ -611,9 +611,13 @@ static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, uns
 }
 
 int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
-                   unsigned long long K, unsigned long long E, float eb, int *d_sp) {
+                   unsigned long long K, unsigned long long E, float eb, int *d_sp, bool try_bits) {
   if (K == 0) return 0;
-  (void)E;
+  if (!d_bins && K <= (unsigned long long)kRankSmall) return rank_small(ctx, d_pairs, K, eb, d_sp);
+  if (!d_bins && try_bits) {
+    const int r = rank_bits_from_pairs(ctx, d_pairs, K, E, eb, d_sp);
+    if (r <= 0) return r;
+  }
   cudaStream_t s = ctx->stream;
   const BinSrc src = {d_bins, eb, 1.0 / (double)eb};
   // 2^9 buckets keep each bucket's bins (slots) within the shared bitmap for
@@ -765,8 +769,8 @@ size_t rank_scratch_bytes(unsigned long long K, int sm_count) {
   // fallback worst case: all K records (two key/value ping-pong buffers + histogram)
   const size_t fb = a256(K * 8) * 2 + a256(K * 4) * 2 + a256(256 * ((K + kRadixTile - 1) / kRadixTile) * 4) +
                     a256(scan_parts(256 * ((K + kRadixTile - 1) / kRadixTile) + K) * 4);
-  // records (8 B) and, for given bins, their permuted bins (4 B)
-  return a256(G * NB * 4) + a256(NB * 4) + a256((NB + 1) * 8) + a256(K * 8) + a256(K * 4) +
+  // records (8 B) and, for given bins, their permuted bins (4 B); the bitmap ranking's tables
+  return (K > (unsigned long long)kRankSmall ? rank_bits_scratch_bytes() : 0) + a256(G * NB * 4) + a256(NB * 4) + a256((NB + 1) * 8) + a256(K * 8) + a256(K * 4) +
          a256(NB * 4) * 3 + a256(16) + fb + a256((NB + 1) * 8) * 2 + 4096;
 }
 
