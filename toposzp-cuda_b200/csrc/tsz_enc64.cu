@@ -14,10 +14,23 @@
 //   * the +-1 neighbours come from the adjacent lanes (shuffles), and each
 //     edge along the row is compared once for both of its points;
 //   * the two other axes are folded into max / min masks one axis at a time,
-//     so that only one neighbour octet pair is live;
+//     so that only one neighbour octet pair is live, and comparisons are sign
+//     bits of differences (FMA pipe) pushed into masks;
 //   * index arithmetic is per octet (one coordinate split), never per point;
-//   * the CTA keeps two tile images and runs one tile behind (its look-back
-//     waits while the next tile's front half is already published).
+//   * the CTA keeps two tile images and runs one tile behind, and a warp of
+//     its own claims tiles and looks back while the others work.
+//
+// What bounds it (512^3 field, abs eb 1e-4, B200): instruction issue, with the
+// ALU pipe 65 % busy (4.2 warp instructions per element, of which
+// classification 0.9).  Its time there, the extrema's codes and the values'
+// bits included, by what it was brought down with:
+//   1110 us  look-back by all warps behind the write-out, 64 registers
+//    994     look-back by a ninth warp beside the front half, which knows full
+//            blocks; claiming a tile ahead instead of just before its front
+//            half costs 350 (every look-back behind the tile waits for it)
+//    894     56 registers: four CTAs per SM instead of three
+//    772     descriptors as one 16-byte word: one load in the look-back
+//    712     comparisons on the FMA pipe, 32-bit coordinate split
 #include "tsz_codec2.cuh"
 #include "tsz_enc64.h"
 #include "tsz_ops.h"
@@ -25,24 +38,71 @@
 
 namespace tsz {
 
-constexpr int kE64Threads = 256;
+constexpr int kE64Threads = 256;                 // the threads that own elements
+constexpr int kE64Warps = kE64Threads / 32;
+constexpr int kE64Cta = kE64Threads + 32;        // and one warp for tile claims and look-backs
 constexpr int kE64Tile = 8 * kE64Threads;        // elements per tile
 constexpr int kE64Blocks = kE64Tile / 64;        // codec blocks per tile
 constexpr unsigned kE64BlockMax = 289;           // block_bytes(64, 33, tags): a safe bound
 constexpr unsigned kE64Img = (kE64Blocks * kE64BlockMax + 64u + 15u) & ~15u;
-constexpr unsigned kE64Stage = kE64Tile * 8u;    // staged critical-point pairs (one per element at most)
-constexpr unsigned kE64Part = kE64Img + kE64Stage;
+// staged critical points, one per element at most: pairs, or codes (extrema
+// from the front, saddles from the back)
+__host__ __device__ constexpr unsigned e64_part(bool bits) { return kE64Img + kE64Tile * (bits ? 4u : 8u); }
 
 struct E64Sh {
-  unsigned long long w64[kE64Threads / 32];
-  unsigned long long gbyte, gcnt;
+  unsigned wb[kE64Warps], wc[kE64Warps];         // block bytes and (extrema << 16 | points) of each warp
+  unsigned long long gbyte, gcnt;                // the tile's place, from the look-back
   unsigned tile_bytes, tile_cps, tile_ext;
   unsigned boff[kE64Blocks];
 };
 
-// hi / lo masks of one axis: bit t set when c[t] is above (below) both of its
-// neighbours at -off and +off.  c > max.NaN(m, p) is exactly (c > m && c > p),
-// NaN operands included.
+// barrier of the warps that own elements
+__device__ __forceinline__ void e64_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// the claim of a tile, from the ninth warp to the others
+__device__ __forceinline__ void e64_claim_post() { asm volatile("bar.arrive 2, 288;" ::: "memory"); }
+__device__ __forceinline__ void e64_claim_wait() { asm volatile("bar.sync 2, 288;" ::: "memory"); }
+
+// A tile's descriptor as one 16-byte word, read and written whole: the status
+// word (2-bit state, bytes) and the counts (points << 32 | extrema) of the
+// tile (state 1) or of all tiles through it (state 2).  Nothing else is
+// published with it, so no access needs an order, and a look-back waits for
+// one load where status, then counts, would be two in a row.
+__device__ __forceinline__ void e64_publish(TileDesc *d, unsigned long long state, unsigned long long bytes,
+                                            unsigned long long cnt) {
+  asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(d),
+               "l"((state << kStatShift) | (bytes & kByteMask)), "l"(cnt)
+               : "memory");
+}
+__device__ __forceinline__ void e64_read(const TileDesc *d, unsigned long long &st, unsigned long long &cnt) {
+  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+               : "=l"(st), "=l"(cnt)
+               : "l"(d)
+               : "memory");
+}
+
+// Shifts the sign bit of f into the low end of mask.
+__device__ __forceinline__ unsigned push_sign(float f, unsigned mask) {
+  return __funnelshift_l(__float_as_uint(f), mask, 1);
+}
+// x with -0 as +0 (NaN stays NaN)
+__device__ __forceinline__ float plus_zero(float x) { return __fadd_rn(x, 0.0f); }
+// float_code of a value that is not -0
+__device__ __forceinline__ unsigned value_code(float x) {
+  const unsigned b = __float_as_uint(x);
+  return b ^ ((unsigned)((int)b >> 31) | 0x80000000u);
+}
+
+// Masks are built from the sign bits of differences: with no -0 among the
+// values, a - b is negative exactly when a < b (a denormal difference is not
+// flushed, equal values give +0, and NaN, which a comparison with NaN and
+// inf - inf give, has a clear sign bit).  A comparison is then one addition on
+// the FMA pipe and one shift, where compare, select and combine are three
+// instructions on the ALU pipe, which bounds this kernel.  Element 0 is the
+// highest bit of a mask.
+
+// hi / lo masks of one axis: bit 7 - t set when c[t] is above (below) both of
+// its neighbours at -off and +off.  c > max.NaN(m, p) is exactly
+// (c > m && c > p), NaN operands included.
 __device__ __forceinline__ void e64_axis(const float *__restrict__ d, long long i0, long long off, unsigned inter,
                                          bool vec, const float (&c)[8], unsigned &hi, unsigned &lo) {
   float m[8], p[8];
@@ -55,7 +115,7 @@ __device__ __forceinline__ void e64_axis(const float *__restrict__ d, long long 
   } else {
 #pragma unroll
     for (int t = 0; t < 8; t++) {
-      const bool in = (inter >> t) & 1u;
+      const bool in = (inter >> (7 - t)) & 1u;
       m[t] = in ? __ldg(d + i0 + t - off) : 0.f;
       p[t] = in ? __ldg(d + i0 + t + off) : 0.f;
     }
@@ -63,27 +123,39 @@ __device__ __forceinline__ void e64_axis(const float *__restrict__ d, long long 
   unsigned h = 0, w = 0;
 #pragma unroll
   for (int t = 0; t < 8; t++) {
-    h |= (c[t] > fmax_nan(m[t], p[t]) ? 1u : 0u) << t;
-    w |= (c[t] < fmin_nan(m[t], p[t]) ? 1u : 0u) << t;
+    h = push_sign(__fsub_rn(plus_zero(fmax_nan(m[t], p[t])), c[t]), h);
+    w = push_sign(__fsub_rn(c[t], fmin_nan(m[t], p[t])), w);
   }
   hi = h;
   lo = w;
 }
 
+// (q, r) = divmod(i, d) of a 32-bit index: fdivmod's product in two 32 x 32
+// multiplications
+__device__ __forceinline__ unsigned divmod32(unsigned i, unsigned d, unsigned long long m, unsigned &r) {
+  const unsigned long long t = (unsigned long long)i * (unsigned)m;
+  const unsigned long long u = (unsigned long long)i * (unsigned)(m >> 32) + (t >> 32);
+  const unsigned q = m ? (unsigned)(u >> 32) : i;
+  r = i - q * d;
+  return q;
+}
+
 // Front half of a tile: load, classify, quantize, pack into img, stage the
-// critical-point pairs, publish the tile's aggregate.  All threads call it.
-template <bool D3>
-__device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, unsigned char *img, uint2 *stage,
+// critical points, publish the tile's aggregate.  The 256 threads that own
+// elements call it.  FULL: every block of the tile has 64 elements, so the only
+// position without a delta is a block's last.
+template <bool D3, bool BITS, bool FULL>
+__device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bool small, unsigned char *img, void *stage,
                                           E64Sh &sh) {
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int l = lane & 7, bi = tid >> 3;
   const long long n = (long long)a.n;
   const long long i0 = tile * kE64Tile + 8 * tid;   // local index of the octet
   const long long g0 = (long long)a.base + i0;       // its global index
   const long long bstart = tile * kE64Tile + 64 * bi;
-  const int len = bstart >= n ? 0 : (n - bstart >= 64 ? 64 : (int)(n - bstart));
+  const int len = FULL ? 64 : (bstart >= n ? 0 : (n - bstart >= 64 ? 64 : (int)(n - bstart)));
   const int e0 = 8 * l;
-  const int nv = len - e0 < 0 ? 0 : (len - e0 > 8 ? 8 : len - e0);
+  const int nv = FULL ? 8 : (len - e0 < 0 ? 0 : (len - e0 > 8 ? 8 : len - e0));
 
   // ---- values of the octet ----
   float x[8];
@@ -95,11 +167,34 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
 #pragma unroll
     for (int t = 0; t < 8; t++) x[t] = t < nv ? __ldg(a.data + g0 + t) : 0.f;
   }
+  // -0 as +0: the same quantized value, value code and comparisons
+#pragma unroll
+  for (int t = 0; t < 8; t++) x[t] = plus_zero(x[t]);
 
-  // ---- interior mask: one coordinate split per octet ----
+  // ---- interior mask (element 0 in bit 7): one coordinate split per octet ----
   unsigned inter = 0;
   bool wrap = false;
-  if (nv > 0) {
+  if (small) {
+    if (nv > 0) {
+      unsigned r, z0, y, xx = 0;
+      const unsigned d3 = (unsigned)a.g.d3;
+      if (D3) {
+        xx = divmod32((unsigned)g0, (unsigned)a.g.plane, a.g.m_plane, r);
+        y = divmod32(r, d3, a.g.m_d3, z0);
+      } else {
+        y = divmod32((unsigned)g0, d3, a.g.m_d3, z0);
+      }
+      if (z0 + 7u < d3) {
+        // a row's first and last columns, and its first and last rows and planes, are boundary
+        const bool row_in = y - 1u < (unsigned)a.g.d2 - 2u && (!D3 || xx - 1u < (unsigned)a.g.d1 - 2u);
+        inter = row_in ? (z0 ? 0xffu : 0x7fu) & (z0 + 8u == d3 ? 0xfeu : 0xffu) : 0u;
+        if (!FULL) inter &= 0xff00u >> nv;
+      } else {
+        wrap = true;   // the octet crosses a row: elements of several rows
+        inter = __brev(octet_interior(g0, nv, a.g)) >> 24;
+      }
+    }
+  } else if (nv > 0) {
     long long r, z0, y, xx = 0;
     if (D3) {
       xx = fdivmod(g0, a.g.plane, a.g.m_plane, r);
@@ -114,10 +209,10 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
         const int ulo = lo > 0 ? (int)lo : 0, uhi = hi < 7 ? (int)hi : 7;
         if (ulo <= uhi) inter = ((2u << uhi) - 1u) & ~((1u << ulo) - 1u);
       }
-      inter &= (nv >= 8) ? 0xffu : ((1u << nv) - 1u);
+      inter = __brev(inter & ((nv >= 8) ? 0xffu : ((1u << nv) - 1u))) >> 24;
     } else {
-      wrap = true;   // the octet crosses a row: elements of several rows
-      inter = octet_interior(g0, nv, a.g);
+      wrap = true;
+      inter = __brev(octet_interior(g0, nv, a.g)) >> 24;
     }
   }
 
@@ -126,22 +221,21 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
   // consecutive elements); the warp's end lanes load their outer neighbour
   float prev = __shfl_up_sync(0xffffffffu, x[7], 1);
   float next = __shfl_down_sync(0xffffffffu, x[0], 1);
-  if (lane == 0 && (inter & 1u)) prev = __ldg(a.data + g0 - 1);
-  if (lane == 31 && (inter & 0x80u)) next = __ldg(a.data + g0 + 8);
-  unsigned types = 0, cpm = 0, exm = 0;
+  if (lane == 0 && (inter & 0x80u)) prev = plus_zero(__ldg(a.data + g0 - 1));
+  if (lane == 31 && (inter & 1u)) next = plus_zero(__ldg(a.data + g0 + 8));
+  unsigned tags = 0, cpm = 0, exm = 0;
   if (__any_sync(0xffffffffu, inter != 0u)) {
-    // edge j (0..8) joins element j-1 and j (element -1 = prev, 8 = next)
+    // edge j (0..8) joins element j-1 and j (element -1 = prev, 8 = next): bit 8 - j
     unsigned gt = 0, lt = 0;
     float cl = prev;
 #pragma unroll
-    for (int t = 0; t < 8; t++) {
-      gt |= (cl > x[t] ? 1u : 0u) << t;
-      lt |= (cl < x[t] ? 1u : 0u) << t;
-      cl = x[t];
+    for (int t = 0; t < 9; t++) {
+      const float cr = t < 8 ? x[t < 8 ? t : 0] : next;
+      lt = push_sign(__fsub_rn(cl, cr), lt);
+      gt = push_sign(__fsub_rn(cr, cl), gt);
+      cl = cr;
     }
-    gt |= (cl > next ? 1u : 0u) << 8;
-    lt |= (cl < next ? 1u : 0u) << 8;
-    const unsigned hz = lt & (gt >> 1), lz = gt & (lt >> 1);
+    const unsigned hz = (lt >> 1) & gt, lz = (gt >> 1) & lt;
     unsigned ha = 0, la = 0, hb = 0, lb = 0;
     if (inter) {
       // vector loads when the octet lies in one row and the offset keeps the
@@ -166,75 +260,105 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
     sd &= inter;
     cpm = mx | mn | sd;
     exm = mx | mn;
-    // 2-bit types: maximum 01, minimum 10, saddle 11 (element t at bits 2t)
-    types = spread2(mx | sd) | (spread2(mn | sd) << 1);
+    // 2-bit types: maximum 01, minimum 10, saddle 11 (element 0 in the top two bits)
+    tags = spread2(mx | sd) | (spread2(mn | sd) << 1);
   }
 
   // ---- quantization and deltas ----
   int q[8];
 #pragma unroll
   for (int t = 0; t < 8; t++) q[t] = t < nv ? quantize(x[t], a.inv) : 0;
-  int qn = __shfl_down_sync(0xffffffffu, q[0], 1, 8);
-  if (l == 7) qn = 0;
+  const int qn = __shfl_down_sync(0xffffffffu, q[0], 1, 8);
   const int cnt = len > 0 ? len - 1 : 0;
-  unsigned negm = 0, maxm = 0, mags[8];
+  unsigned sign = 0, maxm = 0, mags[8];
 #pragma unroll
   for (int t = 0; t < 8; t++) {
-    mags[t] = 0;
-    if (e0 + t < cnt) {
-      const int nx = (t < 7) ? q[t + 1] : qn;
-      const unsigned ud = (unsigned)nx - (unsigned)q[t];
-      const bool ng = (int)ud < 0;
-      mags[t] = ng ? 0u - ud : ud;
-      negm |= (ng ? 1u : 0u) << t;
-      maxm = mags[t] > maxm ? mags[t] : maxm;
-    }
+    int d = (int)((unsigned)((t < 7) ? q[t + 1] : qn) - (unsigned)q[t]);
+    if (FULL ? (t == 7 && l == 7) : e0 + t >= cnt) d = 0;
+    sign = __funnelshift_l((unsigned)d, sign, 1);    // delta e0 + t at bit 7 - t
+    mags[t] = (unsigned)(d < 0 ? 0u - (unsigned)d : (unsigned)d);
+    maxm = mags[t] > maxm ? mags[t] : maxm;
   }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) {
     const unsigned u = __shfl_xor_sync(0xffffffffu, maxm, o, 8);
     maxm = u > maxm ? u : maxm;
   }
-  const unsigned bc = bitcount(maxm);
-  const unsigned bbytes = len ? block_bytes((unsigned)len, bc, true) : 0u;
+  // below 2^16 log2f is off by less than its distance from the next integer
+  const unsigned bc = maxm < 65536u ? 32u - (unsigned)__clz((int)maxm) : bitcount(maxm);
+  const unsigned bbytes = FULL ? 21u + (bc ? 8u + ((bc * 63u + 7u) >> 3) : 0u)
+                               : (len ? block_bytes((unsigned)len, bc, true) : 0u);
 
-  // ---- tile scan: block bytes (bits 0..23), CPs (24..43), extrema (44..63) ----
+  // ---- tile scans: block bytes, and points with extrema above them ----
   unsigned boff, cpo, exo;
   {
-    const unsigned long long v = (unsigned long long)(l == 0 ? bbytes : 0u) |
-                                 ((unsigned long long)__popc(cpm) << 24) |
-                                 ((unsigned long long)__popc(exm) << 44);
-    unsigned long long tot;
-    const unsigned long long ex = cta_excl_scan64<kE64Threads / 32>(v, sh.w64, &tot);
-    // lane 0 of the group added this block's bytes before the other lanes
-    boff = (unsigned)(ex & 0xffffffull) - (l == 0 ? 0u : bbytes);
-    cpo = (unsigned)((ex >> 24) & 0xfffffull);
-    exo = (unsigned)(ex >> 44);
+    // the eight lanes of a block hold its bytes: a scan over the warp's blocks
+    unsigned ib = bbytes, u = __shfl_up_sync(0xffffffffu, ib, 8);
+    if (lane >= 8) ib += u;
+    u = __shfl_up_sync(0xffffffffu, ib, 16);
+    if (lane >= 16) ib += u;
+    const unsigned c = (unsigned)__popc(cpm) | ((unsigned)__popc(exm) << 16);
+    unsigned ic = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      u = __shfl_up_sync(0xffffffffu, ic, o);
+      if (lane >= o) ic += u;
+    }
+    if (lane == 31) { sh.wb[warp] = ib; sh.wc[warp] = ic; }
+    // also the point after which every thread has left the image's last write-out
+    e64_sync();
+    unsigned sb = sh.wb[lane & 7], sc = sh.wc[lane & 7];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const unsigned ub = __shfl_up_sync(0xffffffffu, sb, o, 8), uc = __shfl_up_sync(0xffffffffu, sc, o, 8);
+      if ((lane & 7) >= o) { sb += ub; sc += uc; }
+    }
+    const unsigned tb = __shfl_sync(0xffffffffu, sb, 7), tc = __shfl_sync(0xffffffffu, sc, 7);
+    unsigned pb = __shfl_sync(0xffffffffu, sb, (warp + 7) & 7), pc = __shfl_sync(0xffffffffu, sc, (warp + 7) & 7);
+    if (warp == 0) { pb = 0u; pc = 0u; }
+    boff = pb + ib - bbytes;
+    pc += ic - c;
+    cpo = pc & 0xffffu;
+    exo = pc >> 16;
     if (tid == 0) {
-      sh.tile_bytes = (unsigned)(tot & 0xffffffull);
-      sh.tile_cps = (unsigned)((tot >> 24) & 0xfffffull);
-      sh.tile_ext = (unsigned)(tot >> 44);
-      publish_aggregate(a.desc, tile, tot & 0xffffffull,
-                        (((tot >> 24) & 0xfffffull) << 32) | (tot >> 44));
+      sh.tile_bytes = tb;
+      sh.tile_cps = tc & 0xffffu;
+      sh.tile_ext = tc >> 16;
+      // the first tile's own values are its inclusive ones
+      e64_publish(a.desc + tile, tile ? 1ull : 2ull, tb, ((unsigned long long)(tc & 0xffffu) << 32) | (tc >> 16));
     }
   }
   if (l == 0) sh.boff[bi] = boff;
 
-  // ---- critical-point pairs, staged in raster order ----
+  // ---- critical points, staged ----
   if (cpm) {
-    unsigned ci = cpo, ei = exo;
+    if (BITS) {
+      unsigned *st = static_cast<unsigned *>(stage);
+      unsigned ei = exo, si = kE64Tile - 1u - (cpo - exo);
 #pragma unroll
-    for (int t = 0; t < 8; t++) {
-      if ((cpm >> t) & 1u) {
-        const bool ext = (exm >> t) & 1u;
-        stage[ci++] = make_uint2(float_code(x[t]), ext ? ei : kNoExtremum);
-        ei += ext ? 1u : 0u;
+      for (int t = 0; t < 8; t++) {
+        if ((cpm >> (7 - t)) & 1u) {
+          const bool ext = (exm >> (7 - t)) & 1u;
+          st[ext ? ei : si] = value_code(x[t]);
+          if (ext) ei++; else si--;
+        }
+      }
+    } else {
+      uint2 *st = static_cast<uint2 *>(stage);
+      unsigned ci = cpo, ei = exo;
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        if ((cpm >> (7 - t)) & 1u) {
+          const bool ext = (exm >> (7 - t)) & 1u;
+          st[ci++] = make_uint2(value_code(x[t]), ext ? ei : kNoExtremum);
+          ei += ext ? 1u : 0u;
+        }
       }
     }
   }
 
   // ---- pack the octet into the tile image ----
-  if (nv > 0) {
+  if (FULL || nv > 0) {
     unsigned p = boff;
     if (l == 0) {
       const unsigned an = (unsigned)q[0];
@@ -242,26 +366,28 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
       img[p + 1] = (unsigned char)(an >> 8);
       img[p + 2] = (unsigned char)(an >> 16);
       img[p + 3] = (unsigned char)(an >> 24);
-      if (len > 1) img[p + 4] = (unsigned char)bc;
+      if (FULL || len > 1) img[p + 4] = (unsigned char)bc;
     }
     p += 4;
-    if (len > 1) {
+    if (FULL || len > 1) {
       p += 1;
       if (bc) {
-        const unsigned sbytes = (unsigned)(cnt + 7) / 8u;
-        const bool has_d = e0 < cnt;
-        if (has_d) img[p + l] = (unsigned char)(__brev(negm) >> 24);   // delta e0 + t at bit 7 - t
+        const unsigned sbytes = FULL ? 8u : (unsigned)(cnt + 7) / 8u;
+        const unsigned ucnt = FULL ? 63u : (unsigned)cnt;
+        const bool has_d = FULL || e0 < cnt;
+        if (has_d) img[p + l] = (unsigned char)sign;
         p += sbytes;
         const unsigned fb = bc >> 3, rem = bc & 7u;
         if (has_d) {
           if (fb == 1) {
 #pragma unroll
             for (int t = 0; t < 8; t++)
-              if (e0 + t < cnt) img[p + (unsigned)(e0 + t)] = (unsigned char)(mags[t] >> rem);
+              if (FULL ? (t < 7 || l < 7) : e0 + t < cnt)
+                img[p + (unsigned)(e0 + t)] = (unsigned char)(mags[t] >> rem);
           } else if (fb >= 2) {
 #pragma unroll
             for (int t = 0; t < 8; t++) {
-              if (e0 + t < cnt) {
+              if (e0 + t < (int)ucnt) {
                 unsigned v = mags[t] >> rem;
                 const unsigned o = p + (unsigned)(e0 + t) * fb;
                 for (unsigned u = 0; u < fb; u++) { img[o + u] = (unsigned char)v; v >>= 8; }
@@ -269,19 +395,27 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
             }
           }
         }
-        p += fb * (unsigned)cnt;
+        p += fb * ucnt;
         if (rem) {
-          const unsigned rbytes = (rem * (unsigned)cnt - 1u) / 8u + 1u;
+          // a full block's 63 fields leave less than a byte unused: 8 rem bytes
+          const unsigned rbytes = FULL ? 8u * rem : (rem * ucnt - 1u) / 8u + 1u;
           if (has_d) {
+            // the octet's 8 rem bits, left-aligned in hi:lo: exactly rem bytes at byte l * rem
             const unsigned mask = (1u << rem) - 1u;
-            unsigned long long acc = 0;
+            unsigned h = mags[0] & mask, w = mags[4] & mask;
 #pragma unroll
-            for (int t = 0; t < 8; t++) acc = (acc << rem) | (unsigned long long)(mags[t] & mask);
-            // the octet's 8 rem bits are exactly rem bytes at byte l * rem
-            const unsigned ob = (unsigned)l * rem;
+            for (int t = 1; t < 4; t++) {
+              h = (h << rem) | (mags[t] & mask);
+              w = (w << rem) | (mags[4 + t] & mask);
+            }
+            const unsigned up = 32u - 4u * rem;      // 4 .. 28
+            h <<= up;
+            w <<= up;
+            const unsigned hi = h | (w >> (4u * rem)), lo = w << (32u - 4u * rem);
+            const unsigned ob = p + (unsigned)l * rem, room = FULL ? rem : (rbytes > (unsigned)l * rem ? min(rem, rbytes - (unsigned)l * rem) : 0u);
 #pragma unroll
             for (unsigned u = 0; u < 7; u++)
-              if (u < rem && ob + u < rbytes) img[p + ob + u] = (unsigned char)(acc >> (8 * (rem - 1u - u)));
+              if (u < room) img[ob + u] = (unsigned char)(u < 4 ? hi >> (24u - 8u * u) : lo >> (56u - 8u * u));
           }
           p += rbytes;
         }
@@ -289,41 +423,71 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, un
     }
     // tag byte j: elements 4j .. 4j+3, element 4j in the top two bits
     const unsigned tb = ((unsigned)len + 3u) / 4u;
-    const unsigned t0 = ((types & 3u) << 6) | (((types >> 2) & 3u) << 4) | (((types >> 4) & 3u) << 2) |
-                        ((types >> 6) & 3u);
-    const unsigned t1 = (((types >> 8) & 3u) << 6) | (((types >> 10) & 3u) << 4) | (((types >> 12) & 3u) << 2) |
-                        ((types >> 14) & 3u);
-    if (2u * l < tb) img[p + 2 * l] = (unsigned char)t0;
-    if (2u * l + 1u < tb) img[p + 2 * l + 1] = (unsigned char)t1;
+    if (FULL || 2u * l < tb) img[p + 2 * l] = (unsigned char)(tags >> 8);
+    if (FULL || 2u * l + 1u < tb) img[p + 2 * l + 1] = (unsigned char)tags;
   }
 }
 
-// Back half of a tile: look-back for the tile's stream and CP offsets, block
-// index, write-out of the image and copy-out of the staged pairs.  Ends with
-// a CTA barrier.
+// Look-back of a tile by one warp, four predecessors per lane and round.
+// Publishes the inclusive prefix.
+__device__ __forceinline__ Prefix e64_lookback(TileDesc *desc, long long t, unsigned long long agg_bytes,
+                                               unsigned long long agg_cnt, int *err, int spin_limit) {
+  const int lane = threadIdx.x & 31;
+  const int limit = spin_limit > 0 ? spin_limit : kSpinLimit;
+  Prefix ex{0ull, 0ull};
+  if (t > 0) {
+    bool timed_out = false, found = false;
+    for (long long base = t - 1; !found; base -= 128) {
+      unsigned long long st[4], ct[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const long long idx = base - 32 * u - lane;
+        st[u] = 2ull << kStatShift;
+        ct[u] = 0;
+        if (idx >= 0) e64_read(desc + idx, st[u], ct[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const long long idx = base - 32 * u - lane;
+        if (!found) {
+          int spins = 0;
+          while ((st[u] >> kStatShift) == 0ull) {
+            if (++spins > limit) { timed_out = true; break; }
+            __nanosleep(spins < 64 ? 32 : 256);
+            e64_read(desc + idx, st[u], ct[u]);
+          }
+          unsigned long long flag = st[u] >> kStatShift;
+          if (flag == 0ull) flag = 2ull;   // timed out: an empty inclusive value
+          const unsigned m = __ballot_sync(0xffffffffu, flag == 2ull);
+          const int first = m ? __ffs(m) - 1 : 32;
+          if (lane <= first) {
+            ex.bytes += st[u] & kByteMask;
+            ex.cnt += ct[u];
+          }
+          found = m != 0u;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ex.bytes += __shfl_xor_sync(0xffffffffu, ex.bytes, o);
+      ex.cnt += __shfl_xor_sync(0xffffffffu, ex.cnt, o);
+    }
+    if (timed_out) atomicExch(err, kErrLookbackTimeout);
+  }
+  if (lane == 0) e64_publish(desc + t, 2ull, ex.bytes + agg_bytes, ex.cnt + agg_cnt);
+  return ex;
+}
+
+// Back half of a tile, its place known: block index, write-out of the image
+// and of the staged critical points.  The threads that own elements call it.
 template <bool BITS>
 __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, const unsigned char *img,
-                                         const uint2 *stage, E64Sh &sh, unsigned &nmax, unsigned &cmax) {
+                                         const void *stage, const E64Sh &sh, unsigned &nmax, unsigned &cmax) {
   const int tid = threadIdx.x;
   const long long n = (long long)a.n;
   const long long nblocks = (n + 63) / 64;
-  const long long ntiles = (n + kE64Tile - 1) / kE64Tile;
   const unsigned tile_bytes = sh.tile_bytes;
-  {
-    const Prefix pf = lookback_cta<kE64Threads / 32>(a.desc, tile, tile_bytes,
-                                                      ((unsigned long long)sh.tile_cps << 32) | sh.tile_ext, a.err,
-                                                      a.spin_limit);
-    if (tid == 0) {
-      sh.gbyte = pf.bytes;
-      sh.gcnt = pf.cnt;
-      if (tile == ntiles - 1 && a.total) {
-        a.total[0] = pf.bytes + tile_bytes;
-        a.total[1] = (pf.cnt >> 32) + sh.tile_cps;
-        a.total[2] = (pf.cnt & 0xffffffffull) + sh.tile_ext;
-      }
-    }
-  }
-  __syncthreads();
   const unsigned long long G0 = sh.gbyte;
   const bool fits = (G0 + tile_bytes) <= a.out_cap;
   if (!fits && tid == 0) atomicExch(a.err, kErrOutputOverflow);
@@ -358,82 +522,120 @@ __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, con
     const unsigned t0b = head + 16u * nq;
     if (t0b + tid < tile_bytes) dst[t0b + tid] = img[t0b + tid];
   }
+  const unsigned long long cb = sh.gcnt >> 32, eb0 = sh.gcnt & 0xffffffffull;
+  const unsigned ntc = sh.tile_cps, nte = sh.tile_ext;
   if (BITS) {
     // every value's bit; the extrema's codes in raster order
-    const unsigned long long cb = sh.gcnt >> 32, eb0 = sh.gcnt & 0xffffffffull;
-    const unsigned ntc = sh.tile_cps;
+    const unsigned *st = static_cast<const unsigned *>(stage);
     for (unsigned k = tid; k < ntc; k += kE64Threads) {
-      const uint2 pr = stage[k];
-      const unsigned ext = pr.y == kNoExtremum ? kNoExtremum : (unsigned)eb0 + pr.y;
-      rb_set(a.rb, pr.x, ext);
-      if (cb + k < kRankSmall) a.rb.first[cb + k] = make_uint2(pr.x, ext);
-      nmax = max(nmax, ~pr.x);
-      cmax = max(cmax, pr.x);
-      if (ext != kNoExtremum && eb0 + pr.y < a.cp_cap) a.code_out[eb0 + pr.y] = pr.x;
+      const bool is_ext = k < nte;
+      const unsigned code = st[is_ext ? k : kE64Tile - 1u - (k - nte)];
+      const unsigned ext = is_ext ? (unsigned)eb0 + k : kNoExtremum;
+      rb_set(a.rb, code, ext);
+      if (cb + k < kRankSmall) a.rb.first[cb + k] = make_uint2(code, ext);
+      nmax = max(nmax, ~code);
+      cmax = max(cmax, code);
+      if (is_ext && eb0 + k < a.cp_cap) a.code_out[eb0 + k] = code;
     }
-    if (tid == 0 && eb0 + sh.tile_ext > a.cp_cap) atomicExch(a.err, kErrCapacity);
+    if (tid == 0 && eb0 + nte > a.cp_cap) atomicExch(a.err, kErrCapacity);
   } else {
     // critical-point pairs in raster order
-    const unsigned long long cb = sh.gcnt >> 32;
-    const uint32_t eb0 = (uint32_t)(sh.gcnt & 0xffffffffull);
-    const unsigned ntc = sh.tile_cps;
+    const uint2 *st = static_cast<const uint2 *>(stage);
     uint2 *cp = a.cp_out;
     for (unsigned k = tid; k < ntc; k += kE64Threads) {
       if (cb + k < a.cp_cap) {
-        uint2 pr = stage[k];
-        if (pr.y != kNoExtremum) pr.y += eb0;
+        uint2 pr = st[k];
+        if (pr.y != kNoExtremum) pr.y += (unsigned)eb0;
         cp[cb + k] = pr;
       }
     }
     if (tid == 0 && cb + ntc > a.cp_cap) atomicExch(a.err, kErrCapacity);
   }
-  __syncthreads();
 }
 
-// Persistent CTAs claim tiles in order; each keeps two images and runs one
-// tile behind (tile k's aggregate is published before tile k-1 looks back),
-// so a look-back only ever waits for tiles held by running CTAs.
+// Persistent CTAs claim tiles in order.  Eight warps own the elements and keep
+// two images: they run one tile behind (the front half of tile k, whose
+// aggregate is published in it, then the write-out of tile k-1).  A ninth warp
+// claims the tiles and looks back for tile k-1 while the others are in the
+// front half of tile k.
+// A look-back waits for the aggregates of earlier tiles only, and a tile's
+// aggregate waits, through its CTA's barrier, for look-backs of earlier tiles
+// only, so the waits cannot form a cycle.
 template <bool D3, bool BITS>
-__global__ void __launch_bounds__(kE64Threads, 4) enc64_kernel(Enc64Args a) {
+__global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   __shared__ E64Sh sh[2];
-  __shared__ long long s_claim;
+  __shared__ long long s_claim[2];
+  constexpr unsigned kPart = e64_part(BITS);
   const long long ntiles = ((long long)a.n + kE64Tile - 1) / kE64Tile;
+  const long long nfull = (long long)a.n / kE64Tile;
   const long long tend = a.tile_hi ? (long long)a.tile_hi : ntiles;
+  const bool owner = threadIdx.x < kE64Threads;
+  // flat indices and extents of the field in 32 bits
+  const bool small = a.g.d1 * a.g.plane < (1ll << 32);
   long long prev = -1;
   int cur = 0;
   unsigned nmax = 0, cmax = 0;
   while (true) {
-    if (threadIdx.x == 0) s_claim = (long long)a.tile_lo + (long long)atomicAdd(a.tile_ctr, 1u);
-    __syncthreads();
-    const long long tile = s_claim;
+    // claimed only now (while the other warps write the last tile out), not a
+    // tile ahead: every look-back behind a claimed tile waits for its front half
+    long long tile;
+    if (owner) {
+      e64_claim_wait();
+      tile = s_claim[cur];
+    } else {
+      tile = 0;
+      if (threadIdx.x == kE64Threads) tile = (long long)a.tile_lo + (long long)atomicAdd(a.tile_ctr, 1u);
+      tile = __shfl_sync(0xffffffffu, tile, 0);
+      if (threadIdx.x == kE64Threads) s_claim[cur] = tile;
+      __syncwarp();
+      e64_claim_post();
+    }
     const bool more = tile < tend;
-    unsigned char *part = smem_dyn + (size_t)cur * kE64Part;
-    if (more) e64_front<D3>(a, tile, part, reinterpret_cast<uint2 *>(part + kE64Img), sh[cur]);
+    if (owner) {
+      unsigned char *part = smem_dyn + (size_t)cur * kPart;
+      if (more) {
+        if (tile < nfull) e64_front<D3, BITS, true>(a, tile, small, part, part + kE64Img, sh[cur]);
+        else e64_front<D3, BITS, false>(a, tile, small, part, part + kE64Img, sh[cur]);
+      }
+    } else {
+      if (prev >= 0) {
+        E64Sh &sp = sh[cur ^ 1];
+        const unsigned tb = sp.tile_bytes, tc = sp.tile_cps, te = sp.tile_ext;
+        const Prefix pf = e64_lookback(a.desc, prev, tb, ((unsigned long long)tc << 32) | te, a.err, a.spin_limit);
+        if (threadIdx.x == kE64Threads) {
+          sp.gbyte = pf.bytes;
+          sp.gcnt = pf.cnt;
+          if (prev == ntiles - 1 && a.total) {
+            a.total[0] = pf.bytes + tb;
+            a.total[1] = (pf.cnt >> 32) + tc;
+            a.total[2] = (pf.cnt & 0xffffffffull) + te;
+          }
+        }
+      }
+    }
     __syncthreads();
-    if (prev >= 0) {
-      const unsigned char *pp = smem_dyn + (size_t)(cur ^ 1) * kE64Part;
-      e64_back<BITS>(a, prev, pp, reinterpret_cast<const uint2 *>(pp + kE64Img), sh[cur ^ 1], nmax, cmax);
+    if (owner && prev >= 0) {
+      const unsigned char *pp = smem_dyn + (size_t)(cur ^ 1) * kPart;
+      e64_back<BITS>(a, prev, pp, pp + kE64Img, sh[cur ^ 1], nmax, cmax);
     }
     if (!more) break;
     prev = tile;
     cur ^= 1;
   }
-  if (BITS) rb_extent(a.rb, nmax, cmax);
+  if (BITS && owner) rb_extent(a.rb, nmax, cmax);
 }
 
 unsigned long long enc64_tiles(unsigned long long n) { return (n + kE64Tile - 1) / kE64Tile; }
 
-size_t enc64_smem_bytes() { return 2 * (size_t)kE64Part; }
-
 static cudaError_t launch_enc64(const Enc64Args &a, cudaStream_t s, int sm_count) {
-  const size_t smem = enc64_smem_bytes();
+  const size_t smem = 2 * (size_t)e64_part(a.code_out != nullptr);
   auto k = a.code_out ? (a.g.nd == 3 ? enc64_kernel<true, true> : enc64_kernel<false, true>)
                       : (a.g.nd == 3 ? enc64_kernel<true, false> : enc64_kernel<false, false>);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kE64Threads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kE64Cta, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   const unsigned long long ntiles = enc64_tiles(a.n);
@@ -442,7 +644,7 @@ static cudaError_t launch_enc64(const Enc64Args &a, cudaStream_t s, int sm_count
   unsigned long long grid = (unsigned long long)sm_count * per_sm;
   if (grid > span) grid = span;
   if (grid < 1) grid = 1;
-  k<<<(unsigned)grid, kE64Threads, smem, s>>>(a);
+  k<<<(unsigned)grid, kE64Cta, smem, s>>>(a);
   return cudaGetLastError();
 }
 
