@@ -150,13 +150,12 @@ __device__ __forceinline__ int classify_at(const float *__restrict__ d, long lon
                    __ldg(d + i + g.d3), __ldg(d + i - 1), __ldg(d + i + 1));
 }
 
-// Decoupled look-back tile descriptor: a status/bytes word plus two count
-// words (aggregate and inclusive), each count word written before its status.
-struct TileDesc {
+// Decoupled look-back tile descriptor: the status and count words are one
+// 16-byte word to readers and writers (tsz_lookback.cuh).
+struct alignas(16) TileDesc {
   unsigned long long status;   // bits 63..62: 0 none, 1 aggregate, 2 inclusive; 61..0 bytes
-  unsigned long long agg_cnt;  // (cps << 32) | extrema, this tile only
-  unsigned long long inc_cnt;  // inclusive counts up to and including this tile
-  unsigned long long pad;
+  unsigned long long cnt;      // (cps << 32) | extrema, of this tile or of all tiles through it
+  unsigned long long pad[2];   // the stream parser's exit entry
 };
 
 constexpr unsigned long long kStatShift = 62;

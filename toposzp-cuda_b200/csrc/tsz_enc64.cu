@@ -62,24 +62,6 @@ __device__ __forceinline__ void e64_sync() { asm volatile("bar.sync 1, 256;" :::
 __device__ __forceinline__ void e64_claim_post() { asm volatile("bar.arrive 2, 288;" ::: "memory"); }
 __device__ __forceinline__ void e64_claim_wait() { asm volatile("bar.sync 2, 288;" ::: "memory"); }
 
-// A tile's descriptor as one 16-byte word, read and written whole: the status
-// word (2-bit state, bytes) and the counts (points << 32 | extrema) of the
-// tile (state 1) or of all tiles through it (state 2).  Nothing else is
-// published with it, so no access needs an order, and a look-back waits for
-// one load where status, then counts, would be two in a row.
-__device__ __forceinline__ void e64_publish(TileDesc *d, unsigned long long state, unsigned long long bytes,
-                                            unsigned long long cnt) {
-  asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(d),
-               "l"((state << kStatShift) | (bytes & kByteMask)), "l"(cnt)
-               : "memory");
-}
-__device__ __forceinline__ void e64_read(const TileDesc *d, unsigned long long &st, unsigned long long &cnt) {
-  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
-               : "=l"(st), "=l"(cnt)
-               : "l"(d)
-               : "memory");
-}
-
 // Shifts the sign bit of f into the low end of mask.
 __device__ __forceinline__ unsigned push_sign(float f, unsigned mask) {
   return __funnelshift_l(__float_as_uint(f), mask, 1);
@@ -324,8 +306,7 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
       sh.tile_bytes = tb;
       sh.tile_cps = tc & 0xffffu;
       sh.tile_ext = tc >> 16;
-      // the first tile's own values are its inclusive ones
-      e64_publish(a.desc + tile, tile ? 1ull : 2ull, tb, ((unsigned long long)(tc & 0xffffu) << 32) | (tc >> 16));
+      publish_aggregate(a.desc, tile, tb, ((unsigned long long)(tc & 0xffffu) << 32) | (tc >> 16));
     }
   }
   if (l == 0) sh.boff[bi] = boff;
@@ -444,7 +425,7 @@ __device__ __forceinline__ Prefix e64_lookback(TileDesc *desc, long long t, unsi
         const long long idx = base - 32 * u - lane;
         st[u] = 2ull << kStatShift;
         ct[u] = 0;
-        if (idx >= 0) e64_read(desc + idx, st[u], ct[u]);
+        if (idx >= 0) desc_read(desc + idx, st[u], ct[u]);
       }
 #pragma unroll
       for (int u = 0; u < 4; u++) {
@@ -454,7 +435,7 @@ __device__ __forceinline__ Prefix e64_lookback(TileDesc *desc, long long t, unsi
           while ((st[u] >> kStatShift) == 0ull) {
             if (++spins > limit) { timed_out = true; break; }
             __nanosleep(spins < 64 ? 32 : 256);
-            e64_read(desc + idx, st[u], ct[u]);
+            desc_read(desc + idx, st[u], ct[u]);
           }
           unsigned long long flag = st[u] >> kStatShift;
           if (flag == 0ull) flag = 2ull;   // timed out: an empty inclusive value
@@ -475,7 +456,7 @@ __device__ __forceinline__ Prefix e64_lookback(TileDesc *desc, long long t, unsi
     }
     if (timed_out) atomicExch(err, kErrLookbackTimeout);
   }
-  if (lane == 0) e64_publish(desc + t, 2ull, ex.bytes + agg_bytes, ex.cnt + agg_cnt);
+  if (lane == 0) desc_publish(desc + t, 2ull, ex.bytes + agg_bytes, ex.cnt + agg_cnt);
   return ex;
 }
 

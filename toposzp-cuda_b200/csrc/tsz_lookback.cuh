@@ -12,18 +12,10 @@ namespace tsz {
 
 constexpr int kSpinLimit = 1 << 22;
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
-}
-__device__ __forceinline__ void st_release_u64(unsigned long long *p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -34,17 +26,29 @@ struct Prefix {
   unsigned long long cnt;  // (cps << 32) | extrema
 };
 
+// A tile's descriptor is one 16-byte word, read and written whole: the status
+// word (2-bit state, bytes) and the counts of the tile (state 1) or of all
+// tiles through it (state 2).  Nothing else is published with it, so no access
+// needs an order, and a look-back waits for one load where status, then
+// counts, would be two in a row.
+__device__ __forceinline__ void desc_publish(TileDesc *d, unsigned long long state, unsigned long long bytes,
+                                             unsigned long long cnt) {
+  asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(d),
+               "l"((state << kStatShift) | (bytes & kByteMask)), "l"(cnt)
+               : "memory");
+}
+__device__ __forceinline__ void desc_read(const TileDesc *d, unsigned long long &st, unsigned long long &cnt) {
+  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+               : "=l"(st), "=l"(cnt)
+               : "l"(d)
+               : "memory");
+}
+
 // Publishes tile t's aggregate as early as possible (one thread).  Tile 0's
 // aggregate is its inclusive prefix.
 __device__ __forceinline__ void publish_aggregate(TileDesc *desc, long long t, unsigned long long agg_bytes,
                                                   unsigned long long agg_cnt) {
-  if (t == 0) {
-    st_relaxed_u64(&desc[0].inc_cnt, agg_cnt);
-    st_release_u64(&desc[0].status, (2ull << kStatShift) | agg_bytes);
-  } else {
-    st_relaxed_u64(&desc[t].agg_cnt, agg_cnt);
-    st_release_u64(&desc[t].status, (1ull << kStatShift) | agg_bytes);
-  }
+  desc_publish(desc + t, t == 0 ? 2ull : 1ull, agg_bytes, agg_cnt);
 }
 
 // Called by all 32 lanes of one warp.  Returns the exclusive prefix of tile t.
@@ -62,14 +66,14 @@ __device__ inline Prefix lookback(TileDesc *desc, long long t, unsigned long lon
   bool timed_out = false;
   while (true) {
     long long idx = base - lane;
-    unsigned long long st = (2ull << kStatShift);
+    unsigned long long st = (2ull << kStatShift), ct = 0;
     if (idx >= 0) {
-      st = ld_acquire_u64(&desc[idx].status);
+      desc_read(desc + idx, st, ct);
       int spins = 0;
       while ((st >> kStatShift) == 0ull) {
         if (++spins > kSpinLimit) { timed_out = true; break; }
         __nanosleep(spins < 64 ? 32 : 256);
-        st = ld_acquire_u64(&desc[idx].status);
+        desc_read(desc + idx, st, ct);
       }
     }
     unsigned long long flag = st >> kStatShift;
@@ -79,7 +83,7 @@ __device__ inline Prefix lookback(TileDesc *desc, long long t, unsigned long lon
     unsigned long long b = 0, c = 0;
     if (lane <= first && idx >= 0 && (st >> kStatShift) != 0ull) {
       b = st & kByteMask;
-      c = (flag == 2ull) ? ld_relaxed_u64(&desc[idx].inc_cnt) : ld_relaxed_u64(&desc[idx].agg_cnt);
+      c = ct;
     }
     for (int o = 16; o > 0; o >>= 1) {
       b += __shfl_xor_sync(0xffffffffu, b, o);
@@ -91,10 +95,7 @@ __device__ inline Prefix lookback(TileDesc *desc, long long t, unsigned long lon
     base -= 32;
   }
   if (__any_sync(0xffffffffu, timed_out) && lane == 0) atomicExch(err, kErrLookbackTimeout);
-  if (lane == 0) {
-    st_relaxed_u64(&desc[t].inc_cnt, ex.cnt + agg_cnt);
-    st_release_u64(&desc[t].status, (2ull << kStatShift) | ((ex.bytes + agg_bytes) & kByteMask));
-  }
+  if (lane == 0) desc_publish(desc + t, 2ull, ex.bytes + agg_bytes, ex.cnt + agg_cnt);
   __syncwarp();
   return ex;
 }
@@ -126,14 +127,14 @@ __device__ inline Prefix lookback_cta(TileDesc *desc, long long t, unsigned long
   bool timed_out = false;
   for (int r = 0;; r ^= 1) {
     const long long idx = base - (long long)threadIdx.x;
-    unsigned long long st = (2ull << kStatShift);
+    unsigned long long st = (2ull << kStatShift), ct = 0;
     if (idx >= 0) {
-      st = ld_acquire_u64(&desc[idx].status);
+      desc_read(desc + idx, st, ct);
       int spins = 0;
       while ((st >> kStatShift) == 0ull) {
         if (++spins > limit) { timed_out = true; break; }
         __nanosleep(spins < 64 ? 32 : 256);
-        st = ld_acquire_u64(&desc[idx].status);
+        desc_read(desc + idx, st, ct);
       }
     }
     unsigned long long flag = st >> kStatShift;
@@ -144,7 +145,7 @@ __device__ inline Prefix lookback_cta(TileDesc *desc, long long t, unsigned long
     unsigned long long b = 0, c = 0;
     if (lane <= wfirst && idx >= 0 && (st >> kStatShift) != 0ull) {
       b = st & kByteMask;
-      c = (flag == 2ull) ? ld_relaxed_u64(&desc[idx].inc_cnt) : ld_relaxed_u64(&desc[idx].agg_cnt);
+      c = ct;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -170,10 +171,7 @@ __device__ inline Prefix lookback_cta(TileDesc *desc, long long t, unsigned long
     base -= WARPS * 32;
   }
   if (timed_out) atomicExch(err, kErrLookbackTimeout);
-  if (threadIdx.x == 0) {
-    st_relaxed_u64(&desc[t].inc_cnt, ex.cnt + agg_cnt);
-    st_release_u64(&desc[t].status, (2ull << kStatShift) | ((ex.bytes + agg_bytes) & kByteMask));
-  }
+  if (threadIdx.x == 0) desc_publish(desc + t, 2ull, ex.bytes + agg_bytes, ex.cnt + agg_cnt);
   return ex;
 }
 

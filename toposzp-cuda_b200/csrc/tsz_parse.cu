@@ -191,7 +191,7 @@ __device__ void compose_group(const ParseTree &t, int l, unsigned grp, unsigned 
 
 // Outcome of the guess and what it shares between segments.
 struct ParseGuess {
-  TileDesc *desc;        // per tile, zeroed: count of blocks; pad = exit entry
+  TileDesc *desc;        // per tile, zeroed: count of blocks; pad[0] = exit entry
   unsigned *words;       // zeroed: [0] tile ticket, [1] a guess failed, [2] look-back status
   unsigned unit;         // segment bytes (a multiple of 16, above 4 M)
   unsigned list;         // entries of a warp's list: blocks of a segment, or M
@@ -483,8 +483,9 @@ __device__ __forceinline__ void guess_back(const ParseGeom &g, const ParseOut &o
   const Prefix pf = lookback_cta<NW>(u.desc, tile, s.total, 0ull, reinterpret_cast<int *>(u.words + 2));
   if (threadIdx.x < NW) {
     const unsigned k = threadIdx.x;
+    __threadfence();   // thread 0 has read the descriptor of the tile before
     // a segment that holds a block of the stream starts where the one before it ended
-    const unsigned before = k ? s.exit[k - 1] : (tile ? (unsigned)ld_relaxed_u64(&u.desc[tile - 1].pad) : 0u);
+    const unsigned before = k ? s.exit[k - 1] : (tile ? (unsigned)ld_relaxed_u64(u.desc[tile - 1].pad) : 0u);
     if (pf.bytes + s.off[k] < d.nb && s.entry[k] != before) u.words[1] = 1u;
   }
   const unsigned long long s0 = ((unsigned long long)tile * NW + w) * u.unit, idx0 = pf.bytes + s.off[w];
@@ -592,7 +593,9 @@ parse_guess_kernel(ParseGeom g, unsigned ntiles, ParseOut o, ParseGuess u) {
         if (lane == NW - 1) {
           s.tile = tile;
           s.total = inc;
-          st_relaxed_u64(&u.desc[tile].pad, exit);
+          // the exit first: a reader of the descriptor, past a fence, sees it
+          st_relaxed_u64(u.desc[tile].pad, exit);
+          __threadfence();
           publish_aggregate(u.desc, tile, inc, 0ull);
         }
       }
