@@ -118,3 +118,36 @@ def test_batch_reports_small_buffers(T):
     res = b.compress(items)
     assert res[0][2].topo_bytes > 8
     b.close()
+
+
+def test_batch_rank_tiers_and_encoders(T):
+    """Fields whose points are sorted by one CTA, ranked in bitmaps, sorted per
+    bucket (bins next to zero) and radix-sorted (over 16384 in a bucket), in
+    one batch, equal the per-field calls; once more with one field at an
+    address that is not 16-byte aligned, which the general encoder takes."""
+    import torch
+    rng = np.random.default_rng(5)
+    specs = [((40, 41), 1e-2), ((3, 3), 1e-2), ((600, 700), 1e-3), ((700, 600), 1e-2), ((900, 1000), 0.5),
+             ((60, 70, 80), 1e-3), ((1, 64), 1e-2), ((512, 512), 5.0), ((2048, 3), 1e-2), ((800, 801), 1e-4)]
+    items = []
+    for k, (dims, eb) in enumerate(specs):
+        d = rng.standard_normal(dims).astype(np.float32)
+        if k == 9:
+            d = np.abs(d) + np.float32(1)
+        items.append((torch.from_numpy(d.reshape(-1)).cuda(), dims, eb, False))
+    ctx = T.Context()
+    want = []
+    for x, dims, eb, _ in items:
+        topo, sort, _, sz = ctx.compress(x, dims, eb, 64, index=False)
+        want.append((topo[:sz.topo_bytes].clone(), sort[:sz.sort_bytes].clone(), sz.cp_count, sz.extrema_count))
+    shifted = torch.empty(items[3][0].numel() + 1, dtype=torch.float32, device="cuda")
+    shifted[1:] = items[3][0]
+    b = T.Batch(64)
+    for its in (items, items[:3] + [(shifted[1:],) + items[3][1:]] + items[4:], items):
+        for (tb, sb, sz, _), (t, s, k, e) in zip(b.compress(its), want):
+            assert (sz.cp_count, sz.extrema_count) == (k, e)
+            assert sz.topo_bytes == t.numel() and torch.equal(tb[:sz.topo_bytes], t)
+            assert sz.sort_bytes == s.numel() and torch.equal(sb[:sz.sort_bytes], s)
+    assert b.tuning()["tuned"]
+    ctx.close()
+    b.close()

@@ -5,19 +5,19 @@
 //   upload the field table -> init -> min/max of the relative-bound fields ->
 //   absolute bounds -> ONE persistent topology-encoder launch over a device
 //   tile work-queue spanning every field -> per-field CP / extremum prefix ->
-//   gather all fields' CP pairs into one list with field-disjoint bins ->
 //   results to pinned host memory.
-// Rank: one pass of the bucket/bitmap rank over the whole batch (bins of
-//   different fields never meet: each field's bins are shifted into its own
-//   range).  Should the shifted ranges not fit in 31 bits, fields are ranked
-//   one by one instead.
+// Rank: one pass of the bucket/bitmap rank over the pairs of the whole batch,
+//   where they lie; every field has buckets of its own.
 // Stage C (one CUDA graph): upload the sort-stream table -> ONE persistent
 //   launch of the integer encoder over all fields' sort positions.
 // The streams are byte-identical to the per-field calls.
 //
-// The encoder's CTA shape (warps per CTA, hence codec blocks per tile) and the
-// persistent grid (CTAs per SM) are chosen by an autotuner that times the
-// candidates on the first batch; the format's blockSize is never tuned.
+// blockSize 64 with 16-byte aligned fields takes the blockSize-64 encoder
+// (tsz_enc64.cu; 256 fields, 169 M elements: 1.2 ms against 2.5 ms of the
+// general one).  The general encoder's CTA shape (warps per CTA, hence codec
+// blocks per tile) and persistent grid (CTAs per SM), and the sort-position
+// encoder's, are chosen by an autotuner that times the candidates on the first
+// batch; the format's blockSize is never tuned.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "tsz_codec2.cuh"
+#include "tsz_enc64.h"
 #include "tsz_ops.h"
 #include "tsz_runtime.h"
 
@@ -48,7 +49,7 @@ struct BatchHdr {
   unsigned long long nchunks;     // min/max chunks over all relative-bound fields
 };
 
-constexpr unsigned long long kMinMaxChunk = 1ull << 16;
+constexpr unsigned long long kMinMaxChunk = 1ull << 15;   // a multiple of 32 values per thread
 constexpr int kAuxThreads = 256;
 
 // ---- table layout (host pinned copy and device copy are identical) ----
@@ -73,7 +74,7 @@ struct ResultLayout {
     kbase = o; o += a256(8 * ((size_t)cap + 1));
     ebase = o; o += a256(8 * ((size_t)cap + 1));
     eb = o; o += a256(4 * (size_t)cap);
-    flags = o; o += a256(8 * 8);   // [0] bin overflow, [1] encoder status, [2] bad bound
+    flags = o; o += a256(8 * 8);   // [1] encoder status, [2] bad bound
     bytes = o;
   }
 };
@@ -87,14 +88,11 @@ __device__ __forceinline__ int last_le(const unsigned long long *a, int n, unsig
   return lo;
 }
 
-__global__ void batch_init_kernel(const BatchHdr *hdr, const BatchFieldDev *fields, unsigned *minmax,
-                                  int *binmm) {
+__global__ void batch_init_kernel(const BatchHdr *hdr, const BatchFieldDev *fields, unsigned *minmax) {
   const unsigned nf = hdr->nf;
   for (unsigned f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
     minmax[2 * f] = 0xFFFFFFFFu;
     minmax[2 * f + 1] = 0u;
-    binmm[2 * f] = INT_MAX;
-    binmm[2 * f + 1] = INT_MIN;
     unsigned char *t = fields[f].topo;
     for (int i = 0; i < 8; i++) t[i] = 0;   // offset table of a single-chunk stream
   }
@@ -119,10 +117,29 @@ __global__ void __launch_bounds__(kAuxThreads) batch_minmax_kernel(const BatchHd
     const unsigned long long b0 = (c - fd.chunk0) * kMinMaxChunk;
     const unsigned long long b1 = min(fd.n, b0 + kMinMaxChunk);
     unsigned mn = 0xFFFFFFFFu, mx = 0u;
-    for (unsigned long long i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
-      const unsigned v = float_code(__ldg(fd.data + i));
-      mn = min(mn, v);
-      mx = max(mx, v);
+    // a whole chunk of an aligned field: 16-byte loads, eight in flight a thread
+    if (b1 - b0 == kMinMaxChunk && (reinterpret_cast<uintptr_t>(fd.data) & 15) == 0) {
+      const float4 *p = reinterpret_cast<const float4 *>(fd.data + b0);
+      for (unsigned i = threadIdx.x; i < kMinMaxChunk / 4; i += 8 * kAuxThreads) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = __ldg(p + i + u * kAuxThreads);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const unsigned c[4] = {float_code(v[u].x), float_code(v[u].y), float_code(v[u].z), float_code(v[u].w)};
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            mn = min(mn, c[k]);
+            mx = max(mx, c[k]);
+          }
+        }
+      }
+    } else {
+      for (unsigned long long i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
+        const unsigned v = float_code(__ldg(fd.data + i));
+        mn = min(mn, v);
+        mx = max(mx, v);
+      }
     }
     for (int o = 16; o > 0; o >>= 1) {
       mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
@@ -191,77 +208,6 @@ __global__ void batch_plan_kernel(const BatchHdr *hdr, const unsigned long long 
     __syncthreads();
   }
   if (threadIdx.x == 0) { kbase[nf] = s_ck; ebase[nf] = s_ce; }
-}
-
-// all fields' CP pairs into one list: extremum destinations made global and
-// bins computed with each field's bound; per-field bin range reduced
-__global__ void __launch_bounds__(kAuxThreads) batch_gather_kernel(
-    const BatchHdr *hdr, const BatchFieldDev *fields, const EncArgs *args, const uint2 *pairs,
-    const unsigned long long *kbase, const unsigned long long *ebase, uint2 *pairs_all, int *bins,
-    int *binmm) {
-  const int nf = (int)hdr->nf;
-  const unsigned long long K = kbase[nf];
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long k0 = (unsigned long long)blockIdx.x * blockDim.x; k0 < K; k0 += stride) {
-    const unsigned long long k = k0 + threadIdx.x;
-    const bool in = k < K;
-    int f = 0, bin = 0;
-    if (in) {
-      f = last_le(kbase, nf, k);
-      const uint2 p = pairs[fields[f].pairs_off + (k - kbase[f])];
-      bin = quant_bin(code_float(p.x), args[f].eb, args[f].inv);
-      pairs_all[k] = make_uint2(p.x, p.y == kNoExtremum ? kNoExtremum : (uint32_t)(p.y + ebase[f]));
-      bins[k] = bin;
-    }
-    const unsigned act = __ballot_sync(0xffffffffu, in);
-    const int f0 = __shfl_sync(0xffffffffu, f, 0);
-    const bool same = __all_sync(0xffffffffu, !in || f == f0);
-    if (same) {
-      int mn = in ? bin : INT_MAX, mx = in ? bin : INT_MIN;
-      for (int o = 16; o > 0; o >>= 1) {
-        mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      }
-      if ((threadIdx.x & 31) == 0 && act) {
-        atomicMin(&binmm[2 * f0], mn);
-        atomicMax(&binmm[2 * f0 + 1], mx);
-      }
-    } else if (in) {
-      atomicMin(&binmm[2 * f], bin);
-      atomicMax(&binmm[2 * f + 1], bin);
-    }
-  }
-}
-
-// field-disjoint bin ranges: field f's bins move to [base_f, base_f + range_f)
-__global__ void batch_offsets_kernel(const BatchHdr *hdr, const unsigned long long *totals, const int *binmm,
-                                     long long *off, unsigned long long *flags) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const unsigned nf = hdr->nf;
-  long long base = 0;
-  bool over = false;
-  for (unsigned f = 0; f < nf; f++) {
-    off[f] = 0;
-    if (totals[3 * f + 1] == 0) continue;
-    off[f] = base - (long long)binmm[2 * f];
-    base += (long long)binmm[2 * f + 1] - (long long)binmm[2 * f] + 1;
-    if (base > (long long)INT_MAX) over = true;
-  }
-  flags[0] = over ? 1ull : 0ull;
-}
-
-__global__ void __launch_bounds__(kAuxThreads) batch_apply_kernel(const BatchHdr *hdr,
-                                                                  const unsigned long long *kbase,
-                                                                  const long long *off,
-                                                                  const unsigned long long *flags, int *bins) {
-  if (flags[0]) return;   // ranges overflow: fields are ranked one by one
-  const int nf = (int)hdr->nf;
-  const unsigned long long K = kbase[nf];
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < K; k += stride) {
-    const int f = last_le(kbase, nf, k);
-    bins[k] = (int)((long long)bins[k] + off[f]);
-  }
 }
 
 // offset table of every non-empty sort-position stream
@@ -338,6 +284,7 @@ struct szp_b200_batch {
   bool use_graphs = true;
   int autotune = 1;
   bool tuned = false;
+  bool tuned_topo = false;  // the general topology encoder's shape too
   EncTune tune[2];          // [0] topology encoder, [1] sort-position encoder
   float tune_ms[2][16] = {};
   int tune_count[2] = {0, 0};
@@ -350,10 +297,10 @@ struct szp_b200_batch {
   unsigned char *d_tab = nullptr, *d_itab = nullptr, *d_res = nullptr, *d_ires = nullptr;
   TileDesc *d_desc = nullptr, *d_idesc = nullptr;
   unsigned *d_minmax = nullptr, *d_queue = nullptr;
-  int *d_binmm = nullptr;
-  long long *d_off = nullptr;
-  uint2 *d_pairs = nullptr, *d_pairs_all = nullptr;
-  int *d_bins = nullptr, *d_sp = nullptr;
+  uint2 *d_pairs = nullptr;
+  int *d_sp = nullptr;
+  bool use64 = false;       // the blockSize-64 encoder applies to the current batch
+  int per_sm64 = 0;
   unsigned long long *d_dummy = nullptr;
   cudaGraphExec_t graph_a = nullptr, graph_c = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -368,15 +315,13 @@ static void batch_free_buffers(szp_b200_batch *b) {
   cudaFreeHost(b->h_tab); cudaFreeHost(b->h_itab); cudaFreeHost(b->h_res); cudaFreeHost(b->h_ires);
   b->h_tab = b->h_itab = b->h_res = b->h_ires = nullptr;
   void *dv[] = {b->d_tab, b->d_itab, b->d_res, b->d_ires, b->d_desc, b->d_idesc, b->d_minmax, b->d_queue,
-                b->d_binmm, b->d_off, b->d_pairs, b->d_pairs_all, b->d_bins, b->d_sp, b->d_dummy};
+                b->d_pairs, b->d_sp, b->d_dummy};
   for (void *p : dv) if (p) cudaFree(p);
   b->d_tab = b->d_itab = b->d_res = b->d_ires = nullptr;
   b->d_desc = b->d_idesc = nullptr;
   b->d_minmax = b->d_queue = nullptr;
-  b->d_binmm = nullptr;
-  b->d_off = nullptr;
-  b->d_pairs = b->d_pairs_all = nullptr;
-  b->d_bins = b->d_sp = nullptr;
+  b->d_pairs = nullptr;
+  b->d_sp = nullptr;
   b->d_dummy = nullptr;
   b->cap_f = 0;
   b->cap_tiles = b->cap_pairs = b->cap_itiles = 0;
@@ -414,9 +359,8 @@ static bool batch_reserve(szp_b200_batch *b, int nf, unsigned long long tiles, u
   memset(b->h_itab, 0, b->tl.bytes);
   if (!dalloc(&b->d_tab, b->tl.bytes) || !dalloc(&b->d_itab, b->tl.bytes) || !dalloc(&b->d_res, b->rl.bytes) ||
       !dalloc(&b->d_ires, b->rl.bytes) || !dalloc(&b->d_desc, ct + cf + 1) || !dalloc(&b->d_idesc, ci + cf + 1) ||
-      !dalloc(&b->d_minmax, 2 * (size_t)cf) || !dalloc(&b->d_queue, 8) || !dalloc(&b->d_binmm, 2 * (size_t)cf) ||
-      !dalloc(&b->d_off, (size_t)cf) || !dalloc(&b->d_pairs, cp) || !dalloc(&b->d_pairs_all, cp) ||
-      !dalloc(&b->d_bins, cp) || !dalloc(&b->d_sp, cp) || !dalloc(&b->d_dummy, 8))
+      !dalloc(&b->d_minmax, 2 * (size_t)cf) || !dalloc(&b->d_queue, 8) ||
+      !dalloc(&b->d_pairs, cp) || !dalloc(&b->d_sp, cp) || !dalloc(&b->d_dummy, 8))
     return false;
   b->cap_f = cf;
   b->cap_tiles = ct;
@@ -448,20 +392,17 @@ static int enqueue_stage_a(szp_b200_batch *b, cudaStream_t s) {
       cuda_fail(cudaMemsetAsync(b->d_desc, 0, (b->cap_tiles + b->cap_f + 1) * sizeof(TileDesc), s), "memset") ||
       cuda_fail(cudaMemsetAsync(b->d_queue, 0, 8 * sizeof(unsigned), s), "memset"))
     return -1;
-  batch_init_kernel<<<(b->cap_f + 255) / 256, 256, 0, s>>>(hdr, fields, b->d_minmax, b->d_binmm);
+  batch_init_kernel<<<(b->cap_f + 255) / 256, 256, 0, s>>>(hdr, fields, b->d_minmax);
   batch_minmax_kernel<<<aux_grid, kAuxThreads, 0, s>>>(hdr, fields, b->d_minmax);
   batch_eb_kernel<<<(b->cap_f + 255) / 256, 256, 0, s>>>(hdr, fields, b->d_minmax, args, eb_out, flags);
   if (cuda_fail(cudaGetLastError(), "batch setup kernels")) return -1;
-  if (cuda_fail(launch_batch_encode(kEncClassify, b->tune[0].warps, args, tstart, &hdr->nf, b->d_queue, b->B,
-                                    persistent_grid(b, b->tune[0]), s),
+  if (cuda_fail(b->use64 ? launch_enc64_batch(args, tstart, &hdr->nf, b->d_queue, s, b->ctx->sm_count * b->per_sm64)
+                         : launch_batch_encode(kEncClassify, b->tune[0].warps, args, tstart, &hdr->nf, b->d_queue,
+                                               b->B, persistent_grid(b, b->tune[0]), s),
                 "batched topology encoder"))
     return -1;
   batch_plan_kernel<<<1, 1024, 0, s>>>(hdr, totals, kbase, ebase);
-  batch_gather_kernel<<<aux_grid, kAuxThreads, 0, s>>>(hdr, fields, args, b->d_pairs, kbase, ebase,
-                                                       b->d_pairs_all, b->d_bins, b->d_binmm);
-  batch_offsets_kernel<<<1, 32, 0, s>>>(hdr, totals, b->d_binmm, b->d_off, flags);
-  batch_apply_kernel<<<aux_grid, kAuxThreads, 0, s>>>(hdr, kbase, b->d_off, flags, b->d_bins);
-  if (cuda_fail(cudaGetLastError(), "batch gather kernels") ||
+  if (cuda_fail(cudaGetLastError(), "batch kernels") ||
       cuda_fail(cudaMemcpyAsync(b->h_res, b->d_res, R.bytes, cudaMemcpyDeviceToHost, s), "D2H batch results"))
     return -1;
   return 0;
@@ -491,11 +432,15 @@ static int enqueue_stage_c(szp_b200_batch *b, cudaStream_t s) {
 static int run_stage(szp_b200_batch *b, int which) {
   cudaStream_t s = b->ctx->stream;
   cudaGraphExec_t &ge = which == 0 ? b->graph_a : b->graph_c;
-  if (cuda_fail(launch_batch_encode(which == 0 ? kEncClassify : kEncInts, b->tune[which].warps, nullptr, nullptr,
-                                    nullptr, nullptr, b->B, 1, s, true),
-                "encoder attributes"))
+  if (which == 0 && b->use64) {
+    if (b->per_sm64 == 0 && cuda_fail(enc64_batch_prepare(&b->per_sm64), "encoder attributes")) return -1;
+    b->per_sm64 = std::max(1, b->per_sm64);
+  } else if (cuda_fail(launch_batch_encode(which == 0 ? kEncClassify : kEncInts, b->tune[which].warps, nullptr, nullptr,
+                                           nullptr, nullptr, b->B, 1, s, true),
+                       "encoder attributes")) {
     return -1;
-  b->ctx->launches += which == 0 ? 8 : 2;
+  }
+  b->ctx->launches += which == 0 ? 5 : 2;
   if (!b->use_graphs) {
     return which == 0 ? enqueue_stage_a(b, s) : enqueue_stage_c(b, s);
   }
@@ -537,7 +482,7 @@ static void fill_topo_table(szp_b200_batch *b, const szp_b200_batch_field *fs, i
   const ResultLayout &R = b->rl;
   unsigned long long *totals = reinterpret_cast<unsigned long long *>(b->d_res + R.totals);
   unsigned long long *flags = reinterpret_cast<unsigned long long *>(b->d_res + R.flags);
-  const int TB = tile_blocks_w(b->B, b->tune[0].warps);
+  const int TB = b->use64 ? enc_tile_blocks(64) : tile_blocks_w(b->B, b->tune[0].warps);
   unsigned long long t = 0, p = 0, ch = 0;
   for (int f = 0; f < nf; f++) {
     const FieldPlan &P = plan[f];
@@ -651,7 +596,7 @@ static int autotune_encoder(szp_b200_batch *b, int which, const szp_b200_batch_f
       if (which == 0) {
         // the relative bounds are resolved once before the timed encoder run
         const BatchFieldDev *fields = reinterpret_cast<const BatchFieldDev *>(d + T.fields);
-        batch_init_kernel<<<(b->cap_f + 255) / 256, 256, 0, s>>>(hdr, fields, b->d_minmax, b->d_binmm);
+        batch_init_kernel<<<(b->cap_f + 255) / 256, 256, 0, s>>>(hdr, fields, b->d_minmax);
         batch_minmax_kernel<<<b->ctx->sm_count * 4, kAuxThreads, 0, s>>>(hdr, fields, b->d_minmax);
         batch_eb_kernel<<<(b->cap_f + 255) / 256, 256, 0, s>>>(
             hdr, fields, b->d_minmax, const_cast<EncArgs *>(args),
@@ -704,7 +649,10 @@ szp_b200_batch *szp_b200_batch_create(void *cuda_stream, int blockSize) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   for (int m = 0; m < 2; m++)
     for (auto &kv : g_tune_cache)
-      if (kv.first == tune_key(b->ctx->device, blockSize, m)) { b->tune[m] = kv.second; b->tuned = true; }
+      if (kv.first == tune_key(b->ctx->device, blockSize, m)) {
+        b->tune[m] = kv.second;
+        (m == 0 ? b->tuned_topo : b->tuned) = true;
+      }
   return b;
 }
 
@@ -723,7 +671,7 @@ int szp_b200_batch_configure(szp_b200_batch *b, int use_graphs, int autotune) {
   if (!b) { set_error("null batch"); return -1; }
   b->use_graphs = use_graphs != 0;
   b->autotune = autotune;
-  if (autotune > 1) b->tuned = false;   // tune again on the next batch
+  if (autotune > 1) b->tuned = b->tuned_topo = false;   // tune again on the next batch
   drop_graphs(b);
   return 0;
 }
@@ -760,7 +708,7 @@ int szp_b200_batch_reserve(szp_b200_batch *b, int max_fields, size_t max_element
   if (b->cap_f != oldcap || b->cap_tiles != oldt || b->cap_pairs != oldp || b->cap_itiles != oldi) drop_graphs(b);
   szp_b200_ctx *ctx = b->ctx;
   if (!ctx->scratch.reserve(std::max(rank_scratch_bytes(N, ctx->sm_count),
-                                     rank_scratch_bytes_seg(N, max_fields, ctx->sm_count)) + 8192))
+                                     rank_scratch_bytes_fields(N, max_fields, ctx->sm_count)) + 8192))
     return -1;
   return cuda_fail(cudaStreamSynchronize(ctx->stream), "batch reserve") ? -1 : 0;
 }
@@ -797,19 +745,30 @@ int szp_b200_batch_compress(szp_b200_batch *b, szp_b200_batch_field *fs, int cou
   if (b->cap_f != oldcap || b->cap_tiles != oldt || b->cap_pairs != oldp || b->cap_itiles != oldi) drop_graphs(b);
   szp_b200_ctx *ctx = b->ctx;
   cudaStream_t s = ctx->stream;
-  if (b->autotune == 1 && !b->tuned) {
+  bool use64 = B == 64 && enc_tile_blocks(64) == kEnc64TileBlocks;
+  for (int f = 0; f < count; f++) use64 = use64 && (reinterpret_cast<uintptr_t>(fs[f].d_data) & 15) == 0;
+  if (use64 != b->use64) {
+    b->use64 = use64;
+    drop_graphs(b);
+  }
+  if (b->autotune == 1 && (!b->tuned || (!use64 && !b->tuned_topo))) {
     // shapes already tuned on this device by another batch object
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    int found = 0;
+    bool found[2] = {false, false};
     for (int m = 0; m < 2; m++)
       for (auto &kv : g_tune_cache)
-        if (kv.first == tune_key(ctx->device, B, m)) { b->tune[m] = kv.second; found++; }
-    if (found == 2) { b->tuned = true; drop_graphs(b); }
+        if (kv.first == tune_key(ctx->device, B, m)) { b->tune[m] = kv.second; found[m] = true; }
+    if (found[0] || found[1]) drop_graphs(b);
+    b->tuned_topo = b->tuned_topo || found[0];
+    b->tuned = b->tuned || (found[1] && (found[0] || use64));
   }
   const bool tune_now = b->autotune && !b->tuned;
   tl_begin(ctx);
-  if (tune_now) {
+  // the general encoder's shape is tuned when it first runs
+  const bool tune_topo = b->autotune && !use64 && (tune_now || !b->tuned_topo);
+  if (tune_topo) {
     if (autotune_encoder(b, 0, fs, count, plan, nullptr, nullptr)) return -1;
+    b->tuned_topo = true;
     drop_graphs(b);
   }
   fill_topo_table(b, fs, count, plan);
@@ -841,21 +800,14 @@ int szp_b200_batch_compress(szp_b200_batch *b, szp_b200_batch_field *fs, int cou
   std::vector<unsigned long long> eb_base(ebase, ebase + count + 1);
   // ranks of the whole batch
   if (Etot > 0) {
-    if (!ctx->scratch.reserve(std::max(rank_scratch_bytes(Ktot, ctx->sm_count),
-                                       rank_scratch_bytes_seg(Ktot, count, ctx->sm_count)) + 8192))
-      return -1;
-    if (!flags[0]) {
-      std::vector<unsigned long long> Kf(count);
-      for (int f = 0; f < count; f++) Kf[f] = totals[3 * f + 1];
-      if (rank_positions_seg(ctx, b->d_pairs_all, b->d_bins, Kf.data(), count, b->d_sp)) return -1;
-    } else {
-      for (int f = 0; f < count; f++) {
-        const unsigned long long Kf = totals[3 * f + 1];
-        if (!E[f]) continue;
-        ctx->scratch.reset();
-        if (rank_positions(ctx, b->d_pairs_all + kbase[f], nullptr, Kf, E[f], ebv[f], b->d_sp)) return -1;
-      }
+    if (!ctx->scratch.reserve(rank_scratch_bytes_fields(Ktot, count, ctx->sm_count) + 8192)) return -1;
+    std::vector<RankField> rf(count);
+    unsigned long long off = 0;
+    for (int f = 0; f < count; f++) {
+      rf[f] = {off, totals[3 * f + 1], E[f], ebase[f], ebv[f]};
+      off += plan[f].interior;
     }
+    if (rank_positions_fields(ctx, b->d_pairs, rf.data(), count, b->d_sp)) return -1;
   }
   tl_mark(ctx, "batch_rank");
   // sort-position streams of the whole batch

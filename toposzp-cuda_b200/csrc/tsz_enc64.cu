@@ -534,6 +534,21 @@ __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, con
   }
 }
 
+// The ninth warp's part of a tile: its place, and the totals after the last one.
+__device__ __forceinline__ void e64_place(const Enc64Args &a, long long tile, E64Sh &sh) {
+  const unsigned tb = sh.tile_bytes, tc = sh.tile_cps, te = sh.tile_ext;
+  const Prefix pf = e64_lookback(a.desc, tile, tb, ((unsigned long long)tc << 32) | te, a.err, a.spin_limit);
+  if ((threadIdx.x & 31) == 0) {
+    sh.gbyte = pf.bytes;
+    sh.gcnt = pf.cnt;
+    if (tile == ((long long)a.n + kE64Tile - 1) / kE64Tile - 1 && a.total) {
+      a.total[0] = pf.bytes + tb;
+      a.total[1] = (pf.cnt >> 32) + tc;
+      a.total[2] = (pf.cnt & 0xffffffffull) + te;
+    }
+  }
+}
+
 // Persistent CTAs claim tiles in order.  Eight warps own the elements and keep
 // two images: they run one tile behind (the front half of tile k, whose
 // aggregate is published in it, then the write-out of tile k-1).  A ninth warp
@@ -580,20 +595,7 @@ __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
         else e64_front<D3, BITS, false>(a, tile, small, part, part + kE64Img, sh[cur]);
       }
     } else {
-      if (prev >= 0) {
-        E64Sh &sp = sh[cur ^ 1];
-        const unsigned tb = sp.tile_bytes, tc = sp.tile_cps, te = sp.tile_ext;
-        const Prefix pf = e64_lookback(a.desc, prev, tb, ((unsigned long long)tc << 32) | te, a.err, a.spin_limit);
-        if (threadIdx.x == kE64Threads) {
-          sp.gbyte = pf.bytes;
-          sp.gcnt = pf.cnt;
-          if (prev == ntiles - 1 && a.total) {
-            a.total[0] = pf.bytes + tb;
-            a.total[1] = (pf.cnt >> 32) + tc;
-            a.total[2] = (pf.cnt & 0xffffffffull) + te;
-          }
-        }
-      }
+      if (prev >= 0) e64_place(a, prev, sh[cur ^ 1]);
     }
     __syncthreads();
     if (owner && prev >= 0) {
@@ -605,6 +607,112 @@ __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
     cur ^= 1;
   }
   if (BITS && owner) rb_extent(a.rb, nmax, cmax);
+}
+
+// The fields of a batch.  The ninth warp maps a claim to its field (the claims
+// of a CTA only move forward) and leaves the field's arguments in shared
+// memory, three tiles' worth: the tile being claimed, the one before it and
+// the one that is still written out.
+__global__ void __launch_bounds__(kE64Cta, 4)
+enc64_batch_kernel(const EncArgs *__restrict__ fields, const unsigned long long *__restrict__ tstart,
+                   const unsigned *__restrict__ nfields_dev, unsigned *queue) {
+  extern __shared__ __align__(16) unsigned char smem_dyn[];
+  __shared__ E64Sh sh[2];
+  __shared__ Enc64Args s_args[3];
+  __shared__ long long s_claim[3];
+  constexpr unsigned kPart = e64_part(false);
+  const int nf = (int)*nfields_dev;
+  const unsigned long long total = tstart[nf];
+  const bool owner = threadIdx.x < kE64Threads;
+  const int lane = threadIdx.x & 31;
+  int field = 0, have[3] = {-1, -1, -1};
+  bool pending = false;
+  unsigned unused0 = 0, unused1 = 0;
+  for (int it = 0, cur = 0, slot = 0;; it++, cur ^= 1) {
+    const int before = slot == 0 ? 2 : slot - 1;
+    if (owner) {
+      e64_claim_wait();
+    } else {
+      unsigned long long t = 0;
+      if (lane == 0) t = atomicAdd(queue, 1u);
+      t = __shfl_sync(0xffffffffu, t, 0);
+      if (t < total) {
+        // the last field that starts at or before t, 32 fields a step from the last claim's
+        while (true) {
+          const int i = field + 1 + lane;
+          const unsigned m = __ballot_sync(0xffffffffu, i < nf && tstart[i < nf ? i : nf] <= t);
+          field += __popc(m);      // starts ascend: the set lanes are the first ones
+          if (m != 0xffffffffu) break;
+        }
+        if (lane == 0) {
+          if (have[slot] != field) {
+            const EncArgs &e = fields[field];
+            Enc64Args &a = s_args[slot];
+            a.data = e.data;
+            a.n = e.n;
+            a.inv = e.inv;
+            a.g = e.g;
+            a.out = e.out;
+            a.out_cap = e.out_cap;
+            a.blk_off = e.blk_off;
+            a.desc = e.desc;
+            a.err = e.err;
+            a.total = e.total;
+            a.cp_out = reinterpret_cast<uint2 *>(e.cp_out);
+            a.cp_cap = e.cp_cap;
+            a.spin_limit = 0;
+            a.base = 0;
+          }
+          s_claim[slot] = (long long)(t - tstart[field]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          if (k == slot) have[k] = field;
+      } else if (lane == 0) {
+        s_claim[slot] = -1;
+      }
+      __syncwarp();
+      e64_claim_post();
+    }
+    const long long tile = s_claim[slot];
+    if (owner) {
+      if (tile >= 0) {
+        const Enc64Args &a = s_args[slot];
+        const bool small = a.g.d1 * a.g.plane < (1ll << 32), full = tile < (long long)(a.n / kE64Tile);
+        unsigned char *part = smem_dyn + (size_t)cur * kPart;
+        if (a.g.nd == 3) {
+          if (full) e64_front<true, false, true>(a, tile, small, part, part + kE64Img, sh[cur]);
+          else e64_front<true, false, false>(a, tile, small, part, part + kE64Img, sh[cur]);
+        } else {
+          if (full) e64_front<false, false, true>(a, tile, small, part, part + kE64Img, sh[cur]);
+          else e64_front<false, false, false>(a, tile, small, part, part + kE64Img, sh[cur]);
+        }
+      }
+    } else if (pending) {
+      e64_place(s_args[before], s_claim[before], sh[cur ^ 1]);
+    }
+    __syncthreads();
+    if (owner && pending) {
+      const unsigned char *pp = smem_dyn + (size_t)(cur ^ 1) * kPart;
+      e64_back<false>(s_args[before], s_claim[before], pp, pp + kE64Img, sh[cur ^ 1], unused0, unused1);
+    }
+    if (tile < 0) break;
+    pending = true;
+    slot = slot == 2 ? 0 : slot + 1;
+  }
+}
+
+cudaError_t enc64_batch_prepare(int *per_sm) {
+  const int smem = 2 * (int)e64_part(false);
+  cudaError_t e = cudaFuncSetAttribute(enc64_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, enc64_batch_kernel, kE64Cta, smem);
+  return e;
+}
+
+cudaError_t launch_enc64_batch(const EncArgs *fields, const unsigned long long *tstart, const unsigned *nfields_dev,
+                               unsigned *queue, cudaStream_t s, int grid) {
+  enc64_batch_kernel<<<grid, kE64Cta, 2 * e64_part(false), s>>>(fields, tstart, nfields_dev, queue);
+  return cudaGetLastError();
 }
 
 unsigned long long enc64_tiles(unsigned long long n) { return (n + kE64Tile - 1) / kE64Tile; }

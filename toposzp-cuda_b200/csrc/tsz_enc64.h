@@ -4,6 +4,8 @@
 
 namespace tsz {
 
+constexpr int kEnc64TileBlocks = 32;   // codec blocks per tile
+
 struct Enc64Args {
   const float *data;            // the field, 16-byte aligned
   unsigned long long n;
@@ -34,6 +36,12 @@ bool enc64_applies(const EncArgs &a, int mode);
 // Launches it over the tiles of a (persistent grid sized by occupancy).
 cudaError_t launch_enc64_from(const EncArgs &a, cudaStream_t s, int sm_count);
 cudaError_t launch_enc64_args(const Enc64Args &a, cudaStream_t s, int sm_count);
+// The same over the fields of a batch (blockSize 64, 16-byte aligned fields,
+// pairs): tiles of all fields in one queue (tstart[f]: first tile of field f,
+// tstart[*nfields] their number), claimed in order.
+cudaError_t launch_enc64_batch(const EncArgs *fields, const unsigned long long *tstart, const unsigned *nfields_dev,
+                               unsigned *queue, cudaStream_t s, int grid);
+cudaError_t enc64_batch_prepare(int *per_sm);   // its shared-memory limit and CTAs per SM
 unsigned long long enc64_tiles(unsigned long long n);
 
 // Bounded-wait checks (tests): a look-back whose predecessor never

@@ -73,11 +73,22 @@ int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig,
 
 size_t rank_scratch_bytes(unsigned long long K, int sm_count);
 
-// Ranks of F segments in one pass (h_seg_K: records per segment, host);
-// bins disjoint across segments.
-int rank_positions_seg(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
-                       const unsigned long long *h_seg_K, int F, int *d_sp);
-size_t rank_scratch_bytes_seg(unsigned long long K, int F, int sm_count);
+// Ranks of the F fields of a batch in one pass.  A field's pairs start at
+// pairs_off, their extremum indices are its own, its E positions go to
+// d_sp[ebase ...].
+struct RankField {
+  unsigned long long pairs_off, K, E, ebase;
+  float eb;
+};
+int rank_positions_fields(szp_b200_ctx *ctx, const uint2 *d_pairs, const RankField *h_fields, int F, int *d_sp);
+size_t rank_scratch_bytes_fields(unsigned long long K, int F, int sm_count);
+// the fields among them of up to kRankSmall pairs
+struct SmallField {
+  unsigned long long pairs_off, ebase;
+  unsigned K;
+  float eb;
+};
+int rank_small_fields(szp_b200_ctx *ctx, const uint2 *d_pairs, const SmallField *d_fields, unsigned count, int *d_sp);
 size_t post_scratch_bytes(unsigned long long n);
 int compact_extrema(szp_b200_ctx *ctx, const int *d_cps, int stride, unsigned long long K, int *d_sp,
                     unsigned long long *E_out);

@@ -433,9 +433,18 @@ int rank_bits_from_pairs(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long 
 constexpr int kSmallThreads = 1024;
 static_assert(kRankSmall == 2 * kSmallThreads, "two items per thread");
 
+// with fields: CTA f takes fields[f] of a batch
 __global__ void __launch_bounds__(kSmallThreads)
 rank_small_kernel(const uint2 *__restrict__ pairs, unsigned K, float eb, double inv, int *__restrict__ out,
-                  RankBits rb) {
+                  RankBits rb, const SmallField *__restrict__ fields) {
+  if (fields) {
+    const SmallField f = fields[blockIdx.x];
+    pairs += f.pairs_off;
+    K = f.K;
+    eb = f.eb;
+    inv = 1.0 / (double)eb;
+    out += f.ebase;
+  }
   __shared__ unsigned long long key[kRankSmall];
   __shared__ unsigned s_w[kSmallThreads / 32];
   unsigned P = 64;
@@ -508,8 +517,14 @@ rank_small_kernel(const uint2 *__restrict__ pairs, unsigned K, float eb, double 
 int rank_small(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long long K, float eb, int *d_sp,
                const RankBits *rb) {
   rank_small_kernel<<<1, kSmallThreads, 0, ctx->stream>>>(d_pairs, (unsigned)K, eb, 1.0 / (double)eb, d_sp,
-                                                          rb ? *rb : RankBits{});
+                                                          rb ? *rb : RankBits{}, nullptr);
   if (rb) ctx->rank_bits_dirty = false;
+  ctx->launches += 1;
+  return cuda_fail(cudaGetLastError(), "rank kernel") ? -1 : 0;
+}
+
+int rank_small_fields(szp_b200_ctx *ctx, const uint2 *d_pairs, const SmallField *d_fields, unsigned count, int *d_sp) {
+  rank_small_kernel<<<count, kSmallThreads, 0, ctx->stream>>>(d_pairs, 0, 1.0f, 1.0, d_sp, RankBits{}, d_fields);
   ctx->launches += 1;
   return cuda_fail(cudaGetLastError(), "rank kernel") ? -1 : 0;
 }

@@ -11,8 +11,12 @@
 //      every point sets the bit of its value code, and the dense rank is the
 //      popcount of the bits below its own code;
 //   3. buckets whose slots do not fit (bins spanning huge code ranges, e.g.
-//      values next to zero, or too many bins) fall back to a device-wide LSD
-//      radix sort on (bin, code) followed by a segmented distinct count.
+//      values next to zero, or too many bins) are sorted by one CTA each, and
+//      only larger ones fall back to a device-wide LSD radix sort on (bin,
+//      code) followed by a segmented distinct count.
+// One field's ranks take this way only where the bitmap over its values does
+// not apply (tsz_rankbits.cuh); a batch's fields take it together, each with
+// buckets of its own.
 #include <algorithm>
 #include <vector>
 
@@ -30,6 +34,13 @@ constexpr int kBitmapWords = 5120;   // 20 KB bitmap + 20 KB prefix per CTA
 // index}).  Its bin is recomputed from the code, or, when the caller supplies
 // bins (batches, whose bins carry per-field offsets, or a given CP list), read
 // from a bin array permuted together with the records.
+// What a batch's field brings to its buckets.
+struct SegField {
+  unsigned long long ebase;   // where its extrema's positions start
+  float eb;
+  int logNB;
+};
+
 struct BinSrc {
   const int *bins;   // bins in record order, or nullptr
   float eb;
@@ -40,10 +51,20 @@ struct BinSrc {
 };
 
 // A chunk of records that belongs to one segment (one field of a batch):
-// records [k0, k1) use buckets bbase .. bbase + NB - 1.
+// records [k0, k1) use buckets bbase .. bbase + NB - 1 and the histogram row
+// at moff.
 struct SegChunk {
   unsigned long long k0, k1;
-  unsigned long long bbase;
+  unsigned long long bbase, moff;
+  float eb;
+  int logNB;
+};
+
+// first bucket of every field and its histogram rows (matrix offset, rows)
+struct SegRows {
+  unsigned long long bbase, moff;
+  unsigned rows;
+  int logNB;
 };
 
 // exclusive scan of one value per thread over a CTA of T threads; the total
@@ -80,6 +101,10 @@ __global__ void __launch_bounds__(kHistThreads)
 bucket_hist_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, unsigned long long K, int logNB,
                    unsigned long long chunk, unsigned *__restrict__ M, const SegChunk *__restrict__ seg = nullptr) {
   extern __shared__ unsigned sh[];
+  if (seg) {
+    logNB = seg[blockIdx.x].logNB;
+    bin_of = {nullptr, seg[blockIdx.x].eb, 1.0 / (double)seg[blockIdx.x].eb};
+  }
   const int NB = 1 << logNB;
   for (int b = threadIdx.x; b < NB; b += blockDim.x) sh[b] = 0;
   __syncthreads();
@@ -99,7 +124,8 @@ bucket_hist_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, unsigned long
     }
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < NB; b += blockDim.x) M[(size_t)blockIdx.x * NB + b] = sh[b];
+  M += seg ? seg[blockIdx.x].moff : (unsigned long long)blockIdx.x * NB;
+  for (int b = threadIdx.x; b < NB; b += blockDim.x) M[b] = sh[b];
 }
 
 // ---- 1b. column scan: M[g][b] <- exclusive prefix over g; tot[b] ----------
@@ -128,36 +154,37 @@ __global__ void bucket_colscan_kernel(unsigned *__restrict__ M, int G, int NB, u
   tot[b] = colscan_rows(M, 0, (unsigned)G, NB, b);
 }
 
-// segmented column scan: bucket b of segment f scans the rows (chunks)
-// crow[f] .. crow[f+1]-1; its totals go to tot[f * NB + b]
-__global__ void bucket_colscan_seg_kernel(unsigned *__restrict__ M, const unsigned *__restrict__ crow, int F,
-                                          int NB, unsigned *__restrict__ tot) {
-  const long long gb = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gb >= (long long)F * NB) return;
-  const int f = (int)(gb / NB), b = (int)(gb % NB);
-  tot[gb] = colscan_rows(M, crow[f], crow[f + 1], NB, b);
+// segmented column scan: thread b of CTA f scans bucket b over the rows of
+// field f; also the field of every bucket
+__global__ void bucket_colscan_seg_kernel(unsigned *__restrict__ M, const SegRows *__restrict__ rows,
+                                          unsigned *__restrict__ tot, unsigned *__restrict__ bfield) {
+  const SegRows r = rows[blockIdx.x];
+  const int b = threadIdx.x, NB = 1 << r.logNB;
+  if (r.rows == 0 || b >= NB) return;
+  tot[r.bbase + b] = colscan_rows(M + r.moff, 0, r.rows, NB, b);
+  bfield[r.bbase + b] = blockIdx.x;
 }
 
-// ---- 1c. exclusive scan of bucket totals (one CTA) -------------------------
-__global__ void bucket_start_kernel(const unsigned *__restrict__ tot, int NB,
-                                    unsigned long long *__restrict__ start) {
-  __shared__ unsigned long long part[1024];
-  const int per = (NB + blockDim.x - 1) / blockDim.x;
-  const int b0 = threadIdx.x * per;
-  unsigned long long s = 0;
-  for (int i = 0; i < per; i++) if (b0 + i < NB) s += tot[b0 + i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 1; o < (int)blockDim.x; o <<= 1) {
-    unsigned long long v = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
+// ---- 1c. exclusive scan of bucket totals (one CTA, four totals a thread) ---
+__global__ void __launch_bounds__(1024)
+bucket_start_kernel(const unsigned *__restrict__ tot, int NB, unsigned long long *__restrict__ start) {
+  __shared__ unsigned s_w[32];
+  unsigned long long base = 0;
+  for (int b0 = 0; b0 < NB; b0 += 4096) {
+    const int b = b0 + 4 * (int)threadIdx.x;
+    unsigned v[4], total;
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = b + u < NB ? tot[b + u] : 0u;
+    // a sweep's records are fewer than 2^32 (a batch holds fewer)
+    unsigned run = block_excl_scan<1024>(v[0] + v[1] + v[2] + v[3], s_w, &total);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (b + u < NB) start[b + u] = base + run;
+      run += v[u];
+    }
+    base += total;
   }
-  unsigned long long run = part[threadIdx.x] - s;
-  for (int i = 0; i < per; i++)
-    if (b0 + i < NB) { start[b0 + i] = run; run += tot[b0 + i]; }
-  if (threadIdx.x == blockDim.x - 1) start[NB] = part[threadIdx.x];
+  if (threadIdx.x == 0) start[NB] = base;
 }
 
 // ---- 1d. scatter into buckets, coalesced ---------------------------------
@@ -180,7 +207,12 @@ bucket_scatter_sorted_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, uns
                              const unsigned long long *__restrict__ start_all, uint2 *__restrict__ recs,
                              int *__restrict__ rbins, const SegChunk *__restrict__ seg = nullptr) {
   extern __shared__ unsigned long long smx[];
+  if (seg) {
+    logNB = seg[blockIdx.x].logNB;
+    bin_of = {nullptr, seg[blockIdx.x].eb, 1.0 / (double)seg[blockIdx.x].eb};
+  }
   const int NB = 1 << logNB;
+  M += seg ? seg[blockIdx.x].moff : (unsigned long long)blockIdx.x * NB;
   unsigned long long *base = smx;                              // next global position per bucket
   unsigned *hist = reinterpret_cast<unsigned *>(base + NB);    // per sub-chunk counts
   unsigned *off = hist + NB;                                   // per sub-chunk exclusive offsets
@@ -191,7 +223,7 @@ bucket_scatter_sorted_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, uns
   const unsigned long long c1 = seg ? seg[blockIdx.x].k1 : ((c0 + chunk < K) ? c0 + chunk : K);
   const unsigned long long *start = start_all + (seg ? seg[blockIdx.x].bbase : 0ull);
   for (int b = threadIdx.x; b < NB; b += blockDim.x) {
-    base[b] = start[b] + M[(size_t)blockIdx.x * NB + b];
+    base[b] = start[b] + M[b];
     hist[b] = 0;
   }
   uint2 pr[kScatterPer];
@@ -269,7 +301,8 @@ constexpr int kRankUnroll = 4;
 __global__ void __launch_bounds__(kRankThreads)
 bucket_rank_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const unsigned long long *__restrict__ start,
                    int logNB, int *__restrict__ out, unsigned *__restrict__ fb_list,
-                   unsigned *__restrict__ fb_count) {
+                   unsigned *__restrict__ fb_count, const unsigned *__restrict__ bfield,
+                   const SegField *__restrict__ fields) {
   __shared__ unsigned s_min[kMaxSlots], s_max[kMaxSlots], s_wbase[kMaxSlots + 1];
   __shared__ unsigned bm[kBitmapWords];
   __shared__ unsigned pref[kBitmapWords];
@@ -278,6 +311,12 @@ bucket_rank_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const unsigned
   const unsigned b = blockIdx.x;
   const unsigned long long r0 = start[b], r1 = start[b + 1];
   if (r1 == r0) return;
+  if (fields) {
+    const SegField f = fields[bfield[b]];
+    logNB = f.logNB;
+    out += f.ebase;
+    bin_of = {nullptr, f.eb, 1.0 / (double)f.eb};
+  }
   const unsigned long long cnt = r1 - r0;
   constexpr unsigned long long kStep = (unsigned long long)kRankUnroll * kRankThreads;
   // bins of this bucket are b + k * NB; slot = k mod kMaxSlots is one-to-one
@@ -457,6 +496,143 @@ bucket_sort_rank_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const uns
 
 static size_t sort_rank_smem() { return (size_t)kSortCap * 12; }
 
+// The same for buckets whose bins follow from the codes, up to 1024 PER
+// records: keys are (code, extremum index), PER in a thread's registers.
+// Exchanges within 32 PER keys are registers and shuffles; of the 105 steps of
+// 16384 keys 15 go through shared memory.  Buckets a kernel does not take go
+// on to the next: PER 2 (most of them, two CTAs per SM), 4 and 16.  256 mixed
+// fields: the barrier-per-step sort of (bin, code, index) in 96 KB took 674 us
+// over 131072 CTAs, 16 keys a thread for every bucket 1839.
+__device__ __forceinline__ void key_exchange(unsigned long long &a, unsigned long long &b, bool up) {
+  if ((a > b) == up) {
+    const unsigned long long t = a;
+    a = b;
+    b = t;
+  }
+}
+
+// one step of the bitonic sort among a thread's own keys
+template <int J, int PER>
+__device__ __forceinline__ void key_step_own(unsigned long long (&v)[PER], unsigned k, unsigned e0) {
+#pragma unroll
+  for (int u = 0; u < PER; u++)
+    if (!(u & J) && (u | J) < PER) key_exchange(v[u], v[u | J], ((e0 + u) & k) == 0);
+}
+
+template <int PER>
+__global__ void __launch_bounds__(kSortThreads)
+bucket_sort_codes_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const unsigned long long *__restrict__ start,
+                         const unsigned *__restrict__ fb_list, const unsigned *__restrict__ fb_count,
+                         int *__restrict__ out_all, unsigned *__restrict__ fb2_list, unsigned *__restrict__ fb2_count,
+                         const unsigned *__restrict__ bfield, const SegField *__restrict__ fields) {
+  extern __shared__ unsigned long long sk[];
+  __shared__ unsigned s_w[kSortThreads / 32];
+  const unsigned t = threadIdx.x, e0 = PER * t;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned nfb = *fb_count;
+  for (unsigned i = blockIdx.x; i < nfb; i += gridDim.x) {
+    const unsigned bk = fb_list[i];
+    const unsigned long long r0 = start[bk], cnt64 = start[bk + 1] - r0;
+    if (cnt64 > (unsigned long long)(PER * kSortThreads)) {
+      if (t == 0) fb2_list[atomicAdd(fb2_count, 1u)] = bk;
+      continue;
+    }
+    const unsigned cnt = (unsigned)cnt64;
+    int *out = out_all;
+    if (fields) {
+      const SegField f = fields[bfield[bk]];
+      out += f.ebase;
+      bin_of = {nullptr, f.eb, 1.0 / (double)f.eb};
+    }
+    unsigned P = PER;
+    while (P < cnt) P <<= 1;
+    unsigned long long v[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      v[u] = ~0ull;
+      if (e0 + u < cnt) {
+        const uint2 p = recs[r0 + e0 + u];
+        v[u] = ((unsigned long long)p.x << 32) | p.y;
+      }
+    }
+    for (unsigned k = 2; k <= P; k <<= 1) {
+      for (unsigned j = k >> 1; j >= 32u * PER; j >>= 1) {
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < PER; u++) sk[u * kSortThreads + t] = v[u];
+        __syncthreads();
+        const unsigned o = t ^ (j / PER);
+        const bool keep_min = ((e0 & j) == 0) == ((e0 & k) == 0);
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+          const unsigned long long x = sk[u * kSortThreads + o];
+          v[u] = (v[u] < x) == keep_min ? v[u] : x;
+        }
+      }
+      for (unsigned j = min(k >> 1, 16u * PER); j >= PER; j >>= 1) {
+        const bool keep_min = ((e0 & j) == 0) == ((e0 & k) == 0);
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+          const unsigned long long x = __shfl_xor_sync(0xffffffffu, v[u], j / PER);
+          v[u] = (v[u] < x) == keep_min ? v[u] : x;
+        }
+      }
+      if (PER > 8 && k > 8) key_step_own<8, PER>(v, k, e0);
+      if (PER > 4 && k > 4) key_step_own<4, PER>(v, k, e0);
+      if (PER > 2 && k > 2) key_step_own<2, PER>(v, k, e0);
+      key_step_own<1, PER>(v, k, e0);
+    }
+    // D: distinct codes up to a key; H: the D of its bin's first key; its position is D - H
+    __syncthreads();
+    sk[t] = v[PER - 1];
+    __syncthreads();
+    const bool any = e0 < cnt;
+    unsigned prev = t ? (unsigned)(sk[t - 1] >> 32) : 0u;
+    unsigned d = 0, first_of_bin = 0;
+    unsigned nc = 0, nb = 0;                        // bit u: key u has a new code, a new bin
+    int pbin = any && t ? bin_of({prev, 0u}, 0) : 0;
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      if (e0 + u < cnt) {
+        const unsigned c = (unsigned)(v[u] >> 32);
+        const int bin = bin_of({c, 0u}, 0);
+        if (e0 + u == 0 || c != prev) { nc |= 1u << u; d++; }
+        if (e0 + u == 0 || bin != pbin) nb |= 1u << u;
+        prev = c;
+        pbin = bin;
+      }
+    }
+    unsigned total;
+    unsigned D = block_excl_scan<kSortThreads>(d, s_w, &total);
+    {
+      unsigned run = D;
+#pragma unroll
+      for (int u = 0; u < PER; u++) {
+        run += (nc >> u) & 1u;
+        if ((nb >> u) & 1u) first_of_bin = run;
+      }
+    }
+    unsigned hi = first_of_bin;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned x = __shfl_up_sync(0xffffffffu, hi, o);
+      if (lane >= o) hi = max(hi, x);
+    }
+    if (lane == 31) s_w[warp] = hi;
+    unsigned H = __shfl_up_sync(0xffffffffu, hi, 1);
+    if (lane == 0) H = 0u;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) H = max(H, s_w[w]);
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      D += (nc >> u) & 1u;
+      if ((nb >> u) & 1u) H = D;
+      if (e0 + u < cnt && (unsigned)v[u] != kNoExtremum) out[(unsigned)v[u]] = (int)(D - H);
+    }
+    __syncthreads();
+  }
+}
+
 // ---- 3. fallback: device-wide LSD radix sort on (bin, code) ---------------
 // gather the records of the failed buckets into a contiguous list
 __global__ void fb_gather_count_kernel(const unsigned *__restrict__ fb_list, unsigned nfb,
@@ -471,10 +647,21 @@ __global__ void fb_gather_kernel(const unsigned *__restrict__ fb_list, unsigned 
                                  const unsigned long long *__restrict__ fb_off,
                                  const uint2 *__restrict__ recs, BinSrc bin_of, bool code_keys,
                                  unsigned long long *__restrict__ key,
-                                 unsigned *__restrict__ val) {
+                                 unsigned *__restrict__ val, const unsigned *__restrict__ bfield,
+                                 const SegField *__restrict__ fields) {
   for (unsigned f = blockIdx.x; f < nfb; f += gridDim.x) {
     const unsigned long long r0 = start[fb_list[f]], r1 = start[fb_list[f] + 1];
     const unsigned long long o = fb_off[f];
+    if (fields) {
+      // keys (field, code); the positions of all fields are one array
+      const unsigned fi = bfield[fb_list[f]], eb0 = (unsigned)fields[fi].ebase;
+      for (unsigned long long i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
+        const uint2 r = recs[i];
+        key[o + (i - r0)] = ((unsigned long long)fi << 32) | r.x;
+        val[o + (i - r0)] = r.y == kNoExtremum ? kNoExtremum : r.y + eb0;
+      }
+      continue;
+    }
     for (unsigned long long i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
       const uint2 r = recs[i];
       key[o + (i - r0)] = code_keys ? (unsigned long long)r.x
@@ -545,7 +732,12 @@ __global__ void radix_scatter_kernel(const unsigned long long *__restrict__ key,
 //   rank[i] = D[i] - Dh[i]  (distinct keys of the bin before key i)
 // Keys are (bin, code) pairs, or codes alone when the bins follow from the
 // codes (a bin is a monotone function of the value).
-__device__ __forceinline__ unsigned long long fb_bin(unsigned long long k, bool code_keys, float eb, double inv) {
+__device__ __forceinline__ unsigned long long fb_bin(unsigned long long k, bool code_keys, float eb, double inv,
+                                                     const SegField *__restrict__ fields) {
+  if (fields) {
+    const float e = fields[k >> 32].eb;
+    return (k & 0xffffffff00000000ull) | (unsigned)quant_bin(code_float((unsigned)k), e, 1.0 / (double)e);
+  }
   return code_keys ? (unsigned long long)(unsigned)quant_bin(code_float((unsigned)k), eb, inv) : (k >> 32);
 }
 
@@ -557,10 +749,11 @@ __global__ void fb_distinct_kernel(const unsigned long long *__restrict__ key, u
 
 __global__ void fb_heads_kernel(const unsigned long long *__restrict__ key, unsigned long long n,
                                 const unsigned *__restrict__ D, bool code_keys, float eb, double inv,
-                                unsigned *__restrict__ H) {
+                                const SegField *__restrict__ fields, unsigned *__restrict__ H) {
   const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const bool head = i == 0 || fb_bin(key[i], code_keys, eb, inv) != fb_bin(key[i - 1], code_keys, eb, inv);
+  const bool head = i == 0 || fb_bin(key[i], code_keys, eb, inv, fields) !=
+                                  fb_bin(key[i - 1], code_keys, eb, inv, fields);
   H[i] = head ? D[i] : 0u;
 }
 
@@ -571,13 +764,15 @@ __global__ void fb_out_kernel(const unsigned *__restrict__ val, unsigned long lo
 }
 
 static int rank_fallback(szp_b200_ctx *ctx, const uint2 *recs, BinSrc bin_of, const unsigned long long *start,
-                         const unsigned *fb_list, unsigned nfb, int *d_sp);
+                         const unsigned *fb_list, unsigned nfb, int *d_sp, const unsigned *bfield = nullptr,
+                         const SegField *fields = nullptr, int nfields = 0);
 
 // bucket stages shared by the single-field and segmented drivers, launched
 // after the histogram matrix M and the bucket starts exist
 static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, unsigned long long K, int logNB,
                         unsigned nbk, unsigned C, unsigned long long chunk, const unsigned *M,
-                        const unsigned long long *start, const SegChunk *d_chunks, int *d_sp) {
+                        const unsigned long long *start, const SegChunk *d_chunks, int *d_sp,
+                        const unsigned *bfield = nullptr, const SegField *fields = nullptr, int nfields = 0) {
   cudaStream_t s = ctx->stream;
   Arena &A = ctx->scratch;
   uint2 *recs = A.take<uint2>(K);
@@ -596,10 +791,25 @@ static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, uns
   // past the scatter, bins (when given) are read in record order
   const BinSrc rsrc = {rbins, src.eb, src.inv};
   if (cuda_fail(cudaMemsetAsync(fb_cnt, 0, 16, s), "memset")) return -1;
-  bucket_rank_kernel<<<nbk, kRankThreads, 0, s>>>(recs, rsrc, start, logNB, d_sp, fb_list, fb_cnt);
-  cudaFuncSetAttribute(bucket_sort_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_rank_smem());
-  bucket_sort_rank_kernel<<<nbk, kSortThreads, sort_rank_smem(), s>>>(recs, rsrc, start, fb_list, fb_cnt, d_sp,
-                                                                      fb2_list, fb_cnt + 1);
+  bucket_rank_kernel<<<nbk, kRankThreads, 0, s>>>(recs, rsrc, start, logNB, d_sp, fb_list, fb_cnt, bfield, fields);
+  if (src.bins) {
+    cudaFuncSetAttribute(bucket_sort_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_rank_smem());
+    bucket_sort_rank_kernel<<<nbk, kSortThreads, sort_rank_smem(), s>>>(recs, rsrc, start, fb_list, fb_cnt, d_sp,
+                                                                        fb2_list, fb_cnt + 1);
+  } else {
+    // each takes what fits it from the list before and passes the rest on
+    unsigned *l3 = A.take<unsigned>(nbk), *l4 = A.take<unsigned>(nbk);
+    if (!l3 || !l4) { set_error("scratch arena too small for the rank stage"); return -1; }
+    cudaFuncSetAttribute(bucket_sort_codes_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         16 * kSortThreads * 8);
+    bucket_sort_codes_kernel<2><<<std::min(nbk, 2u * ctx->sm_count), kSortThreads, 2 * kSortThreads * 8, s>>>(
+        recs, rsrc, start, fb_list, fb_cnt, d_sp, l3, fb_cnt + 2, bfield, fields);
+    bucket_sort_codes_kernel<4><<<std::min(nbk, 2u * ctx->sm_count), kSortThreads, 4 * kSortThreads * 8, s>>>(
+        recs, rsrc, start, l3, fb_cnt + 2, d_sp, l4, fb_cnt + 3, bfield, fields);
+    bucket_sort_codes_kernel<16><<<std::min(nbk, (unsigned)ctx->sm_count), kSortThreads, 16 * kSortThreads * 8, s>>>(
+        recs, rsrc, start, l4, fb_cnt + 3, d_sp, fb2_list, fb_cnt + 1, bfield, fields);
+    ctx->launches += 2;
+  }
   ctx->launches += 3;
   if (cuda_fail(cudaGetLastError(), "rank kernels")) return -1;
   unsigned nfb = 0;
@@ -607,7 +817,21 @@ static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, uns
       cuda_fail(cudaStreamSynchronize(s), "rank"))
     return -1;
   if (nfb == 0) return 0;
-  return rank_fallback(ctx, recs, rsrc, start, fb2_list, nfb, d_sp);
+  return rank_fallback(ctx, recs, rsrc, start, fb2_list, nfb, d_sp, bfield, fields, nfields);
+}
+
+// records of a chunk of a batch (two chunks per SM)
+static unsigned long long rank_seg_chunk(unsigned long long K, int sm_count) {
+  return std::max<unsigned long long>(4096, (K + 2 * sm_count - 1) / (2 * sm_count));
+}
+
+// buckets of a list of K records: 2^9 keep each bucket's bins (slots) within
+// the shared bitmap for typical fields while giving the coalesced scatter long
+// runs; fewer where that leaves a bucket below 2048 records
+static int rank_log_buckets(unsigned long long K) {
+  int lg = 6;
+  while (lg < 9 && (K >> lg) > 2048) lg++;
+  return lg;
 }
 
 int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
@@ -620,10 +844,7 @@ int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
   }
   cudaStream_t s = ctx->stream;
   const BinSrc src = {d_bins, eb, 1.0 / (double)eb};
-  // 2^9 buckets keep each bucket's bins (slots) within the shared bitmap for
-  // typical fields while giving the coalesced scatter long runs
-  int logNB = 6;
-  while (logNB < 9 && (K >> logNB) > 2048) logNB++;
+  const int logNB = rank_log_buckets(K);
   const int NB = 1 << logNB;
   int G = ctx->sm_count * 2;
   unsigned long long chunk = (K + G - 1) / G;
@@ -649,7 +870,8 @@ int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
 // alone when the bins follow from the codes -- and a parallel segmented
 // distinct count.
 static int rank_fallback(szp_b200_ctx *ctx, const uint2 *recs, BinSrc bin_of, const unsigned long long *start,
-                         const unsigned *fb_list, unsigned nfb, int *d_sp) {
+                         const unsigned *fb_list, unsigned nfb, int *d_sp, const unsigned *bfield,
+                         const SegField *fields, int nfields) {
   cudaStream_t s = ctx->stream;
   Arena &A = ctx->scratch;
   unsigned long long *fb_len = A.take<unsigned long long>(nfb + 1);
@@ -676,8 +898,10 @@ static int rank_fallback(szp_b200_ctx *ctx, const uint2 *recs, BinSrc bin_of, co
   const bool code_keys = bin_of.bins == nullptr;
   cudaMemcpyAsync(fb_off, h_off.data(), nfb * 8, cudaMemcpyHostToDevice, s);
   fb_gather_kernel<<<std::min(nfb, 4096u), 256, 0, s>>>(fb_list, nfb, start, fb_off, recs, bin_of, code_keys, k1,
-                                                          v1);
-  const int bits = code_keys ? 32 : 64;
+                                                          v1, bfield, fields);
+  int bits = code_keys ? 32 : 64;
+  if (fields)
+    for (bits = 32; (nfields - 1) >> (bits - 32) > 0; bits += 8) {}
   for (int shift = 0; shift < bits; shift += 8) {
     radix_hist_kernel<<<ntiles, 256, 0, s>>>(k1, nf, shift, H, ntiles);
     if (cuda_fail(device_scan_u32<OpAdd>(H, H, hn, part, false, s), "scan")) return -1;
@@ -691,7 +915,7 @@ static int rank_fallback(szp_b200_ctx *ctx, const uint2 *recs, BinSrc bin_of, co
   const unsigned g = (unsigned)((nf + 255) / 256);
   fb_distinct_kernel<<<g, 256, 0, s>>>(k1, nf, D);
   if (cuda_fail(device_scan_u32<OpAdd>(D, D, nf, part, true, s), "scan")) return -1;
-  fb_heads_kernel<<<g, 256, 0, s>>>(k1, nf, D, code_keys, bin_of.eb, bin_of.inv, Dh);
+  fb_heads_kernel<<<g, 256, 0, s>>>(k1, nf, D, code_keys, bin_of.eb, bin_of.inv, fields, Dh);
   if (cuda_fail(device_scan_u32<OpMax>(Dh, Dh, nf, part, true, s), "scan")) return -1;
   fb_out_kernel<<<g, 256, 0, s>>>(v1, nf, D, Dh, d_sp);
   ctx->launches += 3 + (bits / 8) * 5 + 9;
@@ -701,77 +925,105 @@ static int rank_fallback(szp_b200_ctx *ctx, const uint2 *recs, BinSrc bin_of, co
   return 0;
 }
 
-// Ranks of many segments (fields of a batch) in one pass: every segment gets
-// its own NB buckets and chunks never straddle segments, so records of
-// different segments never share a bucket.  bins must be disjoint across
-// segments (the fallback sorts all failing buckets together by bin).
-int rank_positions_seg(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
-                       const unsigned long long *h_seg_K, int F, int *d_sp) {
-  unsigned long long K = 0;
-  for (int f = 0; f < F; f++) K += h_seg_K[f];
-  if (K == 0) return 0;
+// Ranks of the fields of a batch in one pass: fields of up to 2048 points are
+// sorted by one CTA each; every other field gets buckets of its own (as many
+// as its points ask for), chunks never straddle fields, and bins follow from
+// the codes and the field's bound, so nothing but the pairs is read.
+int rank_positions_fields(szp_b200_ctx *ctx, const uint2 *d_pairs, const RankField *h_fields, int F, int *d_sp) {
   cudaStream_t s = ctx->stream;
-  const int logNB = 9, NB = 1 << logNB;
-  unsigned long long chunk = std::max<unsigned long long>(4096, (K + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count));
+  unsigned long long K = 0;
+  for (int f = 0; f < F; f++)
+    if (h_fields[f].K > kRankSmall) K += h_fields[f].K;
+  const unsigned long long chunk = rank_seg_chunk(K, ctx->sm_count);
   std::vector<SegChunk> chunks;
-  std::vector<unsigned> crow(F + 1);
-  unsigned long long k = 0;
+  std::vector<SegRows> rows(F);
+  std::vector<SegField> fields(F);
+  std::vector<unsigned> small;
+  unsigned long long nbk = 0, moff = 0;
+  int lgmax = 6;
   for (int f = 0; f < F; f++) {
-    crow[f] = (unsigned)chunks.size();
-    const unsigned long long k1 = k + h_seg_K[f];
-    for (unsigned long long c = k; c < k1; c += chunk)
-      chunks.push_back({c, std::min(c + chunk, k1), (unsigned long long)f * NB});
-    k = k1;
+    const RankField &r = h_fields[f];
+    const int lg = rank_log_buckets(r.K);
+    fields[f] = {r.ebase, r.eb, lg};
+    rows[f] = {nbk, moff, 0u, lg};
+    if (r.K <= kRankSmall) {
+      if (r.E) small.push_back((unsigned)f);
+      continue;
+    }
+    if (!r.E) continue;
+    lgmax = std::max(lgmax, lg);
+    for (unsigned long long k = 0; k < r.K; k += chunk) {
+      chunks.push_back({r.pairs_off + k, r.pairs_off + std::min(k + chunk, r.K), nbk, moff, r.eb, lg});
+      moff += 1ull << lg;
+      rows[f].rows++;
+    }
+    nbk += 1ull << lg;
   }
-  crow[F] = (unsigned)chunks.size();
   const unsigned C = (unsigned)chunks.size();
-  const unsigned long long nbk = (unsigned long long)F * NB;
   Arena &A = ctx->scratch;
+  SegField *d_fields = A.take<SegField>(F);
+  if (!d_fields) { set_error("scratch arena too small for the batched rank stage"); return -1; }
+  if (cuda_fail(cudaMemcpyAsync(d_fields, fields.data(), F * sizeof(SegField), cudaMemcpyHostToDevice, s),
+                "H2D fields"))
+    return -1;
+  if (!small.empty()) {
+    SmallField *d_small = A.take<SmallField>(small.size());
+    if (!d_small) { set_error("scratch arena too small for the batched rank stage"); return -1; }
+    std::vector<SmallField> hs;
+    for (unsigned f : small)
+      hs.push_back({h_fields[f].pairs_off, h_fields[f].ebase, (unsigned)h_fields[f].K, h_fields[f].eb});
+    if (cuda_fail(cudaMemcpyAsync(d_small, hs.data(), hs.size() * sizeof(SmallField), cudaMemcpyHostToDevice, s),
+                  "H2D fields"))
+      return -1;
+    if (rank_small_fields(ctx, d_pairs, d_small, (unsigned)hs.size(), d_sp)) return -1;
+  }
+  if (C == 0) return 0;
   SegChunk *d_chunks = A.take<SegChunk>(C);
-  unsigned *d_crow = A.take<unsigned>(F + 1);
-  unsigned *M = A.take<unsigned>((size_t)C * NB);
-  unsigned *tot = A.take<unsigned>(nbk);
+  SegRows *d_rows = A.take<SegRows>(F);
+  unsigned *M = A.take<unsigned>(moff);
+  unsigned *tot = A.take<unsigned>(nbk), *bfield = A.take<unsigned>(nbk);
   unsigned long long *start = A.take<unsigned long long>(nbk + 1);
-  if (!d_chunks || !d_crow || !M || !tot || !start) {
+  if (!d_chunks || !d_rows || !M || !tot || !bfield || !start) {
     set_error("scratch arena too small for the batched rank stage");
     return -1;
   }
   if (cuda_fail(cudaMemcpyAsync(d_chunks, chunks.data(), C * sizeof(SegChunk), cudaMemcpyHostToDevice, s),
                 "H2D chunks") ||
-      cuda_fail(cudaMemcpyAsync(d_crow, crow.data(), (F + 1) * sizeof(unsigned), cudaMemcpyHostToDevice, s),
-                "H2D chunk rows"))
+      cuda_fail(cudaMemcpyAsync(d_rows, rows.data(), F * sizeof(SegRows), cudaMemcpyHostToDevice, s), "H2D rows"))
     return -1;
-  const BinSrc src = {d_bins, 1.0f, 1.0};
-  const size_t hsm = (size_t)NB * 4;
-  bucket_hist_kernel<<<C, kHistThreads, hsm, s>>>(d_pairs, src, K, logNB, chunk, M, d_chunks);
-  bucket_colscan_seg_kernel<<<(unsigned)((nbk + 255) / 256), 256, 0, s>>>(M, d_crow, F, NB, tot);
+  const BinSrc src = {nullptr, 1.0f, 1.0};
+  const size_t hsm = (size_t)4 << lgmax;
+  bucket_hist_kernel<<<C, kHistThreads, hsm, s>>>(d_pairs, src, K, lgmax, chunk, M, d_chunks);
+  bucket_colscan_seg_kernel<<<F, 1 << lgmax, 0, s>>>(M, d_rows, tot, bfield);
   bucket_start_kernel<<<1, 1024, 0, s>>>(tot, (int)nbk, start);
   ctx->launches += 3;
-  return rank_buckets(ctx, d_pairs, src, K, logNB, (unsigned)nbk, C, chunk, M, start, d_chunks, d_sp);
+  return rank_buckets(ctx, d_pairs, src, K, lgmax, (unsigned)nbk, C, chunk, M, start, d_chunks, d_sp, bfield, d_fields,
+                      F);
 }
 
-size_t rank_scratch_bytes_seg(unsigned long long K, int F, int sm_count) {
+size_t rank_scratch_bytes_fields(unsigned long long K, int F, int sm_count) {
   const size_t NB = 512;
-  const unsigned long long chunk = std::max<unsigned long long>(4096, (K + 2 * sm_count - 1) / (2 * sm_count));
-  const size_t C = (size_t)(K / chunk) + (size_t)F + 1;
-  const size_t nbk = (size_t)F * NB;
+  const unsigned long long chunk = rank_seg_chunk(K, sm_count);
+  // every field may end in a partial chunk; a field of buckets has over 2048 points
+  const size_t G = std::min<size_t>((size_t)F, (size_t)(K / kRankSmall));
+  const size_t C = (size_t)(K / std::min<unsigned long long>(chunk, 4096)) + G + 1;
+  const size_t nbk = std::max<size_t>(G, 1) * NB;
   const size_t fb = a256(K * 8) * 2 + a256(K * 4) * 2 + a256(256 * ((K + kRadixTile - 1) / kRadixTile) * 4) +
                     a256(scan_parts(256 * ((K + kRadixTile - 1) / kRadixTile) + K) * 4);
-  return a256(C * sizeof(SegChunk)) + a256((F + 1) * 4) + a256(C * NB * 4) + a256(nbk * 4) +
-         a256((nbk + 1) * 8) + a256(K * 8) + a256(K * 4) + a256(nbk * 4) * 2 + a256(16) + fb + a256(nbk * 8) + 8192;
+  return a256(F * sizeof(SegField)) + a256(F * sizeof(SmallField)) + a256(C * sizeof(SegChunk)) +
+         a256(F * sizeof(SegRows)) + a256(C * NB * 4) + a256(nbk * 4) * 2 + a256((nbk + 1) * 8) + a256(K * 8) +
+         a256(nbk * 4) * 4 + a256(16) + fb + a256(nbk * 8) * 2 + 8192;
 }
 
 size_t rank_scratch_bytes(unsigned long long K, int sm_count) {
-  int logNB = 6;
-  while (logNB < 9 && (K >> logNB) > 2048) logNB++;
-  const size_t NB = (size_t)1 << logNB;
+  const size_t NB = (size_t)1 << rank_log_buckets(K);
   const size_t G = (size_t)sm_count * 2 + 1;
   // fallback worst case: all K records (two key/value ping-pong buffers + histogram)
   const size_t fb = a256(K * 8) * 2 + a256(K * 4) * 2 + a256(256 * ((K + kRadixTile - 1) / kRadixTile) * 4) +
                     a256(scan_parts(256 * ((K + kRadixTile - 1) / kRadixTile) + K) * 4);
   // records (8 B) and, for given bins, their permuted bins (4 B); the bitmap ranking's tables
   return (K > (unsigned long long)kRankSmall ? rank_bits_scratch_bytes() : 0) + a256(G * NB * 4) + a256(NB * 4) + a256((NB + 1) * 8) + a256(K * 8) + a256(K * 4) +
-         a256(NB * 4) * 3 + a256(16) + fb + a256((NB + 1) * 8) * 2 + 4096;
+         a256(NB * 4) * 5 + a256(16) + fb + a256((NB + 1) * 8) * 2 + 4096;
 }
 
 // ---------------------------------------------------------------------------
