@@ -302,13 +302,16 @@ __global__ void __launch_bounds__(kRankThreads)
 bucket_rank_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const unsigned long long *__restrict__ start,
                    int logNB, int *__restrict__ out, unsigned *__restrict__ fb_list,
                    unsigned *__restrict__ fb_count, const unsigned *__restrict__ bfield,
-                   const SegField *__restrict__ fields) {
+                   const SegField *__restrict__ fields, const unsigned *__restrict__ list,
+                   const unsigned *__restrict__ list_count) {
   __shared__ unsigned s_min[kMaxSlots], s_max[kMaxSlots], s_wbase[kMaxSlots + 1];
   __shared__ unsigned bm[kBitmapWords];
   __shared__ unsigned pref[kBitmapWords];
   __shared__ unsigned s_w[kRankThreads / 32];
   __shared__ int s_bmin, s_bmax;
-  const unsigned b = blockIdx.x;
+  // the buckets of a list, or all
+  if (list && blockIdx.x >= *list_count) return;
+  const unsigned b = list ? list[blockIdx.x] : blockIdx.x;
   const unsigned long long r0 = start[b], r1 = start[b + 1];
   if (r1 == r0) return;
   if (fields) {
@@ -502,7 +505,8 @@ static size_t sort_rank_smem() { return (size_t)kSortCap * 12; }
 // 16384 keys 15 go through shared memory.  Buckets a kernel does not take go
 // on to the next: PER 2 (most of them, two CTAs per SM), 4 and 16.  256 mixed
 // fields: the barrier-per-step sort of (bin, code, index) in 96 KB took 674 us
-// over 131072 CTAs, 16 keys a thread for every bucket 1839.
+// over 131072 CTAs, 16 keys a thread for every bucket 1839, these three 544,
+// and 194 since buckets of up to 512 records are sorted by warps (2c, 42 us).
 __device__ __forceinline__ void key_exchange(unsigned long long &a, unsigned long long &b, bool up) {
   if ((a > b) == up) {
     const unsigned long long t = a;
@@ -631,6 +635,109 @@ bucket_sort_codes_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const un
     }
     __syncthreads();
   }
+}
+
+// ---- 2c. buckets of up to 512 records: sorted by one warp -----------------
+// No barrier and no shared memory: sixteen keys a lane at most, exchanges in
+// registers and by shuffles (about 3600 instructions for 512 records).  Larger
+// buckets go to big_list.
+template <int PER>
+__device__ __forceinline__ void warp_sort_rank(const uint2 *__restrict__ recs, unsigned cnt, const BinSrc &bin_of,
+                                               int *__restrict__ out) {
+  const unsigned lane = threadIdx.x & 31, e0 = PER * lane;
+  unsigned long long v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const unsigned r = u * 32 + lane;   // any order will do
+    v[u] = ~0ull;
+    if (r < cnt) {
+      const uint2 p = recs[r];
+      v[u] = ((unsigned long long)p.x << 32) | p.y;
+    }
+  }
+#pragma unroll 1
+  for (unsigned k = 2; k <= 32u * PER; k <<= 1) {
+#pragma unroll 1
+    for (unsigned j = k >> 1; j >= PER; j >>= 1) {
+      const bool keep_min = ((e0 & j) == 0) == ((e0 & k) == 0);
+#pragma unroll
+      for (int u = 0; u < PER; u++) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, v[u], j / PER);
+        v[u] = (v[u] < x) == keep_min ? v[u] : x;
+      }
+    }
+    if (PER > 8 && k > 8) key_step_own<8, PER>(v, k, e0);
+    if (PER > 4 && k > 4) key_step_own<4, PER>(v, k, e0);
+    if (PER > 2 && k > 2) key_step_own<2, PER>(v, k, e0);
+    key_step_own<1, PER>(v, k, e0);
+  }
+  // D: distinct codes up to a key; H: the D of its bin's first key; its position is D - H
+  const unsigned left = __shfl_up_sync(0xffffffffu, (unsigned)(v[PER - 1] >> 32), 1);
+  unsigned prev = lane ? left : 0u;
+  int pbin = lane && e0 < cnt ? bin_of({prev, 0u}, 0) : 0;
+  unsigned nc = 0, nb = 0, d = 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    if (e0 + u < cnt) {
+      const unsigned c = (unsigned)(v[u] >> 32);
+      const int bin = bin_of({c, 0u}, 0);
+      if (e0 + u == 0 || c != prev) { nc |= 1u << u; d++; }
+      if (e0 + u == 0 || bin != pbin) nb |= 1u << u;
+      prev = c;
+      pbin = bin;
+    }
+  }
+  unsigned inc = d;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned x = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (unsigned)o) inc += x;
+  }
+  unsigned D = inc - d, run = D, hi = 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    run += (nc >> u) & 1u;
+    if ((nb >> u) & 1u) hi = run;
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned x = __shfl_up_sync(0xffffffffu, hi, o);
+    if (lane >= (unsigned)o) hi = max(hi, x);
+  }
+  unsigned H = __shfl_up_sync(0xffffffffu, hi, 1);
+  if (lane == 0) H = 0u;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    D += (nc >> u) & 1u;
+    if ((nb >> u) & 1u) H = D;
+    if (e0 + u < cnt && (unsigned)v[u] != kNoExtremum) out[(unsigned)v[u]] = (int)(D - H);
+  }
+}
+
+constexpr unsigned kWarpSort = 512;
+constexpr int kWarpSortThreads = 128;
+
+__global__ void __launch_bounds__(kWarpSortThreads)
+bucket_warp_sort_kernel(const uint2 *__restrict__ recs, const unsigned long long *__restrict__ start, unsigned nbk,
+                        int *__restrict__ out, unsigned *__restrict__ big_list, unsigned *__restrict__ big_count,
+                        const unsigned *__restrict__ bfield, const SegField *__restrict__ fields) {
+  const unsigned b = (blockIdx.x * kWarpSortThreads + threadIdx.x) >> 5;
+  if (b >= nbk) return;
+  const unsigned long long r0 = start[b], n64 = start[b + 1] - r0;
+  if (n64 == 0) return;
+  if (n64 > kWarpSort) {
+    if ((threadIdx.x & 31) == 0) big_list[atomicAdd(big_count, 1u)] = b;
+    return;
+  }
+  const SegField f = fields[bfield[b]];
+  const BinSrc bin_of = {nullptr, f.eb, 1.0 / (double)f.eb};
+  const unsigned cnt = (unsigned)n64;
+  recs += r0;
+  out += f.ebase;
+  if (cnt <= 64) warp_sort_rank<2>(recs, cnt, bin_of, out);
+  else if (cnt <= 128) warp_sort_rank<4>(recs, cnt, bin_of, out);
+  else if (cnt <= 256) warp_sort_rank<8>(recs, cnt, bin_of, out);
+  else warp_sort_rank<16>(recs, cnt, bin_of, out);
 }
 
 // ---- 3. fallback: device-wide LSD radix sort on (bin, code) ---------------
@@ -779,7 +886,7 @@ static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, uns
   int *rbins = src.bins ? A.take<int>(K) : nullptr;
   unsigned *fb_list = A.take<unsigned>(nbk);
   unsigned *fb2_list = A.take<unsigned>(nbk);
-  unsigned *fb_cnt = A.take<unsigned>(4);
+  unsigned *fb_cnt = A.take<unsigned>(8);
   if (!recs || (src.bins && !rbins) || !fb_list || !fb2_list || !fb_cnt) {
     set_error("scratch arena too small for the rank stage");
     return -1;
@@ -790,8 +897,21 @@ static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, uns
                                                                rbins, d_chunks);
   // past the scatter, bins (when given) are read in record order
   const BinSrc rsrc = {rbins, src.eb, src.inv};
-  if (cuda_fail(cudaMemsetAsync(fb_cnt, 0, 16, s), "memset")) return -1;
-  bucket_rank_kernel<<<nbk, kRankThreads, 0, s>>>(recs, rsrc, start, logNB, d_sp, fb_list, fb_cnt, bfield, fields);
+  if (cuda_fail(cudaMemsetAsync(fb_cnt, 0, 32, s), "memset")) return -1;
+  unsigned *big = nullptr;
+  unsigned nbig = nbk;
+  if (fields) {
+    // a batch's buckets are mostly small: sorted by warps, the others listed
+    // (at most one in 513 records)
+    big = A.take<unsigned>(nbk);
+    if (!big) { set_error("scratch arena too small for the rank stage"); return -1; }
+    bucket_warp_sort_kernel<<<(nbk * 32 + kWarpSortThreads - 1) / kWarpSortThreads, kWarpSortThreads, 0, s>>>(
+        recs, start, nbk, d_sp, big, fb_cnt + 4, bfield, fields);
+    ctx->launches += 1;
+    nbig = (unsigned)std::min<unsigned long long>(nbk, K / (kWarpSort + 1) + 1);
+  }
+  bucket_rank_kernel<<<nbig, kRankThreads, 0, s>>>(recs, rsrc, start, logNB, d_sp, fb_list, fb_cnt, bfield, fields,
+                                                   big, fb_cnt + 4);
   if (src.bins) {
     cudaFuncSetAttribute(bucket_sort_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_rank_smem());
     bucket_sort_rank_kernel<<<nbk, kSortThreads, sort_rank_smem(), s>>>(recs, rsrc, start, fb_list, fb_cnt, d_sp,
@@ -828,9 +948,9 @@ static unsigned long long rank_seg_chunk(unsigned long long K, int sm_count) {
 // buckets of a list of K records: 2^9 keep each bucket's bins (slots) within
 // the shared bitmap for typical fields while giving the coalesced scatter long
 // runs; fewer where that leaves a bucket below 2048 records
-static int rank_log_buckets(unsigned long long K) {
+static int rank_log_buckets(unsigned long long K, unsigned most = 2048) {
   int lg = 6;
-  while (lg < 9 && (K >> lg) > 2048) lg++;
+  while (lg < 9 && (K >> lg) > most) lg++;
   return lg;
 }
 
@@ -943,7 +1063,7 @@ int rank_positions_fields(szp_b200_ctx *ctx, const uint2 *d_pairs, const RankFie
   int lgmax = 6;
   for (int f = 0; f < F; f++) {
     const RankField &r = h_fields[f];
-    const int lg = rank_log_buckets(r.K);
+    const int lg = rank_log_buckets(r.K, 256);   // buckets that a warp sorts, up to 131072 points
     fields[f] = {r.ebase, r.eb, lg};
     rows[f] = {nbk, moff, 0u, lg};
     if (r.K <= kRankSmall) {
@@ -1012,7 +1132,7 @@ size_t rank_scratch_bytes_fields(unsigned long long K, int F, int sm_count) {
                     a256(scan_parts(256 * ((K + kRadixTile - 1) / kRadixTile) + K) * 4);
   return a256(F * sizeof(SegField)) + a256(F * sizeof(SmallField)) + a256(C * sizeof(SegChunk)) +
          a256(F * sizeof(SegRows)) + a256(C * NB * 4) + a256(nbk * 4) * 2 + a256((nbk + 1) * 8) + a256(K * 8) +
-         a256(nbk * 4) * 4 + a256(16) + fb + a256(nbk * 8) * 2 + 8192;
+         a256(nbk * 4) * 5 + a256(32) + fb + a256(nbk * 8) * 2 + 8192;
 }
 
 size_t rank_scratch_bytes(unsigned long long K, int sm_count) {
@@ -1023,7 +1143,7 @@ size_t rank_scratch_bytes(unsigned long long K, int sm_count) {
                     a256(scan_parts(256 * ((K + kRadixTile - 1) / kRadixTile) + K) * 4);
   // records (8 B) and, for given bins, their permuted bins (4 B); the bitmap ranking's tables
   return (K > (unsigned long long)kRankSmall ? rank_bits_scratch_bytes() : 0) + a256(G * NB * 4) + a256(NB * 4) + a256((NB + 1) * 8) + a256(K * 8) + a256(K * 4) +
-         a256(NB * 4) * 5 + a256(16) + fb + a256((NB + 1) * 8) * 2 + 4096;
+         a256(NB * 4) * 5 + a256(32) + fb + a256((NB + 1) * 8) * 2 + 4096;
 }
 
 // ---------------------------------------------------------------------------

@@ -161,6 +161,14 @@ class BatchField(C.Structure):
                 ("sort_cap", C.c_size_t), ("sizes", Sizes), ("abs_eb", C.c_float)]
 
 
+# BatchField as a numpy record
+BATCH_DT = np.dtype([("d_data", "<u8"), ("geom", [("nd", "<i4"), ("dims", "<i4", (3,))]), ("errBound", "<f4"),
+                     ("rel", "<i4"), ("d_topo", "<u8"), ("topo_cap", "<u8"), ("d_sort", "<u8"), ("sort_cap", "<u8"),
+                     ("sizes", [("topo", "<u8"), ("sort", "<u8"), ("cps", "<u8"), ("extrema", "<u8")]),
+                     ("abs_eb", "<f4")], align=True)
+assert BATCH_DT.itemsize == C.sizeof(BatchField)
+
+
 def build() -> str:
     """Compile the library in place (nvcc, sm_100a)."""
     subprocess.run(["make", "-s", "-C", HERE, "-j8"], check=True)
@@ -688,19 +696,17 @@ class Batch:
         [(topo, sort, Sizes, abs_eb)] with topo / sort the device buffers."""
         if bufs is None:
             bufs = self.buffers(items)
-        arr = (BatchField * len(items))()
-        for k, ((t, shape, err, rel), (tb, sb)) in enumerate(zip(items, bufs)):
-            arr[k].d_data = t.data_ptr()
-            arr[k].geom = geom_of(shape)
-            arr[k].errBound = err
-            arr[k].rel = int(bool(rel))
-            arr[k].d_topo = tb.data_ptr()
-            arr[k].topo_cap = tb.numel()
-            arr[k].d_sort = sb.data_ptr()
-            arr[k].sort_cap = sb.numel()
-        if lib().szp_b200_batch_compress(self.ptr, arr, len(items)):
+        if len(bufs) < len(items):
+            raise ToposzpError("batch: %d buffer pairs for %d fields" % (len(bufs), len(items)))
+        bufs = bufs[:len(items)]
+        # one structured array: filling the ctypes structures field by field
+        # took longer than the ranks of 256 fields
+        arr = np.array([(t.data_ptr(), (len(shape), tuple(shape) + (0,) * (3 - len(shape))), err, bool(rel),
+                         tb.data_ptr(), tb.numel(), sb.data_ptr(), sb.numel(), (0, 0, 0, 0), 0.0)
+                        for (t, shape, err, rel), (tb, sb) in zip(items, bufs)], dtype=BATCH_DT)
+        if lib().szp_b200_batch_compress(self.ptr, arr.ctypes.data_as(C.POINTER(BatchField)), len(items)):
             raise ToposzpError(last_error())
-        return [(tb, sb, arr[k].sizes, float(arr[k].abs_eb)) for k, (tb, sb) in enumerate(bufs)]
+        return [(tb, sb, Sizes(*z), e) for (tb, sb), z, e in zip(bufs, arr["sizes"].tolist(), arr["abs_eb"].tolist())]
 
     def tuning(self):
         shape = (C.c_int * 4)()
