@@ -645,6 +645,7 @@ static cudaError_t launch_dec2_tags(DecArgs a, cudaStream_t s) {
 }
 
 cudaError_t launch_decode(bool tags, DecArgs a, cudaStream_t s) {
+  if (a.B == 64) return launch_decode64(tags, a, s);
   if (a.B <= 256) return tags ? launch_dec2_tags<true>(a, s) : launch_dec2_tags<false>(a, s);
   // the generic decoder stages the payload in 4-byte words: the stream must
   // start on a 4-byte boundary (the octet decoder takes any alignment)

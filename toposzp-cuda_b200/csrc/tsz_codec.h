@@ -71,5 +71,6 @@ size_t enc_smem_bytes(int B, bool tags);
 size_t dec_smem_bytes(int B, bool tags);
 cudaError_t launch_encode(int mode, const EncArgs &a, cudaStream_t s, int grid);
 cudaError_t launch_decode(bool tags, DecArgs a, cudaStream_t s);
+cudaError_t launch_decode64(bool tags, const DecArgs &a, cudaStream_t s);   // blockSize 64
 
 }  // namespace tsz
