@@ -845,7 +845,12 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
   if (!ctx->scratch.reserve(need)) return -1;
   Arena &A = ctx->scratch;
   int *sp = post ? A.take<int>(n) : nullptr;
-  unsigned char *T = d_types ? d_types : A.take<unsigned char>(n);
+  // types: the bytes the caller asked for; for post-processing bit planes,
+  // which the blockSize-64 decoder writes and others make of the bytes
+  const bool planes = post && B == 64;
+  unsigned char *T = d_types || planes ? d_types : A.take<unsigned char>(n);
+  unsigned *TL = nullptr, *TH = nullptr;
+  if (post && !post_planes(ctx, n, &TL, &TH)) { set_error("scratch arena too small for post-processing"); return -1; }
   unsigned long long *idx = parse ? A.take<unsigned long long>(2 * nb)
                                   : reinterpret_cast<unsigned long long *>(const_cast<uint64_t *>(d_blk_index));
   cudaStream_t s = ctx->stream;
@@ -866,6 +871,10 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
   a.eb = absErrBound;
   a.out_f = d_out;
   a.fn_u8 = T;
+  if (planes) {
+    a.pl_lo = reinterpret_cast<unsigned char *>(TL);
+    a.pl_hi = reinterpret_cast<unsigned char *>(TH);
+  }
   a.err = reinterpret_cast<int *>(w + 4);
   a.ext_count = w + 6;
   a.cpu_layout = cpu_layout ? 1 : 0;
@@ -921,9 +930,8 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
   TileDesc *desc = A.take<TileDesc>(ntiles + 1);
   if (!S || !desc) { set_error("scratch arena too small for post-processing"); return -1; }
   int restored = 0;
-  // d_out holds the raw decoded field: the list build gathers the raw values
-  // of the candidates from it before any pass updates it in place
-  return postprocess_with(ctx, d_out, d_out, T, S, desc, spp, spp ? E : 0, g, absErrBound,
+  if (!planes && post_planes_from_bytes(ctx, T, n, TL, TH)) return -1;
+  return postprocess_with(ctx, d_out, d_out, TL, TH, S, desc, spp, spp ? E : 0, g, absErrBound,
                           postprocess == 2, &restored);
 }
 
@@ -953,7 +961,7 @@ int szp_b200_topo_postprocess_dev(szp_b200_ctx *ctx, float *d_data, const float 
   if (!geom_ok(geom, &n, &g)) { set_error("invalid geometry"); return -1; }
   if (!ctx->scratch.reserve(post_scratch_bytes(n) + 8192)) return -1;
   int restored = 0;
-  return postprocess(ctx, d_data, d_orig, nullptr, d_types, d_sp, d_sp ? n_sp : 0, g, absErrBound,
+  return postprocess(ctx, d_data, d_orig, d_types, d_sp, d_sp ? n_sp : 0, g, absErrBound,
                      axis_stencil, &restored);
 }
 

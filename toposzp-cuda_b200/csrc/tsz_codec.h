@@ -50,6 +50,7 @@ struct DecArgs {
   int *out_i;                   // decoded ints (sort-position stream)
   int *fn_i;                    // 2-bit tags as int (optional)
   unsigned char *fn_u8;         // 2-bit tags as bytes (optional)
+  unsigned char *pl_lo, *pl_hi; // bit planes of the tags, bit i % 8 of byte i / 8 (blockSize 64; optional)
   int *err;
   unsigned long long *ext_count;  // optional: number of type-1/2 tags
   unsigned long long img_cap;   // set by the launcher

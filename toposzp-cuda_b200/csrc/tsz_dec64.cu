@@ -183,6 +183,15 @@ __global__ void __launch_bounds__(kD64Threads, 6) decode64_kernel(DecArgs a) {
                     (2u * l + 1u < tb ? (unsigned)img[tsec + 2 * l + 1] : 0u);
       if (nv < 8) tg &= 0xffffu << (16 - 2 * nv);
       n_ext = (unsigned)__popc((tg ^ (tg >> 1)) & 0x5555u);   // types 01 and 10
+      if (a.pl_lo) {
+        // element t to bit t: the compacted fields, element 0 on top, reversed
+        const long long o = i0 >> 3;
+        a.pl_lo[o] = (unsigned char)(__brev(compact2(tg)) >> 24);
+        a.pl_hi[o] = (unsigned char)(__brev(compact2(tg >> 1)) >> 24);
+        // the rest of the planes' last word
+        if (i0 + 8 >= n)
+          for (long long k = o + 1; k & 3; k++) a.pl_lo[k] = a.pl_hi[k] = 0;
+      }
       if (a.fn_u8) {
         if (nv == 8 && ((reinterpret_cast<uintptr_t>(a.fn_u8 + i0) & 7) == 0)) {
           // four two-bit fields of a byte, most significant first, to four bytes

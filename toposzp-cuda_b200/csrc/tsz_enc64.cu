@@ -172,8 +172,17 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
         inter = row_in ? (z0 ? 0xffu : 0x7fu) & (z0 + 8u == d3 ? 0xfeu : 0xffu) : 0u;
         if (!FULL) inter &= 0xff00u >> nv;
       } else {
-        wrap = true;   // the octet crosses a row: elements of several rows
-        inter = __brev(octet_interior(g0, nv, a.g)) >> 24;
+        wrap = true;   // the octet crosses a row
+        if (FULL && d3 > 8u) {
+          // columns z0 .. d3-1 of a row, then 0 .. of the next
+          const unsigned k = d3 - z0;                     // 1 .. 7
+          const bool plane_in = !D3 || xx - 1u < (unsigned)a.g.d1 - 2u;
+          if (plane_in && y - 1u < (unsigned)a.g.d2 - 2u) inter = ((1u << k) - 1u) >> 1;
+          if (plane_in && y < (unsigned)a.g.d2 - 2u) inter |= 0xffu & ~((2u << k) - 1u);
+          inter = __brev(inter) >> 24;
+        } else {
+          inter = __brev(octet_interior(g0, nv, a.g)) >> 24;
+        }
       }
     }
   } else if (nv > 0) {

@@ -65,9 +65,8 @@ int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
                    unsigned long long K, unsigned long long E, float eb, int *d_sp, bool try_bits = true);
 
 // Post-processing of a decoded field in place (serial raster semantics of the
-// reference drivers).  types: u8 per element (or int when types_i != null).
-int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig,
-                const unsigned char *d_types_u8, const int *d_types_i, const int *d_sp,
+// reference drivers).  types: an int per element.
+int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const int *d_types_i, const int *d_sp,
                 unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
                 int *restored_out);
 
@@ -93,8 +92,14 @@ size_t post_scratch_bytes(unsigned long long n);
 int compact_extrema(szp_b200_ctx *ctx, const int *d_cps, int stride, unsigned long long K, int *d_sp,
                     unsigned long long *E_out);
 unsigned long long *post_words(szp_b200_ctx *ctx, unsigned long long n);
-int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, unsigned char *d_T,
-                     unsigned long long *d_S, TileDesc *desc, const int *d_sp,
+// Bit planes of the types (bit i % 32 of word i / 32, zero past the field), in
+// the workspace's scratch; the decoder fills them, or they are made of a byte
+// per point.
+bool post_planes(szp_b200_ctx *ctx, unsigned long long n, unsigned **TL, unsigned **TH);
+int post_planes_from_bytes(szp_b200_ctx *ctx, const unsigned char *d_T, unsigned long long n, unsigned *TL,
+                           unsigned *TH);
+int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const unsigned *d_TL,
+                     const unsigned *d_TH, unsigned long long *d_S, TileDesc *desc, const int *d_sp,
                      unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
                      int *restored_out);
 

@@ -72,12 +72,14 @@ __constant__ double c_w3[27];
 
 struct PostArgs {
   float *F;                     // the field, updated in place
-  // raw decoded value of each entry of the pass's list; null: the field is
-  // the decoded field itself, so an item's raw value is its own F value
-  // before its first write in the pass (F[e] changes only by e's own item)
+  // raw decoded value of a point: OL at its entry of the pass's list, else
+  // ORIG at the point, else (both null: the field is the decoded field itself)
+  // its own F value before its first write in the pass (F[e] changes only by
+  // e's own item)
   const float *OL;
-  float *RAW;                   // fused stencil with OL null: raw values of the items left for enforcement
-  unsigned char *T;             // types in bits 0..1
+  const float *ORIG;
+  float *RAW;                   // fused stencil on the decoded field itself: raw values of the items left for enforcement
+  const unsigned *TL, *TH;      // bit planes of the types
   const int *sp;
   unsigned long long n_sp;
   Geom g;
@@ -110,7 +112,11 @@ __device__ __forceinline__ void st_rlx(unsigned long long *p, unsigned long long
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-__device__ __forceinline__ int ty(const PostArgs &a, long long q) { return a.T[q] & 3; }
+__device__ __forceinline__ int ty(const PostArgs &a, long long q) {
+  const long long w = q >> 5;
+  const unsigned b = (unsigned)(q & 31);
+  return (int)(((a.TL[w] >> b) & 1u) | (((a.TH[w] >> b) & 1u) << 1));
+}
 
 // coordinates of flat index e
 struct C3 { long long x, y, z; };
@@ -160,35 +166,25 @@ __device__ __forceinline__ float valo(const PostArgs &a, long long e, const C3 &
   return a.F[q];
 }
 
-// value of the earlier point e + (dx, dy, dz) as the serial pass sees it,
-// with its loads issued whether or not the caller uses it (exists: the point
-// lies in the field; 0 otherwise)
-template <int PASS>
-__device__ __forceinline__ float far_back(const PostArgs &a, long long e, const C3 &c, int dx, int dy, int dz,
-                                          bool exists) {
-  if (!exists) return 0.f;
-  const long long q = e + (long long)dx * a.g.plane + (long long)dy * a.g.d3 + dz;
-  const bool cand = is_cand_known<PASS>(a, q, interior_off(a, c, dx, dy, dz));
-  const float fv = a.F[q];
-  return cand ? __uint_as_float((unsigned)ld_rlx(&a.S[q])) : fv;
-}
+// The earlier candidates that an RBF / axis-pattern item may read and whose
+// results for this pass it must wait for: the earlier points of the 3x3(x3)
+// box and the points two steps back along each axis.  The candidate tests of
+// all of them are issued first, then the result words of the candidates, so a
+// check waits for two loads in a row, not one per point.
+constexpr int kDepPolls = 1024;
 
-// every earlier candidate that an RBF / axis-pattern item may read has its
-// result for this pass: the earlier points of the 3x3(x3) box and the points
-// two steps back along each axis.  The candidate tests of all of them are
-// issued first, then the result words of the candidates, so an item waits
-// for two loads in a row, not one per point.  polls > 0: while a result is
-// missing, poll the missing words up to polls times (a bounded wait for
-// items of the same launch that are computing them); the item is deferred
-// when one is still missing.
-constexpr int kDepPolls = 256;
+template <int ND>
+struct Deps {
+  static constexpr int NB = ND == 3 ? 13 : 4;   // earlier box points
+  unsigned q[NB + 3];
+  float val[NB + 3];                             // their results
+  unsigned cand, pend;                           // bit i: a candidate; its result is missing
+};
 
 template <int PASS, int ND>
-__device__ bool deps_ready(const PostArgs &a, long long e, const C3 &c, int polls = 0) {
-  constexpr int NB = ND == 3 ? 13 : 4;   // earlier box points
-  long long q[NB + 3];
-  bool cand[NB + 3];
+__device__ __forceinline__ void deps_find(const PostArgs &a, long long e, const C3 &c, Deps<ND> &d) {
   int k = 0;
+  d.cand = 0;
 #pragma unroll
   for (int dx = (ND == 3 ? -1 : 0); dx <= 0; dx++)
 #pragma unroll
@@ -196,28 +192,37 @@ __device__ bool deps_ready(const PostArgs &a, long long e, const C3 &c, int poll
 #pragma unroll
       for (int dz = -1; dz <= 1; dz++) {
         if (dx == 0 && (dy > 0 || (dy == 0 && dz >= 0))) continue;
-        q[k] = e + (long long)dx * a.g.plane + (long long)dy * a.g.d3 + dz;
-        cand[k] = is_cand_known<PASS>(a, q[k], interior_off(a, c, dx, dy, dz));
+        const long long q = e + (long long)dx * a.g.plane + (long long)dy * a.g.d3 + dz;
+        d.q[k] = (unsigned)q;
+        d.cand |= (is_cand_known<PASS>(a, q, interior_off(a, c, dx, dy, dz)) ? 1u : 0u) << k;
         k++;
       }
 #pragma unroll
   for (int j = 0; j < 3; j++) {
     const int dx = j == 0 ? -2 : 0, dy = j == 1 ? -2 : 0, dz = j == 2 ? -2 : 0;
     const bool in = (ND == 3 || j > 0) && c.x + dx >= 0 && c.y + dy >= 0 && c.z + dz >= 0;
-    q[NB + j] = e + (long long)dx * a.g.plane + (long long)dy * a.g.d3 + dz;
-    cand[NB + j] = in && is_cand_known<PASS>(a, q[NB + j], interior_off(a, c, dx, dy, dz));
+    const long long q = e + (long long)dx * a.g.plane + (long long)dy * a.g.d3 + dz;
+    d.q[Deps<ND>::NB + j] = (unsigned)q;
+    d.cand |= (in && is_cand_known<PASS>(a, q, interior_off(a, c, dx, dy, dz)) ? 1u : 0u) << (Deps<ND>::NB + j);
   }
-  unsigned pend = 0;
+  d.pend = d.cand;
+}
+
+// looks at the missing results once (all loads in flight together); true when
+// none is missing any more
+template <int ND>
+__device__ __forceinline__ bool deps_ready(const PostArgs &a, Deps<ND> &d) {
+  constexpr int N = Deps<ND>::NB + 3;
+  unsigned long long w[N];
 #pragma unroll
-  for (int i = 0; i < NB + 3; i++)
-    if (cand[i] && (unsigned)(ld_rlx(&a.S[q[i]]) >> 32) != a.gen) pend |= 1u << i;
-  for (int p = 0; pend && p < polls; p++) {
-    __nanosleep(256);
+  for (int i = 0; i < N; i++) w[i] = ((d.pend >> i) & 1u) ? ld_rlx(&a.S[d.q[i]]) : 0ull;
 #pragma unroll
-    for (int i = 0; i < NB + 3; i++)
-      if (((pend >> i) & 1u) && (unsigned)(ld_rlx(&a.S[q[i]]) >> 32) == a.gen) pend &= ~(1u << i);
-  }
-  return pend == 0;
+  for (int i = 0; i < N; i++)
+    if (((d.pend >> i) & 1u) && (unsigned)(w[i] >> 32) == a.gen) {
+      d.val[i] = __uint_as_float((unsigned)w[i]);
+      d.pend &= ~(1u << i);
+    }
+  return d.pend == 0u;
 }
 
 // ----------------------------------------------------------------------------
@@ -314,10 +319,10 @@ __device__ __forceinline__ void face_item_load(const PostArgs &a, const unsigned
   const long long e = (long long)list[idx];
   const long long pl = a.g.plane, d3 = a.g.d3;
   it.e = e;
-  it.t = ty(a, e);
+  it.t = (a.TL[e >> 5] >> (unsigned)(e & 31)) & 1u ? 1 : 2;   // an extremum: maximum 01, minimum 10
   it.s = (PASS == kPassStencil && idx < a.n_sp) ? a.sp[idx] : 0;
   it.cur = a.F[e];
-  it.o = a.OL ? a.OL[idx] : it.cur;
+  it.o = a.OL ? a.OL[idx] : (a.ORIG ? a.ORIG[e] : it.cur);
   // e is interior: every face neighbour lies in the field
   it.f.xm = ND == 3 ? a.F[e - pl] : 0.f;
   it.f.xp = ND == 3 ? a.F[e + pl] : 0.f;
@@ -428,31 +433,82 @@ __device__ __forceinline__ int cls4_eps(float c, float n, float s, float w, floa
   return ((vh && hl) || (vl && hh)) ? 3 : 0;
 }
 
-// 2D RBF saddle restoration of candidate e (example/test_cuda_topology.cu:227-326)
-__device__ float rbf2(const PostArgs &a, long long e, const C3 &c, float o, bool &ok) {
-  const long long cols = a.g.d3;
-  const long long rows = a.g.d2;
+// What an RBF item reads besides the results it waits for, loaded before it
+// waits: nothing of it changes before the item is done (a later candidate waits
+// for the item, an earlier one's result comes from its word).
+template <int ND>
+struct RbfItem {
+  static constexpr int N = ND == 3 ? 27 : 9, C = N / 2;   // box points, the centre
+  float v[N];          // box value at (dx, dy, dz): v[(dx + 1) * 9 + (dy + 1) * 3 + (dz + 1)] (2D: dx = -1 gone)
+  float far[6];        // two steps out: x-, y-, z- (as the serial pass sees them), x+, y+, z+
+  unsigned chk;        // bit 2 k + s: the neighbour at side s (0 -, 1 +) of axis k is interior and regular
+  unsigned locks;
+  double den;
+  float o;
+};
+
+template <int ND>
+__device__ __forceinline__ double rbf_weight(unsigned locks, int i) {
+  const double ww = ND == 3 ? c_w3[i] : c_w2[i];
+  return ((locks >> i) & 1u) ? __dmul_rn(ww, 0.4) : ww;
+}
+
+template <int ND>
+__device__ __forceinline__ void rbf_load(const PostArgs &a, long long e, const C3 &c, unsigned cand, float o,
+                                         RbfItem<ND> &it) {
+  constexpr int NB = Deps<ND>::NB;
+  const long long pl = a.g.plane, d3 = a.g.d3;
+#pragma unroll
+  for (int i = 0; i < RbfItem<ND>::N; i++) {
+    const int dx = ND == 3 ? i / 9 - 1 : 0, dy = (i / 3) % 3 - 1, dz = i % 3 - 1;
+    // an earlier candidate's value is its result
+    it.v[i] = i < NB && ((cand >> i) & 1u) ? 0.f : a.F[e + dx * pl + dy * d3 + dz];
+  }
+  // the far sides, wherever they exist; used where the serial pass reads them
+  const long long step[3] = {pl, d3, 1};
+  const long long at[3] = {c.x, c.y, c.z}, ext[3] = {a.g.d1, a.g.d2, a.g.d3};
+  it.chk = 0;
+#pragma unroll
+  for (int k = ND == 3 ? 0 : 1; k < 3; k++) {
+    it.far[k] = at[k] >= 2 && !((cand >> (NB + k)) & 1u) ? a.F[e - 2 * step[k]] : 0.f;
+    it.far[3 + k] = at[k] + 2 < ext[k] ? a.F[e + 2 * step[k]] : 0.f;
+    if (at[k] - 1 >= 1 && ty(a, e - step[k]) == 0) it.chk |= 1u << (2 * k);
+    if (at[k] + 1 < ext[k] - 1 && ty(a, e + step[k]) == 0) it.chk |= 2u << (2 * k);
+  }
+  it.locks = box_locks<ND>(a, e, c);
+  it.o = o;
+  double den = 0.0;
+#pragma unroll
+  for (int i = 0; i < RbfItem<ND>::N; i++) den = __dadd_rn(den, rbf_weight<ND>(it.locks, i));
+  it.den = den;
+}
+
+// the results it waited for, and the weighted mean of the box
+template <int ND>
+__device__ __forceinline__ float rbf_mean(const Deps<ND> &d, RbfItem<ND> &it) {
+  constexpr int NB = Deps<ND>::NB;
+#pragma unroll
+  for (int i = 0; i < NB; i++)
+    if ((d.cand >> i) & 1u) it.v[i] = d.val[i];
+#pragma unroll
+  for (int k = ND == 3 ? 0 : 1; k < 3; k++)
+    if ((d.cand >> (NB + k)) & 1u) it.far[k] = d.val[NB + k];
+  double num = 0.0;
+#pragma unroll
+  for (int i = 0; i < RbfItem<ND>::N; i++)
+    num = __dadd_rn(num, __dmul_rn(rbf_weight<ND>(it.locks, i), (double)it.v[i]));
+  return __double2float_rn(__ddiv_rn(num, it.den));
+}
+
+// 2D RBF saddle restoration (example/test_cuda_topology.cu:227-326)
+__device__ __forceinline__ float rbf2(const PostArgs &a, const Deps<2> &d, RbfItem<2> &it, bool &ok) {
   ok = false;
-  // 3x3 neighbourhood values as seen by the serial pass
-  float v[3][3];
-  for (int da = -1; da <= 1; da++)
-    for (int db = -1; db <= 1; db++)
-      v[da + 1][db + 1] = (da == 0 && db == 0) ? a.F[e] : valo<kPassRbf>(a, e, c, 0, da, db);
-  const unsigned lk = box_locks<2>(a, e, c);
-  double num = 0.0, den = 0.0;
-  for (int da = -1; da <= 1; da++)
-    for (int db = -1; db <= 1; db++) {
-      double ww = c_w2[(da + 1) * 3 + (db + 1)];
-      if ((lk >> ((da + 1) * 3 + (db + 1))) & 1u) ww = __dmul_rn(ww, 0.4);
-      num = __dadd_rn(num, __dmul_rn(ww, (double)v[da + 1][db + 1]));
-      den = __dadd_rn(den, ww);
-    }
-  const float old = a.F[e];
-  if (!(den > 0.0)) return old;
-  const float d = __fmul_rn(a.eb, 0.999f);
-  const float lo = __fsub_rn(o, d), hi = __fadd_rn(o, d);
-  const float n = v[0][1], s = v[2][1], w = v[1][0], ea = v[1][2];
-  float cand = __double2float_rn(__ddiv_rn(num, den));
+  const float old = it.v[4];
+  if (!(it.den > 0.0)) return old;
+  float cand = rbf_mean<2>(d, it);
+  const float m = __fmul_rn(a.eb, 0.999f);
+  const float lo = __fsub_rn(it.o, m), hi = __fadd_rn(it.o, m);
+  const float n = it.v[1], s = it.v[7], w = it.v[3], ea = it.v[5];
   {
     const float q = __fmul_rn(0.25f, a.eps);
     float clo = __fsub_rn(fminf(fmaxf(n, s), fmaxf(w, ea)), q);
@@ -467,34 +523,69 @@ __device__ float rbf2(const PostArgs &a, long long e, const C3 &c, float o, bool
   }
   if (cand < lo) cand = lo;
   if (cand > hi) cand = hi;
-  // outer ring values needed by the neighbour validations
-  const bool vu = (c.y - 1 >= 1) && ty(a, e - cols) == 0;
-  const bool vd = (c.y + 1 < rows - 1) && ty(a, e + cols) == 0;
-  const bool vl = (c.z - 1 >= 1) && ty(a, e - 1) == 0;
-  const bool vr = (c.z + 1 < cols - 1) && ty(a, e + 1) == 0;
-  // loaded wherever the points exist, so that the loads overlap
-  const float gu = far_back<kPassRbf>(a, e, c, 0, -2, 0, c.y >= 2);
-  const float gl = far_back<kPassRbf>(a, e, c, 0, 0, -2, c.z >= 2);
-  const float gd = c.y + 2 < rows ? a.F[e + 2 * cols] : 0.f;
-  const float gr = c.z + 2 < cols ? a.F[e + 2] : 0.f;
-  const float u2 = vu ? gu : 0.f, d2 = vd ? gd : 0.f, l2 = vl ? gl : 0.f, r2 = vr ? gr : 0.f;
+  const bool vu = (it.chk >> 2) & 1u, vd = (it.chk >> 3) & 1u, vl = (it.chk >> 4) & 1u, vr = (it.chk >> 5) & 1u;
+  const float u2 = vu ? it.far[1] : 0.f, d2 = vd ? it.far[4] : 0.f, l2 = vl ? it.far[2] : 0.f,
+              r2 = vr ? it.far[5] : 0.f;
   const float step = __fsub_rn(cand, old);
   float alpha = 1.0f;
-  for (int it = 0; it < 10; it++) {
+  for (int k = 0; k < 10; k++) {
     float trial = __fadd_rn(old, __fmul_rn(alpha, step));
     if (trial < lo) trial = lo;
     if (trial > hi) trial = hi;
     const float eps = a.eps;
     bool bad = false;
     // neighbour (i-1, j): its neighbours are (i-2, j), (i, j) = trial, (i-1, j-1), (i-1, j+1)
-    if (vu && cls4_eps(n, u2, trial, v[0][0], v[0][2], eps) != 0) bad = true;
-    if (!bad && vd && cls4_eps(s, trial, d2, v[2][0], v[2][2], eps) != 0) bad = true;
-    if (!bad && vl && cls4_eps(w, v[0][0], v[2][0], l2, trial, eps) != 0) bad = true;
-    if (!bad && vr && cls4_eps(ea, v[0][2], v[2][2], trial, r2, eps) != 0) bad = true;
+    if (vu && cls4_eps(n, u2, trial, it.v[0], it.v[2], eps) != 0) bad = true;
+    if (!bad && vd && cls4_eps(s, trial, d2, it.v[6], it.v[8], eps) != 0) bad = true;
+    if (!bad && vl && cls4_eps(w, it.v[0], it.v[6], l2, trial, eps) != 0) bad = true;
+    if (!bad && vr && cls4_eps(ea, it.v[2], it.v[8], trial, r2, eps) != 0) bad = true;
     if (!bad && cls4_eps(trial, n, s, w, ea, eps) != 3) bad = true;
     if (!bad) { ok = true; return trial; }
     alpha = __fmul_rn(alpha, 0.5f);
   }
+  return old;
+}
+
+// 3D RBF (example/test_cuda_topology_3d.cu:317-434).  A trial changes only the
+// centre value.
+__device__ __forceinline__ float rbf3(const PostArgs &a, const Deps<3> &d, RbfItem<3> &it, bool &ok) {
+  ok = false;
+  const float old = it.v[13];
+  if (!(it.den > 0.0)) return old;
+  float cand = rbf_mean<3>(d, it);
+  const float m = __fmul_rn(a.eb, 0.999f);
+  const float lo = __fsub_rn(it.o, m), hi = __fadd_rn(it.o, m);
+  if (cand < lo) cand = lo;
+  if (cand > hi) cand = hi;
+  const bool cxm = it.chk & 1u, cxp = (it.chk >> 1) & 1u, cym = (it.chk >> 2) & 1u, cyp = (it.chk >> 3) & 1u,
+             czm = (it.chk >> 4) & 1u, czp = (it.chk >> 5) & 1u;
+  const float fxm = cxm ? it.far[0] : 0.f, fym = cym ? it.far[1] : 0.f, fzm = czm ? it.far[2] : 0.f;
+  const float fxp = cxp ? it.far[3] : 0.f, fyp = cyp ? it.far[4] : 0.f, fzp = czp ? it.far[5] : 0.f;
+#define V3(dx, dy, dz) it.v[((dx) + 1) * 9 + ((dy) + 1) * 3 + ((dz) + 1)]
+  const float step = __fsub_rn(cand, old);
+  float alpha = 1.0f;
+  for (int k = 0; k < 10; k++) {
+    float tr = __fadd_rn(old, __fmul_rn(alpha, step));
+    if (tr < lo) tr = lo;
+    if (tr > hi) tr = hi;
+    // classify6(centre, x-, x+, y-, y+, z-, z+) of the centre and of each checked neighbour
+    bool good = classify6(tr, V3(-1, 0, 0), V3(1, 0, 0), V3(0, -1, 0), V3(0, 1, 0), V3(0, 0, -1), V3(0, 0, 1)) == 3;
+    if (good && cxm)
+      good = classify6(V3(-1, 0, 0), fxm, tr, V3(-1, -1, 0), V3(-1, 1, 0), V3(-1, 0, -1), V3(-1, 0, 1)) == 0;
+    if (good && cxp)
+      good = classify6(V3(1, 0, 0), tr, fxp, V3(1, -1, 0), V3(1, 1, 0), V3(1, 0, -1), V3(1, 0, 1)) == 0;
+    if (good && cym)
+      good = classify6(V3(0, -1, 0), V3(-1, -1, 0), V3(1, -1, 0), fym, tr, V3(0, -1, -1), V3(0, -1, 1)) == 0;
+    if (good && cyp)
+      good = classify6(V3(0, 1, 0), V3(-1, 1, 0), V3(1, 1, 0), tr, fyp, V3(0, 1, -1), V3(0, 1, 1)) == 0;
+    if (good && czm)
+      good = classify6(V3(0, 0, -1), V3(-1, 0, -1), V3(1, 0, -1), V3(0, -1, -1), V3(0, 1, -1), fzm, tr) == 0;
+    if (good && czp)
+      good = classify6(V3(0, 0, 1), V3(-1, 0, 1), V3(1, 0, 1), V3(0, -1, 1), V3(0, 1, 1), tr, fzp) == 0;
+    if (good) { ok = true; return tr; }
+    alpha = __fmul_rn(alpha, 0.5f);
+  }
+#undef V3
   return old;
 }
 
@@ -540,90 +631,6 @@ __device__ bool valid3(const PostArgs &a, long long e, const C3 &c, Win3 &W, flo
   return true;
 }
 
-// 3D RBF (example/test_cuda_topology_3d.cu:317-434).  Every value the
-// validation can read is loaded once into registers (compile-time indices):
-// the 3x3x3 box around e and the points two steps out along each axis, the
-// latter loaded wherever they exist and used only where the serial code reads
-// them (the neighbour on that side is interior and regular).  The candidate
-// tests come first and every value load after them, so an item waits for a
-// few loads in a row, not one per point.  A trial changes only the centre
-// value.
-__device__ float rbf3(const PostArgs &a, long long e, const C3 &c, float o, bool &ok) {
-  ok = false;
-  const float old = a.F[e];
-  float v[27];   // box value at (dx, dy, dz): v[(dx + 1) * 9 + (dy + 1) * 3 + (dz + 1)]
-  // which earlier box points (i < 13) are candidates, then every value: the
-  // result of an earlier candidate, else F (loads issued together)
-  bool cb[13];
-#pragma unroll
-  for (int i = 0; i < 13; i++) {
-    const int dx = i / 9 - 1, dy = (i / 3) % 3 - 1, dz = i % 3 - 1;
-    cb[i] = is_cand_known<kPassRbf>(a, e + dx * a.g.plane + dy * a.g.d3 + dz, interior_off(a, c, dx, dy, dz));
-  }
-#pragma unroll
-  for (int i = 0; i < 27; i++) {
-    const int dx = i / 9 - 1, dy = (i / 3) % 3 - 1, dz = i % 3 - 1;
-    const long long q = e + dx * a.g.plane + dy * a.g.d3 + dz;
-    v[i] = (i == 13) ? old : (i < 13 && cb[i]) ? __uint_as_float((unsigned)ld_rlx(&a.S[q])) : a.F[q];
-  }
-  // neighbours whose classification the validation checks, and their far sides
-  const long long pl = a.g.plane, d3 = a.g.d3;
-  const bool cxm = c.x - 1 >= 1 && ty(a, e - pl) == 0, cxp = c.x + 1 < a.g.d1 - 1 && ty(a, e + pl) == 0;
-  const bool cym = c.y - 1 >= 1 && ty(a, e - d3) == 0, cyp = c.y + 1 < a.g.d2 - 1 && ty(a, e + d3) == 0;
-  const bool czm = c.z - 1 >= 1 && ty(a, e - 1) == 0, czp = c.z + 1 < a.g.d3 - 1 && ty(a, e + 1) == 0;
-  // the far sides, loaded wherever they exist (not only after the type
-  // tests) so that their loads overlap; used as the serial pass reads them
-  const float gxm = far_back<kPassRbf>(a, e, c, -2, 0, 0, c.x >= 2);
-  const float gym = far_back<kPassRbf>(a, e, c, 0, -2, 0, c.y >= 2);
-  const float gzm = far_back<kPassRbf>(a, e, c, 0, 0, -2, c.z >= 2);
-  const float gxp = c.x + 2 < a.g.d1 ? a.F[e + 2 * pl] : 0.f;
-  const float gyp = c.y + 2 < a.g.d2 ? a.F[e + 2 * d3] : 0.f;
-  const float gzp = c.z + 2 < a.g.d3 ? a.F[e + 2] : 0.f;
-  const float fxm = cxm ? gxm : 0.f, fym = cym ? gym : 0.f, fzm = czm ? gzm : 0.f;
-  const float fxp = cxp ? gxp : 0.f, fyp = cyp ? gyp : 0.f, fzp = czp ? gzp : 0.f;
-  const unsigned lk = box_locks<3>(a, e, c);
-  double num = 0.0, den = 0.0;
-#pragma unroll
-  for (int i = 0; i < 27; i++) {
-    double ww = c_w3[i];
-    if ((lk >> i) & 1u) ww = __dmul_rn(ww, 0.4);
-    num = __dadd_rn(num, __dmul_rn(ww, (double)v[i]));
-    den = __dadd_rn(den, ww);
-  }
-  if (!(den > 0.0)) return old;
-  const float d = __fmul_rn(a.eb, 0.999f);
-  const float lo = __fsub_rn(o, d), hi = __fadd_rn(o, d);
-  float cand = __double2float_rn(__ddiv_rn(num, den));
-  if (cand < lo) cand = lo;
-  if (cand > hi) cand = hi;
-#define V3(dx, dy, dz) v[((dx) + 1) * 9 + ((dy) + 1) * 3 + ((dz) + 1)]
-  const float step = __fsub_rn(cand, old);
-  float alpha = 1.0f;
-  for (int it = 0; it < 10; it++) {
-    float tr = __fadd_rn(old, __fmul_rn(alpha, step));
-    if (tr < lo) tr = lo;
-    if (tr > hi) tr = hi;
-    // classify6(centre, x-, x+, y-, y+, z-, z+) of the centre and of each checked neighbour
-    bool good = classify6(tr, V3(-1, 0, 0), V3(1, 0, 0), V3(0, -1, 0), V3(0, 1, 0), V3(0, 0, -1), V3(0, 0, 1)) == 3;
-    if (good && cxm)
-      good = classify6(V3(-1, 0, 0), fxm, tr, V3(-1, -1, 0), V3(-1, 1, 0), V3(-1, 0, -1), V3(-1, 0, 1)) == 0;
-    if (good && cxp)
-      good = classify6(V3(1, 0, 0), tr, fxp, V3(1, -1, 0), V3(1, 1, 0), V3(1, 0, -1), V3(1, 0, 1)) == 0;
-    if (good && cym)
-      good = classify6(V3(0, -1, 0), V3(-1, -1, 0), V3(1, -1, 0), fym, tr, V3(0, -1, -1), V3(0, -1, 1)) == 0;
-    if (good && cyp)
-      good = classify6(V3(0, 1, 0), V3(-1, 1, 0), V3(1, 1, 0), tr, fyp, V3(0, 1, -1), V3(0, 1, 1)) == 0;
-    if (good && czm)
-      good = classify6(V3(0, 0, -1), V3(-1, 0, -1), V3(1, 0, -1), V3(0, -1, -1), V3(0, 1, -1), fzm, tr) == 0;
-    if (good && czp)
-      good = classify6(V3(0, 0, 1), V3(-1, 0, 1), V3(1, 0, 1), V3(0, -1, 1), V3(0, 1, 1), tr, fzp) == 0;
-    if (good) { ok = true; return tr; }
-    alpha = __fmul_rn(alpha, 0.5f);
-  }
-#undef V3
-  return old;
-}
-
 // 3D axis-pattern saddle stencil (example/test_cuda_topology_3d.cu:187-314)
 __device__ float axis3(const PostArgs &a, long long e, const C3 &c, float o, bool &ok) {
   ok = false;
@@ -662,26 +669,24 @@ __device__ float axis3(const PostArgs &a, long long e, const C3 &c, float o, boo
 // candidate lists
 // ----------------------------------------------------------------------------
 
-// Interior extrema (X) and interior saddles (Z) in raster order plus the
-// interior-extremum bitmap Eb, in one pass over the types: persistent
-// CTAs take tiles of kListTile points in order (32 consecutive points per
-// thread), publish their counts and find their list offsets by decoupled
-// look-back (extrema in the byte word, saddles in the count word), then write
-// their entries through shared memory so each tile's slice of X and Z is
-// stored contiguously (X staged from the front of one buffer, Z from its back:
-// a point is in at most one list).  The last tile writes the totals to
-// tot[0] = (extrema << 32) | saddles.  The raw decoded value of every list
-// entry (Ox / Oz at its point) goes to OX / OZ beside it, for each list whose
-// source is given (none is needed when the passes read raw values from the
-// field itself).
+// Interior extrema in raster order (X), the interior-extremum and
+// interior-saddle bitmaps (Eb, Sb) and, with Z given, the interior saddles in
+// raster order, in one pass over the types' bit planes: persistent CTAs take
+// tiles of kListTile points in order (one word of 32 points per thread),
+// publish their counts and find their list offsets by decoupled look-back
+// (extrema in the byte word, saddles in the count word), then write their
+// entries through shared memory so each tile's slice of X and Z is stored
+// contiguously (X staged from the front of one buffer, Z from its back: a
+// point is in at most one list).  The last tile writes the totals to tot[0] =
+// (extrema << 32) | saddles.  512^3 field: 241 us from a byte per type with
+// both lists, 149 from the planes with X alone.
 constexpr int kListPer = 32;
 constexpr int kListTile = kPostThreads * kListPer;
 
 __global__ void __launch_bounds__(kPostThreads)
-list_build_kernel(const unsigned char *__restrict__ T, Geom g, long long n, TileDesc *desc, unsigned *tile_ctr,
-                  int *err, unsigned *X, unsigned *Z, unsigned char *Eb,
-                  unsigned long long *tot, const float *__restrict__ Ox, const float *__restrict__ Oz,
-                  float *OX, float *OZ, unsigned *XP) {
+list_build_kernel(const unsigned *__restrict__ TL, const unsigned *__restrict__ TH, Geom g, long long n,
+                  TileDesc *desc, unsigned *tile_ctr, int *err, unsigned *X, unsigned *Z, unsigned *Eb, unsigned *Sb,
+                  unsigned long long *tot, unsigned *XP) {
   __shared__ unsigned s_w1[kWarps], s_w2[kWarps];
   __shared__ unsigned s_buf[kListTile];
   __shared__ long long s_tile;
@@ -695,6 +700,7 @@ list_build_kernel(const unsigned char *__restrict__ T, Geom g, long long n, Tile
     const long long i0 = tile * kListTile + (long long)threadIdx.x * kListPer;
     unsigned em = 0, sm = 0, im = 0;
     if (i0 < n) {
+      const unsigned tl = TL[i0 >> 5], th = TH[i0 >> 5];
       long long r, x, y, z;
       if (g.nd == 2) { x = 0; y = fdivmod(i0, g.d3, g.m_d3, r); z = r; }
       else { x = fdivmod(i0, g.plane, g.m_plane, r); y = fdivmod(r, g.d3, g.m_d3, z); }
@@ -706,6 +712,12 @@ list_build_kernel(const unsigned char *__restrict__ T, Geom g, long long n, Tile
           const int ulo = lo > 0 ? (int)lo : 0, uhi = hi < kListPer - 1 ? (int)hi : kListPer - 1;
           if (ulo <= uhi) im = (uhi == 31 ? 0xffffffffu : ((2u << uhi) - 1u)) & ~((1u << ulo) - 1u);
         }
+      } else if (g.d3 > kListPer && i0 + kListPer <= n) {
+        // two rows: columns z .. d3-1 of one, then 0 .. of the next
+        const unsigned k = (unsigned)(g.d3 - z);          // 1 .. 31
+        const bool plane_in = g.nd == 2 || (x >= 1 && x <= g.d1 - 2);
+        if (plane_in && y >= 1 && y <= g.d2 - 2) im = ((1u << k) - 1u) >> 1;
+        if (plane_in && y + 1 <= g.d2 - 2) im |= ~((2u << k) - 1u);
       } else {
         for (int u = 0; u < kListPer && i0 + u < n; u++) {
           bool in = y >= 1 && y <= g.d2 - 2 && z >= 1 && z <= g.d3 - 2;
@@ -715,38 +727,10 @@ list_build_kernel(const unsigned char *__restrict__ T, Geom g, long long n, Tile
           while (z >= g.d3) { z -= g.d3; y++; if (y >= g.d2) { y -= g.d2; x++; } }
         }
       }
-      if (im) {
-        const bool vec = i0 + kListPer <= n && ((reinterpret_cast<uintptr_t>(T + i0) & 15) == 0);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          unsigned long long w0 = 0, w1 = 0;
-          if (vec) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(T + i0) + h);
-            w0 = ((unsigned long long)v.y << 32) | v.x;
-            w1 = ((unsigned long long)v.w << 32) | v.z;
-          } else {
-            for (int u = 0; u < 8; u++) {
-              if (i0 + 16 * h + u < n) w0 |= (unsigned long long)T[i0 + 16 * h + u] << (8 * u);
-              if (i0 + 16 * h + 8 + u < n) w1 |= (unsigned long long)T[i0 + 16 * h + 8 + u] << (8 * u);
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < 16; u++) {
-            const unsigned t = (unsigned)((u < 8 ? w0 : w1) >> (8 * (u & 7))) & 3u;
-            const unsigned bit = 1u << (16 * h + u);
-            if (im & bit) {
-              if (t == 1u || t == 2u) em |= bit;
-              if (t == 3u) sm |= bit;
-            }
-          }
-        }
-      }
-      // 4 bitmap bytes of this thread's 32 points (i0 is a multiple of 32)
-      if (i0 + kListPer <= n) {
-        reinterpret_cast<unsigned *>(Eb)[i0 >> 5] = em;
-      } else {
-        for (int k = 0; k < 4 && i0 + 8 * k < n; k++) Eb[(i0 >> 3) + k] = (unsigned char)(em >> (8 * k));
-      }
+      em = (tl ^ th) & im;
+      sm = tl & th & im;
+      Eb[i0 >> 5] = em;
+      Sb[i0 >> 5] = sm;
     }
     unsigned te, ts;
     const unsigned eo = cta_excl_scan_post((unsigned)__popc(em), s_w1, &te);
@@ -756,7 +740,7 @@ list_build_kernel(const unsigned char *__restrict__ T, Geom g, long long n, Tile
       unsigned xe = eo, xs = so;
       unsigned mm = em;
       while (mm) { const int u = __ffs(mm) - 1; mm &= mm - 1; s_buf[xe++] = (unsigned)(i0 + u); }
-      mm = sm;
+      mm = Z ? sm : 0u;
       while (mm) { const int u = __ffs(mm) - 1; mm &= mm - 1; s_buf[kListTile - 1 - xs++] = (unsigned)(i0 + u); }
     }
     const Prefix pf = lookback_cta<kWarps>(desc, tile, te, ts, err);
@@ -769,81 +753,68 @@ list_build_kernel(const unsigned char *__restrict__ T, Geom g, long long n, Tile
     const unsigned long long xb = s_xb, zb = s_zb;
     // list position of the first extremum of this thread's bitmap word
     if (i0 < n) XP[i0 >> 5] = (unsigned)(xb + eo);
-    // entries four at a time per thread: the raw-value gathers of a batch
-    // are in flight together
-    for (unsigned k0 = threadIdx.x; k0 < te; k0 += 4 * kPostThreads) {
-      unsigned q[4];
-      float v[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const unsigned k = k0 + u * kPostThreads;
-        q[u] = k < te ? s_buf[k] : 0u;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (Ox && k0 + u * kPostThreads < te) v[u] = Ox[q[u]];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const unsigned k = k0 + u * kPostThreads;
-        if (k < te) {
-          // a list position past n means corrupt tile offsets: recorded, not written
-          if (xb + k < (unsigned long long)n) {
-            X[xb + k] = q[u];
-            if (Ox) OX[xb + k] = v[u];
-          } else {
-            atomicExch(err, kErrMalformed);
-          }
-        }
-      }
-    }
-    for (unsigned k0 = threadIdx.x; k0 < ts; k0 += 4 * kPostThreads) {
-      unsigned q[4];
-      float v[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const unsigned k = k0 + u * kPostThreads;
-        q[u] = k < ts ? s_buf[kListTile - 1 - k] : 0u;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (Oz && k0 + u * kPostThreads < ts) v[u] = Oz[q[u]];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const unsigned k = k0 + u * kPostThreads;
-        if (k < ts) {
-          if (zb + k < (unsigned long long)n) {
-            Z[zb + k] = q[u];
-            if (Oz) OZ[zb + k] = v[u];
-          } else {
-            atomicExch(err, kErrMalformed);
-          }
-        }
-      }
+    // a list position past n means corrupt tile offsets: recorded, not written
+    if (xb + te > (unsigned long long)n || zb + ts > (unsigned long long)n) {
+      if (threadIdx.x == 0) atomicExch(err, kErrMalformed);
+    } else {
+      for (unsigned k = threadIdx.x; k < te; k += kPostThreads) X[xb + k] = s_buf[k];
+      if (Z)
+        for (unsigned k = threadIdx.x; k < ts; k += kPostThreads) Z[zb + k] = s_buf[kListTile - 1 - k];
     }
     __syncthreads();
   }
 }
 
-// lost saddles (RBF candidates): saddles of the original field that F no
-// longer classifies as saddles (example/test_cuda_topology.cu:244-254)
-__global__ void fn_detect_kernel(PostArgs a, const unsigned *__restrict__ Z, unsigned long long nz,
-                                 unsigned *__restrict__ R, unsigned *__restrict__ Y, unsigned *y_count) {
-  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  bool lost = false;
-  long long q = 0;
-  if (i < nz) {
-    q = (long long)Z[i];
-    lost = classify_F(a, q) != 3;
+// Lost saddles (RBF candidates): saddles of the original field that F no
+// longer classifies as saddles (example/test_cuda_topology.cu:244-254).  A
+// warp takes 32 words of the saddle bitmap, lists their points in shared
+// memory in raster order and classifies them 32 at a time, so that its lanes
+// read neighbouring points.
+__global__ void __launch_bounds__(256)
+fn_detect_kernel(PostArgs a, const unsigned *__restrict__ Sb, unsigned nwords, unsigned *__restrict__ R,
+                 unsigned *__restrict__ Y, unsigned *y_count) {
+  __shared__ unsigned short s_pt[8][1024];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned w0 = (blockIdx.x * 8u + warp) * 32u;
+  if (w0 >= nwords) return;
+  unsigned m = w0 + lane < nwords ? Sb[w0 + lane] : 0u;
+  unsigned inc = __popc(m);
+  const unsigned c = inc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
   }
-  const unsigned m = __ballot_sync(0xffffffffu, lost);
-  unsigned base = 0;
-  const int lane = threadIdx.x & 31;
-  if (lane == 0 && m) base = atomicAdd(y_count, (unsigned)__popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (lost) {
-    Y[base + __popc(m & ((1u << lane) - 1u))] = (unsigned)i;
-    atomicOr(&R[q >> 5], 1u << (q & 31));
+  const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
+  unsigned o = inc - c;
+  while (m) {
+    const int u = __ffs(m) - 1;
+    m &= m - 1;
+    s_pt[warp][o++] = (unsigned short)(32 * lane + u);
   }
+  __syncwarp();
+  const long long base = (long long)w0 * 32;
+  for (unsigned k0 = 0; k0 < total; k0 += 32) {
+    const unsigned k = k0 + lane;
+    const long long q = base + (k < total ? s_pt[warp][k] : 0);
+    const bool lost = k < total && classify_F(a, q) != 3;
+    const unsigned lm = __ballot_sync(0xffffffffu, lost);
+    if (!lm) continue;
+    unsigned at = 0;
+    if (lane == 0) at = atomicAdd(y_count, (unsigned)__popc(lm));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (lost) {
+      Y[at + __popc(lm & ((1u << lane) - 1u))] = (unsigned)q;
+      atomicOr(&R[q >> 5], 1u << (q & 31));
+    }
+  }
+}
+
+// raw values of a list's points
+__global__ void gather_kernel(const unsigned *__restrict__ list, unsigned count, const float *__restrict__ src,
+                              float *__restrict__ dst) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count) dst[i] = src[list[i]];
 }
 
 // Outcome of one item of a pass.
@@ -890,24 +861,51 @@ __device__ __forceinline__ int face_item_run(const PostArgs &a, unsigned idx, Fa
   return st;
 }
 
-// One item of the RBF or axis-pattern pass (list index idx): its result goes
-// to F and to S at its point, or it is deferred while an earlier candidate it
-// reads is not final.
+// Items of the RBF or axis-pattern pass (list index idx), one per lane of a
+// warp that calls it whole: an item's result goes to F and to S at its point.
+// While an earlier candidate that an item reads is not final the item looks
+// again, up to polls times, and is deferred after that (returns true).  The
+// lanes look together and the ready ones compute in between: an item often
+// waits for one in a neighbouring lane, which must not wait for it in turn at
+// the end of a loop of its own (1.2 K lost saddles of a 100 x 500 x 500 field
+// in chains: 315 us when it did, @@RBF@@ now).
 template <int PASS, int ND>
-__device__ __forceinline__ int pass_item(const PostArgs &a, const unsigned *__restrict__ list, unsigned idx,
-                                         int polls) {
-  const long long e = (long long)list[idx];
-  bool ok = false;
-  const C3 c = coords(a.g, e);
-  if (!deps_ready<PASS, ND>(a, e, c, polls)) return kItemDeferred;
-  const float o = a.OL ? a.OL[idx] : a.F[e];
-  const float r = PASS == kPassRbf ? ((ND == 2) ? rbf2(a, e, c, o, ok) : rbf3(a, e, c, o, ok)) : axis3(a, e, c, o, ok);
-  if (ok) atomicAdd(a.restored, 1u);
-  // in place: every reader of e's pre-pass value has finished (they are the
-  // earlier candidates e waited for); later readers take e's result from S
-  a.F[e] = r;
-  st_rlx(&a.S[e], ((unsigned long long)a.gen << 32) | __float_as_uint(r));
-  return kItemDone;
+__device__ __forceinline__ bool pass_items(const PostArgs &a, const unsigned *__restrict__ list, unsigned idx,
+                                           bool valid, int polls) {
+  const long long e = valid ? (long long)list[idx] : 0;
+  C3 c = {0, 0, 0};
+  Deps<ND> d;
+  d.pend = 0;
+  if (valid) {
+    c = coords(a.g, e);
+    deps_find<PASS, ND>(a, e, c, d);
+  }
+  float o = 0.f;
+  RbfItem<ND> it;
+  if (valid) {
+    o = a.OL ? a.OL[idx] : (a.ORIG ? a.ORIG[e] : a.F[e]);
+    if (PASS == kPassRbf) rbf_load<ND>(a, e, c, d.cand, o, it);
+  }
+  bool pending = valid;
+  for (int p = 0;; p++) {
+    const bool ready = pending && deps_ready<ND>(a, d);
+    if (ready) {
+      bool ok = false;
+      float r;
+      if constexpr (PASS != kPassRbf) r = axis3(a, e, c, o, ok);
+      else if constexpr (ND == 2) r = rbf2(a, d, it, ok);
+      else r = rbf3(a, d, it, ok);
+      if (ok) atomicAdd(a.restored, 1u);
+      // in place: every reader of e's pre-pass value has finished (they are the
+      // earlier candidates e waited for); later readers take e's result from S
+      a.F[e] = r;
+      st_rlx(&a.S[e], ((unsigned long long)a.gen << 32) | __float_as_uint(r));
+      pending = false;
+    }
+    if (p >= polls || !__any_sync(0xffffffffu, pending)) break;
+    if (!__any_sync(0xffffffffu, ready)) __nanosleep(p < 64 ? 32 : 256);
+  }
+  return pending;
 }
 
 // An item whose earlier candidate is handled by the same CTA at the same
@@ -927,8 +925,7 @@ __device__ __forceinline__ bool pass_item_local(const PostArgs &a, const unsigne
   // RBF and axis-pattern items are long and uneven: a block barrier would make
   // every thread wait for the slowest, so they wait for missing results on
   // their own (bounded, polls) or retry in rounds
-  if (PASS != kPassStencil && PASS != kPassEnforce)
-    return valid && pass_item<PASS, ND>(a, list, idx, polls) == kItemDeferred;
+  if (PASS != kPassStencil && PASS != kPassEnforce) return pass_items<PASS, ND>(a, list, idx, valid, polls);
   bool pending = valid, need = false;
   FaceItem item;
   if (valid) face_item_load<PASS, ND>(a, list, idx, item);
@@ -1041,7 +1038,7 @@ enforce_sparse_kernel(PostArgs a, const unsigned *__restrict__ list, const unsig
 // A round over a worklist whose length is on the device (*nw_dev), in a
 // grid-stride loop over a grid of any size (no barrier inside).
 template <int PASS, int ND>
-__global__ void __launch_bounds__(kPostThreads)
+__global__ void __launch_bounds__(kPostThreads, 2)
 pass_round_dev_kernel(PostArgs a, const unsigned *__restrict__ list, const unsigned *__restrict__ W,
                       const unsigned *nw_dev, unsigned *__restrict__ Wn, unsigned *wn_count) {
   const unsigned nw = *nw_dev;
@@ -1053,7 +1050,7 @@ pass_round_dev_kernel(PostArgs a, const unsigned *__restrict__ list, const unsig
   for (unsigned base = blockIdx.x * blockDim.x; base < nw; base += stride) {
     const unsigned i = base + threadIdx.x;
     unsigned idx = 0;
-    if (i < nw) idx = W[i];
+    if (i < nw) idx = W ? W[i] : i;
     const bool defer = pass_item_local<PASS, ND>(a, list, idx, i < nw, polls);
     const unsigned m = __ballot_sync(0xffffffffu, defer);
     unsigned wb = 0;
@@ -1173,9 +1170,17 @@ pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, const unsigned *
   (void)tot;
 }
 
-__global__ void types_from_int_kernel(const int *__restrict__ fn, unsigned char *__restrict__ T, long long n) {
+// bit planes of the types, from an int or a byte per point (a warp per word)
+template <class V>
+__global__ void type_planes_kernel(const V *__restrict__ fn, long long n, unsigned *__restrict__ TL,
+                                   unsigned *__restrict__ TH) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) T[i] = (unsigned char)(fn[i] & 3);
+  const unsigned t = i < n ? (unsigned)fn[i] : 0u;
+  const unsigned lo = __ballot_sync(0xffffffffu, t & 1u), hi = __ballot_sync(0xffffffffu, t & 2u);
+  if ((threadIdx.x & 31) == 0 && i < n) {
+    TL[i >> 5] = lo;
+    TH[i >> 5] = hi;
+  }
 }
 
 static bool g_weights_ready[64];
@@ -1204,9 +1209,9 @@ static cudaError_t upload_weights(int dev) {
 size_t post_scratch_bytes(unsigned long long n) {
   const unsigned long long ntiles = (n + kPostTile - 1) / kPostTile;
   const unsigned long long words = (n + 31) / 32;
-  // T, descriptors, RBF + extrema bitmaps + extremum word positions, lists X
-  // and Z, worklists (2), Y, raw values of X and Z
-  return a256(n) + a256((ntiles + 1) * sizeof(TileDesc)) + 3 * a256(words * 4 + 4) + 7 * a256(n * 4) + 8192;
+  // type planes, descriptors, RBF + extrema + saddle bitmaps + extremum word
+  // positions, lists X and Z, worklists (2), Y, raw values of X and Z
+  return a256((ntiles + 1) * sizeof(TileDesc)) + 6 * a256(words * 4 + 4) + 7 * a256(n * 4) + 8192;
 }
 
 
@@ -1255,6 +1260,22 @@ static int coop_grid(szp_b200_ctx *ctx) {
     }
   }
   return grid_for_dev[dev] > 0 ? grid_for_dev[dev] : 0;
+}
+
+// CTAs of a round over a list of device-known length that are resident at once
+template <int PASS, int ND>
+static int dev_grid(szp_b200_ctx *ctx) {
+  static int per_sm_for_dev[64];
+  const int dev = ctx->device;
+  if (dev < 0 || dev >= 64) return ctx->sm_count;
+  if (per_sm_for_dev[dev] == 0) {
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pass_round_dev_kernel<PASS, ND>, kPostThreads, 0) !=
+        cudaSuccess)
+      cudaGetLastError();
+    per_sm_for_dev[dev] = nb > 0 ? nb : 1;
+  }
+  return per_sm_for_dev[dev] * ctx->sm_count;
 }
 
 // Rounds over deferred items as ordinary launches, kBurstRounds of them
@@ -1321,7 +1342,7 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
     enforce_sparse_kernel<ND><<<(ni_words + kSparseWords - 1) / kSparseWords, kPostThreads, 0, s>>>(
         a, list, ni_bits, ni_words, W0, n0);
   else if (count_dev)
-    pass_round_dev_kernel<PASS, ND><<<ctx->sm_count * 2, kPostThreads, 0, s>>>(a, list, sel, count_dev, W0, n0);
+    pass_round_dev_kernel<PASS, ND><<<dev_grid<PASS, ND>(ctx), kPostThreads, 0, s>>>(a, list, sel, count_dev, W0, n0);
   else
     pass_round_kernel<PASS, ND><<<(count + kPostThreads - 1) / kPostThreads, kPostThreads, 0, s>>>(
         a, list, sel, count, W0, n0);
@@ -1357,13 +1378,13 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
 template <int ND>
 static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned nx, unsigned *Z, unsigned nz,
                           unsigned *Y, unsigned *W0, unsigned *W1, unsigned *R,
-                          const unsigned *Eb, float *OX, const float *OZ,
+                          const unsigned *Eb, const unsigned *Sb, float *OX, const float *OZ,
                           int axis_stencil, bool raw_in_F) {
   cudaStream_t s = ctx->stream;
   const long long n = a.n;
-  // raw_in_F: OX / OZ were not gathered; OX keeps the raw values of the
-  // items the fused stencil leaves for enforcement
-  a.OL = raw_in_F ? nullptr : OX;
+  // raw_in_F: OX keeps the raw values of the items the fused stencil leaves
+  // for enforcement
+  a.OL = nullptr;
   a.RAW = nullptr;
   a.X = Eb;
   if (a.sp && a.n_sp > 0) {
@@ -1379,7 +1400,7 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
     if (run_pass<kPassStencil, ND>(ctx, a, X, nullptr, nx, nullptr, W0, W1)) return -1;
     a.NI = nullptr;
     a.RAW = nullptr;
-    a.OL = OX;   // raw values of the remaining items (gathered, or stashed by the stencil)
+    a.OL = raw_in_F ? OX : nullptr;   // raw values of the remaining items, stashed by the stencil
     tl_mark(ctx, "post_stencil");
     a.gen = next_gen(ctx);
     if (run_pass<kPassEnforce, ND>(ctx, a, X, nullptr, 0, nullptr, W0, W1, NIb, ni_words)) return -1;
@@ -1395,19 +1416,18 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
   unsigned *ycnt = reinterpret_cast<unsigned *>(ctx->d_words + 8);
   if (cuda_fail(cudaMemsetAsync(ycnt, 0, 4, s), "memset")) return -1;
   a.R = R;
-  if (nz) fn_detect_kernel<<<(nz + 255) / 256, 256, 0, s>>>(a, Z, nz, R, Y, ycnt);
+  if (nz) fn_detect_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(a, Sb, (unsigned)words, R, Y, ycnt);
   ctx->launches += nz ? 1 : 0;
   if (cuda_fail(cudaGetLastError(), "fn detect")) return -1;
   tl_mark(ctx, "post_fn_locks");
-  // RBF runs over Z restricted to the lost saddles (Y holds indices into Z);
-  // their number stays on the device.  Saddles keep their raw values until
-  // RBF itself writes them.
-  a.OL = raw_in_F ? nullptr : OZ;
+  // RBF runs over the lost saddles Y; their number stays on the device.
+  // Saddles keep their raw values until RBF itself writes them.
+  a.OL = nullptr;
   a.gen = next_gen(ctx);
-  if (nz && run_pass<kPassRbf, ND>(ctx, a, Z, Y, 0, ycnt, W0, W1)) return -1;
+  if (nz && run_pass<kPassRbf, ND>(ctx, a, Y, nullptr, 0, ycnt, W0, W1)) return -1;
   tl_mark(ctx, "post_rbf");
   if (axis_stencil && ND == 3 && nz) {
-    a.OL = OZ;   // gathered in every mode: RBF has changed some saddles
+    a.OL = raw_in_F ? OZ : nullptr;   // gathered before the passes: RBF has changed some saddles
     a.gen = next_gen(ctx);
     if (run_pass<kPassAxis, ND>(ctx, a, Z, nullptr, nz, nullptr, W0, W1)) return -1;
     tl_mark(ctx, "post_axis");
@@ -1415,8 +1435,8 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
   return 0;
 }
 
-int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, unsigned char *d_T,
-                     unsigned long long *d_S, TileDesc *desc, const int *d_sp,
+int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const unsigned *d_TL,
+                     const unsigned *d_TH, unsigned long long *d_S, TileDesc *desc, const int *d_sp,
                      unsigned long long n_sp, const Geom &g, float eb, int axis_stencil, int *restored_out) {
   const long long n = g.d1 * g.d2 * g.d3;
   if (g.d2 < 3 || g.d3 < 3 || (g.nd == 3 && g.d1 < 3)) { if (restored_out) *restored_out = 0; return 0; }
@@ -1430,19 +1450,15 @@ int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, unsi
   unsigned *W0 = A.take<unsigned>(n), *W1 = A.take<unsigned>(n);
   unsigned *R = A.take<unsigned>((n + 31) / 32);
   unsigned *Eb = A.take<unsigned>((n + 31) / 32 + 1);
+  unsigned *Sb = A.take<unsigned>((n + 31) / 32 + 1);
   unsigned *XP = A.take<unsigned>((n + 31) / 32 + 1);
   float *OX = A.take<float>(n), *OZ = A.take<float>(n);
-  if (!X || !Z || !Y || !W0 || !W1 || !R || !Eb || !XP || !OX || !OZ) {
+  if (!X || !Z || !Y || !W0 || !W1 || !R || !Eb || !Sb || !XP || !OX || !OZ) {
     set_error("scratch arena too small for post-processing");
     return -1;
   }
   unsigned long long *w = ctx->d_words;  // [9] pass status, [10] round counters
   if (cuda_fail(cudaMemsetAsync(w, 0, 96, s), "memset")) return -1;
-  {
-    // the words past the last written byte of the bitmap must read as zero
-    const long long words = (n + 31) / 32;
-    if (cuda_fail(cudaMemsetAsync(Eb + words - 1, 0, 8, s), "memset")) return -1;
-  }
   unsigned *tile_ctr = reinterpret_cast<unsigned *>(w + 3);
   unsigned long long *d_tot = w + 2;
   const long long ltiles = (n + kListTile - 1) / kListTile;
@@ -1454,10 +1470,8 @@ int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, unsi
   const bool axis_raw = axis_stencil && g.nd == 3;
   {
     const unsigned grid = (unsigned)std::min<long long>(ltiles, (long long)ctx->sm_count * 6);
-    list_build_kernel<<<grid, kPostThreads, 0, s>>>(d_T, g, n, desc, tile_ctr, reinterpret_cast<int *>(w + 4), X,
-                                                    Z, reinterpret_cast<unsigned char *>(Eb), d_tot,
-                                                    raw_in_F ? nullptr : d_orig,
-                                                    raw_in_F && !axis_raw ? nullptr : d_orig, OX, OZ, XP);
+    list_build_kernel<<<grid, kPostThreads, 0, s>>>(d_TL, d_TH, g, n, desc, tile_ctr, reinterpret_cast<int *>(w + 4),
+                                                    X, axis_raw ? Z : nullptr, Eb, Sb, d_tot, XP);
   }
   ctx->launches += 1;
   unsigned long long tot = 0;
@@ -1466,10 +1480,16 @@ int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, unsi
       cuda_fail(cudaStreamSynchronize(s), "lists"))
     return -1;
   const unsigned nx = (unsigned)(tot >> 32), nz = (unsigned)(tot & 0xffffffffull);
+  if (axis_raw && raw_in_F && nz) {
+    gather_kernel<<<(nz + 255) / 256, 256, 0, s>>>(Z, nz, d_data, OZ);
+    ctx->launches += 1;
+  }
   tl_mark(ctx, "post_lists");
   PostArgs a{};
   a.F = d_data;
-  a.T = d_T;
+  a.TL = d_TL;
+  a.TH = d_TH;
+  a.ORIG = raw_in_F ? nullptr : d_orig;
   a.sp = d_sp;
   a.n_sp = d_sp ? n_sp : 0;
   a.g = g;
@@ -1481,9 +1501,9 @@ int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, unsi
   a.err = reinterpret_cast<int *>(w + 4);
   a.restored = reinterpret_cast<unsigned *>(w + 5);
   const int rc = (g.nd == 2)
-                     ? run_all_passes<2>(ctx, a, X, nx, Z, nz, Y, W0, W1, R, Eb, OX, OZ, axis_stencil,
+                     ? run_all_passes<2>(ctx, a, X, nx, Z, nz, Y, W0, W1, R, Eb, Sb, OX, OZ, axis_stencil,
                                          raw_in_F)
-                     : run_all_passes<3>(ctx, a, X, nx, Z, nz, Y, W0, W1, R, Eb, OX, OZ, axis_stencil,
+                     : run_all_passes<3>(ctx, a, X, nx, Z, nz, Y, W0, W1, R, Eb, Sb, OX, OZ, axis_stencil,
                                          raw_in_F);
   if (rc) return -1;
   if (cuda_fail(cudaMemcpyAsync(ctx->h_words, w, 96, cudaMemcpyDeviceToHost, s), "D2H") ||
@@ -1529,25 +1549,35 @@ int selftest_grid_barrier(int spin_limit, int *status, float *ms) {
   return rc;
 }
 
-int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig,
-                const unsigned char *d_types_u8, const int *d_types_i, const int *d_sp,
+bool post_planes(szp_b200_ctx *ctx, unsigned long long n, unsigned **TL, unsigned **TH) {
+  *TL = ctx->scratch.take<unsigned>((n + 31) / 32 + 1);
+  *TH = ctx->scratch.take<unsigned>((n + 31) / 32 + 1);
+  return *TL && *TH;
+}
+
+int post_planes_from_bytes(szp_b200_ctx *ctx, const unsigned char *d_T, unsigned long long n, unsigned *TL,
+                           unsigned *TH) {
+  type_planes_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(d_T, (long long)n, TL, TH);
+  ctx->launches += 1;
+  return cuda_fail(cudaGetLastError(), "type planes") ? -1 : 0;
+}
+
+int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const int *d_types_i, const int *d_sp,
                 unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
                 int *restored_out) {
   const long long n = g.d1 * g.d2 * g.d3;
   Arena &A = ctx->scratch;
   unsigned long long *S = post_words(ctx, (unsigned long long)n);
-  unsigned char *T = A.take<unsigned char>(n);
+  unsigned *TL, *TH;
   const unsigned long long ntiles = (n + kPostTile - 1) / kPostTile;
   TileDesc *desc = A.take<TileDesc>(ntiles + 1);
-  if (!S || !T || !desc) { set_error("scratch arena too small for post-processing"); return -1; }
-  cudaStream_t s = ctx->stream;
-  if (d_types_i) {
-    types_from_int_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_types_i, T, n);
-    ctx->launches += 1;
-  } else if (cuda_fail(cudaMemcpyAsync(T, d_types_u8, n, cudaMemcpyDeviceToDevice, s), "copy types")) {
+  if (!S || !desc || !post_planes(ctx, n, &TL, &TH)) {
+    set_error("scratch arena too small for post-processing");
     return -1;
   }
-  return postprocess_with(ctx, d_data, d_orig, T, S, desc, d_sp, n_sp, g, eb, axis_stencil, restored_out);
+  type_planes_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(d_types_i, n, TL, TH);
+  ctx->launches += 1;
+  return postprocess_with(ctx, d_data, d_orig, TL, TH, S, desc, d_sp, n_sp, g, eb, axis_stencil, restored_out);
 }
 
 }  // namespace tsz
