@@ -868,7 +868,7 @@ __device__ __forceinline__ int face_item_run(const PostArgs &a, unsigned idx, Fa
 // lanes look together and the ready ones compute in between: an item often
 // waits for one in a neighbouring lane, which must not wait for it in turn at
 // the end of a loop of its own (1.2 K lost saddles of a 100 x 500 x 500 field
-// in chains: 315 us when it did, @@RBF@@ now).
+// in chains: 315 us when it did, 109 now).
 template <int PASS, int ND>
 __device__ __forceinline__ bool pass_items(const PostArgs &a, const unsigned *__restrict__ list, unsigned idx,
                                            bool valid, int polls) {
