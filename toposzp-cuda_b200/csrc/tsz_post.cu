@@ -97,6 +97,7 @@ struct PostArgs {
   // stencil pass fused with enforcement (null: plain stencil pass): bitmap
   // over list positions of the items that still need the enforcement pass
   unsigned *NI;
+  const unsigned *ONLY;         // the whole pass in one cooperative launch: bitmap of the list positions it runs (null: all)
 };
 
 // No "memory" clobber: a result word is read whole and carries its own
@@ -836,7 +837,6 @@ __device__ __forceinline__ float stencil_nd(const PostArgs &a, const Face &f, fl
 // runs over them alone.
 template <int PASS, int ND>
 __device__ __forceinline__ int face_item_run(const PostArgs &a, unsigned idx, FaceItem &it) {
-  if (!face_item_ready(a, it)) return kItemDeferred;
   const long long e = it.e;
   float r;
   int st = kItemDone;
@@ -908,34 +908,34 @@ __device__ __forceinline__ bool pass_items(const PostArgs &a, const unsigned *__
   return pending;
 }
 
-// An item whose earlier candidate is handled by the same CTA at the same
-// time (the previous point of a row, or of the previous row) would be
-// deferred to the next round; the CTA instead retries its pending items a
-// few times, a block barrier apart, so that chains inside the CTA resolve in
-// this round.  Every thread of the CTA must call it.  Returns true while the
-// item is still pending.  In the fused stencil pass, the items left for the
+// One item per lane of a warp that calls it whole; true while the item is
+// still pending.  Its state is loaded once; then the warp looks at the missing
+// results of all its items and runs the ready ones, again while that unblocks
+// others (an item often waits for one in a neighbouring lane), and otherwise
+// up to polls times.  In the fused stencil pass, the items left for the
 // enforcement pass are marked in the a.NI bitmap here (one atomic per warp
 // when the warp's items share a bitmap word, as in a round over the whole
 // list).
-constexpr int kLocalRetries = 5;
+constexpr int kShortPolls = 6;   // rounds whose items are not all in flight
 
 template <int PASS, int ND>
 __device__ __forceinline__ bool pass_item_local(const PostArgs &a, const unsigned *__restrict__ list, unsigned idx,
-                                                bool valid, int polls = 0) {
-  // RBF and axis-pattern items are long and uneven: a block barrier would make
-  // every thread wait for the slowest, so they wait for missing results on
-  // their own (bounded, polls) or retry in rounds
+                                                bool valid, int polls) {
   if (PASS != kPassStencil && PASS != kPassEnforce) return pass_items<PASS, ND>(a, list, idx, valid, polls);
   bool pending = valid, need = false;
   FaceItem item;
   if (valid) face_item_load<PASS, ND>(a, list, idx, item);
-  for (int it = 0; it < kLocalRetries; it++) {
-    if (pending) {
-      const int st = face_item_run<PASS, ND>(a, idx, item);
-      pending = st == kItemDeferred;
-      need = need || st == kItemNeedsEnforce;
+  for (int p = 0;; p++) {
+    const bool ready = pending && face_item_ready(a, item);
+    if (ready) {
+      need = face_item_run<PASS, ND>(a, idx, item) == kItemNeedsEnforce;
+      pending = false;
     }
-    if (!__syncthreads_or(pending)) break;
+    if (!__any_sync(0xffffffffu, pending)) break;
+    if (!__any_sync(0xffffffffu, ready)) {
+      if (p >= polls) break;
+      if (p >= kShortPolls) __nanosleep(p < 64 ? 32 : 256);
+    }
   }
   if (PASS == kPassStencil && a.NI) {
     const unsigned m = __ballot_sync(0xffffffffu, need);
@@ -967,7 +967,7 @@ pass_round_kernel(PostArgs a, const unsigned *__restrict__ list, const unsigned 
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned idx = 0;
   if (i < nw) idx = W ? W[i] : i;
-  const bool defer = pass_item_local<PASS, ND>(a, list, idx, i < nw);
+  const bool defer = pass_item_local<PASS, ND>(a, list, idx, i < nw, kShortPolls);
   const unsigned m = __ballot_sync(0xffffffffu, defer);
   const int lane = threadIdx.x & 31;
   unsigned base = 0;
@@ -1026,7 +1026,7 @@ enforce_sparse_kernel(PostArgs a, const unsigned *__restrict__ list, const unsig
     const unsigned i = base + threadIdx.x;
     const bool valid = i < total;
     const unsigned idx = valid ? s_idx[i] : 0u;
-    const bool defer = pass_item_local<kPassEnforce, ND>(a, list, idx, valid);
+    const bool defer = pass_item_local<kPassEnforce, ND>(a, list, idx, valid, kShortPolls);
     const unsigned m = __ballot_sync(0xffffffffu, defer);
     unsigned wb = 0;
     if (lane == 0 && m) wb = atomicAdd(wn_count, (unsigned)__popc(m));
@@ -1045,7 +1045,9 @@ pass_round_dev_kernel(PostArgs a, const unsigned *__restrict__ list, const unsig
   const int lane = threadIdx.x & 31;
   const unsigned stride = gridDim.x * blockDim.x;
   // every item of the round in flight at once: an item may wait for the
-  // earlier ones it reads, which are being computed beside it
+  // earlier ones it reads, which are being computed beside it.  Otherwise one
+  // look: the RBF stage of 1800x3600 is 75 us
+  // so, 95 when a warp looks six times and goes on while a lane is ready.
   const int polls = nw <= stride ? kDepPolls : 0;
   for (unsigned base = blockIdx.x * blockDim.x; base < nw; base += stride) {
     const unsigned i = base + threadIdx.x;
@@ -1128,7 +1130,7 @@ pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, const unsigned *
                  const unsigned *total_dev, const unsigned *W_start, const unsigned *nstart_dev, unsigned *Wx,
                  unsigned *Wy, unsigned *cnts, unsigned *bar, unsigned long long *status) {
   const unsigned tot = total_dev ? __ldcg(total_dev) : total;
-  const unsigned *W = W_start ? W_start : sel;
+  const unsigned *W = W_start ? W_start : sel;   // null: list positions themselves
   unsigned nw = W_start ? __ldcg(nstart_dev) : tot;
   const bool after_round0 = W_start != nullptr;
   int b = 0;
@@ -1150,7 +1152,8 @@ pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, const unsigned *
       const unsigned i = base + threadIdx.x;
       unsigned idx = 0;
       if (i < nw) idx = W ? __ldcg(W + i) : i;
-      const bool defer = pass_item_local<PASS, ND>(a, list, idx, i < nw, nw <= stride ? kDepPolls : 0);
+      const bool defer = pass_item_local<PASS, ND>(a, list, idx, i < nw && (!a.ONLY || bit_at(a.ONLY, idx)),
+                                                   nw <= stride ? kDepPolls : kShortPolls);
       const unsigned m = __ballot_sync(0xffffffffu, defer);
       unsigned wb = 0;
       if (lane == 0 && m) wb = atomicAdd(cnt, (unsigned)__popc(m));
@@ -1322,11 +1325,14 @@ static int finish_rounds(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, u
 // enforcement after the fused stencil) -- then the rounds over the deferred
 // items: in one cooperative launch that reads its counts on the device (after
 // one more ordinary round when round 0 ran over a list), or as bursts of
-// ordinary launches (finish_rounds).
+// ordinary launches (finish_rounds).  most: a bound of the items known on the
+// host; when all of them fit the cooperative grid at once, one launch runs the
+// whole pass (60x90, the stencil 22 -> 13 us, enforcement 19 -> 10, RBF 18 ->
+// 14: such a field spends its time on launches).
 template <int PASS, int ND>
 static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const unsigned *sel, unsigned count,
-                    const unsigned *count_dev, unsigned *W0, unsigned *W1, const unsigned *ni_bits = nullptr,
-                    unsigned ni_words = 0) {
+                    unsigned most, const unsigned *count_dev, unsigned *W0, unsigned *W1,
+                    const unsigned *ni_bits = nullptr, unsigned ni_words = 0) {
   if (ni_bits ? ni_words == 0 : (!count_dev && count == 0)) return 0;
   const int grid = coop_grid<PASS, ND>(ctx);
   cudaStream_t s = ctx->stream;
@@ -1337,6 +1343,23 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
   unsigned *bar = cnts + 3;
   unsigned *n1 = cnts + 6;
   unsigned long long *status = ctx->d_words + 9;
+  const unsigned zero = 0;
+  const unsigned *no_total = nullptr;
+  if (grid && most <= (unsigned)grid * kPostThreads) {
+    // every item in flight at once: one launch, no worklist to start from
+    if (cuda_fail(cudaMemsetAsync(cnts, 0, 32, s), "memset")) return -1;
+    const unsigned *none = nullptr;
+    a.ONLY = ni_bits;
+    void *args[] = {(void *)&a,    (void *)&list, (void *)&none, (void *)&most, (void *)(count_dev ? &count_dev : &no_total),
+                    (void *)&none, (void *)&none, (void *)&W0,   (void *)&W1,   (void *)&cnts,
+                    (void *)&bar,  (void *)&status};
+    const unsigned need = (most + kPostThreads - 1) / kPostThreads;
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)pass_coop_kernel<PASS, ND>,
+                                                      dim3(need ? need : 1), dim3(kPostThreads), args, 0, s);
+    a.ONLY = nullptr;
+    ctx->launches += 1;
+    return cuda_fail(e, "cooperative pass launch") ? -1 : 0;
+  }
   if (cuda_fail(cudaMemsetAsync(n0, 0, 4, s), "memset")) return -1;
   if (ni_bits)
     enforce_sparse_kernel<ND><<<(ni_words + kSparseWords - 1) / kSparseWords, kPostThreads, 0, s>>>(
@@ -1362,8 +1385,6 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
     Wx = W0;
     Wy = W1;
   }
-  const unsigned zero = 0;
-  const unsigned *no_total = nullptr;
   void *args[] = {(void *)&a,       (void *)&list,   (void *)&sel, (void *)&zero, (void *)&no_total,
                   (void *)&W_start, (void *)&nstart, (void *)&Wx,  (void *)&Wy,   (void *)&cnts,
                   (void *)&bar,     (void *)&status};
@@ -1397,16 +1418,16 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
     a.gen = next_gen(ctx);
     a.NI = NIb;
     a.RAW = raw_in_F ? OX : nullptr;
-    if (run_pass<kPassStencil, ND>(ctx, a, X, nullptr, nx, nullptr, W0, W1)) return -1;
+    if (run_pass<kPassStencil, ND>(ctx, a, X, nullptr, nx, nx, nullptr, W0, W1)) return -1;
     a.NI = nullptr;
     a.RAW = nullptr;
     a.OL = raw_in_F ? OX : nullptr;   // raw values of the remaining items, stashed by the stencil
     tl_mark(ctx, "post_stencil");
     a.gen = next_gen(ctx);
-    if (run_pass<kPassEnforce, ND>(ctx, a, X, nullptr, 0, nullptr, W0, W1, NIb, ni_words)) return -1;
+    if (run_pass<kPassEnforce, ND>(ctx, a, X, nullptr, 0, nx, nullptr, W0, W1, NIb, ni_words)) return -1;
   } else {
     a.gen = next_gen(ctx);
-    if (run_pass<kPassEnforce, ND>(ctx, a, X, nullptr, nx, nullptr, W0, W1)) return -1;
+    if (run_pass<kPassEnforce, ND>(ctx, a, X, nullptr, nx, nx, nullptr, W0, W1)) return -1;
   }
   tl_mark(ctx, "post_enforce");
   // the lost saddles (from F after enforcement); RBF reads the locks from the
@@ -1424,12 +1445,12 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
   // Saddles keep their raw values until RBF itself writes them.
   a.OL = nullptr;
   a.gen = next_gen(ctx);
-  if (nz && run_pass<kPassRbf, ND>(ctx, a, Y, nullptr, 0, ycnt, W0, W1)) return -1;
+  if (nz && run_pass<kPassRbf, ND>(ctx, a, Y, nullptr, 0, nz, ycnt, W0, W1)) return -1;
   tl_mark(ctx, "post_rbf");
   if (axis_stencil && ND == 3 && nz) {
     a.OL = raw_in_F ? OZ : nullptr;   // gathered before the passes: RBF has changed some saddles
     a.gen = next_gen(ctx);
-    if (run_pass<kPassAxis, ND>(ctx, a, Z, nullptr, nz, nullptr, W0, W1)) return -1;
+    if (run_pass<kPassAxis, ND>(ctx, a, Z, nullptr, nz, nz, nullptr, W0, W1)) return -1;
     tl_mark(ctx, "post_axis");
   }
   return 0;
