@@ -7,8 +7,12 @@
 //   * a value past a block's last delta is decoded from whatever follows it and
 //     goes nowhere (it could only reach elements that do not exist), so no value
 //     has a bound check of its own;
-//   * the remainder fields of an octet are a 64-bit big-endian window, shifted
-//     left by one field a value;
+//   * the remainder fields of an octet are a 64-bit big-endian window, four
+//     fields in each of two words, moved to the top by a multiply;
+//   * a block's offsets, length, bit count and checks are worked out by one
+//     lane of the CTA's first warp, not by the eight that decode it, and a CTA
+//     of full blocks has no length of its own anywhere (512^3: 316 -> 262 us
+//     for the stage, ALU pipe 76 % busy before);
 //   * signs multiply: q[t + 1] = q[t] + magnitude * (+1 or -1), one multiply-add
 //     per value on the FMA pipe, which also is the octet's prefix sum;
 //   * blocks with full magnitude bytes beyond one take the byte loop.
@@ -32,22 +36,162 @@ __device__ __forceinline__ void ld_window(const unsigned *imgw, unsigned p, unsi
   hi = __funnelshift_r(b, c, sh);
 }
 
+// x >> n for n <= 32 (zero at 32)
+__device__ __forceinline__ unsigned shr_clamp(unsigned x, unsigned n) {
+  unsigned r;
+  asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
+  return r;
+}
+
+constexpr unsigned kD64Ok = 0x10000u;
+
+// A block as its warp of the CTA found it: x: image position of its block, y:
+// anchor, z: image position of its types, w: bit count, kD64Ok.
+// FULL: the block has 64 elements.
+template <bool TAGS, bool FULL>
+__device__ __forceinline__ unsigned d64_octet(const DecArgs &a, const unsigned char *img, const uint4 &h,
+                                              long long base, int len, int l) {
+  const unsigned *imgw = reinterpret_cast<const unsigned *>(img);
+  const bool ok = (h.w & kD64Ok) != 0;
+  const unsigned bc = h.w & 0xffu;
+  const int e0 = 8 * l;
+  const int nv = FULL ? 8 : (len - e0 < 0 ? 0 : (len - e0 > 8 ? 8 : len - e0));
+  const unsigned cnt = FULL ? 63u : (len > 0 ? (unsigned)len - 1u : 0u);
+  // q[t]: sum of the octet's deltas before element t; q[8]: of all of them
+  int q[9];
+#pragma unroll
+  for (int t = 0; t < 9; t++) q[t] = 0;
+  if (ok && bc && (FULL || (unsigned)e0 < cnt)) {
+    const unsigned p = h.x + 5u, sbytes = (cnt + 7u) >> 3;
+    const unsigned neg = (unsigned)img[p + l] << 24;     // sign of delta e0 + t at bit 31 - t
+    const unsigned mag = p + sbytes, fb = bc >> 3, rem = bc & 7u;
+    // rem bytes at byte l rem of the remainder section, most significant bits
+    // first: fields 0 .. 3 on top of w0, 4 .. 7 of w1 (28 bits or fewer each)
+    unsigned rl, rh;
+    ld_window(imgw, mag + fb * cnt + (unsigned)l * rem, rl, rh);
+    const unsigned w0 = __byte_perm(rl, 0u, 0x0123);
+    const unsigned w1 = __funnelshift_l(__byte_perm(rh, 0u, 0x0123), w0, 4u * rem);
+    const unsigned down = 32u - rem, up = 1u << rem;     // no field when rem is 0: a shift by 32
+    const unsigned ups[4] = {1u, up, up * up, up * up * up};
+    if (fb <= 1) {
+      unsigned fl = 0, fh = 0;
+      if (fb) ld_window(imgw, mag + (unsigned)e0, fl, fh);
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        const unsigned full = __byte_perm(t < 4 ? fl : fh, 0u, 0x4440u + (unsigned)(t & 3));
+        const unsigned m = full * up + shr_clamp((t < 4 ? w0 : w1) * ups[t & 3], down);
+        q[t + 1] = (int)(m * (unsigned)(((int)(neg << t) >> 31) | 1) + (unsigned)q[t]);
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        unsigned full = 0;
+        if ((unsigned)(e0 + t) < cnt) {
+          const unsigned o = mag + (unsigned)(e0 + t) * fb;
+          for (unsigned u = 0; u < fb; u++) full |= (unsigned)img[o + u] << (8u * u);
+        }
+        const unsigned m = full * up + shr_clamp((t < 4 ? w0 : w1) * ups[t & 3], down);
+        q[t + 1] = (int)(m * (unsigned)(((int)(neg << t) >> 31) | 1) + (unsigned)q[t]);
+      }
+    }
+  }
+  // exclusive scan of the octet sums over the block's lanes
+  int inc = q[8];
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o, 8);
+    if (l >= o) inc = (int)((unsigned)inc + (unsigned)u);
+  }
+  if (!ok || nv == 0) return 0u;
+  const int v0 = (int)(h.y + (unsigned)inc - (unsigned)q[8]);
+#pragma unroll
+  for (int t = 0; t < 8; t++) q[t] = (int)((unsigned)q[t] + (unsigned)v0);
+  const long long i0 = base + e0;
+  if (a.out_f) {
+    float f[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) f[t] = __fmul_rn((float)q[t], a.eb);
+    // i0 is a multiple of 8: the array's alignment decides
+    if (nv == 8 && ((reinterpret_cast<uintptr_t>(a.out_f) & 15) == 0)) {
+      reinterpret_cast<float4 *>(a.out_f + i0)[0] = make_float4(f[0], f[1], f[2], f[3]);
+      reinterpret_cast<float4 *>(a.out_f + i0)[1] = make_float4(f[4], f[5], f[6], f[7]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < 8; t++) if (t < nv) a.out_f[i0 + t] = f[t];
+    }
+  }
+  if (!TAGS && a.out_i) {
+    if (nv == 8 && ((reinterpret_cast<uintptr_t>(a.out_i) & 15) == 0)) {
+      reinterpret_cast<int4 *>(a.out_i + i0)[0] = make_int4(q[0], q[1], q[2], q[3]);
+      reinterpret_cast<int4 *>(a.out_i + i0)[1] = make_int4(q[4], q[5], q[6], q[7]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < 8; t++) if (t < nv) a.out_i[i0 + t] = q[t];
+    }
+  }
+  if (!TAGS) return 0u;
+  const unsigned tb = FULL ? 16u : ((unsigned)len + 3u) / 4u;
+  // element 0 in the top two of 16 bits; elements past nv as regular points
+  unsigned tg = ((FULL || 2u * l < tb) ? (unsigned)img[h.z + 2 * l] << 8 : 0u) |
+                ((FULL || 2u * l + 1u < tb) ? (unsigned)img[h.z + 2 * l + 1] : 0u);
+  if (!FULL && nv < 8) tg &= 0xffffu << (16 - 2 * nv);
+  if (a.pl_lo) {
+    // element t to bit t: low bits compacted in the lower half, high bits in
+    // the upper, element 0 on top; all reversed
+    unsigned x = (tg & 0x5555u) | ((tg & 0xaaaau) << 15);
+    x = (x | (x >> 1)) & 0x33333333u;
+    x = (x | (x >> 2)) & 0x0f0f0f0fu;
+    x = __brev((x | (x >> 4)) & 0x00ff00ffu);
+    const long long o = i0 >> 3;
+    a.pl_lo[o] = (unsigned char)(x >> 24);
+    a.pl_hi[o] = (unsigned char)(x >> 8);
+    // the rest of the planes' last word
+    if (!FULL && i0 + 8 >= (long long)a.n)
+      for (long long k = o + 1; k & 3; k++) a.pl_lo[k] = a.pl_hi[k] = 0;
+  }
+  if (a.fn_u8) {
+    if (nv == 8 && ((reinterpret_cast<uintptr_t>(a.fn_u8) & 7) == 0)) {
+      // four two-bit fields of a byte, most significant first, to four bytes
+      unsigned w[2];
+#pragma unroll
+      for (int hf = 0; hf < 2; hf++) {
+        const unsigned x = hf ? tg & 0xffu : tg >> 8;
+        const unsigned y = (x | (x << 12)) & 0x000f000fu;        // low nibble, high nibble << 16
+        const unsigned z = (y | (y << 6)) & 0x03030303u;         // fields 3, 2 (low to high byte), 1, 0
+        w[hf] = __byte_perm(z, 0u, 0x0123);
+      }
+      *reinterpret_cast<uint2 *>(a.fn_u8 + i0) = make_uint2(w[0], w[1]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < 8; t++) if (t < nv) a.fn_u8[i0 + t] = (unsigned char)((tg >> (14 - 2 * t)) & 3u);
+    }
+  }
+  if (a.fn_i) {
+#pragma unroll
+    for (int t = 0; t < 8; t++) if (t < nv) a.fn_i[i0 + t] = (int)((tg >> (14 - 2 * t)) & 3u);
+  }
+  return (unsigned)__popc((tg ^ (tg >> 1)) & 0x5555u);   // types 01 and 10
+}
+
 template <bool TAGS>
 __global__ void __launch_bounds__(kD64Threads, 6) decode64_kernel(DecArgs a) {
   __shared__ __align__(16) unsigned char img[d64_img_bytes(TAGS) + 32];
-  __shared__ unsigned long long s_off[kD64Blocks + 1];
+  __shared__ uint4 s_hd[kD64Blocks];
   const int tid = threadIdx.x, l = tid & 7, bi = tid >> 3;
   const long long n = (long long)a.n;
   const long long nblocks = (n + 63) / 64;
   const long long b0 = (long long)blockIdx.x * kD64Blocks;
   const int nb = (int)((nblocks - b0) < kD64Blocks ? (nblocks - b0) : kD64Blocks);
-  if (tid <= nb) s_off[tid] = b0 + tid < nblocks ? a.blk_off[b0 + tid] : a.payload_len;
-  __syncthreads();
   // the image holds the payload bytes from the 16-byte boundary at or below
   // payload + lo: img[ib + k] is payload[lo + k]
-  const unsigned long long lo = s_off[0];
-  unsigned long long hi = s_off[nb];
-  if (hi > a.payload_len) hi = a.payload_len;
+  const unsigned long long lo = a.blk_off[b0];
+  const unsigned long long end = b0 + nb < nblocks ? a.blk_off[b0 + nb] : a.payload_len;
+  const unsigned long long hi = end > a.payload_len ? a.payload_len : end;
+  unsigned long long o0 = 0, o1 = 0;
+  if (tid < nb) {
+    o0 = a.blk_off[b0 + tid];
+    o1 = b0 + tid + 1 < nblocks ? a.blk_off[b0 + tid + 1] : a.payload_len;
+  }
   if (lo > hi || hi - lo > d64_img_bytes(TAGS) - 48u) {
     if (tid == 0) atomicExch(a.err, kErrMalformed);
     return;
@@ -58,11 +202,14 @@ __global__ void __launch_bounds__(kD64Threads, 6) decode64_kernel(DecArgs a) {
     const uintptr_t pb = reinterpret_cast<uintptr_t>(a.payload), pe = pb + a.payload_len;
     const uintptr_t g16 = pb + lo - ib;
     const unsigned nq = (ib + (unsigned)(hi - lo) + 15u) >> 4;
+    // 16-byte pieces inside the payload: all but perhaps the first and the last
+    const unsigned q_lo = lo < ib ? 1u : 0u;
+    const unsigned q_hi = g16 + 16ull * nq <= pe ? nq : nq - 1u;
     uint4 *imgq = reinterpret_cast<uint4 *>(img);
     for (unsigned q = tid; q < nq; q += kD64Threads) {
       const uintptr_t src = g16 + 16u * q;
       uint4 v;
-      if (src >= pb && src + 16 <= pe) {
+      if (q >= q_lo && q < q_hi) {
         v = __ldg(reinterpret_cast<const uint4 *>(src));
       } else {
         unsigned w4[4] = {0u, 0u, 0u, 0u};
@@ -76,144 +223,39 @@ __global__ void __launch_bounds__(kD64Threads, 6) decode64_kernel(DecArgs a) {
     }
   }
   __syncthreads();
-  const unsigned *imgw = reinterpret_cast<const unsigned *>(img);
-  const bool have = bi < nb;
+  // a lane a block: the blocks' fields and checks, once and not once a lane of
+  // the eight that decode it
+  if (tid < kD64Blocks) {
+    uint4 h = make_uint4(0u, 0u, 0u, 0u);
+    if (tid < nb) {
+      const long long left = n - (b0 + tid) * 64;
+      const unsigned len = left < 64 ? (unsigned)left : 64u;
+      bool ok = !(o0 < lo || o0 + 4 > hi || o1 < o0 || o1 > end);
+      if (ok) {
+        h.x = (unsigned)(o0 - lo) + ib;
+        const unsigned bend = (unsigned)((o1 < hi ? o1 : hi) - lo) + ib;
+        unsigned w0, w1;
+        ld_window(reinterpret_cast<const unsigned *>(img), h.x, w0, w1);
+        h.y = w0;
+        const unsigned bc = len > 1u && h.x + 4 < bend ? w1 & 0xffu : 0u;
+        const unsigned bytes = bc > 32u ? 0u : block_bytes_layout(len, bc, TAGS, a.cpu_layout != 0);
+        ok = bc <= 32u && h.x + bytes <= bend;
+        h.z = h.x + bytes - (len + 3u) / 4u;
+        h.w = bc | (ok ? kD64Ok : 0u);
+      }
+      if (!ok) atomicExch(a.err, kErrMalformed);
+    }
+    s_hd[tid] = h;
+  }
+  __syncthreads();
+  const uint4 h = s_hd[bi];
   const long long base = (b0 + bi) * 64;
-  const int len = have ? (int)((n - base) < 64 ? (n - base) : 64) : 0;
-  const int e0 = 8 * l;
-  const int nv = len - e0 < 0 ? 0 : (len - e0 > 8 ? 8 : len - e0);
-  bool ok = have;
-  unsigned start = 0, bend = 0;
-  if (ok) {
-    const unsigned long long o0 = s_off[bi], o1 = s_off[bi + 1];
-    if (o0 < lo || o0 + 4 > hi || o1 < o0 || o1 > s_off[nb]) ok = false;
-    start = (unsigned)(o0 - lo) + ib;
-    bend = (unsigned)((o1 < hi ? o1 : hi) - lo) + ib;
-  }
-  unsigned bc = 0;
-  int anchor = 0;
-  if (ok) {
-    unsigned w0, w1;
-    ld_window(imgw, start, w0, w1);
-    anchor = (int)w0;
-    if (len > 1) bc = start + 4 < bend ? w1 & 0xffu : 0u;
-    if (bc > 32u || start + block_bytes_layout((unsigned)len, bc, TAGS, a.cpu_layout != 0) > bend) ok = false;
-  }
-  if (have && !ok && l == 0) atomicExch(a.err, kErrMalformed);
-  const unsigned cnt = len > 0 ? (unsigned)len - 1u : 0u;
-  // q[t]: sum of the octet's deltas before element t; q[8]: of all of them
-  int q[9];
-#pragma unroll
-  for (int t = 0; t < 9; t++) q[t] = 0;
-  if (ok && bc && (unsigned)e0 < cnt) {
-    const unsigned p = start + 5u, sbytes = (cnt + 7u) >> 3;
-    const unsigned neg = (unsigned)img[p + l] << 24;     // sign of delta e0 + t at bit 31 - t
-    const unsigned mag = p + sbytes, fb = bc >> 3, rem = bc & 7u;
-    // rem bytes at byte l rem of the remainder section, most significant bits first
-    unsigned rl, rh;
-    ld_window(imgw, mag + fb * cnt + (unsigned)l * rem, rl, rh);
-    unsigned wh = __byte_perm(rl, 0u, 0x0123), wl = __byte_perm(rh, 0u, 0x0123);
-    const unsigned down = 31u - rem;                     // a field is (wh >> 1) >> down: nothing when rem is 0
-    unsigned fl = 0, fh = 0;
-    if (fb == 1) ld_window(imgw, mag + (unsigned)e0, fl, fh);
-    const unsigned up = 1u << rem;
-    if (fb <= 1) {
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        const unsigned full = __byte_perm(fl, fh, 0x4440u + (unsigned)t) & 0xffu;
-        const unsigned m = full * up + ((wh >> 1) >> down);
-        wh = __funnelshift_l(wl, wh, rem);
-        wl <<= rem;
-        q[t + 1] = (int)(m * (unsigned)(((int)(neg << t) >> 31) | 1) + (unsigned)q[t]);
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        unsigned full = 0;
-        if ((unsigned)(e0 + t) < cnt) {
-          const unsigned o = mag + (unsigned)(e0 + t) * fb;
-          for (unsigned u = 0; u < fb; u++) full |= (unsigned)img[o + u] << (8u * u);
-        }
-        const unsigned m = full * up + ((wh >> 1) >> down);
-        wh = __funnelshift_l(wl, wh, rem);
-        wl <<= rem;
-        q[t + 1] = (int)(m * (unsigned)(((int)(neg << t) >> 31) | 1) + (unsigned)q[t]);
-      }
-    }
-  }
-  // exclusive scan of the octet sums over the block's lanes
-  int inc = q[8];
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, inc, o, 8);
-    if (l >= o) inc = (int)((unsigned)inc + (unsigned)u);
-  }
-  const int v0 = (int)((unsigned)anchor + (unsigned)inc - (unsigned)q[8]);
-  unsigned n_ext = 0;
-  if (ok && nv > 0) {
-#pragma unroll
-    for (int t = 0; t < 8; t++) q[t] = (int)((unsigned)q[t] + (unsigned)v0);
-    const long long i0 = base + e0;
-    if (a.out_f) {
-      float f[8];
-#pragma unroll
-      for (int t = 0; t < 8; t++) f[t] = __fmul_rn((float)q[t], a.eb);
-      if (nv == 8 && ((reinterpret_cast<uintptr_t>(a.out_f + i0) & 15) == 0)) {
-        reinterpret_cast<float4 *>(a.out_f + i0)[0] = make_float4(f[0], f[1], f[2], f[3]);
-        reinterpret_cast<float4 *>(a.out_f + i0)[1] = make_float4(f[4], f[5], f[6], f[7]);
-      } else {
-#pragma unroll
-        for (int t = 0; t < 8; t++) if (t < nv) a.out_f[i0 + t] = f[t];
-      }
-    }
-    if (!TAGS && a.out_i) {
-      if (nv == 8 && ((reinterpret_cast<uintptr_t>(a.out_i + i0) & 15) == 0)) {
-        reinterpret_cast<int4 *>(a.out_i + i0)[0] = make_int4(q[0], q[1], q[2], q[3]);
-        reinterpret_cast<int4 *>(a.out_i + i0)[1] = make_int4(q[4], q[5], q[6], q[7]);
-      } else {
-#pragma unroll
-        for (int t = 0; t < 8; t++) if (t < nv) a.out_i[i0 + t] = q[t];
-      }
-    }
-    if (TAGS) {
-      const unsigned tb = ((unsigned)len + 3u) / 4u;
-      const unsigned tsec = start + block_bytes_layout((unsigned)len, bc, true, a.cpu_layout != 0) - tb;
-      // element 0 in the top two of 16 bits; elements past nv as regular points
-      unsigned tg = (2u * l < tb ? (unsigned)img[tsec + 2 * l] << 8 : 0u) |
-                    (2u * l + 1u < tb ? (unsigned)img[tsec + 2 * l + 1] : 0u);
-      if (nv < 8) tg &= 0xffffu << (16 - 2 * nv);
-      n_ext = (unsigned)__popc((tg ^ (tg >> 1)) & 0x5555u);   // types 01 and 10
-      if (a.pl_lo) {
-        // element t to bit t: the compacted fields, element 0 on top, reversed
-        const long long o = i0 >> 3;
-        a.pl_lo[o] = (unsigned char)(__brev(compact2(tg)) >> 24);
-        a.pl_hi[o] = (unsigned char)(__brev(compact2(tg >> 1)) >> 24);
-        // the rest of the planes' last word
-        if (i0 + 8 >= n)
-          for (long long k = o + 1; k & 3; k++) a.pl_lo[k] = a.pl_hi[k] = 0;
-      }
-      if (a.fn_u8) {
-        if (nv == 8 && ((reinterpret_cast<uintptr_t>(a.fn_u8 + i0) & 7) == 0)) {
-          // four two-bit fields of a byte, most significant first, to four bytes
-          unsigned w[2];
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const unsigned x = h ? tg & 0xffu : tg >> 8;
-            const unsigned y = (x | (x << 12)) & 0x000f000fu;        // low nibble, high nibble << 16
-            const unsigned z = (y | (y << 6)) & 0x03030303u;         // fields 3, 2 (low to high byte), 1, 0
-            w[h] = __byte_perm(z, 0u, 0x0123);
-          }
-          *reinterpret_cast<uint2 *>(a.fn_u8 + i0) = make_uint2(w[0], w[1]);
-        } else {
-#pragma unroll
-          for (int t = 0; t < 8; t++) if (t < nv) a.fn_u8[i0 + t] = (unsigned char)((tg >> (14 - 2 * t)) & 3u);
-        }
-      }
-      if (a.fn_i) {
-#pragma unroll
-        for (int t = 0; t < 8; t++) if (t < nv) a.fn_i[i0 + t] = (int)((tg >> (14 - 2 * t)) & 3u);
-      }
-    }
+  unsigned n_ext;
+  if ((b0 + kD64Blocks) * 64 <= n) {
+    n_ext = d64_octet<TAGS, true>(a, img, h, base, 64, l);
+  } else {
+    const int len = bi < nb ? (int)((n - base) < 64 ? (n - base) : 64) : 0;
+    n_ext = d64_octet<TAGS, false>(a, img, h, base, len, l);
   }
   if (TAGS && a.ext_count) {
     // one atomic per CTA: every CTA adds to the same word
