@@ -31,6 +31,13 @@
 //    894     56 registers: four CTAs per SM instead of three
 //    772     descriptors as one 16-byte word: one load in the look-back
 //    712     comparisons on the FMA pipe, 32-bit coordinate split
+//
+// The same kernel without the classification encodes integers (with the types
+// of a byte array, or none) and quantized fields, in place of the octet encoder
+// with its look-back in line: plain field of 60 M floats 575 -> 463 us for
+// encoding and decoding, double field of 256^3 217 -> 184, topology of 512^3
+// (its sort positions) 977 -> 941.  Five CTAs per SM (40 registers, spills)
+// measure the same.
 #include "tsz_codec2.cuh"
 #include "tsz_enc64.h"
 #include "tsz_ops.h"
@@ -48,6 +55,10 @@ constexpr unsigned kE64Img = (kE64Blocks * kE64BlockMax + 64u + 15u) & ~15u;
 // staged critical points, one per element at most: pairs, or codes (extrema
 // from the front, saddles from the back)
 __host__ __device__ constexpr unsigned e64_part(bool bits) { return kE64Img + kE64Tile * (bits ? 4u : 8u); }
+// the same of a kernel for mode, whose points are staged only where it classifies
+__host__ __device__ constexpr unsigned e64_part(int mode, bool bits) {
+  return mode == kEncClassify ? e64_part(bits) : kE64Img;
+}
 
 struct E64Sh {
   unsigned wb[kE64Warps], wc[kE64Warps];         // block bytes and (extrema << 16 | points) of each warp
@@ -125,8 +136,10 @@ __device__ __forceinline__ unsigned divmod32(unsigned i, unsigned d, unsigned lo
 // Front half of a tile: load, classify, quantize, pack into img, stage the
 // critical points, publish the tile's aggregate.  The 256 threads that own
 // elements call it.  FULL: every block of the tile has 64 elements, so the only
-// position without a delta is a block's last.
-template <bool D3, bool BITS, bool FULL>
+// position without a delta is a block's last.  The modes without
+// classification take integers as they are or quantize only, and their tags,
+// where they have any, from a byte per element.
+template <int MODE, bool D3, bool BITS, bool FULL>
 __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bool small, unsigned char *img, void *stage,
                                           E64Sh &sh) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -140,8 +153,25 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
   const int nv = FULL ? 8 : (len - e0 < 0 ? 0 : (len - e0 > 8 ? 8 : len - e0));
 
   // ---- values of the octet ----
+  constexpr bool kTags = mode_tags(MODE), kFloats = MODE == kEncClassify || MODE == kEncQuant;
   float x[8];
-  if (nv == 8) {
+  int q[8];
+  unsigned tags = 0, cpm = 0, exm = 0;
+  if (!kFloats) {
+    if (nv == 8) {
+      const int4 *pi = reinterpret_cast<const int4 *>(a.ints + i0);
+      const int4 u = __ldg(pi), v = __ldg(pi + 1);
+      q[0] = u.x; q[1] = u.y; q[2] = u.z; q[3] = u.w; q[4] = v.x; q[5] = v.y; q[6] = v.z; q[7] = v.w;
+    } else {
+#pragma unroll
+      for (int t = 0; t < 8; t++) q[t] = t < nv ? __ldg(a.ints + i0 + t) : 0;
+    }
+    if (kTags && nv > 0) {
+      // element t from bits 2t of the types to the t-th field from the top
+      const unsigned ty = __brev(load_type_octet(a.types, i0, nv)) >> 16;
+      tags = ((ty & 0x5555u) << 1) | ((ty >> 1) & 0x5555u);
+    }
+  } else if (nv == 8) {
     const float4 *px = reinterpret_cast<const float4 *>(a.data + g0);
     const float4 u = __ldg(px), v = __ldg(px + 1);
     x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
@@ -149,6 +179,7 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
 #pragma unroll
     for (int t = 0; t < 8; t++) x[t] = t < nv ? __ldg(a.data + g0 + t) : 0.f;
   }
+  if constexpr (MODE == kEncClassify) {
   // -0 as +0: the same quantized value, value code and comparisons
 #pragma unroll
   for (int t = 0; t < 8; t++) x[t] = plus_zero(x[t]);
@@ -214,7 +245,6 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
   float next = __shfl_down_sync(0xffffffffu, x[0], 1);
   if (lane == 0 && (inter & 0x80u)) prev = plus_zero(__ldg(a.data + g0 - 1));
   if (lane == 31 && (inter & 1u)) next = plus_zero(__ldg(a.data + g0 + 8));
-  unsigned tags = 0, cpm = 0, exm = 0;
   if (__any_sync(0xffffffffu, inter != 0u)) {
     // edge j (0..8) joins element j-1 and j (element -1 = prev, 8 = next): bit 8 - j
     unsigned gt = 0, lt = 0;
@@ -254,11 +284,13 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
     // 2-bit types: maximum 01, minimum 10, saddle 11 (element 0 in the top two bits)
     tags = spread2(mx | sd) | (spread2(mn | sd) << 1);
   }
+  }
 
   // ---- quantization and deltas ----
-  int q[8];
+  if (kFloats) {
 #pragma unroll
-  for (int t = 0; t < 8; t++) q[t] = t < nv ? quantize(x[t], a.inv) : 0;
+    for (int t = 0; t < 8; t++) q[t] = t < nv ? quantize(x[t], a.inv) : 0;
+  }
   const int qn = __shfl_down_sync(0xffffffffu, q[0], 1, 8);
   const int cnt = len > 0 ? len - 1 : 0;
   unsigned sign = 0, maxm = 0, mags[8];
@@ -277,8 +309,8 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
   }
   // below 2^16 log2f is off by less than its distance from the next integer
   const unsigned bc = maxm < 65536u ? 32u - (unsigned)__clz((int)maxm) : bitcount(maxm);
-  const unsigned bbytes = FULL ? 21u + (bc ? 8u + ((bc * 63u + 7u) >> 3) : 0u)
-                               : (len ? block_bytes((unsigned)len, bc, true) : 0u);
+  const unsigned bbytes = FULL ? (kTags ? 21u : 5u) + (bc ? 8u + ((bc * 63u + 7u) >> 3) : 0u)
+                               : (len ? block_bytes((unsigned)len, bc, kTags) : 0u);
 
   // ---- tile scans: block bytes, and points with extrema above them ----
   unsigned boff, cpo, exo;
@@ -290,10 +322,12 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
     if (lane >= 16) ib += u;
     const unsigned c = (unsigned)__popc(cpm) | ((unsigned)__popc(exm) << 16);
     unsigned ic = c;
+    if (MODE == kEncClassify) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      u = __shfl_up_sync(0xffffffffu, ic, o);
-      if (lane >= o) ic += u;
+      for (int o = 1; o < 32; o <<= 1) {
+        u = __shfl_up_sync(0xffffffffu, ic, o);
+        if (lane >= o) ic += u;
+      }
     }
     if (lane == 31) { sh.wb[warp] = ib; sh.wc[warp] = ic; }
     // also the point after which every thread has left the image's last write-out
@@ -321,7 +355,7 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
   if (l == 0) sh.boff[bi] = boff;
 
   // ---- critical points, staged ----
-  if (cpm) {
+  if (MODE == kEncClassify && cpm) {
     if (BITS) {
       unsigned *st = static_cast<unsigned *>(stage);
       unsigned ei = exo, si = kE64Tile - 1u - (cpo - exo);
@@ -413,8 +447,8 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
     }
     // tag byte j: elements 4j .. 4j+3, element 4j in the top two bits
     const unsigned tb = ((unsigned)len + 3u) / 4u;
-    if (FULL || 2u * l < tb) img[p + 2 * l] = (unsigned char)(tags >> 8);
-    if (FULL || 2u * l + 1u < tb) img[p + 2 * l + 1] = (unsigned char)tags;
+    if (kTags && (FULL || 2u * l < tb)) img[p + 2 * l] = (unsigned char)(tags >> 8);
+    if (kTags && (FULL || 2u * l + 1u < tb)) img[p + 2 * l + 1] = (unsigned char)tags;
   }
 }
 
@@ -566,12 +600,12 @@ __device__ __forceinline__ void e64_place(const Enc64Args &a, long long tile, E6
 // A look-back waits for the aggregates of earlier tiles only, and a tile's
 // aggregate waits, through its CTA's barrier, for look-backs of earlier tiles
 // only, so the waits cannot form a cycle.
-template <bool D3, bool BITS>
+template <int MODE, bool D3, bool BITS>
 __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   __shared__ E64Sh sh[2];
   __shared__ long long s_claim[2];
-  constexpr unsigned kPart = e64_part(BITS);
+  constexpr unsigned kPart = e64_part(MODE, BITS);
   const long long ntiles = ((long long)a.n + kE64Tile - 1) / kE64Tile;
   const long long nfull = (long long)a.n / kE64Tile;
   const long long tend = a.tile_hi ? (long long)a.tile_hi : ntiles;
@@ -600,8 +634,8 @@ __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
     if (owner) {
       unsigned char *part = smem_dyn + (size_t)cur * kPart;
       if (more) {
-        if (tile < nfull) e64_front<D3, BITS, true>(a, tile, small, part, part + kE64Img, sh[cur]);
-        else e64_front<D3, BITS, false>(a, tile, small, part, part + kE64Img, sh[cur]);
+        if (tile < nfull) e64_front<MODE, D3, BITS, true>(a, tile, small, part, part + kE64Img, sh[cur]);
+        else e64_front<MODE, D3, BITS, false>(a, tile, small, part, part + kE64Img, sh[cur]);
       }
     } else {
       if (prev >= 0) e64_place(a, prev, sh[cur ^ 1]);
@@ -690,11 +724,11 @@ enc64_batch_kernel(const EncArgs *__restrict__ fields, const unsigned long long 
         const bool small = a.g.d1 * a.g.plane < (1ll << 32), full = tile < (long long)(a.n / kE64Tile);
         unsigned char *part = smem_dyn + (size_t)cur * kPart;
         if (a.g.nd == 3) {
-          if (full) e64_front<true, false, true>(a, tile, small, part, part + kE64Img, sh[cur]);
-          else e64_front<true, false, false>(a, tile, small, part, part + kE64Img, sh[cur]);
+          if (full) e64_front<kEncClassify, true, false, true>(a, tile, small, part, part + kE64Img, sh[cur]);
+          else e64_front<kEncClassify, true, false, false>(a, tile, small, part, part + kE64Img, sh[cur]);
         } else {
-          if (full) e64_front<false, false, true>(a, tile, small, part, part + kE64Img, sh[cur]);
-          else e64_front<false, false, false>(a, tile, small, part, part + kE64Img, sh[cur]);
+          if (full) e64_front<kEncClassify, false, false, true>(a, tile, small, part, part + kE64Img, sh[cur]);
+          else e64_front<kEncClassify, false, false, false>(a, tile, small, part, part + kE64Img, sh[cur]);
         }
       }
     } else if (pending) {
@@ -726,10 +760,14 @@ cudaError_t launch_enc64_batch(const EncArgs *fields, const unsigned long long *
 
 unsigned long long enc64_tiles(unsigned long long n) { return (n + kE64Tile - 1) / kE64Tile; }
 
-static cudaError_t launch_enc64(const Enc64Args &a, cudaStream_t s, int sm_count) {
-  const size_t smem = 2 * (size_t)e64_part(a.code_out != nullptr);
-  auto k = a.code_out ? (a.g.nd == 3 ? enc64_kernel<true, true> : enc64_kernel<false, true>)
-                      : (a.g.nd == 3 ? enc64_kernel<true, false> : enc64_kernel<false, false>);
+static cudaError_t launch_enc64(int mode, const Enc64Args &a, cudaStream_t s, int sm_count) {
+  const size_t smem = 2 * (size_t)e64_part(mode, a.code_out != nullptr);
+  const bool d3 = a.g.nd == 3;
+  auto k = mode == kEncInts       ? enc64_kernel<kEncInts, false, false>
+           : mode == kEncIntTypes ? enc64_kernel<kEncIntTypes, false, false>
+           : mode == kEncQuant    ? enc64_kernel<kEncQuant, false, false>
+           : a.code_out           ? (d3 ? enc64_kernel<kEncClassify, true, true> : enc64_kernel<kEncClassify, false, true>)
+                                  : (d3 ? enc64_kernel<kEncClassify, true, false> : enc64_kernel<kEncClassify, false, false>);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
@@ -778,7 +816,7 @@ int selftest_lookback(int spin_limit, int *status, float *ms) {
     a.tile_hi = 2;
     a.spin_limit = spin_limit;
     cudaEventRecord(e0, 0);
-    const cudaError_t le = launch_enc64(a, 0, 1);
+    const cudaError_t le = launch_enc64(kEncClassify, a, 0, 1);
     cudaEventRecord(e1, 0);
     int h = 0;
     if (!cuda_fail(le, "probe launch") && !cuda_fail(cudaMemcpy(&h, a.err, 4, cudaMemcpyDeviceToHost), "D2H")) {
@@ -794,13 +832,23 @@ int selftest_lookback(int spin_limit, int *status, float *ms) {
 }
 
 bool enc64_applies(const EncArgs &a, int mode) {
-  return mode == kEncClassify && a.B == 64 && (a.cp_mode == kCpPairs || a.cp_mode == kCpBits) && a.out != nullptr &&
-         (reinterpret_cast<uintptr_t>(a.data) & 15) == 0 && enc_tile_blocks(64) == kE64Blocks;
+  if (a.B != 64 || a.out == nullptr || enc_tile_blocks(64) != kE64Blocks) return false;
+  const void *in = a.data;
+  if (mode == kEncClassify) {
+    if (a.cp_mode != kCpPairs && a.cp_mode != kCpBits) return false;
+  } else if (mode == kEncInts || mode == kEncIntTypes) {
+    in = a.ints;
+  } else if (mode != kEncQuant) {
+    return false;
+  }
+  return (reinterpret_cast<uintptr_t>(in) & 15) == 0;
 }
 
-cudaError_t launch_enc64_args(const Enc64Args &a, cudaStream_t s, int sm_count) { return launch_enc64(a, s, sm_count); }
+cudaError_t launch_enc64_args(const Enc64Args &a, cudaStream_t s, int sm_count) {
+  return launch_enc64(kEncClassify, a, s, sm_count);
+}
 
-cudaError_t launch_enc64_from(const EncArgs &e, cudaStream_t s, int sm_count) {
+cudaError_t launch_enc64_from(int mode, const EncArgs &e, cudaStream_t s, int sm_count) {
   Enc64Args a{};
   a.data = e.data;
   a.n = e.n;
@@ -823,7 +871,9 @@ cudaError_t launch_enc64_from(const EncArgs &e, cudaStream_t s, int sm_count) {
   }
   a.cp_cap = e.cp_cap;
   a.spin_limit = 0;
-  return launch_enc64(a, s, sm_count);
+  a.ints = e.ints;
+  a.types = e.types;
+  return launch_enc64(mode, a, s, sm_count);
 }
 
 }  // namespace tsz

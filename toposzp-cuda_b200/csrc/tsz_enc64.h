@@ -8,6 +8,8 @@ constexpr int kEnc64TileBlocks = 32;   // codec blocks per tile
 
 struct Enc64Args {
   const float *data;            // the field, 16-byte aligned
+  const int *ints;              // or its integers, 16-byte aligned, and their types
+  const unsigned char *types;
   unsigned long long n;
   double inv;                   // 1 / (double)eb
   Geom g;
@@ -30,11 +32,12 @@ struct Enc64Args {
                                 // base + local through data (indexed by global element)
 };
 
-// The fused topology encoder (pairs, or bits and codes) applies to blockSize 64 and a
-// 16-byte aligned field; its tiles are the general encoder's (2048 elements).
+// blockSize 64 and a 16-byte aligned field: the fused topology encoder (pairs,
+// or bits and codes), and the encoders of integers and of quantized fields;
+// tiles are the general encoder's (2048 elements).
 bool enc64_applies(const EncArgs &a, int mode);
 // Launches it over the tiles of a (persistent grid sized by occupancy).
-cudaError_t launch_enc64_from(const EncArgs &a, cudaStream_t s, int sm_count);
+cudaError_t launch_enc64_from(int mode, const EncArgs &a, cudaStream_t s, int sm_count);
 cudaError_t launch_enc64_args(const Enc64Args &a, cudaStream_t s, int sm_count);
 // The same over the fields of a batch (blockSize 64, 16-byte aligned fields,
 // pairs): tiles of all fields in one queue (tstart[f]: first tile of field f,
