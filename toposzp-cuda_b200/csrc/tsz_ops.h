@@ -5,6 +5,14 @@
 
 namespace tsz {
 
+// Scratch arrays of the post-processing of one field (tsz_post.cu).
+struct PostLists {
+  unsigned *X, *Z, *Y;          // extrema, saddles (axis pass), lost saddles
+  unsigned *W0, *W1;            // worklists
+  unsigned *R, *Eb, *Sb, *XP;   // bitmaps: lost saddles, extrema, saddles; list position of each word's first extremum
+  float *OX, *OZ;               // raw values of X and Z
+};
+
 // Geometry from extents (nd = 2: rows, cols; nd = 3: d1, d2, d3).
 Geom make_geom(int nd, long long a, long long b, long long c);
 
@@ -99,9 +107,12 @@ bool post_planes(szp_b200_ctx *ctx, unsigned long long n, unsigned **TL, unsigne
 int post_planes_from_bytes(szp_b200_ctx *ctx, const unsigned char *d_T, unsigned long long n, unsigned *TL,
                            unsigned *TH);
 int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const unsigned *d_TL,
-                     const unsigned *d_TH, unsigned long long *d_S, TileDesc *desc, const int *d_sp,
-                     unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
+                     const unsigned *d_TH, unsigned long long *d_S, const PostLists &l, unsigned long long tot,
+                     const int *d_sp, unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
                      int *restored_out);
+bool post_has_work(const Geom &g);
+int post_lists_begin(szp_b200_ctx *ctx, const unsigned *d_TL, const unsigned *d_TH, TileDesc *desc, const Geom &g,
+                     int axis_stencil, PostLists *l);
 
 // Block offsets of a single-chunk stream, parsed on the device (enqueued on
 // ctx->stream, no sync).  d_payload: the bytes after the 8-byte offset table,

@@ -775,10 +775,12 @@ __global__ void __launch_bounds__(256)
 fn_detect_kernel(PostArgs a, const unsigned *__restrict__ Sb, unsigned nwords, unsigned *__restrict__ R,
                  unsigned *__restrict__ Y, unsigned *y_count) {
   __shared__ unsigned short s_pt[8][1024];
+  __shared__ unsigned s_lost[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned w0 = (blockIdx.x * 8u + warp) * 32u;
   if (w0 >= nwords) return;
   unsigned m = w0 + lane < nwords ? Sb[w0 + lane] : 0u;
+  s_lost[warp][lane] = 0u;
   unsigned inc = __popc(m);
   const unsigned c = inc;
 #pragma unroll
@@ -806,9 +808,11 @@ fn_detect_kernel(PostArgs a, const unsigned *__restrict__ Sb, unsigned nwords, u
     at = __shfl_sync(0xffffffffu, at, 0);
     if (lost) {
       Y[at + __popc(lm & ((1u << lane) - 1u))] = (unsigned)q;
-      atomicOr(&R[q >> 5], 1u << (q & 31));
+      atomicOr(&s_lost[warp][(unsigned)(q - base) >> 5], 1u << (q & 31));
     }
   }
+  __syncwarp();
+  if (w0 + lane < nwords) R[w0 + lane] = s_lost[warp][lane];   // every word, with or without lost saddles
 }
 
 // raw values of a list's points
@@ -1283,17 +1287,30 @@ static int dev_grid(szp_b200_ctx *ctx) {
 
 // Rounds over deferred items as ordinary launches, kBurstRounds of them
 // between host checks of the remaining count: W holds the items on entry
-// (their count in word 7), W and Wo alternate.  Every round completes at
+// (their count in the pass's n0), W and Wo alternate.  Every round completes at
 // least the earliest pending item, so a burst that completes none reports an
 // error.
 constexpr int kBurstRounds = 4;
 constexpr int kRoundLimit = 100000;
 
+// The words of a pass: the length of its first worklist, three round counters,
+// the barrier's counter and generation, the length of the second worklist.
+// Each pass has its own, so that one memset clears them for all.
+struct PassWords { unsigned n0, cnts[3], bar[2], n1, unused[9]; };
+constexpr int kPassWord = 24;   // of the workspace's 64 words
+static_assert(sizeof(PassWords) == 64 && kPassWord + 4 * 8 <= 64, "four passes' words");
+
+template <int PASS>
+static PassWords *pass_words(szp_b200_ctx *ctx) {
+  static_assert(PASS >= 0 && PASS < 4, "pass numbers");
+  return reinterpret_cast<PassWords *>(ctx->d_words + kPassWord) + PASS;
+}
+
 template <int PASS, int ND>
 static int finish_rounds(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, unsigned *W, unsigned *Wo) {
   cudaStream_t s = ctx->stream;
-  unsigned *c[3] = {reinterpret_cast<unsigned *>(ctx->d_words + 7), reinterpret_cast<unsigned *>(ctx->d_words + 11),
-                    reinterpret_cast<unsigned *>(ctx->d_words + 12)};
+  PassWords *pw = pass_words<PASS>(ctx);
+  unsigned *c[3] = {&pw->n0, &pw->cnts[0], &pw->cnts[1]};
   unsigned *h_left = reinterpret_cast<unsigned *>(ctx->h_words + 15);
   int ci = 0;
   unsigned prev = 0xffffffffu;
@@ -1336,18 +1353,13 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
   if (ni_bits ? ni_words == 0 : (!count_dev && count == 0)) return 0;
   const int grid = coop_grid<PASS, ND>(ctx);
   cudaStream_t s = ctx->stream;
-  // words 7 (round-0 count) and 10..13: three round counters, the barrier
-  // counter and generation, the length of the round-1 worklist
-  unsigned *n0 = reinterpret_cast<unsigned *>(ctx->d_words + 7);
-  unsigned *cnts = reinterpret_cast<unsigned *>(ctx->d_words + 10);
-  unsigned *bar = cnts + 3;
-  unsigned *n1 = cnts + 6;
+  PassWords *pw = pass_words<PASS>(ctx);
+  unsigned *n0 = &pw->n0, *cnts = pw->cnts, *bar = pw->bar, *n1 = &pw->n1;
   unsigned long long *status = ctx->d_words + 9;
   const unsigned zero = 0;
   const unsigned *no_total = nullptr;
   if (grid && most <= (unsigned)grid * kPostThreads) {
     // every item in flight at once: one launch, no worklist to start from
-    if (cuda_fail(cudaMemsetAsync(cnts, 0, 32, s), "memset")) return -1;
     const unsigned *none = nullptr;
     a.ONLY = ni_bits;
     void *args[] = {(void *)&a,    (void *)&list, (void *)&none, (void *)&most, (void *)(count_dev ? &count_dev : &no_total),
@@ -1360,7 +1372,6 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
     ctx->launches += 1;
     return cuda_fail(e, "cooperative pass launch") ? -1 : 0;
   }
-  if (cuda_fail(cudaMemsetAsync(n0, 0, 4, s), "memset")) return -1;
   if (ni_bits)
     enforce_sparse_kernel<ND><<<(ni_words + kSparseWords - 1) / kSparseWords, kPostThreads, 0, s>>>(
         a, list, ni_bits, ni_words, W0, n0);
@@ -1372,7 +1383,6 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
   ctx->launches += 1;
   if (cuda_fail(cudaGetLastError(), "pass round")) return -1;
   if (!grid) return finish_rounds<PASS, ND>(ctx, a, list, W0, W1);
-  if (cuda_fail(cudaMemsetAsync(cnts, 0, 32, s), "memset")) return -1;
   const unsigned *W_start = W0, *nstart = n0;
   unsigned *Wx = W1, *Wy = W0;
   if (!count_dev) {
@@ -1433,9 +1443,7 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
   // the lost saddles (from F after enforcement); RBF reads the locks from the
   // extremum bitmap (box_locks)
   const long long words = (n + 31) / 32;
-  if (cuda_fail(cudaMemsetAsync(R, 0, words * 4, s), "memset")) return -1;
   unsigned *ycnt = reinterpret_cast<unsigned *>(ctx->d_words + 8);
-  if (cuda_fail(cudaMemsetAsync(ycnt, 0, 4, s), "memset")) return -1;
   a.R = R;
   if (nz) fn_detect_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(a, Sb, (unsigned)words, R, Y, ycnt);
   ctx->launches += nz ? 1 : 0;
@@ -1456,56 +1464,62 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
   return 0;
 }
 
-int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const unsigned *d_TL,
-                     const unsigned *d_TH, unsigned long long *d_S, TileDesc *desc, const int *d_sp,
-                     unsigned long long n_sp, const Geom &g, float eb, int axis_stencil, int *restored_out) {
+// whether there are interior points to work on
+bool post_has_work(const Geom &g) { return g.d2 >= 3 && g.d3 >= 3 && (g.nd != 3 || g.d1 >= 3); }
+
+// Launches the list kernel: totals to word 2 (extrema << 32 | saddles), its
+// status to word 5.  Words 2, 3 and 5 are zero on entry.
+int post_lists_begin(szp_b200_ctx *ctx, const unsigned *d_TL, const unsigned *d_TH, TileDesc *desc, const Geom &g,
+                     int axis_stencil, PostLists *l) {
   const long long n = g.d1 * g.d2 * g.d3;
-  if (g.d2 < 3 || g.d3 < 3 || (g.nd == 3 && g.d1 < 3)) { if (restored_out) *restored_out = 0; return 0; }
-  if (n >= (1ll << 32)) { set_error("post-processing supports fields of fewer than 2^32 points"); return -1; }
+  Arena &A = ctx->scratch;
+  l->X = A.take<unsigned>(n); l->Z = A.take<unsigned>(n); l->Y = A.take<unsigned>(n);
+  l->W0 = A.take<unsigned>(n); l->W1 = A.take<unsigned>(n);
+  l->R = A.take<unsigned>((n + 31) / 32);
+  l->Eb = A.take<unsigned>((n + 31) / 32 + 1);
+  l->Sb = A.take<unsigned>((n + 31) / 32 + 1);
+  l->XP = A.take<unsigned>((n + 31) / 32 + 1);
+  l->OX = A.take<float>(n); l->OZ = A.take<float>(n);
+  if (!l->X || !l->Z || !l->Y || !l->W0 || !l->W1 || !l->R || !l->Eb || !l->Sb || !l->XP || !l->OX || !l->OZ) {
+    set_error("scratch arena too small for post-processing");
+    return -1;
+  }
+  unsigned long long *w = ctx->d_words;
+  const long long ltiles = (n + kListTile - 1) / kListTile;
+  if (cuda_fail(cudaMemsetAsync(desc, 0, (ltiles + 1) * sizeof(TileDesc), ctx->stream), "memset")) return -1;
+  const unsigned grid = (unsigned)std::min<long long>(ltiles, (long long)ctx->sm_count * 6);
+  list_build_kernel<<<grid, kPostThreads, 0, ctx->stream>>>(
+      d_TL, d_TH, g, n, desc, reinterpret_cast<unsigned *>(w + 3), reinterpret_cast<int *>(w + 5), l->X,
+      axis_stencil && g.nd == 3 ? l->Z : nullptr, l->Eb, l->Sb, w + 2, l->XP);
+  ctx->launches += 1;
+  return cuda_fail(cudaGetLastError(), "lists") ? -1 : 0;
+}
+
+// The passes over the lists of post_lists_begin, whose totals the caller has read.
+int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const unsigned *d_TL,
+                     const unsigned *d_TH, unsigned long long *d_S, const PostLists &l, unsigned long long tot,
+                     const int *d_sp, unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
+                     int *restored_out) {
+  const long long n = g.d1 * g.d2 * g.d3;
   int dev = 0;
   cudaGetDevice(&dev);
   if (cuda_fail(upload_weights(dev), "weights")) return -1;
   cudaStream_t s = ctx->stream;
-  Arena &A = ctx->scratch;
-  unsigned *X = A.take<unsigned>(n), *Z = A.take<unsigned>(n), *Y = A.take<unsigned>(n);
-  unsigned *W0 = A.take<unsigned>(n), *W1 = A.take<unsigned>(n);
-  unsigned *R = A.take<unsigned>((n + 31) / 32);
-  unsigned *Eb = A.take<unsigned>((n + 31) / 32 + 1);
-  unsigned *Sb = A.take<unsigned>((n + 31) / 32 + 1);
-  unsigned *XP = A.take<unsigned>((n + 31) / 32 + 1);
-  float *OX = A.take<float>(n), *OZ = A.take<float>(n);
-  if (!X || !Z || !Y || !W0 || !W1 || !R || !Eb || !Sb || !XP || !OX || !OZ) {
-    set_error("scratch arena too small for post-processing");
-    return -1;
-  }
-  unsigned long long *w = ctx->d_words;  // [9] pass status, [10] round counters
-  if (cuda_fail(cudaMemsetAsync(w, 0, 96, s), "memset")) return -1;
-  unsigned *tile_ctr = reinterpret_cast<unsigned *>(w + 3);
-  unsigned long long *d_tot = w + 2;
-  const long long ltiles = (n + kListTile - 1) / kListTile;
-  if (cuda_fail(cudaMemsetAsync(desc, 0, (ltiles + 1) * sizeof(TileDesc), s), "memset")) return -1;
+  // [4] status, [5] restored, [8] lost saddles, [9] pass status, and the words of each pass
+  unsigned long long *w = ctx->d_words;
+  if (cuda_fail(cudaMemsetAsync(w, 0, (kPassWord + 4 * 8) * 8, s), "memset")) return -1;
   // post-processing of the decoded field itself: each item reads its raw
   // value from F before it writes (no gathered raw lists), except the
   // axis-pattern pass, which runs after RBF has changed saddles
   const bool raw_in_F = d_orig == d_data;
   const bool axis_raw = axis_stencil && g.nd == 3;
-  {
-    const unsigned grid = (unsigned)std::min<long long>(ltiles, (long long)ctx->sm_count * 6);
-    list_build_kernel<<<grid, kPostThreads, 0, s>>>(d_TL, d_TH, g, n, desc, tile_ctr, reinterpret_cast<int *>(w + 4),
-                                                    X, axis_raw ? Z : nullptr, Eb, Sb, d_tot, XP);
-  }
-  ctx->launches += 1;
-  unsigned long long tot = 0;
-  if (cuda_fail(cudaGetLastError(), "lists") ||
-      cuda_fail(cudaMemcpyAsync(&tot, d_tot, 8, cudaMemcpyDeviceToHost, s), "D2H") ||
-      cuda_fail(cudaStreamSynchronize(s), "lists"))
-    return -1;
   const unsigned nx = (unsigned)(tot >> 32), nz = (unsigned)(tot & 0xffffffffull);
+  unsigned *Z = l.Z;
+  float *OZ = l.OZ;
   if (axis_raw && raw_in_F && nz) {
     gather_kernel<<<(nz + 255) / 256, 256, 0, s>>>(Z, nz, d_data, OZ);
     ctx->launches += 1;
   }
-  tl_mark(ctx, "post_lists");
   PostArgs a{};
   a.F = d_data;
   a.TL = d_TL;
@@ -1518,14 +1532,14 @@ int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, cons
   a.eb = eb;
   a.eps = fmaxf(1e-6f, 0.1f * eb);
   a.S = d_S;
-  a.XP = XP;
+  a.XP = l.XP;
   a.err = reinterpret_cast<int *>(w + 4);
   a.restored = reinterpret_cast<unsigned *>(w + 5);
   const int rc = (g.nd == 2)
-                     ? run_all_passes<2>(ctx, a, X, nx, Z, nz, Y, W0, W1, R, Eb, Sb, OX, OZ, axis_stencil,
-                                         raw_in_F)
-                     : run_all_passes<3>(ctx, a, X, nx, Z, nz, Y, W0, W1, R, Eb, Sb, OX, OZ, axis_stencil,
-                                         raw_in_F);
+                     ? run_all_passes<2>(ctx, a, l.X, nx, Z, nz, l.Y, l.W0, l.W1, l.R, l.Eb, l.Sb, l.OX, OZ,
+                                         axis_stencil, raw_in_F)
+                     : run_all_passes<3>(ctx, a, l.X, nx, Z, nz, l.Y, l.W0, l.W1, l.R, l.Eb, l.Sb, l.OX, OZ,
+                                         axis_stencil, raw_in_F);
   if (rc) return -1;
   if (cuda_fail(cudaMemcpyAsync(ctx->h_words, w, 96, cudaMemcpyDeviceToHost, s), "D2H") ||
       cuda_fail(cudaStreamSynchronize(s), "postprocess"))
@@ -1587,7 +1601,10 @@ int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const int
                 unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
                 int *restored_out) {
   const long long n = g.d1 * g.d2 * g.d3;
+  if (!post_has_work(g)) { if (restored_out) *restored_out = 0; return 0; }
+  if (n >= (1ll << 32)) { set_error("post-processing supports fields of fewer than 2^32 points"); return -1; }
   Arena &A = ctx->scratch;
+  cudaStream_t s = ctx->stream;
   unsigned long long *S = post_words(ctx, (unsigned long long)n);
   unsigned *TL, *TH;
   const unsigned long long ntiles = (n + kPostTile - 1) / kPostTile;
@@ -1596,9 +1613,19 @@ int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const int
     set_error("scratch arena too small for post-processing");
     return -1;
   }
-  type_planes_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(d_types_i, n, TL, TH);
+  type_planes_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_types_i, n, TL, TH);
   ctx->launches += 1;
-  return postprocess_with(ctx, d_data, d_orig, TL, TH, S, desc, d_sp, n_sp, g, eb, axis_stencil, restored_out);
+  PostLists l;
+  if (cuda_fail(cudaMemsetAsync(ctx->d_words, 0, 64, s), "memset") ||
+      post_lists_begin(ctx, TL, TH, desc, g, axis_stencil, &l) ||
+      cuda_fail(cudaMemcpyAsync(ctx->h_words, ctx->d_words, 64, cudaMemcpyDeviceToHost, s), "D2H") ||
+      cuda_fail(cudaStreamSynchronize(s), "lists"))
+    return -1;
+  tl_mark(ctx, "post_lists");
+  const int err = (int)(ctx->h_words[5] & 0xffffffffu);
+  if (err) { set_error("post-processing status %d", err); return -1; }
+  return postprocess_with(ctx, d_data, d_orig, TL, TH, S, l, ctx->h_words[2], d_sp, n_sp, g, eb, axis_stencil,
+                          restored_out);
 }
 
 }  // namespace tsz
