@@ -78,7 +78,7 @@ struct PostArgs {
   // e's own item)
   const float *OL;
   const float *ORIG;
-  float *RAW;                   // fused stencil on the decoded field itself: raw values of the items left for enforcement
+  float *RAW;                   // fused stencil on the decoded field itself: raw values of the items it leaves
   const unsigned *TL, *TH;      // bit planes of the types
   const int *sp;
   unsigned long long n_sp;
@@ -97,7 +97,7 @@ struct PostArgs {
   // stencil pass fused with enforcement (null: plain stencil pass): bitmap
   // over list positions of the items that still need the enforcement pass
   unsigned *NI;
-  const unsigned *ONLY;         // the whole pass in one cooperative launch: bitmap of the list positions it runs (null: all)
+  const unsigned *ONLY;         // a pass of one launch: bitmap of the list positions that it runs (null: all)
 };
 
 // No "memory" clobber: a result word is read whole and carries its own
@@ -678,9 +678,13 @@ __device__ float axis3(const PostArgs &a, long long e, const C3 &c, float o, boo
 // (extrema in the byte word, saddles in the count word), then write their
 // entries through shared memory so each tile's slice of X and Z is stored
 // contiguously (X staged from the front of one buffer, Z from its back: a
-// point is in at most one list).  The last tile writes the totals to tot[0] =
-// (extrema << 32) | saddles.  512^3 field: 241 us from a byte per type with
-// both lists, 149 from the planes with X alone.
+// point is in at most one list).  A CTA runs one tile behind: it publishes tile
+// k's counts before it looks back for tile k-1, so the tiles that a look-back
+// waits for are held by CTAs that have published them (tiles are claimed in
+// order), and the wait has a tile of work behind it.  The last tile writes the
+// totals to tot[0] = (extrema << 32) | saddles.  512^3 field: 241 us from a
+// byte per type with both lists, 149 from the planes with X alone, 94
+// with the look-back a tile behind and both counts in one scan.
 constexpr int kListPer = 32;
 constexpr int kListTile = kPostThreads * kListPer;
 
@@ -688,81 +692,101 @@ __global__ void __launch_bounds__(kPostThreads)
 list_build_kernel(const unsigned *__restrict__ TL, const unsigned *__restrict__ TH, Geom g, long long n,
                   TileDesc *desc, unsigned *tile_ctr, int *err, unsigned *X, unsigned *Z, unsigned *Eb, unsigned *Sb,
                   unsigned long long *tot, unsigned *XP) {
-  __shared__ unsigned s_w1[kWarps], s_w2[kWarps];
-  __shared__ unsigned s_buf[kListTile];
+  __shared__ unsigned s_w[kWarps];
+  __shared__ unsigned short s_buf[2][kListTile];   // offsets in the tile
   __shared__ long long s_tile;
   __shared__ unsigned long long s_xb, s_zb;
   const long long ntiles = (n + kListTile - 1) / kListTile;
-  while (true) {
+  long long prev = -1;
+  unsigned p_te = 0, p_ts = 0, p_eo = 0;
+  for (int cur = 0;; cur ^= 1) {
     if (threadIdx.x == 0) s_tile = (long long)atomicAdd(tile_ctr, 1u);
     __syncthreads();
     const long long tile = s_tile;
-    if (tile >= ntiles) break;
-    const long long i0 = tile * kListTile + (long long)threadIdx.x * kListPer;
-    unsigned em = 0, sm = 0, im = 0;
-    if (i0 < n) {
-      const unsigned tl = TL[i0 >> 5], th = TH[i0 >> 5];
-      long long r, x, y, z;
-      if (g.nd == 2) { x = 0; y = fdivmod(i0, g.d3, g.m_d3, r); z = r; }
-      else { x = fdivmod(i0, g.plane, g.m_plane, r); y = fdivmod(r, g.d3, g.m_d3, z); }
-      if (z + kListPer - 1 < g.d3 && i0 + kListPer <= n) {
-        // the 32 points share one row: interior columns 1 .. d3-2
-        const bool row_in = y >= 1 && y <= g.d2 - 2 && (g.nd == 2 || (x >= 1 && x <= g.d1 - 2));
-        if (row_in) {
-          const long long lo = 1 - z, hi = g.d3 - 2 - z;   // interior offsets u in [lo, hi]
-          const int ulo = lo > 0 ? (int)lo : 0, uhi = hi < kListPer - 1 ? (int)hi : kListPer - 1;
-          if (ulo <= uhi) im = (uhi == 31 ? 0xffffffffu : ((2u << uhi) - 1u)) & ~((1u << ulo) - 1u);
+    const bool more = tile < ntiles;
+    unsigned te = 0, ts = 0, eo = 0;
+    if (more) {
+      const long long i0 = tile * kListTile + (long long)threadIdx.x * kListPer;
+      unsigned em = 0, sm = 0, im = 0;
+      if (i0 < n) {
+        const unsigned tl = TL[i0 >> 5], th = TH[i0 >> 5];
+        long long r, x, y, z;
+        if (g.nd == 2) { x = 0; y = fdivmod(i0, g.d3, g.m_d3, r); z = r; }
+        else { x = fdivmod(i0, g.plane, g.m_plane, r); y = fdivmod(r, g.d3, g.m_d3, z); }
+        if (z + kListPer - 1 < g.d3 && i0 + kListPer <= n) {
+          // the 32 points share one row: interior columns 1 .. d3-2
+          const bool row_in = y >= 1 && y <= g.d2 - 2 && (g.nd == 2 || (x >= 1 && x <= g.d1 - 2));
+          if (row_in) {
+            const long long lo = 1 - z, hi = g.d3 - 2 - z;   // interior offsets u in [lo, hi]
+            const int ulo = lo > 0 ? (int)lo : 0, uhi = hi < kListPer - 1 ? (int)hi : kListPer - 1;
+            if (ulo <= uhi) im = (uhi == 31 ? 0xffffffffu : ((2u << uhi) - 1u)) & ~((1u << ulo) - 1u);
+          }
+        } else if (g.d3 > kListPer && i0 + kListPer <= n) {
+          // two rows: columns z .. d3-1 of one, then 0 .. of the next
+          const unsigned k = (unsigned)(g.d3 - z);          // 1 .. 31
+          const bool plane_in = g.nd == 2 || (x >= 1 && x <= g.d1 - 2);
+          if (plane_in && y >= 1 && y <= g.d2 - 2) im = ((1u << k) - 1u) >> 1;
+          if (plane_in && y + 1 <= g.d2 - 2) im |= ~((2u << k) - 1u);
+        } else {
+          for (int u = 0; u < kListPer && i0 + u < n; u++) {
+            bool in = y >= 1 && y <= g.d2 - 2 && z >= 1 && z <= g.d3 - 2;
+            if (g.nd == 3) in = in && x >= 1 && x <= g.d1 - 2;
+            if (in) im |= 1u << u;
+            z++;
+            while (z >= g.d3) { z -= g.d3; y++; if (y >= g.d2) { y -= g.d2; x++; } }
+          }
         }
-      } else if (g.d3 > kListPer && i0 + kListPer <= n) {
-        // two rows: columns z .. d3-1 of one, then 0 .. of the next
-        const unsigned k = (unsigned)(g.d3 - z);          // 1 .. 31
-        const bool plane_in = g.nd == 2 || (x >= 1 && x <= g.d1 - 2);
-        if (plane_in && y >= 1 && y <= g.d2 - 2) im = ((1u << k) - 1u) >> 1;
-        if (plane_in && y + 1 <= g.d2 - 2) im |= ~((2u << k) - 1u);
-      } else {
-        for (int u = 0; u < kListPer && i0 + u < n; u++) {
-          bool in = y >= 1 && y <= g.d2 - 2 && z >= 1 && z <= g.d3 - 2;
-          if (g.nd == 3) in = in && x >= 1 && x <= g.d1 - 2;
-          if (in) im |= 1u << u;
-          z++;
-          while (z >= g.d3) { z -= g.d3; y++; if (y >= g.d2) { y -= g.d2; x++; } }
-        }
+        em = (tl ^ th) & im;
+        sm = tl & th & im;
+        Eb[i0 >> 5] = em;
+        Sb[i0 >> 5] = sm;
       }
-      em = (tl ^ th) & im;
-      sm = tl & th & im;
-      Eb[i0 >> 5] = em;
-      Sb[i0 >> 5] = sm;
+      // both counts in one scan: a tile has 8192 points
+      unsigned tc;
+      const unsigned co = cta_excl_scan_post((unsigned)__popc(em) | ((unsigned)__popc(sm) << 16), s_w, &tc);
+      te = tc & 0xffffu;
+      ts = tc >> 16;
+      eo = co & 0xffffu;
+      if (threadIdx.x == 0) publish_aggregate(desc, tile, te, ts);
+      {
+        unsigned short *buf = s_buf[cur];
+        const unsigned at = threadIdx.x * kListPer;
+        unsigned xe = eo, xs = kListTile - 1 - (co >> 16);
+        unsigned mm = em;
+        while (mm) { const int u = __ffs(mm) - 1; mm &= mm - 1; buf[xe++] = (unsigned short)(at + u); }
+        mm = Z ? sm : 0u;
+        while (mm) { const int u = __ffs(mm) - 1; mm &= mm - 1; buf[xs--] = (unsigned short)(at + u); }
+      }
     }
-    unsigned te, ts;
-    const unsigned eo = cta_excl_scan_post((unsigned)__popc(em), s_w1, &te);
-    const unsigned so = cta_excl_scan_post((unsigned)__popc(sm), s_w2, &ts);
-    if (threadIdx.x == 0) publish_aggregate(desc, tile, te, ts);
-    {
-      unsigned xe = eo, xs = so;
-      unsigned mm = em;
-      while (mm) { const int u = __ffs(mm) - 1; mm &= mm - 1; s_buf[xe++] = (unsigned)(i0 + u); }
-      mm = Z ? sm : 0u;
-      while (mm) { const int u = __ffs(mm) - 1; mm &= mm - 1; s_buf[kListTile - 1 - xs++] = (unsigned)(i0 + u); }
+    if (prev >= 0) {
+      const Prefix pf = lookback_cta<kWarps>(desc, prev, p_te, p_ts, err);
+      if (threadIdx.x == 0) {
+        s_xb = pf.bytes;
+        s_zb = pf.cnt;
+        if (prev == ntiles - 1) *tot = ((pf.bytes + p_te) << 32) | (pf.cnt + p_ts);
+      }
+      __syncthreads();
+      const unsigned long long xb = s_xb, zb = s_zb;
+      const long long b0 = prev * kListTile;
+      // list position of the first extremum of this thread's bitmap word
+      const long long i0 = b0 + (long long)threadIdx.x * kListPer;
+      if (i0 < n) XP[i0 >> 5] = (unsigned)(xb + p_eo);
+      // a list position past n means corrupt tile offsets: recorded, not written
+      if (xb + p_te > (unsigned long long)n || zb + p_ts > (unsigned long long)n) {
+        if (threadIdx.x == 0) atomicExch(err, kErrMalformed);
+      } else {
+        const unsigned short *buf = s_buf[cur ^ 1];
+        for (unsigned k = threadIdx.x; k < p_te; k += kPostThreads) X[xb + k] = (unsigned)b0 + buf[k];
+        if (Z)
+          for (unsigned k = threadIdx.x; k < p_ts; k += kPostThreads)
+            Z[zb + k] = (unsigned)b0 + buf[kListTile - 1 - k];
+      }
     }
-    const Prefix pf = lookback_cta<kWarps>(desc, tile, te, ts, err);
-    if (threadIdx.x == 0) {
-      s_xb = pf.bytes;
-      s_zb = pf.cnt;
-      if (tile == ntiles - 1) *tot = ((pf.bytes + te) << 32) | (pf.cnt + ts);
-    }
-    __syncthreads();
-    const unsigned long long xb = s_xb, zb = s_zb;
-    // list position of the first extremum of this thread's bitmap word
-    if (i0 < n) XP[i0 >> 5] = (unsigned)(xb + eo);
-    // a list position past n means corrupt tile offsets: recorded, not written
-    if (xb + te > (unsigned long long)n || zb + ts > (unsigned long long)n) {
-      if (threadIdx.x == 0) atomicExch(err, kErrMalformed);
-    } else {
-      for (unsigned k = threadIdx.x; k < te; k += kPostThreads) X[xb + k] = s_buf[k];
-      if (Z)
-        for (unsigned k = threadIdx.x; k < ts; k += kPostThreads) Z[zb + k] = s_buf[kListTile - 1 - k];
-    }
-    __syncthreads();
+    if (!more) break;
+    prev = tile;
+    p_te = te;
+    p_ts = ts;
+    p_eo = eo;
   }
 }
 
@@ -1362,9 +1386,9 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
     // every item in flight at once: one launch, no worklist to start from
     const unsigned *none = nullptr;
     a.ONLY = ni_bits;
-    void *args[] = {(void *)&a,    (void *)&list, (void *)&none, (void *)&most, (void *)(count_dev ? &count_dev : &no_total),
-                    (void *)&none, (void *)&none, (void *)&W0,   (void *)&W1,   (void *)&cnts,
-                    (void *)&bar,  (void *)&status};
+    const unsigned **total = count_dev ? &count_dev : &no_total;
+    void *args[] = {(void *)&a,    (void *)&list, (void *)&none, (void *)&most, (void *)total,   (void *)&none,
+                    (void *)&none, (void *)&W0,   (void *)&W1,   (void *)&cnts, (void *)&bar,    (void *)&status};
     const unsigned need = (most + kPostThreads - 1) / kPostThreads;
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)pass_coop_kernel<PASS, ND>,
                                                       dim3(need ? need : 1), dim3(kPostThreads), args, 0, s);
