@@ -12,10 +12,9 @@
 //     S[e] = (generation << 32) | float bits: one 64-bit word that a reader
 //     takes whole (relaxed), so value and readiness never need ordering;
 //   * a candidate is computed once every EARLIER candidate it reads has its
-//     result for this pass (read from S); otherwise it is retried (stencil
-//     and enforcement: a few times, a CTA barrier apart; RBF and axis
-//     pattern: bounded polls of the missing words) and then deferred to the
-//     next round;
+//     result for this pass (read from S); otherwise its warp looks again at
+//     the missing words, a bounded number of times, and runs what became
+//     ready in between, and then it is deferred to the next round;
 //   * every LATER point a candidate reads lists that candidate among its own
 //     earlier reads, so it cannot have been updated yet: F still holds its
 //     pre-pass value, exactly as in the serial pass.
@@ -25,8 +24,9 @@
 // candidate face neighbour, and the enforcement pass proper runs only over the
 // rest (face_item_run, enforce_sparse_kernel).  The raw decoded value each
 // point is clamped against is the item's own F value before its write when
-// the field is the decoded field itself, else gathered per list entry when
-// the lists are built.  Floating-point expressions use explicit round-to-nearest
+// the field is the decoded field itself, else the original field's; the
+// axis pass of the decoded field, which follows RBF, has them gathered first.
+// Floating-point expressions use explicit round-to-nearest
 // intrinsics so that no multiply-add is contracted (the reference host code is
 // compiled without contraction).
 #include <cfloat>
@@ -1169,10 +1169,10 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, int spin_l
 }
 
 // The rounds of a pass after round 1 (or all of them) in one cooperative
-// launch: rounds are separated by grid barriers instead of host round trips.  The worklist starts as W_start with
-// *nstart_dev items (the deferred items of a round-0 launch) or, when W_start
-// is null, as sel (list indices; null = the whole list) with the pass's total
-// item count.  The total is *total_dev when that is not null, else total.
+// launch: rounds are separated by grid barriers instead of host round trips.
+// The worklist starts as W_start with *nstart_dev items (the deferred items of
+// a round-0 launch) or, when W_start is null, as the list positions themselves,
+// *total_dev of them when that is not null, else total.
 // Worklists and counters written during the launch are read through L2
 // (__ldcg), since other SMs wrote them.  Every CTA takes the same branch at
 // every barrier: the counts it reads are final after the barrier.
@@ -1183,11 +1183,11 @@ constexpr int kCoopRoundLimit = 100000;
 // resident threads more than registers.
 template <int PASS, int ND>
 __global__ void __launch_bounds__(kPostThreads, 2)
-pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, const unsigned *sel, unsigned total,
+pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, unsigned total,
                  const unsigned *total_dev, const unsigned *W_start, const unsigned *nstart_dev, unsigned *Wx,
                  unsigned *Wy, unsigned *cnts, unsigned *bar, unsigned long long *status) {
   const unsigned tot = total_dev ? __ldcg(total_dev) : total;
-  const unsigned *W = W_start ? W_start : sel;   // null: list positions themselves
+  const unsigned *W = W_start;   // null: list positions themselves
   unsigned nw = W_start ? __ldcg(nstart_dev) : tot;
   const bool after_round0 = W_start != nullptr;
   int b = 0;
@@ -1390,7 +1390,7 @@ static int finish_rounds(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, u
 }
 
 // Runs one pass: round 0 as one launch over all of its items -- list
-// positions 0 .. count-1, or sel[0 .. *count_dev) (count known only on the
+// positions 0 .. count-1, or 0 .. *count_dev-1 (count known only on the
 // device), or the set bits of the bitmap ni_bits of ni_words words (the
 // enforcement after the fused stencil) -- then the rounds over the deferred
 // items: in one cooperative launch that reads its counts on the device (after
@@ -1400,7 +1400,7 @@ static int finish_rounds(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, u
 // whole pass (60x90, the stencil 22 -> 13 us, enforcement 19 -> 10, RBF 18 ->
 // 14: such a field spends its time on launches).
 template <int PASS, int ND>
-static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const unsigned *sel, unsigned count,
+static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, unsigned count,
                     unsigned most, const unsigned *count_dev, unsigned *W0, unsigned *W1,
                     const unsigned *ni_bits = nullptr, unsigned ni_words = 0) {
   if (ni_bits ? ni_words == 0 : (!count_dev && count == 0)) return 0;
@@ -1416,8 +1416,8 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
     const unsigned *none = nullptr;
     a.ONLY = ni_bits;
     const unsigned **total = count_dev ? &count_dev : &no_total;
-    void *args[] = {(void *)&a,    (void *)&list, (void *)&none, (void *)&most, (void *)total,   (void *)&none,
-                    (void *)&none, (void *)&W0,   (void *)&W1,   (void *)&cnts, (void *)&bar,    (void *)&status};
+    void *args[] = {(void *)&a,    (void *)&list, (void *)&most, (void *)total,   (void *)&none,  (void *)&none,
+                    (void *)&W0,   (void *)&W1,   (void *)&cnts, (void *)&bar,    (void *)&status};
     const unsigned need = (most + kPostThreads - 1) / kPostThreads;
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)pass_coop_kernel<PASS, ND>,
                                                       dim3(need ? need : 1), dim3(kPostThreads), args, 0, s);
@@ -1429,10 +1429,10 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
     enforce_sparse_kernel<ND><<<(ni_words + kSparseWords - 1) / kSparseWords, kPostThreads, 0, s>>>(
         a, list, ni_bits, ni_words, W0, n0);
   else if (count_dev)
-    pass_round_dev_kernel<PASS, ND><<<dev_grid<PASS, ND>(ctx), kPostThreads, 0, s>>>(a, list, sel, count_dev, W0, n0);
+    pass_round_dev_kernel<PASS, ND><<<dev_grid<PASS, ND>(ctx), kPostThreads, 0, s>>>(a, list, nullptr, count_dev, W0, n0);
   else
     pass_round_kernel<PASS, ND><<<(count + kPostThreads - 1) / kPostThreads, kPostThreads, 0, s>>>(
-        a, list, sel, count, W0, n0);
+        a, list, nullptr, count, W0, n0);
   ctx->launches += 1;
   if (cuda_fail(cudaGetLastError(), "pass round")) return -1;
   if (!grid) return finish_rounds<PASS, ND>(ctx, a, list, W0, W1);
@@ -1448,7 +1448,7 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, const 
     Wx = W0;
     Wy = W1;
   }
-  void *args[] = {(void *)&a,       (void *)&list,   (void *)&sel, (void *)&zero, (void *)&no_total,
+  void *args[] = {(void *)&a,       (void *)&list,   (void *)&zero, (void *)&no_total,
                   (void *)&W_start, (void *)&nstart, (void *)&Wx,  (void *)&Wy,   (void *)&cnts,
                   (void *)&bar,     (void *)&status};
   if (cuda_fail(cudaLaunchCooperativeKernel((const void *)pass_coop_kernel<PASS, ND>, dim3(grid), dim3(kPostThreads),
@@ -1481,16 +1481,16 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
     a.gen = next_gen(ctx);
     a.NI = NIb;
     a.RAW = raw_in_F ? OX : nullptr;
-    if (run_pass<kPassStencil, ND>(ctx, a, X, nullptr, nx, nx, nullptr, W0, W1)) return -1;
+    if (run_pass<kPassStencil, ND>(ctx, a, X, nx, nx, nullptr, W0, W1)) return -1;
     a.NI = nullptr;
     a.RAW = nullptr;
     a.OL = raw_in_F ? OX : nullptr;   // raw values of the remaining items, stashed by the stencil
     tl_mark(ctx, "post_stencil");
     a.gen = next_gen(ctx);
-    if (run_pass<kPassEnforce, ND>(ctx, a, X, nullptr, 0, nx, nullptr, W0, W1, NIb, ni_words)) return -1;
+    if (run_pass<kPassEnforce, ND>(ctx, a, X, 0, nx, nullptr, W0, W1, NIb, ni_words)) return -1;
   } else {
     a.gen = next_gen(ctx);
-    if (run_pass<kPassEnforce, ND>(ctx, a, X, nullptr, nx, nx, nullptr, W0, W1)) return -1;
+    if (run_pass<kPassEnforce, ND>(ctx, a, X, nx, nx, nullptr, W0, W1)) return -1;
   }
   tl_mark(ctx, "post_enforce");
   // the lost saddles (from F after enforcement); RBF reads the locks from the
@@ -1506,12 +1506,12 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
   // Saddles keep their raw values until RBF itself writes them.
   a.OL = nullptr;
   a.gen = next_gen(ctx);
-  if (nz && run_pass<kPassRbf, ND>(ctx, a, Y, nullptr, 0, nz, ycnt, W0, W1)) return -1;
+  if (nz && run_pass<kPassRbf, ND>(ctx, a, Y, 0, nz, ycnt, W0, W1)) return -1;
   tl_mark(ctx, "post_rbf");
   if (axis_stencil && ND == 3 && nz) {
     a.OL = raw_in_F ? OZ : nullptr;   // gathered before the passes: RBF has changed some saddles
     a.gen = next_gen(ctx);
-    if (run_pass<kPassAxis, ND>(ctx, a, Z, nullptr, nz, nz, nullptr, W0, W1)) return -1;
+    if (run_pass<kPassAxis, ND>(ctx, a, Z, nz, nz, nullptr, W0, W1)) return -1;
     tl_mark(ctx, "post_axis");
   }
   return 0;
