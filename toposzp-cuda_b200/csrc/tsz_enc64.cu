@@ -209,7 +209,8 @@ __device__ __forceinline__ void e64_front(const Enc64Args &a, long long tile, bo
           const unsigned k = d3 - z0;                     // 1 .. 7
           const bool plane_in = !D3 || xx - 1u < (unsigned)a.g.d1 - 2u;
           if (plane_in && y - 1u < (unsigned)a.g.d2 - 2u) inter = ((1u << k) - 1u) >> 1;
-          if (plane_in && y < (unsigned)a.g.d2 - 2u) inter |= 0xffu & ~((2u << k) - 1u);
+          // (y + 2 < d2, not y < d2 - 2: one row a plane must not wrap)
+          if (plane_in && y + 2u < (unsigned)a.g.d2) inter |= 0xffu & ~((2u << k) - 1u);
           inter = __brev(inter) >> 24;
         } else {
           inter = __brev(octet_interior(g0, nv, a.g)) >> 24;
