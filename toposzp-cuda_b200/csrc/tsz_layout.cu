@@ -209,7 +209,8 @@ static int detect_chunks(szp_b200_ctx *ctx, Arena &A, const unsigned char *cmp, 
   };
   auto try_T = [&](int T, unsigned long long bound, bool *ok) -> int {
     if (whole_T(T, bound, ok)) return -1;
-    if (*ok || T == 1) return 0;   // one chunk: the walk was the chunk's own
+    // one chunk from payload offset 0: the walk was the chunk's own
+    if (*ok || (T == 1 && tab[0] == 0)) return 0;
     const unsigned long long hdr = (unsigned long long)T * 8;
     if (hdr >= bound) return 0;
     const unsigned long long bpt = (nb + T - 1) / T;
