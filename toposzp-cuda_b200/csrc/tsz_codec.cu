@@ -412,7 +412,7 @@ decode_kernel(DecArgs a) {
     const int len = (int)((n - base) < B ? (n - base) : B);
     // offsets must be monotone and inside the staged span; otherwise the
     // stream is malformed and the block is skipped (no out-of-range reads)
-    if (s_off[bi] < s_off[0] || s_off[bi] + 4 > hi || s_off[bi + 1] < s_off[bi] ||
+    if (s_off[bi] < s_off[0] || s_off[bi] > hi || hi - s_off[bi] < 4 || s_off[bi + 1] < s_off[bi] ||
         s_off[bi + 1] > s_off[nb]) {
       if (lane == 0) atomicExch(a.err, kErrMalformed);
       continue;

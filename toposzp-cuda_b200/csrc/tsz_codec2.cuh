@@ -748,7 +748,8 @@ decode2_kernel(DecArgs a) {
   bool ok = have;
   unsigned start = 0, bend = 0;
   if (ok) {
-    if (s_off[bi] < s_off[0] || s_off[bi] + 4 > hi || s_off[bi + 1] < s_off[bi] || s_off[bi + 1] > s_off[nb])
+    if (s_off[bi] < s_off[0] || s_off[bi] > hi || hi - s_off[bi] < 4 || s_off[bi + 1] < s_off[bi] ||
+        s_off[bi + 1] > s_off[nb])
       ok = false;
     start = (unsigned)(s_off[bi] - lo) + ib;
     bend = (unsigned)((s_off[bi + 1] < hi ? s_off[bi + 1] : hi) - lo) + ib;

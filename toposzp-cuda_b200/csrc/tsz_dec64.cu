@@ -240,7 +240,8 @@ __global__ void __launch_bounds__(kD64Threads, 16) decode64_kernel(DecArgs a) {
     if (tid < nb) {
       const long long left = n - (b0 + tid) * 64;
       const unsigned len = left < 64 ? (unsigned)left : 64u;
-      bool ok = !(o0 < lo || o0 + 4 > hi || o1 < o0 || o1 > end);
+      // (no sum of an offset, which may be anything in a caller's index)
+      bool ok = !(o0 < lo || o0 > hi || hi - o0 < 4 || o1 < o0 || o1 > end);
       if (ok) {
         h.x = (unsigned)(o0 - lo) + ib;
         const unsigned bend = (unsigned)((o1 < hi ? o1 : hi) - lo) + ib;
