@@ -922,6 +922,7 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
   // sort positions: one per extremum tag, unless the caller knows the count
   const unsigned long long E = sort_count != ~0ull ? sort_count : ctx->h_words[6];
   const int *spp = nullptr;
+  if (post_words_clear(ctx)) return -1;
   if (E > 0 && have_sort) {
     if (parse && (ctx->h_words[18] == 0 || ctx->h_words[19] != 0)) {
       if (parse_failed) *parse_failed = true;
@@ -935,7 +936,8 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
     b.n = E;
     b.B = B;
     b.out_i = sp;
-    b.err = reinterpret_cast<int *>(w + 4);
+    // read back with the status of the passes, which take what it decodes
+    b.err = reinterpret_cast<int *>(w + kSortStatusWord);
     if (cuda_fail(launch_decode(false, b, s), "decode sort")) return -1;
     ctx->launches += 1;
     tl_mark(ctx, "decode_sort");

@@ -106,6 +106,8 @@ unsigned long long *post_words(szp_b200_ctx *ctx, unsigned long long n);
 bool post_planes(szp_b200_ctx *ctx, unsigned long long n, unsigned **TL, unsigned **TH);
 int post_planes_from_bytes(szp_b200_ctx *ctx, const unsigned char *d_T, unsigned long long n, unsigned *TL,
                            unsigned *TH);
+constexpr int kSortStatusWord = 7;   // of d_words: status of the sort positions' decoder
+int post_words_clear(szp_b200_ctx *ctx);
 int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const unsigned *d_TL,
                      const unsigned *d_TH, unsigned long long *d_S, const PostLists &l, unsigned long long tot,
                      const int *d_sp, unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,

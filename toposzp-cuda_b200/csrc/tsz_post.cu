@@ -1548,7 +1548,15 @@ int post_lists_begin(szp_b200_ctx *ctx, const unsigned *d_TL, const unsigned *d_
   return cuda_fail(cudaGetLastError(), "lists") ? -1 : 0;
 }
 
-// The passes over the lists of post_lists_begin, whose totals the caller has read.
+// Clears the words of the passes: [4] status, [5] restored, [7] status of the
+// sort positions' decoder (kSortStatusWord), [8] lost saddles, [9] pass status,
+// and the words of each pass.
+int post_words_clear(szp_b200_ctx *ctx) {
+  return cuda_fail(cudaMemsetAsync(ctx->d_words, 0, (kPassWord + 4 * 8) * 8, ctx->stream), "memset") ? -1 : 0;
+}
+
+// The passes over the lists of post_lists_begin, whose totals the caller has
+// read; between the two, post_words_clear and then what decodes d_sp.
 int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const unsigned *d_TL,
                      const unsigned *d_TH, unsigned long long *d_S, const PostLists &l, unsigned long long tot,
                      const int *d_sp, unsigned long long n_sp, const Geom &g, float eb, int axis_stencil,
@@ -1558,9 +1566,7 @@ int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, cons
   cudaGetDevice(&dev);
   if (cuda_fail(upload_weights(dev), "weights")) return -1;
   cudaStream_t s = ctx->stream;
-  // [4] status, [5] restored, [8] lost saddles, [9] pass status, and the words of each pass
   unsigned long long *w = ctx->d_words;
-  if (cuda_fail(cudaMemsetAsync(w, 0, (kPassWord + 4 * 8) * 8, s), "memset")) return -1;
   // post-processing of the decoded field itself: each item reads its raw
   // value from F before it writes (no gathered raw lists), except the
   // axis-pattern pass, which runs after RBF has changed saddles
@@ -1597,6 +1603,10 @@ int postprocess_with(szp_b200_ctx *ctx, float *d_data, const float *d_orig, cons
   if (cuda_fail(cudaMemcpyAsync(ctx->h_words, w, 96, cudaMemcpyDeviceToHost, s), "D2H") ||
       cuda_fail(cudaStreamSynchronize(s), "postprocess"))
     return -1;
+  if (ctx->h_words[kSortStatusWord] & 0xffffffffu) {
+    set_error("decoder reported malformed sort-position stream");
+    return -1;
+  }
   const int err = (int)(ctx->h_words[4] & 0xffffffffu);
   if (err) { set_error("post-processing status %d", err); return -1; }
   if (ctx->h_words[9] == 1) { set_error("post-processing pass did not converge"); return -1; }
@@ -1677,6 +1687,7 @@ int postprocess(szp_b200_ctx *ctx, float *d_data, const float *d_orig, const int
   tl_mark(ctx, "post_lists");
   const int err = (int)(ctx->h_words[5] & 0xffffffffu);
   if (err) { set_error("post-processing status %d", err); return -1; }
+  if (post_words_clear(ctx)) return -1;
   return postprocess_with(ctx, d_data, d_orig, TL, TH, S, l, ctx->h_words[2], d_sp, n_sp, g, eb, axis_stencil,
                           restored_out);
 }
