@@ -521,7 +521,9 @@ SZP_B200_API double szp_b200_server_now(szp_b200_server *s);
  * elements, and its batch compressor for the largest merged launch (up to
  * max_batch fields of 2^24 elements in total), so that serving them allocates
  * nothing (an allocation while other workers run would stall the device for
- * all of them).  A relative-bound compression of more than 2^24 elements runs
+ * all of them).  For requests of 2^21 elements and more each worker also takes
+ * the rank stage's bitmap (118 MB), where the device has room for it; without
+ * it the same streams take longer.  A relative-bound compression of more than 2^24 elements runs
  * as a batch of one and still grows its worker's batch compressor the first
  * time.  Call it while no request is in flight.  Returns 0 on success. */
 SZP_B200_API int szp_b200_server_reserve(szp_b200_server *s, size_t max_elements);

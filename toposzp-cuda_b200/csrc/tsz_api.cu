@@ -72,7 +72,6 @@ int ctx_reserve_for(szp_b200_ctx *ctx, unsigned long long n, int B) {
                      parse_scratch_bytes(stream_bound(n, B, true) - 8, B, true) +
                      parse_scratch_bytes(stream_bound(n, B, false) - 8, B, false);
   if (!ctx->scratch.reserve(comp > dec ? comp : dec)) return -1;
-  if (rank_bits_reserve(ctx)) return -1;
   return post_words(ctx, n) ? 0 : -1;
 }
 

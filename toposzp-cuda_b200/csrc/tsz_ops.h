@@ -53,7 +53,8 @@ int encode_pass(szp_b200_ctx *ctx, int mode, const float *d_data, const int *d_i
 // Returns 0, -1 on an error, or 1 when the values are left to the bucket
 // ranking (which needs pairs).
 constexpr int kRbStatWord = 8;   // of d_words: RankBits::stat (32 bytes)
-int rank_bits_reserve(szp_b200_ctx *ctx);
+bool rank_bits_reserve(szp_b200_ctx *ctx);
+size_t rank_bits_bytes();        // that a workspace keeps for it
 bool rank_bits_begin(szp_b200_ctx *ctx, float eb, RankBits *rb);
 int rank_bits_finish(szp_b200_ctx *ctx, const RankBits &rb, const unsigned *h_stat, float eb, const unsigned *d_codes,
                      const uint2 *d_pairs, unsigned long long K, unsigned long long E, int *d_sp);
@@ -62,7 +63,6 @@ int rank_bits_from_pairs(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long 
 // rb: the bits that the pairs set, to be cleared (null: none)
 int rank_small(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long long K, float eb, int *d_sp,
                const RankBits *rb = nullptr);
-size_t rank_bits_scratch_bytes();
 
 // Dense rank of every extremum inside its quantization bin.
 //   pairs[k] = (orderable value code, extremum index or kNoExtremum), k < K
@@ -143,7 +143,8 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
                         bool cpu_layout = false, unsigned long long sort_count = ~0ull);
 
 // Grows a workspace so that compressing or decompressing (with
-// post-processing) a field of n elements allocates nothing more.
+// post-processing) a field of n elements allocates nothing more (but the rank
+// stage's bitmap, which is optional: rank_bits_reserve).
 int ctx_reserve_for(szp_b200_ctx *ctx, unsigned long long n, int B);
 
 }  // namespace tsz

@@ -321,17 +321,36 @@ static int host_bin(unsigned code, float eb, double inv) {
 
 static size_t rb_bytes() { return (size_t)kRbUnits * 16; }
 
-int rank_bits_reserve(szp_b200_ctx *ctx) {
-  if (ctx->rank_bits) return 0;
+// The workspace's allocation: the bits, the values aside and the first pairs,
+// the bins' prefix counts and the tiles' counts.
+struct RbStore {
+  size_t side, first, bins, cnt, bytes;
+  RbStore() {
+    side = rb_bytes();
+    first = side + kSideCap * sizeof(uint2);
+    bins = first + kRankSmall * sizeof(uint2);
+    cnt = bins + (size_t)kMaxBins * 4;
+    bytes = cnt + ((size_t)kRbUnits / kRbTile + 2) * 4;
+  }
+};
+
+size_t rank_bits_bytes() { return RbStore().bytes; }
+
+// Whether the workspace has the bitmap, or could get it.  It is optional (the
+// bucket ranking gives the same positions without it): no room for it is no
+// error, and is remembered, so that later calls do not try again.
+bool rank_bits_reserve(szp_b200_ctx *ctx) {
+  if (ctx->rank_bits) return true;
+  if (ctx->rank_bits_no_room) return false;
   void *p = nullptr;
-  if (cudaMalloc(&p, rb_bytes() + (kSideCap + kRankSmall) * sizeof(uint2)) != cudaSuccess) {
+  if (cudaMalloc(&p, rank_bits_bytes()) != cudaSuccess) {
     cudaGetLastError();
-    set_error("device allocation of %zu bytes failed", rb_bytes());
-    return -1;
+    ctx->rank_bits_no_room = true;
+    return false;
   }
   ctx->rank_bits = static_cast<unsigned *>(p);
   ctx->rank_bits_dirty = true;
-  return 0;
+  return true;
 }
 
 bool rank_bits_begin(szp_b200_ctx *ctx, float eb, RankBits *rb) {
@@ -346,12 +365,14 @@ bool rank_bits_begin(szp_b200_ctx *ctx, float eb, RankBits *rb) {
   memcpy(&hb, &h, 4);
   if (zb == 0) zb = 1;
   if (hb <= zb || 2ull * (hb - zb) / kRbBits + 2 > kRbUnits) return false;
-  if (rank_bits_reserve(ctx)) { clear_error(); return false; }
+  if (!rank_bits_reserve(ctx)) return false;
+  const RbStore at;
+  unsigned char *base = reinterpret_cast<unsigned char *>(ctx->rank_bits);
   rb->bits = ctx->rank_bits;
   rb->rz = zb;
   rb->rh = hb;
-  rb->side = reinterpret_cast<uint2 *>(reinterpret_cast<unsigned char *>(ctx->rank_bits) + rb_bytes());
-  rb->first = rb->side + kSideCap;
+  rb->side = reinterpret_cast<uint2 *>(base + at.side);
+  rb->first = reinterpret_cast<uint2 *>(base + at.first);
   rb->stat = reinterpret_cast<unsigned *>(ctx->d_words + kRbStatWord);
   cudaStream_t s = ctx->stream;
   if (ctx->rank_bits_dirty && cuda_fail(cudaMemsetAsync(ctx->rank_bits, 0, rb_bytes(), s), "memset")) return false;
@@ -383,11 +404,10 @@ int rank_bits_finish(szp_b200_ctx *ctx, const RankBits &rb, const unsigned *h_st
   cudaStream_t s = ctx->stream;
   const unsigned s0 = lo / kRbBits, s1 = hi > lo ? (hi - 1u) / kRbBits + 1u : s0;
   if (E) {
-    Arena &A = ctx->scratch;
-    unsigned *binp = A.take<unsigned>(g.nbins);
+    const RbStore at;
+    unsigned char *base = reinterpret_cast<unsigned char *>(ctx->rank_bits);
+    unsigned *binp = reinterpret_cast<unsigned *>(base + at.bins), *cnt = reinterpret_cast<unsigned *>(base + at.cnt);
     const unsigned ntiles = (s1 - s0 + kRbTile - 1) / kRbTile;
-    unsigned *cnt = A.take<unsigned>(ntiles + 1);
-    if (!binp || !cnt) { set_error("scratch arena too small for the rank stage"); return -1; }
     if (ntiles) {
       rank_bits_count_kernel<<<ntiles, kThreads, 0, s>>>(rb.bits, s0, s1, cnt);
       rank_bits_prefix_kernel<<<ntiles, kThreads, 0, s>>>(rb.bits, s0, s1, cnt);
@@ -527,10 +547,6 @@ int rank_small_fields(szp_b200_ctx *ctx, const uint2 *d_pairs, const SmallField 
   rank_small_kernel<<<count, kSmallThreads, 0, ctx->stream>>>(d_pairs, 0, 1.0f, 1.0, d_sp, RankBits{}, d_fields);
   ctx->launches += 1;
   return cuda_fail(cudaGetLastError(), "rank kernel") ? -1 : 0;
-}
-
-size_t rank_bits_scratch_bytes() {
-  return a256((size_t)kMaxBins * 4) + a256(((size_t)kRbUnits / kRbTile + 2) * 4);
 }
 
 }  // namespace tsz

@@ -46,6 +46,7 @@ struct szp_b200_ctx {
   unsigned post_gen = 0;
   unsigned *rank_bits = nullptr;           // bitmap of the rank stage, zero between calls unless dirty
   bool rank_bits_dirty = false;
+  bool rank_bits_no_room = false;          // its allocation failed once
   // stage timeline of the last call (CUDA events on the workspace stream)
   static constexpr int kMaxStages = 24;
   cudaEvent_t ev[kMaxStages + 1] = {};

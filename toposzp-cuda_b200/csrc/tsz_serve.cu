@@ -72,13 +72,21 @@ struct szp_b200_server {
 
 namespace tsz {
 
+// A compression of at least this many elements fills the GPU by itself: it
+// runs alone through the fused single-field path (the blockSize-64 encoder
+// and the single-field rank), and smaller ones are merged into batched
+// launches behind a small head.
+constexpr size_t kAloneElems = (size_t)1 << 21;
+
 // Estimated device working set of a request beyond its caller-owned buffers
 // (bytes per element: compression keeps CP pairs, bins, ranks and encoder
-// scratch; decompression keeps the raw copy, tags, ranks and the
-// post-processing lists).
+// scratch, and alone the bitmap of its rank stage; decompression keeps the raw
+// copy, tags, ranks and the post-processing lists).
 static size_t request_cost(const szp_b200_request *r) {
   const size_t n = elems_of(r->geom);
-  return r->op == SZP_B200_OP_COMPRESS ? 40 * n + (1u << 20) : 32 * n + (1u << 20);
+  if (r->op != SZP_B200_OP_COMPRESS) return 32 * n + (1u << 20);
+  const bool alone = n >= kAloneElems && r->blockSize == 64 && !r->rel;
+  return 40 * n + (1u << 20) + (alone ? rank_bits_bytes() : 0);
 }
 
 static void fail_request(szp_b200_request *r, const char *msg) {
@@ -113,11 +121,6 @@ static int compress_group(Slot &sl, szp_b200_request **rs, int count) {
   return rc;
 }
 
-// A compression of at least this many elements fills the GPU by itself: it
-// runs alone through the fused single-field path (the blockSize-64 encoder
-// and the single-field rank), and smaller ones are merged into batched
-// launches behind a small head.
-constexpr size_t kAloneElems = (size_t)1 << 21;
 // Elements of one merged launch at most: the workers' batch compressors are
 // sized for it up front (szp_b200_server_reserve), so serving allocates
 // nothing -- a buffer that grew would free memory, which waits for every
@@ -317,6 +320,13 @@ int szp_b200_server_reserve(szp_b200_server *S, size_t max_elements) {
     if (ctx_reserve_for(sl.ctx, max_elements, S->cfg.blockSize) ||
         szp_b200_batch_reserve(sl.batch, S->cfg.max_batch, kBatchElems))
       return -1;
+  // after every worker has what it cannot do without: the bitmaps of the rank
+  // stage, for the requests that run alone; one that finds no room is done without
+  if (max_elements >= kAloneElems && S->cfg.blockSize == 64)
+    for (auto &sl : S->slots) {
+      DeviceGuard dg(sl.ctx);
+      rank_bits_reserve(sl.ctx);
+    }
   return 0;
 }
 

@@ -1141,9 +1141,9 @@ size_t rank_scratch_bytes(unsigned long long K, int sm_count) {
   // fallback worst case: all K records (two key/value ping-pong buffers + histogram)
   const size_t fb = a256(K * 8) * 2 + a256(K * 4) * 2 + a256(256 * ((K + kRadixTile - 1) / kRadixTile) * 4) +
                     a256(scan_parts(256 * ((K + kRadixTile - 1) / kRadixTile) + K) * 4);
-  // records (8 B) and, for given bins, their permuted bins (4 B); the bitmap ranking's tables
-  return (K > (unsigned long long)kRankSmall ? rank_bits_scratch_bytes() : 0) + a256(G * NB * 4) + a256(NB * 4) + a256((NB + 1) * 8) + a256(K * 8) + a256(K * 4) +
-         a256(NB * 4) * 5 + a256(32) + fb + a256((NB + 1) * 8) * 2 + 4096;
+  // records (8 B) and, for given bins, their permuted bins (4 B)
+  return a256(G * NB * 4) + a256(NB * 4) + a256((NB + 1) * 8) + a256(K * 8) + a256(K * 4) + a256(NB * 4) * 5 +
+         a256(32) + fb + a256((NB + 1) * 8) * 2 + 4096;
 }
 
 // ---------------------------------------------------------------------------
