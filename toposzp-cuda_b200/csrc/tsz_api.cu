@@ -66,7 +66,7 @@ int ctx_reserve_for(szp_b200_ctx *ctx, unsigned long long n, int B) {
   const unsigned long long nb = (n + B - 1) / B;
   // the largest scratch of a fused compression and of a fused decompression
   // with post-processing and device stream parsing
-  const size_t comp = a256(n * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 3 +
+  const size_t comp = a256(n * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 2 +
                       rank_scratch_bytes(n, ctx->sm_count) + 8192;
   const size_t dec = post_scratch_bytes(n) + a256(n * 4) + a256(n) + 8192 + a256(2 * nb * 8) +
                      parse_scratch_bytes(stream_bound(n, B, true) - 8, B, true) +
@@ -719,7 +719,7 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
   const int B = blockSize;
   const unsigned long long nb = (n + B - 1) / B;
   const unsigned long long kcap = n;
-  const size_t need = a256(kcap * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 3 +
+  const size_t need = a256(kcap * 8) + a256(n * 4) + a256((nb / enc_tile_blocks(B) + 2) * sizeof(TileDesc)) * 2 +
                       rank_scratch_bytes(kcap, ctx->sm_count) + 8192;
   if (!ctx->scratch.reserve(need)) return -1;
   Arena &A = ctx->scratch;
@@ -727,7 +727,7 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
   int *sp = A.take<int>(n);
   unsigned long long tot[3];
   // From 2^18 values on the encoder sets the rank's bits itself and hands
-  // over the extrema's codes (in the pairs' place): no pair is written or
+  // over the values' codes (in the pairs' place): no pair is written or
   // read.  Below, the pairs are few and the rank picks its way by their count.
   RankBits rb;
   const EncArgs probe = [&] { EncArgs e{}; e.B = B; e.data = d_data; e.out = d_topo + 8; e.cp_mode = kCpBits; return e; }();
@@ -763,28 +763,16 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
       return -1;
   }
   const unsigned long long K = tot[1], E = tot[2];
-  int left = bits && K == 0 ? 0 : 1;   // 1: to be ranked from pairs
+  if (bits && K == 0) ctx->rank_bits_dirty = false;   // nothing was set
   if (bits && K) {
     unsigned h_stat[8];
     memcpy(h_stat, ctx->h_words + kRbStatWord, sizeof(h_stat));
-    left = rank_bits_finish(ctx, rb, h_stat, absErrBound, reinterpret_cast<const unsigned *>(pairs), nullptr, K, E, sp);
-    if (left < 0) return -1;
-  } else if (bits) {
-    ctx->rank_bits_dirty = false;      // nothing was set
+    const unsigned *codes = reinterpret_cast<const unsigned *>(pairs);
+    const int r = rank_bits_finish(ctx, rb, h_stat, absErrBound, codes, nullptr, K, E, sp);
+    if (r < 0 || (r > 0 && E && rank_positions_codes(ctx, codes, kcap, K, E, absErrBound, sp))) return -1;
   }
   if (E == 0) return 0;
-  if (left) {
-    if (bits) {
-      // values the bits do not cover: the same encoding once more, for its pairs
-      if (ctx->d2h_stream && cuda_fail(cudaStreamSynchronize(ctx->d2h_stream), "sync")) return -1;
-      if (ctx->copy_stream && cuda_fail(cudaStreamSynchronize(ctx->copy_stream), "sync")) return -1;
-      if (encode_pass(ctx, kEncClassify, d_data, nullptr, nullptr, n, B, absErrBound, g, d_topo,
-                      stream_bound(n, B, true), reinterpret_cast<unsigned long long *>(d_blk_index), kCpPairs, pairs,
-                      kcap, tot))
-        return -1;
-    }
-    if (rank_positions(ctx, pairs, nullptr, K, E, absErrBound, sp, !bits)) return -1;
-  }
+  if (!bits && rank_positions(ctx, pairs, nullptr, K, E, absErrBound, sp)) return -1;
   tl_mark(ctx, "rank");
   unsigned long long st[3];
   if (encode_pass(ctx, kEncInts, nullptr, sp, nullptr, E, B, absErrBound, g, d_sort,

@@ -11,7 +11,8 @@ enum EncMode { kEncClassify = 0, kEncTypes = 1, kEncInts = 2, kEncIntTypes = 3, 
 
 // whether the blocks of a mode carry 2-bit tags
 __host__ __device__ constexpr bool mode_tags(int mode) { return mode != kEncInts && mode != kEncQuant; }
-// kCpBits: every value's bit (rb) and the extrema's codes in raster order (blockSize 64 encoder)
+// kCpBits: every value's bit (rb), the extrema's codes in raster order and, from
+// cp_cap codes on, the saddles' (blockSize 64 encoder)
 enum CpMode { kCpNone = 0, kCpRecords = 1, kCpPairs = 2, kCpBits = 3 };
 
 struct EncArgs {
@@ -35,7 +36,7 @@ struct EncArgs {
   int cp_mode;                  // CpMode (kEncClassify only)
   void *cp_out;                 // CriticalPoint / CriticalPoint3D records or uint2 pairs
   unsigned long long cp_cap;
-  RankBits rb;                  // kCpBits (cp_out: extremum codes)
+  RankBits rb;                  // kCpBits (cp_out: 2 cp_cap codes)
   unsigned img_stride;          // octet encoder: bytes of one of its two tile images (0: one image, no pipelining)
 };
 

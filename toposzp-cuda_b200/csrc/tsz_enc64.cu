@@ -508,7 +508,8 @@ __device__ __forceinline__ Prefix e64_lookback(TileDesc *desc, long long t, unsi
 // and of the staged critical points.  The threads that own elements call it.
 template <bool BITS>
 __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, const unsigned char *img,
-                                         const void *stage, const E64Sh &sh, unsigned &nmax, unsigned &cmax) {
+                                         const void *stage, const E64Sh &sh, unsigned &nmax, unsigned &cmax,
+                                         bool &full) {
   const int tid = threadIdx.x;
   const long long n = (long long)a.n;
   const long long nblocks = (n + 63) / 64;
@@ -550,19 +551,25 @@ __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, con
   const unsigned long long cb = sh.gcnt >> 32, eb0 = sh.gcnt & 0xffffffffull;
   const unsigned ntc = sh.tile_cps, nte = sh.tile_ext;
   if (BITS) {
-    // every value's bit; the extrema's codes in raster order
-    const unsigned *st = static_cast<const unsigned *>(stage);
-    for (unsigned k = tid; k < ntc; k += kE64Threads) {
-      const bool is_ext = k < nte;
-      const unsigned code = st[is_ext ? k : kE64Tile - 1u - (k - nte)];
-      const unsigned ext = is_ext ? (unsigned)eb0 + k : kNoExtremum;
-      rb_set(a.rb, code, ext);
-      if (cb + k < kRankSmall) a.rb.first[cb + k] = make_uint2(code, ext);
-      nmax = max(nmax, ~code);
-      cmax = max(cmax, code);
-      if (is_ext && eb0 + k < a.cp_cap) a.code_out[eb0 + k] = code;
+    // every value's bit; the codes of the extrema, and those of the saddles, in
+    // raster order: what the bucket ranking takes where the bits do not do
+    if (cb + ntc > a.cp_cap) {
+      if (tid == 0) atomicExch(a.err, kErrCapacity);
+    } else {
+      const unsigned *st = static_cast<const unsigned *>(stage);
+      unsigned *eo = a.code_out + eb0, *so = a.code_out + a.cp_cap + (cb - eb0) - nte;
+      const bool head = cb < kRankSmall;
+      for (unsigned k = tid; k < ntc; k += kE64Threads) {
+        const bool is_ext = k < nte;
+        const unsigned code = st[is_ext ? k : kE64Tile - 1u + nte - k];
+        const unsigned ext = is_ext ? (unsigned)eb0 + k : kNoExtremum;
+        rb_set(a.rb, code, ext, full);
+        if (head && cb + k < kRankSmall) a.rb.first[cb + k] = make_uint2(code, ext);
+        nmax = max(nmax, ~code);
+        cmax = max(cmax, code);
+        (is_ext ? eo : so)[k] = code;
+      }
     }
-    if (tid == 0 && eb0 + nte > a.cp_cap) atomicExch(a.err, kErrCapacity);
   } else {
     // critical-point pairs in raster order
     const uint2 *st = static_cast<const uint2 *>(stage);
@@ -616,6 +623,7 @@ __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
   long long prev = -1;
   int cur = 0;
   unsigned nmax = 0, cmax = 0;
+  bool full = false;
   while (true) {
     // claimed only now (while the other warps write the last tile out), not a
     // tile ahead: every look-back behind a claimed tile waits for its front half
@@ -644,7 +652,7 @@ __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
     __syncthreads();
     if (owner && prev >= 0) {
       const unsigned char *pp = smem_dyn + (size_t)(cur ^ 1) * kPart;
-      e64_back<BITS>(a, prev, pp, pp + kE64Img, sh[cur ^ 1], nmax, cmax);
+      e64_back<BITS>(a, prev, pp, pp + kE64Img, sh[cur ^ 1], nmax, cmax, full);
     }
     if (!more) break;
     prev = tile;
@@ -672,6 +680,7 @@ enc64_batch_kernel(const EncArgs *__restrict__ fields, const unsigned long long 
   int field = 0, have[3] = {-1, -1, -1};
   bool pending = false;
   unsigned unused0 = 0, unused1 = 0;
+  bool unused2 = false;
   for (int it = 0, cur = 0, slot = 0;; it++, cur ^= 1) {
     const int before = slot == 0 ? 2 : slot - 1;
     if (owner) {
@@ -738,7 +747,8 @@ enc64_batch_kernel(const EncArgs *__restrict__ fields, const unsigned long long 
     __syncthreads();
     if (owner && pending) {
       const unsigned char *pp = smem_dyn + (size_t)(cur ^ 1) * kPart;
-      e64_back<false>(s_args[before], s_claim[before], pp, pp + kE64Img, sh[cur ^ 1], unused0, unused1);
+      e64_back<false>(s_args[before], s_claim[before], pp, pp + kE64Img, sh[cur ^ 1], unused0, unused1,
+                      unused2);
     }
     if (tile < 0) break;
     pending = true;

@@ -23,7 +23,7 @@ struct Enc64Args {
   int *err;                     // status word
   unsigned long long *total;    // [payload bytes, cps, extrema]
   uint2 *cp_out;                // critical-point pairs {value code, extremum index or ~0}, or null:
-  unsigned *code_out;           // extremum codes in raster order, every value's bit in rb
+  unsigned *code_out;           // extremum codes in raster order, from cp_cap on the saddles', every value's bit in rb
   RankBits rb;
   unsigned long long cp_cap;
   int spin_limit;               // look-back polls before giving up (0: default)

@@ -51,7 +51,7 @@ int encode_pass(szp_b200_ctx *ctx, int mode, const float *d_data, const int *d_i
 // finish: positions of the E extrema, from their codes in raster order or
 // from K pairs, h_stat the call's statistics; enqueued, and the bits cleared.
 // Returns 0, -1 on an error, or 1 when the values are left to the bucket
-// ranking (which needs pairs).
+// ranking.
 constexpr int kRbStatWord = 8;   // of d_words: RankBits::stat (32 bytes)
 bool rank_bits_reserve(szp_b200_ctx *ctx);
 size_t rank_bits_bytes();        // that a workspace keeps for it
@@ -68,9 +68,13 @@ int rank_small(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long long K, fl
 //   pairs[k] = (orderable value code, extremum index or kNoExtremum), k < K
 //   writes sp[e] for every extremum e < E.  bins come from the value
 //   (bin = quant_bin(value, eb)); mode_given_bins = true uses bins[k] instead.
-// (try_bits: through the bitmap over the values where it applies)
+// (through the bitmap over the values where it applies)
 int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
-                   unsigned long long K, unsigned long long E, float eb, int *d_sp, bool try_bits = true);
+                   unsigned long long K, unsigned long long E, float eb, int *d_sp);
+// The same, in buckets, from the codes that an encode_pass with kCpBits left:
+// the extrema's, and from cap codes on the K - E saddles'.
+int rank_positions_codes(szp_b200_ctx *ctx, const unsigned *d_codes, unsigned long long cap, unsigned long long K,
+                         unsigned long long E, float eb, int *d_sp);
 
 // Post-processing of a decoded field in place (serial raster semantics of the
 // reference drivers).  types: an int per element.

@@ -55,10 +55,11 @@ __device__ __forceinline__ void sort_keys_2048(unsigned long long (&v)[2], unsig
 __global__ void __launch_bounds__(256)
 rank_bits_pairs_kernel(const uint2 *__restrict__ pairs, unsigned long long K, RankBits rb) {
   unsigned nmax = 0, cmax = 0;
+  bool full = false;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < K; k += stride) {
     const uint2 p = pairs[k];
-    rb_set(rb, p.x, p.y);
+    rb_set(rb, p.x, p.y, full);
     nmax = max(nmax, ~p.x);
     cmax = max(cmax, p.x);
   }
@@ -381,29 +382,38 @@ bool rank_bits_begin(szp_b200_ctx *ctx, float eb, RankBits *rb) {
   return true;
 }
 
+// bits below a code's: its own place, or that of the gap it lies in
+static unsigned rb_place(const RankBits &rb, unsigned code, bool *in) {
+  const unsigned S = rb.rh - rb.rz, mag = ((code >> 31) ? code : ~code) & 0x7FFFFFFFu;
+  unsigned idx;
+  *in = rb_index(rb.rz, rb.rh, code, &idx);
+  return *in ? idx : (mag < rb.rz ? S : ((code >> 31) ? 2u * S : 0u));
+}
+
 int rank_bits_finish(szp_b200_ctx *ctx, const RankBits &rb, const unsigned *h_stat, float eb, const unsigned *d_codes,
                      const uint2 *d_pairs, unsigned long long K, unsigned long long E, int *d_sp) {
   if (!d_pairs && K <= kRankSmall) return rank_small(ctx, rb.first, K, eb, d_sp, &rb);
-  if (h_stat[3] || h_stat[2] > kSideCap) return 1;
   const unsigned cmin = ~h_stat[0], cmax = h_stat[1];
   RbRange g;
   g.rz = rb.rz;
   g.rh = rb.rh;
   g.eb = eb;
   g.inv = 1.0 / (double)eb;
-  const unsigned S = rb.rh - rb.rz;
-  unsigned lo, hi;
-  if (!rb_index(rb.rz, rb.rh, cmin, &lo)) lo = S;
-  hi = rb_index(rb.rz, rb.rh, cmax, &hi) ? hi + 1u : S;
+  // the bits that may be set are those between the smallest and the largest value's
+  bool in;
+  const unsigned lo = rb_place(rb, cmin, &in), top = rb_place(rb, cmax, &in), hi = in ? top + 1u : top;
   g.lo = lo;
   g.hi = hi;
-  g.b0 = host_bin(cmin, eb, g.inv);
-  const long long nb = (long long)host_bin(cmax, eb, g.inv) - g.b0 + 1;
-  if (nb < 1 || nb > (long long)kMaxBins) return 1;
-  g.nbins = (unsigned)nb;
   cudaStream_t s = ctx->stream;
   const unsigned s0 = lo / kRbBits, s1 = hi > lo ? (hi - 1u) / kRbBits + 1u : s0;
-  if (E) {
+  bool apply = !h_stat[3] && h_stat[2] <= kSideCap;
+  if (apply) {
+    g.b0 = host_bin(cmin, eb, g.inv);
+    const long long nb = (long long)host_bin(cmax, eb, g.inv) - g.b0 + 1;
+    apply = nb >= 1 && nb <= (long long)kMaxBins;
+    g.nbins = (unsigned)nb;
+  }
+  if (E && apply) {
     const RbStore at;
     unsigned char *base = reinterpret_cast<unsigned char *>(ctx->rank_bits);
     unsigned *binp = reinterpret_cast<unsigned *>(base + at.bins), *cnt = reinterpret_cast<unsigned *>(base + at.cnt);
@@ -429,7 +439,7 @@ int rank_bits_finish(szp_b200_ctx *ctx, const RankBits &rb, const unsigned *h_st
   // the words that were set, for the next call
   if (s1 > s0 && cuda_fail(cudaMemsetAsync(rb.bits + 4ull * s0, 0, 16ull * (s1 - s0), s), "memset")) return -1;
   ctx->rank_bits_dirty = false;
-  return 0;
+  return apply ? 0 : 1;
 }
 
 int rank_bits_from_pairs(szp_b200_ctx *ctx, const uint2 *d_pairs, unsigned long long K, unsigned long long E, float eb,

@@ -23,7 +23,16 @@
 //
 // Values nearer to zero than 2^-6 eb (two bins share them) are kept aside and
 // sorted; values from 2^30 eb on, more than kSideCap aside, or more than
-// kMaxBins bins are left to the bucket ranking.
+// kMaxBins bins are left to the bucket ranking, which takes the codes that the
+// encoder leaves beside the bits (from a pair list, the pairs).  Such fields,
+// in buckets alone / encoded a second time for pairs / from the codes:
+//   512^3 of zero mean, bound 1/50 of its deviation       6.29 / 6.55 / 5.2 ms
+//   512^3 with seven eighths below the bound              78.0 / 78.9 / 33.8
+//   512^3 in 10 M bins                                    5.38 / 5.74 / 5.0
+//   1800 x 3600 noise below the bound                     3.30 / 3.41 / 2.2
+// (most of it from the gather of the buckets that are radix-sorted, which had
+// one CTA a bucket).  A field with bits for all values pays nothing for the
+// saddles' codes that measures: compression of 512^3 929 / 930 us.
 #pragma once
 #include "tsz_common.cuh"
 
@@ -53,19 +62,32 @@ __host__ __device__ __forceinline__ bool rb_index(unsigned rz, unsigned rh, unsi
   return mag - rz < rh - rz;
 }
 
-__device__ __forceinline__ void rb_set(const RankBits &rb, unsigned code, unsigned ext) {
+// Keeps a value without a bit aside.  The lanes that are here together take
+// their places with one atomic, and a thread that has seen that the bits will
+// not do (full) takes none: in a field that lies near zero every value comes here.
+__device__ __forceinline__ void rb_aside(const RankBits &rb, unsigned code, unsigned ext, bool &full) {
+  const unsigned mag = ((code >> 31) ? code : ~code) & 0x7FFFFFFFu;
+  if (mag >= rb.rh) {
+    rb.stat[3] = 1u;
+    full = true;
+    return;
+  }
+  const unsigned m = __activemask(), lane = threadIdx.x & 31u, first = (unsigned)__ffs((int)m) - 1u;
+  unsigned k = 0;
+  if (lane == first) k = atomicAdd(rb.stat + 2, (unsigned)__popc(m));
+  k = __shfl_sync(m, k, (int)first);
+  full = k + (unsigned)__popc(m) > kSideCap;
+  k += (unsigned)__popc(m & ((1u << lane) - 1u));
+  if (k < kSideCap) rb.side[k] = make_uint2(code, ext);
+}
+
+__device__ __forceinline__ void rb_set(const RankBits &rb, unsigned code, unsigned ext, bool &full) {
   unsigned idx;
   if (rb_index(rb.rz, rb.rh, code, &idx)) {
     const unsigned q = idx / kRbBits, r = idx - q * kRbBits;
     atomicOr(rb.bits + 4u * q + 1u + (r >> 5), 1u << (r & 31u));
-  } else {
-    const unsigned mag = ((code >> 31) ? code : ~code) & 0x7FFFFFFFu;
-    if (mag >= rb.rh) {
-      rb.stat[3] = 1u;
-    } else {
-      const unsigned k = atomicAdd(rb.stat + 2, 1u);
-      if (k < kSideCap) rb.side[k] = make_uint2(code, ext);
-    }
+  } else if (!full) {
+    rb_aside(rb, code, ext, full);
   }
 }
 

@@ -30,10 +30,6 @@ constexpr int kRankThreads = 512;
 constexpr int kMaxSlots = 256;
 constexpr int kBitmapWords = 5120;   // 20 KB bitmap + 20 KB prefix per CTA
 
-// A bucketed record is the critical-point pair itself ({value code, extremum
-// index}).  Its bin is recomputed from the code, or, when the caller supplies
-// bins (batches, whose bins carry per-field offsets, or a given CP list), read
-// from a bin array permuted together with the records.
 // What a batch's field brings to its buckets.
 struct SegField {
   unsigned long long ebase;   // where its extrema's positions start
@@ -41,6 +37,23 @@ struct SegField {
   int logNB;
 };
 
+// The critical points of a list: pairs {value code, extremum index}, or (CODES)
+// the codes of its E extrema in order and, from cap codes on, those of the others.
+struct PairSrc {
+  const uint2 *pairs;
+  const unsigned *codes;
+  unsigned long long E, cap;
+};
+template <bool CODES>
+__device__ __forceinline__ uint2 pair_at(const PairSrc &src, unsigned long long k) {
+  if (!CODES) return src.pairs[k];
+  const bool ext = k < src.E;
+  return make_uint2(src.codes[ext ? k : src.cap + (k - src.E)], ext ? (unsigned)k : kNoExtremum);
+}
+
+// A bucketed record is the critical-point pair itself.  Its bin is recomputed
+// from the code, or, when the caller supplies bins (a given CP list), read from
+// a bin array permuted together with the records.
 struct BinSrc {
   const int *bins;   // bins in record order, or nullptr
   float eb;
@@ -97,8 +110,9 @@ __device__ __forceinline__ unsigned block_excl_scan(unsigned v, unsigned *s_w, u
 constexpr int kHistThreads = 512;
 constexpr int kHistUnroll = 4;
 
+template <bool CODES>
 __global__ void __launch_bounds__(kHistThreads)
-bucket_hist_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, unsigned long long K, int logNB,
+bucket_hist_kernel(PairSrc src, BinSrc bin_of, unsigned long long K, int logNB,
                    unsigned long long chunk, unsigned *__restrict__ M, const SegChunk *__restrict__ seg = nullptr) {
   extern __shared__ unsigned sh[];
   if (seg) {
@@ -115,7 +129,7 @@ bucket_hist_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, unsigned long
 #pragma unroll
     for (int u = 0; u < kHistUnroll; u++) {
       const unsigned long long j = k + (unsigned long long)u * kHistThreads;
-      if (j < c1) r[u] = pairs[j];
+      if (j < c1) r[u] = pair_at<CODES>(src, j);
     }
 #pragma unroll
     for (int u = 0; u < kHistUnroll; u++) {
@@ -201,8 +215,9 @@ __host__ __device__ constexpr size_t scatter_smem(int NB) {
   return (size_t)NB * 16 + (size_t)kSub * 12;
 }
 
-__global__ void __launch_bounds__(kScatterThreads)
-bucket_scatter_sorted_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, unsigned long long K, int logNB,
+template <bool CODES>
+__global__ void __launch_bounds__(kScatterThreads, 2)
+bucket_scatter_sorted_kernel(PairSrc src, BinSrc bin_of, unsigned long long K, int logNB,
                              unsigned long long chunk, const unsigned *__restrict__ M,
                              const unsigned long long *__restrict__ start_all, uint2 *__restrict__ recs,
                              int *__restrict__ rbins, const SegChunk *__restrict__ seg = nullptr) {
@@ -230,7 +245,7 @@ bucket_scatter_sorted_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, uns
 #pragma unroll
   for (int u = 0; u < kScatterPer; u++) {
     const unsigned long long k = c0 + threadIdx.x + u * kScatterThreads;
-    if (k < c1) pr[u] = pairs[k];
+    if (k < c1) pr[u] = pair_at<CODES>(src, k);
   }
   __syncthreads();
   for (unsigned long long sub = c0; sub < c1; sub += kSub) {
@@ -273,7 +288,7 @@ bucket_scatter_sorted_kernel(const uint2 *__restrict__ pairs, BinSrc bin_of, uns
 #pragma unroll
       for (int u = 0; u < kScatterPer; u++) {
         const unsigned long long k = sub + kSub + threadIdx.x + u * kScatterThreads;
-        if (k < c1) pr[u] = pairs[k];
+        if (k < c1) pr[u] = pair_at<CODES>(src, k);
       }
     }
     // write in staged (bucket) order: global = base[b] + (i - off[b])
@@ -749,6 +764,7 @@ __global__ void fb_gather_count_kernel(const unsigned *__restrict__ fb_list, uns
   if (i < nfb) fb_len[i] = start[fb_list[i] + 1] - start[fb_list[i]];
 }
 
+// (gridDim.y CTAs share a bucket: two buckets of 58 K records took 113 us with one each)
 __global__ void fb_gather_kernel(const unsigned *__restrict__ fb_list, unsigned nfb,
                                  const unsigned long long *__restrict__ start,
                                  const unsigned long long *__restrict__ fb_off,
@@ -756,20 +772,22 @@ __global__ void fb_gather_kernel(const unsigned *__restrict__ fb_list, unsigned 
                                  unsigned long long *__restrict__ key,
                                  unsigned *__restrict__ val, const unsigned *__restrict__ bfield,
                                  const SegField *__restrict__ fields) {
+  const unsigned long long t0 = (unsigned long long)blockIdx.y * blockDim.x + threadIdx.x;
+  const unsigned long long step = (unsigned long long)gridDim.y * blockDim.x;
   for (unsigned f = blockIdx.x; f < nfb; f += gridDim.x) {
     const unsigned long long r0 = start[fb_list[f]], r1 = start[fb_list[f] + 1];
     const unsigned long long o = fb_off[f];
     if (fields) {
       // keys (field, code); the positions of all fields are one array
       const unsigned fi = bfield[fb_list[f]], eb0 = (unsigned)fields[fi].ebase;
-      for (unsigned long long i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
+      for (unsigned long long i = r0 + t0; i < r1; i += step) {
         const uint2 r = recs[i];
         key[o + (i - r0)] = ((unsigned long long)fi << 32) | r.x;
         val[o + (i - r0)] = r.y == kNoExtremum ? kNoExtremum : r.y + eb0;
       }
       continue;
     }
-    for (unsigned long long i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
+    for (unsigned long long i = r0 + t0; i < r1; i += step) {
       const uint2 r = recs[i];
       key[o + (i - r0)] = code_keys ? (unsigned long long)r.x
                                     : (((unsigned long long)((unsigned)bin_of(r, i) ^ 0x80000000u) << 32) | r.x);
@@ -876,7 +894,7 @@ static int rank_fallback(szp_b200_ctx *ctx, const uint2 *recs, BinSrc bin_of, co
 
 // bucket stages shared by the single-field and segmented drivers, launched
 // after the histogram matrix M and the bucket starts exist
-static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, unsigned long long K, int logNB,
+static int rank_buckets(szp_b200_ctx *ctx, const PairSrc &points, BinSrc src, unsigned long long K, int logNB,
                         unsigned nbk, unsigned C, unsigned long long chunk, const unsigned *M,
                         const unsigned long long *start, const SegChunk *d_chunks, int *d_sp,
                         const unsigned *bfield = nullptr, const SegField *fields = nullptr, int nfields = 0) {
@@ -892,9 +910,9 @@ static int rank_buckets(szp_b200_ctx *ctx, const uint2 *d_pairs, BinSrc src, uns
     return -1;
   }
   const size_t ssm = scatter_smem(1 << logNB);
-  cudaFuncSetAttribute(bucket_scatter_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm);
-  bucket_scatter_sorted_kernel<<<C, kScatterThreads, ssm, s>>>(d_pairs, src, K, logNB, chunk, M, start, recs,
-                                                               rbins, d_chunks);
+  auto scatter = points.codes ? bucket_scatter_sorted_kernel<true> : bucket_scatter_sorted_kernel<false>;
+  cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm);
+  scatter<<<C, kScatterThreads, ssm, s>>>(points, src, K, logNB, chunk, M, start, recs, rbins, d_chunks);
   // past the scatter, bins (when given) are read in record order
   const BinSrc rsrc = {rbins, src.eb, src.inv};
   if (cuda_fail(cudaMemsetAsync(fb_cnt, 0, 32, s), "memset")) return -1;
@@ -954,14 +972,9 @@ static int rank_log_buckets(unsigned long long K, unsigned most = 2048) {
   return lg;
 }
 
-int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
-                   unsigned long long K, unsigned long long E, float eb, int *d_sp, bool try_bits) {
-  if (K == 0) return 0;
-  if (!d_bins && K <= (unsigned long long)kRankSmall) return rank_small(ctx, d_pairs, K, eb, d_sp);
-  if (!d_bins && try_bits) {
-    const int r = rank_bits_from_pairs(ctx, d_pairs, K, E, eb, d_sp);
-    if (r <= 0) return r;
-  }
+// the bucket ranking of one list
+static int rank_list(szp_b200_ctx *ctx, const PairSrc &points, const int *d_bins, unsigned long long K, float eb,
+                     int *d_sp) {
   cudaStream_t s = ctx->stream;
   const BinSrc src = {d_bins, eb, 1.0 / (double)eb};
   const int logNB = rank_log_buckets(K);
@@ -978,11 +991,28 @@ int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
     return -1;
   }
   const size_t hsm = (size_t)NB * 4;
-  bucket_hist_kernel<<<G, kHistThreads, hsm, s>>>(d_pairs, src, K, logNB, chunk, M);
+  auto hist = points.codes ? bucket_hist_kernel<true> : bucket_hist_kernel<false>;
+  hist<<<G, kHistThreads, hsm, s>>>(points, src, K, logNB, chunk, M, nullptr);
   bucket_colscan_kernel<<<(NB + 255) / 256, 256, 0, s>>>(M, G, NB, tot);
   bucket_start_kernel<<<1, 1024, 0, s>>>(tot, NB, start);
   ctx->launches += 3;
-  return rank_buckets(ctx, d_pairs, src, K, logNB, (unsigned)NB, (unsigned)G, chunk, M, start, nullptr, d_sp);
+  return rank_buckets(ctx, points, src, K, logNB, (unsigned)NB, (unsigned)G, chunk, M, start, nullptr, d_sp);
+}
+
+int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
+                   unsigned long long K, unsigned long long E, float eb, int *d_sp) {
+  if (K == 0) return 0;
+  if (!d_bins && K <= (unsigned long long)kRankSmall) return rank_small(ctx, d_pairs, K, eb, d_sp);
+  if (!d_bins) {
+    const int r = rank_bits_from_pairs(ctx, d_pairs, K, E, eb, d_sp);
+    if (r <= 0) return r;
+  }
+  return rank_list(ctx, {d_pairs, nullptr, 0, 0}, d_bins, K, eb, d_sp);
+}
+
+int rank_positions_codes(szp_b200_ctx *ctx, const unsigned *d_codes, unsigned long long cap, unsigned long long K,
+                         unsigned long long E, float eb, int *d_sp) {
+  return rank_list(ctx, {nullptr, d_codes, E, cap}, nullptr, K, eb, d_sp);
 }
 
 // Buckets that did not fit the bitmap rank: their records are gathered and
@@ -1017,8 +1047,8 @@ static int rank_fallback(szp_b200_ctx *ctx, const uint2 *recs, BinSrc bin_of, co
   }
   const bool code_keys = bin_of.bins == nullptr;
   cudaMemcpyAsync(fb_off, h_off.data(), nfb * 8, cudaMemcpyHostToDevice, s);
-  fb_gather_kernel<<<std::min(nfb, 4096u), 256, 0, s>>>(fb_list, nfb, start, fb_off, recs, bin_of, code_keys, k1,
-                                                          v1, bfield, fields);
+  const dim3 gg(std::min(nfb, 4096u), (unsigned)std::min<unsigned long long>(nf / nfb / 2048 + 1, 1024));
+  fb_gather_kernel<<<gg, 256, 0, s>>>(fb_list, nfb, start, fb_off, recs, bin_of, code_keys, k1, v1, bfield, fields);
   int bits = code_keys ? 32 : 64;
   if (fields)
     for (bits = 32; (nfields - 1) >> (bits - 32) > 0; bits += 8) {}
@@ -1113,11 +1143,12 @@ int rank_positions_fields(szp_b200_ctx *ctx, const uint2 *d_pairs, const RankFie
     return -1;
   const BinSrc src = {nullptr, 1.0f, 1.0};
   const size_t hsm = (size_t)4 << lgmax;
-  bucket_hist_kernel<<<C, kHistThreads, hsm, s>>>(d_pairs, src, K, lgmax, chunk, M, d_chunks);
+  const PairSrc points = {d_pairs, nullptr, 0, 0};
+  bucket_hist_kernel<false><<<C, kHistThreads, hsm, s>>>(points, src, K, lgmax, chunk, M, d_chunks);
   bucket_colscan_seg_kernel<<<F, 1 << lgmax, 0, s>>>(M, d_rows, tot, bfield);
   bucket_start_kernel<<<1, 1024, 0, s>>>(tot, (int)nbk, start);
   ctx->launches += 3;
-  return rank_buckets(ctx, d_pairs, src, K, lgmax, (unsigned)nbk, C, chunk, M, start, d_chunks, d_sp, bfield, d_fields,
+  return rank_buckets(ctx, points, src, K, lgmax, (unsigned)nbk, C, chunk, M, start, d_chunks, d_sp, bfield, d_fields,
                       F);
 }
 
