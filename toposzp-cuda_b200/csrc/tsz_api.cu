@@ -726,12 +726,12 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
   uint2 *pairs = A.take<uint2>(kcap);
   int *sp = A.take<int>(n);
   unsigned long long tot[3];
-  // From 2^18 values on the encoder sets the rank's bits itself and hands
-  // over the values' codes (in the pairs' place): no pair is written or
-  // read.  Below, the pairs are few and the rank picks its way by their count.
+  // From kRankBitsFieldMin values on the encoder sets the rank's bits itself
+  // and hands over the values' codes (in the pairs' place): no pair is written
+  // or read.  Below, the rank picks its way by the number of pairs.
   RankBits rb;
   const EncArgs probe = [&] { EncArgs e{}; e.B = B; e.data = d_data; e.out = d_topo + 8; e.cp_mode = kCpBits; return e; }();
-  const bool bits = n >= (1ull << 18) && enc64_applies(probe, kEncClassify) && rank_bits_begin(ctx, absErrBound, &rb);
+  const bool bits = n >= kRankBitsFieldMin && enc64_applies(probe, kEncClassify) && rank_bits_begin(ctx, absErrBound, &rb);
   const int cp_mode = bits ? kCpBits : kCpPairs;
   tl_begin(ctx);
   // a field still on the host (h_src) is copied in parts that overlap the encoder

@@ -43,6 +43,20 @@ constexpr unsigned kRbBelow = 6, kRbAbove = 30;   // binades below and above eb
 constexpr unsigned kSideCap = 4096;
 constexpr unsigned kRankSmall = 2048;      // lists that one CTA sorts
 constexpr unsigned kMaxBins = 1u << 22;
+
+// Pairs from which bits are set for them, which is a launch and a wait of its
+// own.  Ranking a list (us, bits / buckets): values spread over many bins,
+// 16384 pairs 67 / 60, 32768 75 / 60, 65536 77 / 63, 131072 83 / 87, 1 M
+// 104 / 147; a thousand and more in a bin, 16384 70 / 72, 32768 75 / 97, 65536
+// 79 / 186, 131072 82 / 429.
+constexpr unsigned long long kRankBitsMin = 1ull << 16;
+// Values of a field from which the encoder sets them, for nothing in launches or
+// waits; fewer are not worth the 118 MB.  Compression of 2D noise (us, bits from
+// the encoder / pairs in buckets): 8100 values 106 / 118, 16384 102 / 117, 32761
+// 108 / 118, with a thousand points in a bin 104 / 118, 104 / 122, 104 / 163; of
+// a smooth field, whose few points one CTA sorts either way, 74.4 / 75.0,
+// 70.0 / 69.9, 69.3 / 70.3.
+constexpr unsigned long long kRankBitsFieldMin = 1ull << 14;
 constexpr unsigned kRbUnits = (unsigned)((2ull * (kRbBelow + kRbAbove) << 23) / kRbBits) + 2u;
 
 struct RankBits {

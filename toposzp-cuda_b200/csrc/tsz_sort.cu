@@ -539,6 +539,101 @@ __device__ __forceinline__ void key_step_own(unsigned long long (&v)[PER], unsig
 }
 
 template <int PER>
+__device__ __forceinline__ void cta_sort_rank(const uint2 *__restrict__ recs, unsigned cnt, const BinSrc &bin_of,
+                                              int *__restrict__ out, unsigned long long *sk, unsigned *s_w) {
+  const unsigned t = threadIdx.x, e0 = PER * t;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned P = PER;
+  while (P < cnt) P <<= 1;
+  unsigned long long v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    v[u] = ~0ull;
+    if (e0 + u < cnt) {
+      const uint2 p = recs[e0 + u];
+      v[u] = ((unsigned long long)p.x << 32) | p.y;
+    }
+  }
+  for (unsigned k = 2; k <= P; k <<= 1) {
+    for (unsigned j = k >> 1; j >= 32u * PER; j >>= 1) {
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < PER; u++) sk[u * kSortThreads + t] = v[u];
+      __syncthreads();
+      const unsigned o = t ^ (j / PER);
+      const bool keep_min = ((e0 & j) == 0) == ((e0 & k) == 0);
+#pragma unroll
+      for (int u = 0; u < PER; u++) {
+        const unsigned long long x = sk[u * kSortThreads + o];
+        v[u] = (v[u] < x) == keep_min ? v[u] : x;
+      }
+    }
+    for (unsigned j = min(k >> 1, 16u * PER); j >= PER; j >>= 1) {
+      const bool keep_min = ((e0 & j) == 0) == ((e0 & k) == 0);
+#pragma unroll
+      for (int u = 0; u < PER; u++) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, v[u], j / PER);
+        v[u] = (v[u] < x) == keep_min ? v[u] : x;
+      }
+    }
+    if (PER > 8 && k > 8) key_step_own<8, PER>(v, k, e0);
+    if (PER > 4 && k > 4) key_step_own<4, PER>(v, k, e0);
+    if (PER > 2 && k > 2) key_step_own<2, PER>(v, k, e0);
+    key_step_own<1, PER>(v, k, e0);
+  }
+  // D: distinct codes up to a key; H: the D of its bin's first key; its position is D - H
+  __syncthreads();
+  sk[t] = v[PER - 1];
+  __syncthreads();
+  const bool any = e0 < cnt;
+  unsigned prev = t ? (unsigned)(sk[t - 1] >> 32) : 0u;
+  unsigned d = 0, first_of_bin = 0;
+  unsigned nc = 0, nb = 0;                        // bit u: key u has a new code, a new bin
+  int pbin = any && t ? bin_of({prev, 0u}, 0) : 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    if (e0 + u < cnt) {
+      const unsigned c = (unsigned)(v[u] >> 32);
+      const int bin = bin_of({c, 0u}, 0);
+      if (e0 + u == 0 || c != prev) { nc |= 1u << u; d++; }
+      if (e0 + u == 0 || bin != pbin) nb |= 1u << u;
+      prev = c;
+      pbin = bin;
+    }
+  }
+  unsigned total;
+  unsigned D = block_excl_scan<kSortThreads>(d, s_w, &total);
+  {
+    unsigned run = D;
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      run += (nc >> u) & 1u;
+      if ((nb >> u) & 1u) first_of_bin = run;
+    }
+  }
+  unsigned hi = first_of_bin;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned x = __shfl_up_sync(0xffffffffu, hi, o);
+    if (lane >= o) hi = max(hi, x);
+  }
+  if (lane == 31) s_w[warp] = hi;
+  unsigned H = __shfl_up_sync(0xffffffffu, hi, 1);
+  if (lane == 0) H = 0u;
+  __syncthreads();
+  for (int w = 0; w < warp; w++) H = max(H, s_w[w]);
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    D += (nc >> u) & 1u;
+    if ((nb >> u) & 1u) H = D;
+    if (e0 + u < cnt && (unsigned)v[u] != kNoExtremum) out[(unsigned)v[u]] = (int)(D - H);
+  }
+  __syncthreads();
+}
+
+// The buckets of fb_list of up to 1024 PER records; the others to fb2_list.
+// ANY: with the 2, 4, 8 or 16 keys a thread that a bucket asks for (up to PER).
+template <int PER, bool ANY>
 __global__ void __launch_bounds__(kSortThreads)
 bucket_sort_codes_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const unsigned long long *__restrict__ start,
                          const unsigned *__restrict__ fb_list, const unsigned *__restrict__ fb_count,
@@ -546,14 +641,12 @@ bucket_sort_codes_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const un
                          const unsigned *__restrict__ bfield, const SegField *__restrict__ fields) {
   extern __shared__ unsigned long long sk[];
   __shared__ unsigned s_w[kSortThreads / 32];
-  const unsigned t = threadIdx.x, e0 = PER * t;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned nfb = *fb_count;
   for (unsigned i = blockIdx.x; i < nfb; i += gridDim.x) {
     const unsigned bk = fb_list[i];
     const unsigned long long r0 = start[bk], cnt64 = start[bk + 1] - r0;
     if (cnt64 > (unsigned long long)(PER * kSortThreads)) {
-      if (t == 0) fb2_list[atomicAdd(fb2_count, 1u)] = bk;
+      if (threadIdx.x == 0) fb2_list[atomicAdd(fb2_count, 1u)] = bk;
       continue;
     }
     const unsigned cnt = (unsigned)cnt64;
@@ -563,92 +656,10 @@ bucket_sort_codes_kernel(const uint2 *__restrict__ recs, BinSrc bin_of, const un
       out += f.ebase;
       bin_of = {nullptr, f.eb, 1.0 / (double)f.eb};
     }
-    unsigned P = PER;
-    while (P < cnt) P <<= 1;
-    unsigned long long v[PER];
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      v[u] = ~0ull;
-      if (e0 + u < cnt) {
-        const uint2 p = recs[r0 + e0 + u];
-        v[u] = ((unsigned long long)p.x << 32) | p.y;
-      }
-    }
-    for (unsigned k = 2; k <= P; k <<= 1) {
-      for (unsigned j = k >> 1; j >= 32u * PER; j >>= 1) {
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < PER; u++) sk[u * kSortThreads + t] = v[u];
-        __syncthreads();
-        const unsigned o = t ^ (j / PER);
-        const bool keep_min = ((e0 & j) == 0) == ((e0 & k) == 0);
-#pragma unroll
-        for (int u = 0; u < PER; u++) {
-          const unsigned long long x = sk[u * kSortThreads + o];
-          v[u] = (v[u] < x) == keep_min ? v[u] : x;
-        }
-      }
-      for (unsigned j = min(k >> 1, 16u * PER); j >= PER; j >>= 1) {
-        const bool keep_min = ((e0 & j) == 0) == ((e0 & k) == 0);
-#pragma unroll
-        for (int u = 0; u < PER; u++) {
-          const unsigned long long x = __shfl_xor_sync(0xffffffffu, v[u], j / PER);
-          v[u] = (v[u] < x) == keep_min ? v[u] : x;
-        }
-      }
-      if (PER > 8 && k > 8) key_step_own<8, PER>(v, k, e0);
-      if (PER > 4 && k > 4) key_step_own<4, PER>(v, k, e0);
-      if (PER > 2 && k > 2) key_step_own<2, PER>(v, k, e0);
-      key_step_own<1, PER>(v, k, e0);
-    }
-    // D: distinct codes up to a key; H: the D of its bin's first key; its position is D - H
-    __syncthreads();
-    sk[t] = v[PER - 1];
-    __syncthreads();
-    const bool any = e0 < cnt;
-    unsigned prev = t ? (unsigned)(sk[t - 1] >> 32) : 0u;
-    unsigned d = 0, first_of_bin = 0;
-    unsigned nc = 0, nb = 0;                        // bit u: key u has a new code, a new bin
-    int pbin = any && t ? bin_of({prev, 0u}, 0) : 0;
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      if (e0 + u < cnt) {
-        const unsigned c = (unsigned)(v[u] >> 32);
-        const int bin = bin_of({c, 0u}, 0);
-        if (e0 + u == 0 || c != prev) { nc |= 1u << u; d++; }
-        if (e0 + u == 0 || bin != pbin) nb |= 1u << u;
-        prev = c;
-        pbin = bin;
-      }
-    }
-    unsigned total;
-    unsigned D = block_excl_scan<kSortThreads>(d, s_w, &total);
-    {
-      unsigned run = D;
-#pragma unroll
-      for (int u = 0; u < PER; u++) {
-        run += (nc >> u) & 1u;
-        if ((nb >> u) & 1u) first_of_bin = run;
-      }
-    }
-    unsigned hi = first_of_bin;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned x = __shfl_up_sync(0xffffffffu, hi, o);
-      if (lane >= o) hi = max(hi, x);
-    }
-    if (lane == 31) s_w[warp] = hi;
-    unsigned H = __shfl_up_sync(0xffffffffu, hi, 1);
-    if (lane == 0) H = 0u;
-    __syncthreads();
-    for (int w = 0; w < warp; w++) H = max(H, s_w[w]);
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      D += (nc >> u) & 1u;
-      if ((nb >> u) & 1u) H = D;
-      if (e0 + u < cnt && (unsigned)v[u] != kNoExtremum) out[(unsigned)v[u]] = (int)(D - H);
-    }
-    __syncthreads();
+    if (ANY && cnt <= 2u * kSortThreads) cta_sort_rank<2>(recs + r0, cnt, bin_of, out, sk, s_w);
+    else if (ANY && cnt <= 4u * kSortThreads) cta_sort_rank<4>(recs + r0, cnt, bin_of, out, sk, s_w);
+    else if (ANY && cnt <= 8u * kSortThreads) cta_sort_rank<8>(recs + r0, cnt, bin_of, out, sk, s_w);
+    else cta_sort_rank<PER>(recs + r0, cnt, bin_of, out, sk, s_w);
   }
 }
 
@@ -934,19 +945,27 @@ static int rank_buckets(szp_b200_ctx *ctx, const PairSrc &points, BinSrc src, un
     cudaFuncSetAttribute(bucket_sort_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_rank_smem());
     bucket_sort_rank_kernel<<<nbk, kSortThreads, sort_rank_smem(), s>>>(recs, rsrc, start, fb_list, fb_cnt, d_sp,
                                                                         fb2_list, fb_cnt + 1);
-  } else {
+  } else if (fields || K >= kRankBitsMin) {
     // each takes what fits it from the list before and passes the rest on
     unsigned *l3 = A.take<unsigned>(nbk), *l4 = A.take<unsigned>(nbk);
     if (!l3 || !l4) { set_error("scratch arena too small for the rank stage"); return -1; }
-    cudaFuncSetAttribute(bucket_sort_codes_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(bucket_sort_codes_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          16 * kSortThreads * 8);
-    bucket_sort_codes_kernel<2><<<std::min(nbk, 2u * ctx->sm_count), kSortThreads, 2 * kSortThreads * 8, s>>>(
+    bucket_sort_codes_kernel<2, false><<<std::min(nbk, 2u * ctx->sm_count), kSortThreads, 2 * kSortThreads * 8, s>>>(
         recs, rsrc, start, fb_list, fb_cnt, d_sp, l3, fb_cnt + 2, bfield, fields);
-    bucket_sort_codes_kernel<4><<<std::min(nbk, 2u * ctx->sm_count), kSortThreads, 4 * kSortThreads * 8, s>>>(
+    bucket_sort_codes_kernel<4, false><<<std::min(nbk, 2u * ctx->sm_count), kSortThreads, 4 * kSortThreads * 8, s>>>(
         recs, rsrc, start, l3, fb_cnt + 2, d_sp, l4, fb_cnt + 3, bfield, fields);
-    bucket_sort_codes_kernel<16><<<std::min(nbk, (unsigned)ctx->sm_count), kSortThreads, 16 * kSortThreads * 8, s>>>(
-        recs, rsrc, start, l4, fb_cnt + 3, d_sp, fb2_list, fb_cnt + 1, bfield, fields);
+    bucket_sort_codes_kernel<16, false><<<std::min(nbk, (unsigned)ctx->sm_count), kSortThreads, 16 * kSortThreads * 8,
+                                          s>>>(recs, rsrc, start, l4, fb_cnt + 3, d_sp, fb2_list, fb_cnt + 1, bfield,
+                                               fields);
     ctx->launches += 2;
+  } else {
+    // a short list: at most 64 buckets, and often none of them is here (one
+    // launch for three: 62 -> 57 us for 8192 spread values)
+    cudaFuncSetAttribute(bucket_sort_codes_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         16 * kSortThreads * 8);
+    bucket_sort_codes_kernel<16, true><<<nbk, kSortThreads, 16 * kSortThreads * 8, s>>>(
+        recs, rsrc, start, fb_list, fb_cnt, d_sp, fb2_list, fb_cnt + 1, nullptr, nullptr);
   }
   ctx->launches += 3;
   if (cuda_fail(cudaGetLastError(), "rank kernels")) return -1;
@@ -1003,7 +1022,7 @@ int rank_positions(szp_b200_ctx *ctx, const uint2 *d_pairs, const int *d_bins,
                    unsigned long long K, unsigned long long E, float eb, int *d_sp) {
   if (K == 0) return 0;
   if (!d_bins && K <= (unsigned long long)kRankSmall) return rank_small(ctx, d_pairs, K, eb, d_sp);
-  if (!d_bins) {
+  if (!d_bins && K >= kRankBitsMin) {
     const int r = rank_bits_from_pairs(ctx, d_pairs, K, E, eb, d_sp);
     if (r <= 0) return r;
   }
