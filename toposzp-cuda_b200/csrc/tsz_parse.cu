@@ -422,12 +422,14 @@ __device__ __forceinline__ unsigned stage_steps(const ParseGeom &g, unsigned lon
 }
 
 // Walks from the block starts e < M up to place dist (step: the table at the
-// first start's bit count byte): the smallest and largest distance past it at
-// which one that does not stop leaves, in *lo and *hi.  All lanes of a warp.
-// Most starts have an invalid bit count byte; the rest go through `keep` to
-// the lanes, a new one whenever a lane's walk ends.
-__device__ __forceinline__ void warm_walks(const unsigned short *step, unsigned dist, unsigned M, unsigned short *keep,
-                                           unsigned *lo_out, unsigned *hi_out) {
+// first start's bit count byte): the distance past it at which all that do not
+// stop leave, or kNoEntry where none arrives or two leave in different places.
+// All lanes of a warp.  Most starts have an invalid bit count byte; the rest
+// go through `keep` to the lanes, a new one whenever a lane's walk ends.
+// Of blocks of zeros every start is valid and no walk meets another: a look
+// every 16 rounds ends it once two places differ, or after `rounds` of them.
+__device__ __forceinline__ unsigned warm_walks(const unsigned short *step, unsigned dist, unsigned M, unsigned rounds,
+                                               unsigned short *keep) {
   const unsigned lane = threadIdx.x & 31;
   unsigned kept = 0;
 #pragma unroll 2
@@ -441,11 +443,12 @@ __device__ __forceinline__ void warm_walks(const unsigned short *step, unsigned 
   __syncwarp();
   unsigned lo = kNoEntry, hi = 0u;
   unsigned next = 32, p = lane < kept ? keep[lane] : kNoEntry;
-  while (__any_sync(0xffffffffu, p != kNoEntry)) {
+  bool open = false;
+  for (unsigned r = 1; __any_sync(0xffffffffu, p != kNoEntry); r++) {
     // four blocks between refills; a walk that stops stays where it is
     unsigned last = p;
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
+    for (int k = 0; k < 4; k++) {
       last = p;
       if (p < dist) p += step[p];
     }
@@ -462,10 +465,16 @@ __device__ __forceinline__ void warm_walks(const unsigned short *step, unsigned 
     const unsigned mine = next + __popc(m & ((1u << lane) - 1u));
     if (p == kNoEntry && mine < kept) p = keep[mine];
     next += (unsigned)__popc(m);
+    if ((r & 15u) == 0u) {
+      const unsigned l = __reduce_min_sync(0xffffffffu, lo);
+      open = r >= rounds || (l != kNoEntry && l != __reduce_max_sync(0xffffffffu, hi));
+      if (open) break;
+    }
   }
-  *lo_out = __reduce_min_sync(0xffffffffu, lo);
-  *hi_out = __reduce_max_sync(0xffffffffu, hi);
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
   __syncwarp();
+  return open || lo != hi ? kNoEntry : lo;
 }
 
 // State of a tile between its two halves.
@@ -520,6 +529,12 @@ parse_guess_kernel(ParseGeom g, unsigned ntiles, ParseOut o, ParseGuess u) {
   unsigned short *lists_all = tab + (size_t)(NW + 2) * u.unit + 48;
   const ParseDims d(g, o);
   const BlockLen lens(g);
+  // rounds (of four blocks) of 64 KB of the shortest blocks: more than
+  // blockSize 64 can take, where ordinary data takes a few tens.  Decoding 4 M
+  // zeros (us, every entry of 16 KB segments walked / no end but the last walk's
+  // / now): plain codec, blockSize 64 1390 / 950 / 458, 128 1670 / 2380 / 493,
+  // 256 2250 / 8530 / 860; topology, 64 544 / 306 / 189, 256 313 / 806 / 154.
+  const unsigned rounds = 16384u / lens.base;
   unsigned cur = 0;
   bool pending = false;
   while (true) {
@@ -544,17 +559,17 @@ parse_guess_kernel(ParseGeom g, unsigned ntiles, ParseOut o, ParseGuess u) {
       {
         const unsigned at = w * u.unit;                  // this warp's segment
         const unsigned long long s0 = t0 + at;
-        unsigned lo = kNoEntry, hi = 0u;
+        unsigned entry = kNoEntry;
         if (s0 == 0) {
-          lo = hi = 0u;
+          entry = 0u;
         } else if (s0 < g.len) {
           // a walk from payload offset 0 is the true one
           unsigned short *keep = lists + (size_t)w * u.list;
-          warm_walks(step + at - u.unit, u.unit, s0 == u.unit ? 1u : g.M, keep, &lo, &hi);
-          if (lo != hi && w == 0)
-            warm_walks(step - 2u * u.unit, 2u * u.unit, s0 == 2u * u.unit ? 1u : g.M, keep, &lo, &hi);
+          entry = warm_walks(step + at - u.unit, u.unit, s0 == u.unit ? 1u : g.M, rounds, keep);
+          if (entry == kNoEntry && w == 0)
+            entry = warm_walks(step - 2u * u.unit, 2u * u.unit, s0 == 2u * u.unit ? 1u : g.M, rounds, keep);
         }
-        if (lane == 0) s.entry[w] = lo == hi ? lo : kNoEntry;
+        if (lane == 0) s.entry[w] = entry;
       }
       __syncthreads();
       if (w == 0) {
