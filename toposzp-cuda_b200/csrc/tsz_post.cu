@@ -1205,12 +1205,17 @@ pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, unsigned total,
     // clearing it now cannot hide a count from a slower CTA.
     unsigned *cnt = cnts + (round % 3);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(cnts + ((round + 1) % 3), 0u);
+    // in a worklist of many times the grid most items wait for ones that this
+    // round does not reach: one look each (checkerboards, whose points wait for
+    // one another in long chains: 1500x1700 574 ms with kShortPolls, 447 so;
+    // 160x170x180 225, 163; 700x800, below the line, 42.9 with kShortPolls, 46.7
+    // with one look)
+    const int polls = nw <= stride ? kDepPolls : ((nw >> 3) <= stride ? kShortPolls : 0);
     for (unsigned base = blockIdx.x * blockDim.x; base < nw; base += stride) {
       const unsigned i = base + threadIdx.x;
       unsigned idx = 0;
       if (i < nw) idx = W ? __ldcg(W + i) : i;
-      const bool defer = pass_item_local<PASS, ND>(a, list, idx, i < nw && (!a.ONLY || bit_at(a.ONLY, idx)),
-                                                   nw <= stride ? kDepPolls : kShortPolls);
+      const bool defer = pass_item_local<PASS, ND>(a, list, idx, i < nw && (!a.ONLY || bit_at(a.ONLY, idx)), polls);
       const unsigned m = __ballot_sync(0xffffffffu, defer);
       unsigned wb = 0;
       if (lane == 0 && m) wb = atomicAdd(cnt, (unsigned)__popc(m));
