@@ -509,7 +509,7 @@ __device__ __forceinline__ Prefix e64_lookback(TileDesc *desc, long long t, unsi
 template <bool BITS>
 __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, const unsigned char *img,
                                          const void *stage, const E64Sh &sh, unsigned &nmax, unsigned &cmax,
-                                         bool &full) {
+                                         unsigned &seen) {
   const int tid = threadIdx.x;
   const long long n = (long long)a.n;
   const long long nblocks = (n + 63) / 64;
@@ -563,7 +563,7 @@ __device__ __forceinline__ void e64_back(const Enc64Args &a, long long tile, con
         const bool is_ext = k < nte;
         const unsigned code = st[is_ext ? k : kE64Tile - 1u + nte - k];
         const unsigned ext = is_ext ? (unsigned)eb0 + k : kNoExtremum;
-        rb_set(a.rb, code, ext, full);
+        rb_set(a.rb, code, ext, seen);
         if (head && cb + k < kRankSmall) a.rb.first[cb + k] = make_uint2(code, ext);
         nmax = max(nmax, ~code);
         cmax = max(cmax, code);
@@ -622,8 +622,7 @@ __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
   const bool small = a.g.d1 * a.g.plane < (1ll << 32);
   long long prev = -1;
   int cur = 0;
-  unsigned nmax = 0, cmax = 0;
-  bool full = false;
+  unsigned nmax = 0, cmax = 0, seen = 0;
   while (true) {
     // claimed only now (while the other warps write the last tile out), not a
     // tile ahead: every look-back behind a claimed tile waits for its front half
@@ -652,7 +651,7 @@ __global__ void __launch_bounds__(kE64Cta, 4) enc64_kernel(Enc64Args a) {
     __syncthreads();
     if (owner && prev >= 0) {
       const unsigned char *pp = smem_dyn + (size_t)(cur ^ 1) * kPart;
-      e64_back<BITS>(a, prev, pp, pp + kE64Img, sh[cur ^ 1], nmax, cmax, full);
+      e64_back<BITS>(a, prev, pp, pp + kE64Img, sh[cur ^ 1], nmax, cmax, seen);
     }
     if (!more) break;
     prev = tile;
@@ -679,8 +678,7 @@ enc64_batch_kernel(const EncArgs *__restrict__ fields, const unsigned long long 
   const int lane = threadIdx.x & 31;
   int field = 0, have[3] = {-1, -1, -1};
   bool pending = false;
-  unsigned unused0 = 0, unused1 = 0;
-  bool unused2 = false;
+  unsigned unused0 = 0, unused1 = 0, unused2 = 0;
   for (int it = 0, cur = 0, slot = 0;; it++, cur ^= 1) {
     const int before = slot == 0 ? 2 : slot - 1;
     if (owner) {

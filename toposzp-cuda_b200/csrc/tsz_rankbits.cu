@@ -55,11 +55,11 @@ __device__ __forceinline__ void sort_keys_2048(unsigned long long (&v)[2], unsig
 __global__ void __launch_bounds__(256)
 rank_bits_pairs_kernel(const uint2 *__restrict__ pairs, unsigned long long K, RankBits rb) {
   unsigned nmax = 0, cmax = 0;
-  bool full = false;
+  unsigned seen = 0;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < K; k += stride) {
     const uint2 p = pairs[k];
-    rb_set(rb, p.x, p.y, full);
+    rb_set(rb, p.x, p.y, seen);
     nmax = max(nmax, ~p.x);
     cmax = max(cmax, p.x);
   }
@@ -188,10 +188,18 @@ __global__ void rank_bits_bins_kernel(const unsigned *__restrict__ bits, RbRange
 // ---- 3b. the values aside (bins 0 and 1), sorted by one CTA ----------------
 // A value of bin 0 comes after the bin's set bits, all negative; one of bin 1
 // before them, so the distinct ones of bin 1 are added to that bin's positions
-// (its table entry less their number).
+// (its table entry less their number).  A key of its own for the zeros (zero:
+// there are some), whose position goes to *zero_pos.
 __global__ void __launch_bounds__(1024)
-rank_bits_side_kernel(const unsigned *__restrict__ bits, RbRange g, const uint2 *__restrict__ side, unsigned cnt,
-                      unsigned *__restrict__ binp, int *__restrict__ out) {
+rank_bits_side_kernel(const unsigned *__restrict__ bits, RbRange g, const uint2 *__restrict__ side, unsigned nside,
+                      bool zero, unsigned *__restrict__ binp, int *__restrict__ out, unsigned *__restrict__ zero_pos) {
+  const unsigned cnt = nside + (zero ? 1u : 0u);
+  auto load = [&](unsigned i) {
+    if (i >= cnt) return ~0ull;
+    if (i == nside) return ((unsigned long long)kZeroCode << 32) | kNoExtremum;
+    const uint2 v = side[i];
+    return ((unsigned long long)v.x << 32) | v.y;
+  };
   __shared__ unsigned long long key[kSideCap];
   __shared__ unsigned s_w[32];
   unsigned P = 64;
@@ -200,8 +208,7 @@ rank_bits_side_kernel(const unsigned *__restrict__ bits, RbRange g, const uint2 
     unsigned long long v2[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const unsigned i = 2u * threadIdx.x + u;
-      v2[u] = i < cnt ? ((unsigned long long)side[i].x << 32) | side[i].y : ~0ull;
+      v2[u] = load(2u * threadIdx.x + u);
     }
     sort_keys_2048(v2, P, key);
     key[2u * threadIdx.x] = v2[0];
@@ -209,7 +216,7 @@ rank_bits_side_kernel(const unsigned *__restrict__ bits, RbRange g, const uint2 
     __syncthreads();
   } else {
     for (unsigned i = threadIdx.x; i < P; i += blockDim.x)
-      key[i] = i < cnt ? ((unsigned long long)side[i].x << 32) | side[i].y : ~0ull;
+      key[i] = load(i);
     __syncthreads();
     for (unsigned k = 2; k <= P; k <<= 1)
       for (unsigned j = k >> 1; j > 0; j >>= 1) {
@@ -255,8 +262,9 @@ rank_bits_side_kernel(const unsigned *__restrict__ bits, RbRange g, const uint2 
   unsigned run = pre & 0xffffu;   // distinct values before the thread's first
   for (unsigned i = i0; i < i1; i++) {
     if (i == 0 || (key[i] >> 32) != (key[i - 1] >> 32)) run++;
-    const unsigned e = (unsigned)key[i];
-    if (e != kNoExtremum) out[e] = (int)(bin_of(i) <= 0 ? base0 + run - 1u : run - 1u - D0);
+    const unsigned e = (unsigned)key[i], pos = bin_of(i) <= 0 ? base0 + run - 1u : run - 1u - D0;
+    if (e != kNoExtremum) out[e] = (int)pos;
+    if ((unsigned)(key[i] >> 32) == kZeroCode) *zero_pos = pos;
   }
   __syncthreads();
   if (threadIdx.x == 0 && D1 && g.b0 <= 1 && 1 - (long long)g.b0 < (long long)g.nbins) binp[1 - g.b0] -= D1;
@@ -273,7 +281,8 @@ __device__ __forceinline__ int rb_rank(const unsigned *__restrict__ bits, const 
 // sectors in flight together)
 __global__ void __launch_bounds__(256)
 rank_bits_codes_kernel(const unsigned *__restrict__ codes, unsigned long long E, const unsigned *__restrict__ bits,
-                       RbRange g, const unsigned *__restrict__ binp, int *__restrict__ out) {
+                       RbRange g, const unsigned *__restrict__ binp, const unsigned *__restrict__ zero_pos,
+                       int *__restrict__ out) {
   const unsigned long long e0 = 4ull * ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x);
   if (e0 >= E) return;
   if (e0 + 4 <= E) {
@@ -290,28 +299,34 @@ rank_bits_codes_kernel(const unsigned *__restrict__ codes, unsigned long long E,
     if (in[0] && in[1] && in[2] && in[3]) {
       *reinterpret_cast<int4 *>(out + e0) = make_int4(r[0], r[1], r[2], r[3]);
     } else {
-      // values aside have their positions already
+      // values aside have their positions already, but the zeros
 #pragma unroll
-      for (int k = 0; k < 4; k++)
+      for (int k = 0; k < 4; k++) {
         if (in[k]) out[e0 + k] = r[k];
+        else if (cc[k] == kZeroCode) out[e0 + k] = (int)*zero_pos;
+      }
     }
   } else {
     for (unsigned long long e = e0; e < E; e++) {
       unsigned idx;
       const unsigned c = codes[e];
       if (rb_index(g.rz, g.rh, c, &idx)) out[e] = rb_rank(bits, g, binp, c, idx);
+      else if (c == kZeroCode) out[e] = (int)*zero_pos;
     }
   }
 }
 
 __global__ void __launch_bounds__(256)
 rank_bits_pair_out_kernel(const uint2 *__restrict__ pairs, unsigned long long K, const unsigned *__restrict__ bits,
-                          RbRange g, const unsigned *__restrict__ binp, int *__restrict__ out) {
+                          RbRange g, const unsigned *__restrict__ binp, const unsigned *__restrict__ zero_pos,
+                          int *__restrict__ out) {
   const unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= K) return;
   const uint2 p = pairs[k];
   unsigned idx;
-  if (p.y != kNoExtremum && rb_index(g.rz, g.rh, p.x, &idx)) out[p.y] = rb_rank(bits, g, binp, p.x, idx);
+  if (p.y == kNoExtremum) return;
+  if (rb_index(g.rz, g.rh, p.x, &idx)) out[p.y] = rb_rank(bits, g, binp, p.x, idx);
+  else if (p.x == kZeroCode) out[p.y] = (int)*zero_pos;
 }
 
 // ---- host ------------------------------------------------------------------
@@ -406,7 +421,8 @@ int rank_bits_finish(szp_b200_ctx *ctx, const RankBits &rb, const unsigned *h_st
   g.hi = hi;
   cudaStream_t s = ctx->stream;
   const unsigned s0 = lo / kRbBits, s1 = hi > lo ? (hi - 1u) / kRbBits + 1u : s0;
-  bool apply = !h_stat[3] && h_stat[2] <= kSideCap;
+  const bool zero = h_stat[4] != 0u;
+  bool apply = !h_stat[3] && h_stat[2] + (zero ? 1u : 0u) <= kSideCap;
   if (apply) {
     g.b0 = host_bin(cmin, eb, g.inv);
     const long long nb = (long long)host_bin(cmax, eb, g.inv) - g.b0 + 1;
@@ -425,14 +441,17 @@ int rank_bits_finish(szp_b200_ctx *ctx, const RankBits &rb, const unsigned *h_st
     }
     rank_bits_bins_kernel<<<(g.nbins + 127) / 128, 128, 0, s>>>(rb.bits, g, binp);
     ctx->launches += 1;
-    if (h_stat[2]) {
-      rank_bits_side_kernel<<<1, 1024, 0, s>>>(rb.bits, g, rb.side, h_stat[2], binp, d_sp);
+    unsigned *zero_pos = rb.stat + 5;
+    if (h_stat[2] || zero) {
+      rank_bits_side_kernel<<<1, 1024, 0, s>>>(rb.bits, g, rb.side, h_stat[2], zero, binp, d_sp, zero_pos);
       ctx->launches += 1;
     }
     if (d_codes)
-      rank_bits_codes_kernel<<<(unsigned)((E + 1023) / 1024), 256, 0, s>>>(d_codes, E, rb.bits, g, binp, d_sp);
+      rank_bits_codes_kernel<<<(unsigned)((E + 1023) / 1024), 256, 0, s>>>(d_codes, E, rb.bits, g, binp,
+                                                                              zero_pos, d_sp);
     else
-      rank_bits_pair_out_kernel<<<(unsigned)((K + 255) / 256), 256, 0, s>>>(d_pairs, K, rb.bits, g, binp, d_sp);
+      rank_bits_pair_out_kernel<<<(unsigned)((K + 255) / 256), 256, 0, s>>>(d_pairs, K, rb.bits, g, binp,
+                                                                                 zero_pos, d_sp);
     ctx->launches += 1;
     if (cuda_fail(cudaGetLastError(), "rank kernels")) return -1;
   }

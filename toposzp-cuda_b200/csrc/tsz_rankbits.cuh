@@ -22,7 +22,9 @@
 // random 32-byte sector that every extremum reads (95 of the 141 us).
 //
 // Values nearer to zero than 2^-6 eb (two bins share them) are kept aside and
-// sorted; values from 2^30 eb on, more than kSideCap aside, or more than
+// sorted, all zeros as one of them (a field of small integers, us, buckets /
+// each zero aside / so: 300 x 400 126 / 193 / 123, 160 x 170 x 180 520 / 636 /
+// 226); values from 2^30 eb on, more than kSideCap aside, or more than
 // kMaxBins bins are left to the bucket ranking, which takes the codes that the
 // encoder leaves beside the bits (from a pair list, the pairs).  Such fields,
 // in buckets alone / encoded a second time for pairs / from the codes:
@@ -64,8 +66,13 @@ struct RankBits {
   unsigned rz, rh;     // magnitudes (float bits) [rz, rh) have a bit
   uint2 *side;         // {code, extremum index or ~0} of the values below rz
   uint2 *first;        // the first kRankSmall pairs of an encoder launch: a field with no more needs no scan
-  unsigned *stat;      // zeroed: [0] largest ~code, [1] largest code, [2] values aside, [3] out of range
+  unsigned *stat;      // zeroed: [0] largest ~code, [1] largest code, [2] values aside (but zeros), [3] out of
+                       // range, [4] zeros among them, [5] their position
 };
+
+constexpr unsigned kZeroCode = 0x80000000u;   // of +0 and -0
+// what a thread has seen: the bits will not do; a zero
+enum : unsigned { kRbFull = 1u, kRbZero = 2u };
 
 // bit of a value code, by value: the negative half, then the positive one;
 // false when the value has none
@@ -76,32 +83,40 @@ __host__ __device__ __forceinline__ bool rb_index(unsigned rz, unsigned rh, unsi
   return mag - rz < rh - rz;
 }
 
-// Keeps a value without a bit aside.  The lanes that are here together take
-// their places with one atomic, and a thread that has seen that the bits will
-// not do (full) takes none: in a field that lies near zero every value comes here.
-__device__ __forceinline__ void rb_aside(const RankBits &rb, unsigned code, unsigned ext, bool &full) {
+// Keeps a value without a bit aside.  Zeros, of which a masked or quantized
+// field is full, leave a mark only.  Of the others, the lanes that are here
+// together take their places with one atomic, and a thread that has seen that
+// the bits will not do takes none: in a field that lies near zero every value
+// comes here.
+__device__ __forceinline__ void rb_aside(const RankBits &rb, unsigned code, unsigned ext, unsigned &seen) {
   const unsigned mag = ((code >> 31) ? code : ~code) & 0x7FFFFFFFu;
+  if (code == kZeroCode) {
+    if (!(seen & kRbZero)) rb.stat[4] = 1u;
+    seen |= kRbZero;
+    return;
+  }
+  if (seen & kRbFull) return;
   if (mag >= rb.rh) {
     rb.stat[3] = 1u;
-    full = true;
+    seen |= kRbFull;
     return;
   }
   const unsigned m = __activemask(), lane = threadIdx.x & 31u, first = (unsigned)__ffs((int)m) - 1u;
   unsigned k = 0;
   if (lane == first) k = atomicAdd(rb.stat + 2, (unsigned)__popc(m));
   k = __shfl_sync(m, k, (int)first);
-  full = k + (unsigned)__popc(m) > kSideCap;
+  if (k + (unsigned)__popc(m) > kSideCap) seen |= kRbFull;
   k += (unsigned)__popc(m & ((1u << lane) - 1u));
   if (k < kSideCap) rb.side[k] = make_uint2(code, ext);
 }
 
-__device__ __forceinline__ void rb_set(const RankBits &rb, unsigned code, unsigned ext, bool &full) {
+__device__ __forceinline__ void rb_set(const RankBits &rb, unsigned code, unsigned ext, unsigned &seen) {
   unsigned idx;
   if (rb_index(rb.rz, rb.rh, code, &idx)) {
     const unsigned q = idx / kRbBits, r = idx - q * kRbBits;
     atomicOr(rb.bits + 4u * q + 1u + (r >> 5), 1u << (r & 31u));
-  } else if (!full) {
-    rb_aside(rb, code, ext, full);
+  } else {
+    rb_aside(rb, code, ext, seen);
   }
 }
 
