@@ -812,7 +812,7 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
                         const uint64_t *d_blk_index, szp_b200_geom geom, float absErrBound,
                         int blockSize, float *d_out, unsigned char *d_types, int postprocess,
                         bool ref_bound, bool *parse_failed, cudaEvent_t sort_ready, bool cpu_layout,
-                        unsigned long long sort_count) {
+                        unsigned long long sort_count, const std::vector<ChunkSpan> *sort_chunks) {
   if (parse_failed) *parse_failed = false;
   if (!ctx || !d_topo || !d_out) { set_error("null argument"); return -1; }
   if (!check_block_size(blockSize, "szp_b200_topo_decompress_dev")) return -1;
@@ -925,8 +925,22 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
     b.out_i = sp;
     // read back with the status of the passes, which take what it decodes
     b.err = reinterpret_cast<int *>(w + kSortStatusWord);
-    if (cuda_fail(launch_decode(false, b, s), "decode sort")) return -1;
-    ctx->launches += 1;
+    if (sort_chunks && !sort_chunks->empty()) {
+      // chunks that need not follow one another: each is a stream of its own
+      // to the decoder, whose tiles hold blocks that do
+      for (const ChunkSpan &c : *sort_chunks) {
+        DecArgs k = b;
+        k.payload_len = c.end;
+        k.blk_off = b.blk_off + c.b0;
+        k.n = std::min(c.nb * B, E - c.b0 * B);
+        k.out_i = sp + c.b0 * B;
+        if (cuda_fail(launch_decode(false, k, s), "decode sort")) return -1;
+        ctx->launches += 1;
+      }
+    } else {
+      if (cuda_fail(launch_decode(false, b, s), "decode sort")) return -1;
+      ctx->launches += 1;
+    }
     tl_mark(ctx, "decode_sort");
     spp = sp;
   }

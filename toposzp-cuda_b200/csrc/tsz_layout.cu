@@ -95,11 +95,14 @@ static unsigned long long ones_of(unsigned long long n, int B) {
 
 // Parses the block offsets of one chunk of a stream on the device: blocks
 // [b0, b0 + nbc) starting at payload offset off (relative to pay), within
-// lim bytes of pay.  Offsets go to d_offs[b0 ..] (relative to pay).
+// lim bytes of pay.  Offsets go to d_offs[b0 ..] (relative to pay), the payload
+// offset after its last block to *end.
 static int parse_chunk(szp_b200_ctx *ctx, Arena &A, const unsigned char *pay, unsigned long long lim,
                        unsigned long long off, unsigned long long b0, unsigned long long nbc, unsigned long long n,
-                       int B, bool tags, unsigned long long *d_offs, unsigned long long *d_status, bool *ok) {
+                       int B, bool tags, unsigned long long *d_offs, unsigned long long *d_status, bool *ok,
+                       unsigned long long *end) {
   *ok = false;
+  *end = off;
   if (nbc == 0) { *ok = true; return 0; }
   if (off >= lim) return 0;
   const unsigned long long e0 = b0 * (unsigned long long)B;
@@ -118,6 +121,7 @@ static int parse_chunk(szp_b200_ctx *ctx, Arena &A, const unsigned char *pay, un
     return -1;
   if (st[0] != 0 && st[1] == 0) {
     *ok = true;
+    *end = off + (st[0] - 1);
     add_base_kernel<<<(unsigned)((nbc + 255) / 256), 256, 0, ctx->stream>>>(tmp, nbc, off, d_offs + b0);
     if (cuda_fail(cudaGetLastError(), "offsets")) return -1;
     ctx->launches += 1;
@@ -170,11 +174,14 @@ __global__ void chunk_verify_kernel(const unsigned char *__restrict__ cmp, const
 // len: its bytes, n: elements; first_try: 1 for the topology stream, 2 for
 // the sort positions (whose detection assumes one thread unless a larger
 // count validates).  Writes the payload-relative offsets of every block to
-// d_offs and returns T (0 when no candidate, not even one thread, walks).
+// d_offs and returns T (0 when no candidate, not even one thread, walks).  The
+// chunks of a table that does not describe one walk, which need not follow one
+// another (the rule can take a smaller T than the writer's), go to *chunks.
 static int detect_chunks(szp_b200_ctx *ctx, Arena &A, const unsigned char *cmp, unsigned long long len,
                          unsigned long long n, int B, bool tags, int first_try, unsigned long long *d_offs,
-                         unsigned long long *d_status) {
+                         unsigned long long *d_status, std::vector<ChunkSpan> *chunks) {
   cudaStream_t s = ctx->stream;
+  chunks->clear();
   const unsigned long long nb = (n + B - 1) / B;
   const unsigned long long maxc = tags ? 8ull * n + 1024ull : 4ull * n + 4ull;
   const unsigned long long bound = std::min(maxc, len);
@@ -208,19 +215,24 @@ static int detect_chunks(szp_b200_ctx *ctx, Arena &A, const unsigned char *cmp, 
     return 0;
   };
   auto try_T = [&](int T, unsigned long long bound, bool *ok) -> int {
+    chunks->clear();
     if (whole_T(T, bound, ok)) return -1;
     // one chunk from payload offset 0: the walk was the chunk's own
     if (*ok || (T == 1 && tab[0] == 0)) return 0;
     const unsigned long long hdr = (unsigned long long)T * 8;
     if (hdr >= bound) return 0;
     const unsigned long long bpt = (nb + T - 1) / T;
+    chunks->clear();
     for (int t = 0; t < T; t++) {
       const unsigned long long b0 = (unsigned long long)t * bpt;
       if (b0 >= nb) break;
       const unsigned long long nbc = std::min(bpt, nb - b0);
+      unsigned long long end = 0;
       bool cok = false;
-      if (parse_chunk(ctx, A, cmp + hdr, bound - hdr, tab[t], b0, nbc, n, B, tags, d_offs, d_status, &cok)) return -1;
+      if (parse_chunk(ctx, A, cmp + hdr, bound - hdr, tab[t], b0, nbc, n, B, tags, d_offs, d_status, &cok, &end))
+        return -1;
       if (!cok) return 0;
+      chunks->push_back({b0, nbc, end});
     }
     *ok = true;
     return 0;
@@ -367,13 +379,14 @@ int szp_b200_container_decompress_dev(szp_b200_ctx *ctx, const unsigned char *d_
   unsigned long long *idx = ctx->io.take<unsigned long long>(nb + nbs + 1);
   if (!ctx->scratch.reserve(need)) return -1;
   unsigned long long *w = ctx->d_words;
-  const int Tt = detect_chunks(ctx, ctx->scratch, d_in, topo_size, n, B, true, 1, idx, w + 16);
+  std::vector<ChunkSpan> chunks;
+  const int Tt = detect_chunks(ctx, ctx->scratch, d_in, topo_size, n, B, true, 1, idx, w + 16, &chunks);
   if (Tt < 0) return -1;
   if (Tt == 0) { set_error("topology stream: no thread count walks inside the stream"); return -1; }
   int Ts = 0;
   if (E) {
     ctx->scratch.reset();
-    Ts = detect_chunks(ctx, ctx->scratch, sort_cmp, sort_len, E, B, false, 2, idx + nb, w + 18);
+    Ts = detect_chunks(ctx, ctx->scratch, sort_cmp, sort_len, E, B, false, 2, idx + nb, w + 18, &chunks);
     if (Ts < 0) return -1;
     if (Ts == 0) { set_error("sort-position stream: no thread count walks inside the stream"); return -1; }
   }
@@ -384,7 +397,8 @@ int szp_b200_container_decompress_dev(szp_b200_ctx *ctx, const unsigned char *d_
   const unsigned char *sptr = E ? sort_cmp + 8ull * Ts - 8 : nullptr;
   const unsigned long long sbytes = E ? sort_len - 8ull * Ts + 8 : 0;
   return decompress_dev_impl(ctx, tptr, tbytes, sptr, sbytes, reinterpret_cast<const uint64_t *>(idx), geom,
-                             absErrBound, B, d_out, d_types, postprocess, false, nullptr, nullptr, true, E);
+                             absErrBound, B, d_out, d_types, postprocess, false, nullptr, nullptr, true, E,
+                             E ? &chunks : nullptr);
 }
 
 }  // extern "C"

@@ -1,9 +1,16 @@
 // Internal operators shared by the API layer (not part of the C ABI).
 #pragma once
+#include <vector>
+
 #include "tsz_codec.h"
 #include "tsz_runtime.h"
 
 namespace tsz {
+
+// Blocks [b0, b0 + nb) of a stream, which end at payload offset `end`.
+struct ChunkSpan {
+  unsigned long long b0, nb, end;
+};
 
 // Scratch arrays of the post-processing of one field (tsz_post.cu).
 struct PostLists {
@@ -144,7 +151,8 @@ int decompress_dev_impl(szp_b200_ctx *ctx, const unsigned char *d_topo, size_t t
                         const uint64_t *d_blk_index, szp_b200_geom geom, float absErrBound,
                         int blockSize, float *d_out, unsigned char *d_types, int postprocess,
                         bool ref_bound, bool *parse_failed, cudaEvent_t sort_ready = nullptr,
-                        bool cpu_layout = false, unsigned long long sort_count = ~0ull);
+                        bool cpu_layout = false, unsigned long long sort_count = ~0ull,
+                        const std::vector<ChunkSpan> *sort_chunks = nullptr);
 
 // Grows a workspace so that compressing or decompressing (with
 // post-processing) a field of n elements allocates nothing more (but the rank
