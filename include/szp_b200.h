@@ -455,7 +455,10 @@ SZP_B200_API int szp_b200_batch_reserve(szp_b200_batch *b, int max_fields, size_
 
 /* Chosen shapes: shape[0..3] = topology encoder threads per CTA, CTAs per SM,
  * sort-position encoder threads per CTA, CTAs per SM; ms[] = the autotuner's
- * timings of the topology-encoder candidates.  Returns 1 once tuned. */
+ * timings of the topology-encoder candidates.  The blockSize-64 encoder, which
+ * takes batches of 16-byte aligned fields at that blockSize, has one shape:
+ * shape[0..1] and ms[] are then what the general encoder would use, zeros in
+ * ms[] until it has run.  Returns 1 once tuned. */
 SZP_B200_API int szp_b200_batch_tuning(szp_b200_batch *b, int *shape, float *ms, int max);
 
 /* The batch's workspace (stage times, launch counter). */

@@ -17,9 +17,12 @@
 // Reading follows the reference's thread-count detection
 // (SZp/include/szp_detect_threads.h:153-190 for the sort positions, :282-309
 // for the topology): the first candidate T whose table is non-decreasing and
-// bounded and whose every chunk walks inside the validation bound.  Each
-// candidate's chunks are walked by the device parser, one chunk at a time,
-// not by a serial walk on the host.
+// bounded and whose every chunk walks inside the validation bound.  The first
+// blocks of all candidates' chunks are probed in one launch, which leaves few
+// candidates; a candidate's payload is then walked once by the device parser,
+// and its table compared with where the blocks lie (100x500x500 of 8 chunks:
+// 4.6 -> 0.5 ms against a parse per chunk and candidate).  Only where they
+// differ are the chunks walked one at a time.
 #include <algorithm>
 #include <vector>
 

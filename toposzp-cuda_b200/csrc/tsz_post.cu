@@ -1186,9 +1186,8 @@ __global__ void __launch_bounds__(kPostThreads, 2)
 pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, unsigned total,
                  const unsigned *total_dev, const unsigned *W_start, const unsigned *nstart_dev, unsigned *Wx,
                  unsigned *Wy, unsigned *cnts, unsigned *bar, unsigned long long *status) {
-  const unsigned tot = total_dev ? __ldcg(total_dev) : total;
   const unsigned *W = W_start;   // null: list positions themselves
-  unsigned nw = W_start ? __ldcg(nstart_dev) : tot;
+  unsigned nw = W_start ? __ldcg(nstart_dev) : (total_dev ? __ldcg(total_dev) : total);
   const bool after_round0 = W_start != nullptr;
   int b = 0;
   const unsigned stride = gridDim.x * blockDim.x;
@@ -1232,7 +1231,6 @@ pass_coop_kernel(PostArgs a, const unsigned *__restrict__ list, unsigned total,
     nw = next;
     b ^= 1;
   }
-  (void)tot;
 }
 
 // bit planes of the types, from an int or a byte per point (a warp per word)
@@ -1433,7 +1431,8 @@ static int run_pass(szp_b200_ctx *ctx, PostArgs &a, const unsigned *list, unsign
   if (ni_bits)
     enforce_sparse_kernel<ND><<<(ni_words + kSparseWords - 1) / kSparseWords, kPostThreads, 0, s>>>(
         a, list, ni_bits, ni_words, W0, n0);
-  else if (count_dev)
+  else if constexpr (PASS == kPassRbf)
+    // its items are counted on the device
     pass_round_dev_kernel<PASS, ND><<<dev_grid<PASS, ND>(ctx), kPostThreads, 0, s>>>(a, list, nullptr, count_dev, W0, n0);
   else
     pass_round_kernel<PASS, ND><<<(count + kPostThreads - 1) / kPostThreads, kPostThreads, 0, s>>>(
@@ -1513,11 +1512,13 @@ static int run_all_passes(szp_b200_ctx *ctx, PostArgs &a, unsigned *X, unsigned 
   a.gen = next_gen(ctx);
   if (nz && run_pass<kPassRbf, ND>(ctx, a, Y, 0, nz, ycnt, W0, W1)) return -1;
   tl_mark(ctx, "post_rbf");
-  if (axis_stencil && ND == 3 && nz) {
-    a.OL = raw_in_F ? OZ : nullptr;   // gathered before the passes: RBF has changed some saddles
-    a.gen = next_gen(ctx);
-    if (run_pass<kPassAxis, ND>(ctx, a, Z, nz, nz, nullptr, W0, W1)) return -1;
-    tl_mark(ctx, "post_axis");
+  if constexpr (ND == 3) {
+    if (axis_stencil && nz) {
+      a.OL = raw_in_F ? OZ : nullptr;   // gathered before the passes: RBF has changed some saddles
+      a.gen = next_gen(ctx);
+      if (run_pass<kPassAxis, ND>(ctx, a, Z, nz, nz, nullptr, W0, W1)) return -1;
+      tl_mark(ctx, "post_axis");
+    }
   }
   return 0;
 }
