@@ -728,10 +728,11 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
   unsigned long long tot[3];
   // From kRankBitsFieldMin values on the encoder sets the rank's bits itself
   // and hands over the values' codes (in the pairs' place): no pair is written
-  // or read.  Below, the rank picks its way by the number of pairs.
+  // or read.  Else the rank picks its way by the number of pairs.
   RankBits rb;
   const EncArgs probe = [&] { EncArgs e{}; e.B = B; e.data = d_data; e.out = d_topo + 8; e.cp_mode = kCpBits; return e; }();
-  const bool bits = n >= kRankBitsFieldMin && enc64_applies(probe, kEncClassify) && rank_bits_begin(ctx, absErrBound, &rb);
+  const bool may_set = n >= kRankBitsFieldMin && enc64_applies(probe, kEncClassify);
+  const bool bits = may_set && (n >= kRankBitsAlways || ctx->rank_bits) && rank_bits_begin(ctx, absErrBound, &rb);
   const int cp_mode = bits ? kCpBits : kCpPairs;
   tl_begin(ctx);
   // a field still on the host (h_src) is copied in parts that overlap the encoder
@@ -773,6 +774,7 @@ static int compress_dev_impl(szp_b200_ctx *ctx, const float *d_data, szp_b200_ge
   }
   if (E == 0) return 0;
   if (!bits && rank_positions(ctx, pairs, nullptr, K, E, absErrBound, sp)) return -1;
+  if (may_set && K > kRankSmall) rank_bits_reserve(ctx);   // for the fields that follow
   tl_mark(ctx, "rank");
   unsigned long long st[3];
   if (encode_pass(ctx, kEncInts, nullptr, sp, nullptr, E, B, absErrBound, g, d_sort,

@@ -53,12 +53,15 @@ constexpr unsigned kMaxBins = 1u << 22;
 // 79 / 186, 131072 82 / 429.
 constexpr unsigned long long kRankBitsMin = 1ull << 16;
 // Values of a field from which the encoder sets them, for nothing in launches or
-// waits; fewer are not worth the 118 MB.  Compression of 2D noise (us, bits from
-// the encoder / pairs in buckets): 8100 values 106 / 118, 16384 102 / 117, 32761
-// 108 / 118, with a thousand points in a bin 104 / 118, 104 / 122, 104 / 163; of
-// a smooth field, whose few points one CTA sorts either way, 74.4 / 75.0,
-// 70.0 / 69.9, 69.3 / 70.3.
+// waits, in a workspace that has the bitmap; fewer are not worth it.  Compression
+// of 2D noise (us, bits from the encoder / pairs in buckets): 8100 values 106 /
+// 118, 16384 102 / 117, 32761 108 / 118, with a thousand points in a bin 104 /
+// 118, 104 / 122, 104 / 163; of a smooth field, whose few points one CTA sorts
+// either way, 74.4 / 75.0, 70.0 / 69.9, 69.3 / 70.3.
 constexpr unsigned long long kRankBitsFieldMin = 1ull << 14;
+// Values from which a workspace gets the bitmap for it (118 MB; 0.25 ms, once).
+// Below, one that has met a field of more points than one CTA sorts has it.
+constexpr unsigned long long kRankBitsAlways = 1ull << 18;
 constexpr unsigned kRbUnits = (unsigned)((2ull * (kRbBelow + kRbAbove) << 23) / kRbBits) + 2u;
 
 struct RankBits {
